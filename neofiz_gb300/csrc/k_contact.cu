@@ -265,8 +265,9 @@ __device__ void grid_from_box(const Dev &d, int nodes, Grid &g) {
     g.cellSize = cellSize;
     g.r0 = rlo;
     g.z0 = zlo;
-    const int a = jd2i((rhi - rlo) / cellSize) + 1;
-    const int b = jd2i((zhi - zlo) / cellSize) + 1;
+    const nf_divisor byCell = nf_divisor_of(cellSize);
+    const int a = jd2i(nf_div_by(rhi - rlo, cellSize, byCell)) + 1;
+    const int b = jd2i(nf_div_by(zhi - zlo, cellSize, byCell)) + 1;
     g.cols = a > 1 ? a : 1;
     g.rows = b > 1 ? b : 1;
     g.cells = (long long)g.cols * (long long)g.rows;
@@ -326,26 +327,27 @@ __device__ void resolve_pair(const Dev &d, int n, int q) {
     const double len = d.slen[q];
     const double tr = -d.snz[q];                            // parameter, :655-661 (the
     const double tz = d.snr[q];                             // tangent as in depth_of)
-    const double t = ((d.cr[n] - d.cr[a]) * tr + (d.cz[n] - d.cz[a]) * tz) / len;
+    const double t = nf_div((d.cr[n] - d.cr[a]) * tr + (d.cz[n] - d.cz[a]) * tz, len);
     const double wa = 1.0 - t, wb = t;
     const double ma = d.mass[a], mb = d.mass[b];
     // 0.25 / m is 0.25 (1 / m) exactly for a normal mass below 2^1000 (a power of two scales
     // a rounded quotient without rounding again), and 1 / m is the kept invMass
-    const double qa = normal_below_2p1000(ma) ? 0.25 * d.invMass[a] : 0.25 / ma;
-    const double qb = normal_below_2p1000(mb) ? 0.25 * d.invMass[b] : 0.25 / mb;
+    const double qa = normal_below_2p1000(ma) ? 0.25 * d.invMass[a] : nf_div(0.25, ma);
+    const double qb = normal_below_2p1000(mb) ? 0.25 * d.invMass[b] : nf_div(0.25, mb);
     const double invMaster = qa + qb;
     if (!(invMaster > 0.0)) return;
-    const double mMaster = 1.0 / invMaster;
+    const double mMaster = nf_div(1.0, invMaster);
     const double mSlave = d.mass[n];
-    const double mStar = mSlave * mMaster / (mSlave + mMaster);
-    const double k = d.cScale * mStar / (reference * reference);
+    const double mStar = nf_div(mSlave * mMaster, mSlave + mMaster);
+    const double k = nf_div(d.cScale * mStar, reference * reference);
     const double nR = d.snr[q], nZ = d.snz[q];
-    const double mTrue = 1.0 / (wa * wa / ma + wb * wb / mb);
-    const double mTangent = mSlave * mTrue / (mSlave + mTrue);
+    const double mTrue = nf_div(1.0, nf_div(wa * wa, ma) + nf_div(wb * wb, mb));
+    const double mTangent = nf_div(mSlave * mTrue, mSlave + mTrue);
+    const nf_divisor byTangent = nf_divisor_of(mTangent);
     const double2 vn = d.V[n], va = d.V[a], vb = d.V[b];
     const double closing = (vn.x - wa * va.x - wb * vb.x) * nR
                            + (vn.y - wa * va.y - wb * vb.y) * nZ;
-    const double damper = 2.0 * d.cDamping * mStar * d.cSqrtScale / reference;
+    const double damper = nf_div(2.0 * d.cDamping * mStar * d.cSqrtScale, reference);
     const double normal = jmax(0.0, k * depth - damper * closing);
     double *pv = d.pairVal + 12 * (size_t)n;
     pv[0] = normal * nR;
@@ -360,7 +362,7 @@ __device__ void resolve_pair(const Dev &d, int n, int q) {
     double dthis = 0.0;
     const double damperForce = normal - k * depth;
     if (damperForce != 0.0) {
-        const double closingAfter = closing + damperForce * dt / mTangent;
+        const double closingAfter = closing + nf_div_by(damperForce * dt, mTangent, byTangent);
         dthis -= damperForce * 0.5 * (closing + closingAfter) * dt;
     }
     uint8_t state = NF_CONTACT_PAIR;
@@ -368,7 +370,7 @@ __device__ void resolve_pair(const Dev &d, int n, int q) {
         const double tR = -nZ, tZ = nR;
         const double slide = (vn.x - wa * va.x - wb * vb.x) * tR
                              + (vn.y - wa * va.y - wb * vb.y) * tZ;
-        double tangent = -STICK_RELAXATION * mTangent * slide / dt;
+        double tangent = nf_div(-STICK_RELAXATION * mTangent * slide, dt);
         const double cone = d.cFriction * normal;
         bool slipped = false;
         if (tangent > cone) { tangent = cone; slipped = true; }
@@ -379,7 +381,7 @@ __device__ void resolve_pair(const Dev &d, int n, int q) {
         pv[7] = -(wa * tangent * tZ);
         pv[10] = -(wb * tangent * tR);
         pv[11] = -(wb * tangent * tZ);
-        const double after = slide + tangent * dt / mTangent;
+        const double after = slide + nf_div_by(tangent * dt, mTangent, byTangent);
         dthis += -tangent * 0.5 * (slide + after) * dt;
         state |= slipped ? NF_CONTACT_SLIP : NF_CONTACT_STICK;
     }
@@ -766,11 +768,12 @@ __global__ void __launch_bounds__(CB, 2) k_contact_pass(Dev d) {
             const double2 xa = d.X0[a], ua = d.U[a], xb = d.X0[b], ub = d.U[b];
             const double dr = (xb.x + ub.x) - (xa.x + ua.x);
             const double dz = (xb.y + ub.y) - (xa.y + ua.y);
-            const double len = sqrt(dr * dr + dz * dz);
+            const double len = nf_sqrt(dr * dr + dz * dz);
             d.slen[q] = len;
             if (len > 0.0) {
-                d.snr[q] = dz / len;
-                d.snz[q] = -dr / len;
+                const nf_divisor byLen = nf_divisor_of(len);
+                d.snr[q] = nf_div_by(dz, len, byLen);
+                d.snz[q] = nf_div_by(-dr, len, byLen);
             } else {
                 d.snr[q] = 0.0;
                 d.snz[q] = 0.0;
@@ -835,12 +838,14 @@ __global__ void __launch_bounds__(CB, 2) k_contact_pass(Dev d) {
             sr += d.snr[own[k]];
             sz += d.snz[own[k]];
         }
-        const double len = sqrt(sr * sr + sz * sz);
-        d.pnr[n] = len > 0.0 ? sr / len : 0.0;
-        d.pnz[n] = len > 0.0 ? sz / len : 0.0;
+        const double len = nf_sqrt(sr * sr + sz * sz);
+        const nf_divisor byLen = nf_divisor_of(len);
+        d.pnr[n] = len > 0.0 ? nf_div_by(sr, len, byLen) : 0.0;
+        d.pnz[n] = len > 0.0 ? nf_div_by(sz, len, byLen) : 0.0;
         // Contact.cellOf, Contact.java:553-557
-        const int ci = iclamp(jd2i((d.cr[n] - g.r0) / g.cellSize), g.cols);
-        const int cj = iclamp(jd2i((d.cz[n] - g.z0) / g.cellSize), g.rows);
+        const nf_divisor byCell = nf_divisor_of(g.cellSize);
+        const int ci = iclamp(jd2i(nf_div_by(d.cr[n] - g.r0, g.cellSize, byCell)), g.cols);
+        const int cj = iclamp(jd2i(nf_div_by(d.cz[n] - g.z0, g.cellSize, byCell)), g.rows);
         d.nodeCell[n] = make_int2(ci, cj);
         const long long cell = (long long)cj * g.cols + ci;
         // the node's ends, two at a time: both slots are claimed before either is written, so

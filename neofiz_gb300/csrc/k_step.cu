@@ -95,8 +95,9 @@ __global__ void __launch_bounds__(BLOCK) k_nodal(Dev d) {
     if (threadIdx.x == 0) {
         const double avg = 0.5 * (s->dtPrevious + dt);
         const double half = 0.5 * d.damping * avg;
-        coef[0] = (1.0 - half) / (1.0 + half);
-        coef[1] = avg / (1.0 + half);
+        const nf_divisor by = nf_divisor_of(1.0 + half);
+        coef[0] = nf_div_by(1.0 - half, 1.0 + half, by);
+        coef[1] = nf_div_by(avg, 1.0 + half, by);
         coef[2] = avg;
         if (blockIdx.x == 0) {
             s->decay = coef[0];
@@ -472,7 +473,7 @@ __global__ void __launch_bounds__(BLOCK) k_element_full(Dev d, int zeroStrain) {
                 const double J10 = dN0e * r0 + dN1e * r1 + dN2e * r2 + dN3e * r3;
                 const double J11 = dN0e * z0 + dN1e * z1 + dN2e * z2 + dN3e * z3;
                 const double det = J00 * J11 - J01 * J10;
-                const double inv = 1.0 / det;
+                const double inv = nf_div(1.0, det);
 
                 const double d0r = (J11 * dN0x - J01 * dN0e) * inv;
                 const double d1r = (J11 * dN1x - J01 * dN1e) * inv;
@@ -490,9 +491,11 @@ __global__ void __launch_bounds__(BLOCK) k_element_full(Dev d, int zeroStrain) {
                 const double dGamRZ = dRdZ + dZdR;
 
                 double rg = 0.0, dEpsT = 0.0;
+                nf_divisor byRg{};
                 if (d.axi) {
                     rg = N0 * r0 + N1 * r1 + N2 * r2 + N3 * r3;
-                    dEpsT = (N0 * a0 + N1 * a1 + N2 * a2 + N3 * a3) / rg;
+                    byRg = nf_divisor_of(rg);
+                    dEpsT = nf_div_by(N0 * a0 + N1 * a1 + N2 * a2 + N3 * a3, rg, byRg);
                 }
                 const int p = e * 4 + g;
                 double sg[4], bk[4];
@@ -506,7 +509,8 @@ __global__ void __launch_bounds__(BLOCK) k_element_full(Dev d, int zeroStrain) {
                 if (d.finite) {
                     const double spinDt = 0.5 * (dZdR - dRdZ);
                     if (!is_zero(spinDt)) {
-                        const double cs = corot_cos(spinDt), sn = corot_sin(spinDt);
+                        double cs, sn;
+                        corot_angles(spinDt, cs, sn);
                         corot_rotate(sg, cs, sn);
                         corot_rotate(bk, cs, sn);
                     }
@@ -538,7 +542,7 @@ __global__ void __launch_bounds__(BLOCK) k_element_full(Dev d, int zeroStrain) {
                 const double sR = sg[0], sZ = sg[1], sT = sg[2], sRZ = sg[3];
                 const double dV = d.axi ? 2.0 * NF_PI * rg * det : d.thickness * det;
                 if (d.axi) {
-                    const double hh = sT / rg * dV;
+                    const double hh = nf_div_by(sT, rg, byRg) * dV;
                     g0r -= (d0r * sR + d0z * sRZ) * dV + N0 * hh;
                     g1r -= (d1r * sR + d1z * sRZ) * dV + N1 * hh;
                     g2r -= (d2r * sR + d2z * sRZ) * dV + N2 * hh;
@@ -689,7 +693,7 @@ __global__ void __launch_bounds__(1024) k_end(Dev d, int nodeBlocks, int elemBlo
     if (updateDt) {
         if (d.finite) {
             s->dtPrevious = s->dt;
-            s->dt = d.cfl * sqrt(minEdge * d.massScale) / d.fastestWave;
+            s->dt = nf_div(d.cfl * nf_sqrt(minEdge * d.massScale), d.fastestWave);
         }
         s->stepsTaken += 1;
     }

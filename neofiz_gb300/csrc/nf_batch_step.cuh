@@ -66,8 +66,9 @@ __device__ __forceinline__ void block_step_coef(BlockStep &bs, const BatchInst &
     const double dtAvg = 0.5 * (dtPrev + dt);
     const double half = 0.5 * in.damping * dtAvg;
     bs.dt = dt;
-    bs.decay = (1.0 - half) / (1.0 + half);
-    bs.gain = dtAvg / (1.0 + half);
+    const nf_divisor by = nf_divisor_of(1.0 + half);
+    bs.decay = nf_div_by(1.0 - half, 1.0 + half, by);
+    bs.gain = nf_div_by(dtAvg, 1.0 + half, by);
     bs.dtAvg = dtAvg;
     bs.fdt = (float)bs.dt;
     bs.fdecay = (float)bs.decay;
@@ -97,7 +98,7 @@ static __device__ __noinline__ void block_step_advance(double *sh, int warps, Bl
     for (int w = 1; w < warps; w++) m = min(m, bbits(sh[w]));
     const double me = bdouble(m);
     sh[warps] = me;
-    if (finite) block_step_coef(*bs, in, in.cfl * sqrt(me * in.massScale) / in.wave, dt);
+    if (finite) block_step_coef(*bs, in, nf_div(in.cfl * nf_sqrt(me * in.massScale), in.wave), dt);
     else block_step_coef(*bs, in, dt, dtPrev);
 }
 
@@ -151,7 +152,9 @@ __device__ __forceinline__ double batch_step(const Dev &d, const BatchInst &in, 
     } else {
         const double dtAvg = 0.5 * (dtPrev + dt);                   // :947-956
         const double half = 0.5 * in.damping * dtAvg;
-        co = NodalCoef{(1.0 - half) / (1.0 + half), dtAvg / (1.0 + half), dtAvg, dt};
+        const nf_divisor by = nf_divisor_of(1.0 + half);
+        co = NodalCoef{nf_div_by(1.0 - half, 1.0 + half, by), nf_div_by(dtAvg, 1.0 + half, by),
+                       dtAvg, dt};
     }
     const WallRef w{in.hasWall, in.wallPlane, in.wallFriction, wallContact, wallStuck};
     if (COMP) {                                                  // requires bs
@@ -196,7 +199,7 @@ __device__ __forceinline__ double batch_step(const Dev &d, const BatchInst &in, 
     }
     if (d.finite) {                                                   // :985-990
         dtPrev = dt;
-        dt = bs ? bs->dt : in.cfl * sqrt(me * in.massScale) / in.wave;
+        dt = bs ? bs->dt : nf_div(in.cfl * nf_sqrt(me * in.massScale), in.wave);
     }
     return me;
 }

@@ -46,7 +46,7 @@ static __device__ __forceinline__ void nodal_node(const Dev &d, int i, const Nod
     } else if (resting && w.friction > 0.0) {
         // RigidWall.slide, RigidWall.java:236-259
         const double normal = -f.y;
-        const double trial = -m * decay * v.x / gain - f.x;
+        const double trial = nf_div(-m * decay * v.x, gain) - f.x;
         const double limit = isinf(w.friction) ? INFINITY : w.friction * normal;
         if (fabs(trial) <= limit) {
             loss += 0.5 * m * v.x * v.x;
@@ -55,7 +55,7 @@ static __device__ __forceinline__ void nodal_node(const Dev &d, int i, const Nod
             v.x = 0.0;
         } else {
             const double tangential = copysign(limit, trial);
-            const double slid = decay * v.x + gain * (f.x + tangential) / m;
+            const double slid = decay * v.x + nf_div(gain * (f.x + tangential), m);
             fric += -tangential * slid * dt;
             ws |= NF_WALL_SLID;
             v.x = slid;
@@ -208,7 +208,7 @@ static __device__ __forceinline__ void element_reduced(const Dev &d, int e, doub
         double det, d0r, d1r, d0z, d1z;
         if (moderate_or_zero(S00) && moderate_or_zero(S01) && moderate_or_zero(S10) &&
             moderate_or_zero(S11) && moderate_or_zero(D)) {
-            const double invD = 1.0 / D;
+            const double invD = nf_div(1.0, D);
             det = 0.0625 * D;
             d0r = (S01 - S11) * invD;
             d1r = (S01 + S11) * invD;
@@ -217,7 +217,7 @@ static __device__ __forceinline__ void element_reduced(const Dev &d, int e, doub
         } else {
             const double J00 = 0.25 * S00, J01 = 0.25 * S01, J10 = 0.25 * S10, J11 = 0.25 * S11;
             det = J00 * J11 - J01 * J10;
-            const double inv = 1.0 / det;
+            const double inv = nf_div(1.0, det);
             d0r = 0.25 * (J01 - J11) * inv;
             d1r = 0.25 * (J01 + J11) * inv;
             d0z = 0.25 * (J10 - J00) * inv;
@@ -235,9 +235,11 @@ static __device__ __forceinline__ void element_reduced(const Dev &d, int e, doub
         const double dGamRZ = dRdZ + dZdR;
 
         double rg = 0.0, dEpsT = 0.0;
+        nf_divisor byRg{};
         if (d.axi) {
             rg = 0.25 * (r0 + r1 + r2 + r3);
-            dEpsT = 0.25 * (a0 + a1 + a2 + a3) / rg;
+            byRg = nf_divisor_of(rg);
+            dEpsT = nf_div_by(0.25 * (a0 + a1 + a2 + a3), rg, byRg);
         }
         double sg[4], bk[4];
         {
@@ -250,7 +252,8 @@ static __device__ __forceinline__ void element_reduced(const Dev &d, int e, doub
         if (d.finite) {
             const double spinDt = 0.5 * (dZdR - dRdZ);
             if (!is_zero(spinDt)) {
-                const double cs = corot_cos(spinDt), sn = corot_sin(spinDt);
+                double cs, sn;
+                corot_angles(spinDt, cs, sn);
                 corot_rotate(sg, cs, sn);
                 // a back stress of +0s (no kinematic hardening) rotates to itself
                 if (!(all_plus_zero(bk[0], bk[1], bk[2], bk[3]) && corot_keeps_zero(cs, sn)))
@@ -287,7 +290,7 @@ static __device__ __forceinline__ void element_reduced(const Dev &d, int e, doub
 
         double g0r, g1r, g2r, g3r;
         if (d.axi) {
-            const double hh = sT / rg * dV * 0.25;
+            const double hh = nf_div_by(sT, rg, byRg) * dV * 0.25;
             g0r = -((d0r * sR + d0z * sRZ) * dV + hh);
             g1r = -((d1r * sR + d1z * sRZ) * dV + hh);
             g2r = -((d2r * sR + d2z * sRZ) * dV + hh);
@@ -349,7 +352,8 @@ static __device__ __forceinline__ void point_update_mixed(const Dev &d, int e, i
         bk[0] = b.x; bk[1] = b.y; bk[2] = b.z; bk[3] = b.w;
     }
     if (d.finite && spinDt != 0.0f) {
-        const float cs = corot_cos(spinDt), sn = corot_sin(spinDt);
+        float cs, sn;
+        corot_angles(spinDt, cs, sn);
         corot_rotate(sg, cs, sn);
         corot_rotate(bk, cs, sn);
     }
@@ -477,7 +481,7 @@ static __device__ __forceinline__ void pressure_edge(const Dev &d, int e, double
                                                      double rampDuration) {
     double p = target;
     if (rampDuration > 0.0) {
-        const double s = jmin(1.0, t / rampDuration);
+        const double s = jmin(1.0, nf_div(t, rampDuration));
         p = target * s * s * (3.0 - 2.0 * s);
     }
     double *c = d.contribution + 8 * (size_t)(d.E + e);
@@ -493,18 +497,19 @@ static __device__ __forceinline__ void pressure_edge(const Dev &d, int e, double
     }
     const double tr = rb - ra;
     const double tz = zb - za;
-    const double len = sqrt(tr * tr + tz * tz);
+    const double len = nf_sqrt(tr * tr + tz * tz);
     if (len == 0.0) {
         c[0] = 0.0; c[1] = 0.0; c[4] = 0.0; c[5] = 0.0;
         return;
     }
-    const double nr = tz / len;
-    const double nz = -tr / len;
+    const nf_divisor byLen = nf_divisor_of(len);
+    const double nr = nf_div_by(tz, len, byLen);
+    const double nz = nf_div_by(-tr, len, byLen);
     double wa, wb;
     if (d.axi) {
         const double circumference = 2.0 * NF_PI * len;
-        wa = circumference * (ra / 3.0 + rb / 6.0);
-        wb = circumference * (ra / 6.0 + rb / 3.0);
+        wa = circumference * (nf_div(ra, 3.0) + nf_div(rb, 6.0));
+        wb = circumference * (nf_div(ra, 6.0) + nf_div(rb, 3.0));
     } else {
         wa = d.thickness * len * 0.5;
         wb = wa;
@@ -520,7 +525,7 @@ static __device__ __forceinline__ void pressure_edge_f32(const Dev &d, int e, do
                                                          double target, double rampDuration) {
     double p = target;
     if (rampDuration > 0.0) {
-        const double s = jmin(1.0, t / rampDuration);
+        const double s = jmin(1.0, nf_div(t, rampDuration));
         p = target * s * s * (3.0 - 2.0 * s);
     }
     float *c = d.contribF + 8 * (size_t)(d.E + e);
@@ -532,17 +537,18 @@ static __device__ __forceinline__ void pressure_edge_f32(const Dev &d, int e, do
         ra += ua.x; rb += ub.x; za += ua.y; zb += ub.y;
     }
     const double tr = rb - ra, tz = zb - za;
-    const double len = sqrt(tr * tr + tz * tz);
+    const double len = nf_sqrt(tr * tr + tz * tz);
     if (len == 0.0) {
         c[0] = 0.f; c[1] = 0.f; c[4] = 0.f; c[5] = 0.f;
         return;
     }
-    const double nr = tz / len, nz = -tr / len;
+    const nf_divisor byLen = nf_divisor_of(len);
+    const double nr = nf_div_by(tz, len, byLen), nz = nf_div_by(-tr, len, byLen);
     double wa, wb;
     if (d.axi) {
         const double circumference = 2.0 * NF_PI * len;
-        wa = circumference * (ra / 3.0 + rb / 6.0);
-        wb = circumference * (ra / 6.0 + rb / 3.0);
+        wa = circumference * (nf_div(ra, 3.0) + nf_div(rb, 6.0));
+        wb = circumference * (nf_div(ra, 6.0) + nf_div(rb, 3.0));
     } else {
         wa = d.thickness * len * 0.5;
         wb = wa;
@@ -689,7 +695,7 @@ static __device__ __forceinline__ void pressure_edge_comp(const Dev &d, int e, d
                                                           double target, double rampDuration) {
     double p = target;
     if (rampDuration > 0.0) {
-        const double s = jmin(1.0, t / rampDuration);
+        const double s = jmin(1.0, nf_div(t, rampDuration));
         p = target * s * s * (3.0 - 2.0 * s);
     }
     float *c = d.contribF + 8 * (size_t)(d.E + e);
@@ -703,17 +709,18 @@ static __device__ __forceinline__ void pressure_edge_comp(const Dev &d, int e, d
         za += (double)ua.z + (double)ua.w; zb += (double)ub.z + (double)ub.w;
     }
     const double tr = rb - ra, tz = zb - za;
-    const double len = sqrt(tr * tr + tz * tz);
+    const double len = nf_sqrt(tr * tr + tz * tz);
     if (len == 0.0) {
         c[0] = 0.f; c[1] = 0.f; c[4] = 0.f; c[5] = 0.f;
         return;
     }
-    const double nr = tz / len, nz = -tr / len;
+    const nf_divisor byLen = nf_divisor_of(len);
+    const double nr = nf_div_by(tz, len, byLen), nz = nf_div_by(-tr, len, byLen);
     double wa, wb;
     if (d.axi) {
         const double circumference = 2.0 * NF_PI * len;
-        wa = circumference * (ra / 3.0 + rb / 6.0);
-        wb = circumference * (ra / 6.0 + rb / 3.0);
+        wa = circumference * (nf_div(ra, 3.0) + nf_div(rb, 6.0));
+        wb = circumference * (nf_div(ra, 6.0) + nf_div(rb, 3.0));
     } else {
         wa = d.thickness * len * 0.5;
         wb = wa;

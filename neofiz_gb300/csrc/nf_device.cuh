@@ -14,6 +14,7 @@
 
 #include <cstdint>
 #include "nf_math.h"
+#include "nf_ifp.h"
 
 namespace nf {
 
@@ -42,7 +43,14 @@ template <typename T> struct Fn;
 template <> struct Fn<double> {
     static __device__ __forceinline__ double pow(double a, double b) { return nf_pow(a, b); }
     static __device__ __forceinline__ double log(double a) { return nf_log(a); }
-    static __device__ __forceinline__ double sqrt(double a) { return ::sqrt(a); }
+    // IEEE quotient and root, in integer arithmetic (nf_ifp.h)
+    static __device__ __forceinline__ double sqrt(double a) { return nf_sqrt(a); }
+    static __device__ __forceinline__ double div(double a, double b) { return nf_div(a, b); }
+    using Divisor = nf_divisor;
+    static __device__ __forceinline__ Divisor divisor(double b) { return nf_divisor_of(b); }
+    static __device__ __forceinline__ double div_by(double a, double b, const Divisor &v) {
+        return nf_div_by(a, b, v);
+    }
     static __device__ __forceinline__ double hypot(double a, double b) { return nf_hypot(a, b); }
     static __device__ __forceinline__ double atan2(double a, double b) { return nf_atan2(a, b); }
     static __device__ __forceinline__ double sin(double a) { return nf_sin(a); }
@@ -58,6 +66,12 @@ template <> struct Fn<float> {
     static __device__ __forceinline__ float pow(float a, float b) { return __powf(a, b); }
     static __device__ __forceinline__ float log(float a) { return __logf(a); }
     static __device__ __forceinline__ float sqrt(float a) { return ::sqrtf(a); }
+    static __device__ __forceinline__ float div(float a, float b) { return a / b; }
+    struct Divisor {};
+    static __device__ __forceinline__ Divisor divisor(float) { return Divisor{}; }
+    static __device__ __forceinline__ float div_by(float a, float b, const Divisor &) {
+        return a / b;
+    }
     static __device__ __forceinline__ float hypot(float a, float b) { return ::hypotf(a, b); }
     static __device__ __forceinline__ float atan2(float a, float b) { return ::atan2f(a, b); }
     static __device__ __forceinline__ float sin(float a) { return ::sinf(a); }
@@ -126,7 +140,7 @@ template <typename T>
 __device__ __forceinline__ T jc_rateTerm(const MatT<T> &f, T rate) {
     if (rate <= f.refRate) return T(1);
     // rate / 1 is rate exactly: the common reference rate of 1/s skips the division
-    return T(1) + f.c * Fn<T>::log(f.refRate == T(1) ? rate : rate / f.refRate);
+    return T(1) + f.c * Fn<T>::log(f.refRate == T(1) ? rate : Fn<T>::div(rate, f.refRate));
 }
 // isfinite by the exponent field (an integer test, off the FP64 pipe)
 __device__ __forceinline__ bool finite_bits(double x) {
@@ -146,7 +160,7 @@ __device__ __forceinline__ T jc_thermalTerm(const MatT<T> &f, T temperature) {
     // a point that has done no plastic work sits at room temperature: 0 / span is +-0, whose
     // term is 1, for any span but 0 and NaN (which the division below turns into NaN)
     if (is_zero(above) && (span > T(0) || span < T(0))) return T(1);
-    const T homologous = above / span;
+    const T homologous = Fn<T>::div(above, span);
     if (homologous <= T(0)) return T(1);
     if (homologous >= T(1)) return T(0);
     return T(1) - Fn<T>::pow(homologous, f.m);
@@ -179,23 +193,24 @@ static __device__ __noinline__ SolveOut<T> j2_solve(T norm, T stiffness, T plast
                                                     T thermal, T dt, const MatT<T> &jc) {
     const T tolerance = Fn<T>::tolerance * jc.a;
     T lo = T(0);
-    T hi = norm / stiffness;
+    T hi = Fn<T>::div(norm, stiffness);
     T dGamma = hi;
+    const typename Fn<T>::Divisor byDt = Fn<T>::divisor(dt);     // shared by the iterations
     for (int iteration = 0; iteration < SOLVE_ITERATIONS; iteration++) {
         const T dEps = T(SQRT_2_3) * dGamma;
         const T eps = plasticStrain + dEps;
-        const T rate = dt > T(0) ? dEps / dt : T(0);
+        const T rate = dt > T(0) ? Fn<T>::div_by(dEps, dt, byDt) : T(0);
         const T strain = jc_strainTerm(jc, eps);
         const T rateFactor = jc_rateTerm(jc, rate);
         const T g = norm - stiffness * dGamma - T(SQRT_2_3) * strain * rateFactor * thermal;
         if (g > T(0)) lo = dGamma; else hi = dGamma;
         if (Fn<T>::abs(g) <= tolerance) return SolveOut<T>{dGamma, strain, iteration + 1, 1};
         T slope = -stiffness
-                  - T(TWO_THIRDS) * (jc.n * (strain - jc.a) / eps) * rateFactor * thermal;
+                  - T(TWO_THIRDS) * Fn<T>::div(jc.n * (strain - jc.a), eps) * rateFactor * thermal;
         if (!(rate <= jc.refRate)) {
-            slope -= T(SQRT_2_3) * strain * jc.c * thermal / dGamma;
+            slope -= Fn<T>::div(T(SQRT_2_3) * strain * jc.c * thermal, dGamma);
         }
-        T next = dGamma - g / slope;
+        T next = dGamma - Fn<T>::div(g, slope);
         if (!(next > lo && next < hi)) next = T(0.5) * (lo + hi);
         dGamma = next;
     }
@@ -306,9 +321,9 @@ __device__ __forceinline__ T j2_update(T *s, T *bk, T &epsP, T &work, T dRR, T d
     T strainNew = T(0);                   // the strain term at the new plastic strain, if known
     bool haveStrain = false;
     if (!jc || softening) {
-        dGamma = (norm - radius) / (stiffness + T(TWO_THIRDS) * hardening);
+        dGamma = Fn<T>::div(norm - radius, stiffness + T(TWO_THIRDS) * hardening);
         if (softening && flowStress + hardening * T(SQRT_2_3) * dGamma < T(0)) {
-            dGamma = norm / stiffness;
+            dGamma = Fn<T>::div(norm, stiffness);
         }
     } else {
         const SolveOut<T> r = j2_solve(norm, stiffness, epsP, thermal, strainDt, flow);
@@ -319,7 +334,7 @@ __device__ __forceinline__ T j2_update(T *s, T *bk, T &epsP, T &work, T dRR, T d
         haveStrain = r.converged != 0;
         if (cost) *cost = 1 + r.iterations;
     }
-    const T inv = T(1) / norm;
+    const T inv = Fn<T>::div(T(1), norm);
     const T nRR = xRR * inv, nZZ = xZZ * inv, nTT = xTT * inv, nRZ = xRZ * inv;
 
     const T pull = T(2) * mu * dGamma;
@@ -365,15 +380,14 @@ __device__ __forceinline__ void corot_rotate(T *t, T c, T sn) {
     t[1] = ss * rr + T(2) * cs * rz + cc * zz;
     t[3] = cs * (rr - zz) + (cc - ss) * rz;
 }
+// The cosine (1 - h^2) / (1 + h^2) and sine 2 h / (1 + h^2), h = spinDt / 2.
 template <typename T>
-__device__ __forceinline__ T corot_cos(T spinDt) {
+__device__ __forceinline__ void corot_angles(T spinDt, T &c, T &sn) {
     const T h = T(0.5) * spinDt;
-    return (T(1) - h * h) / (T(1) + h * h);
-}
-template <typename T>
-__device__ __forceinline__ T corot_sin(T spinDt) {
-    const T h = T(0.5) * spinDt;
-    return T(2) * h / (T(1) + h * h);
+    const T below = T(1) + h * h;
+    const typename Fn<T>::Divisor by = Fn<T>::divisor(below);    // one divisor, two quotients
+    c = Fn<T>::div_by(T(1) - h * h, below, by);
+    sn = Fn<T>::div_by(T(2) * h, below, by);
 }
 
 // corot_rotate of a tensor whose rr, zz and rz are +0 gives +0 in all three when c and sn are
@@ -430,7 +444,7 @@ template <typename T>
 __device__ __forceinline__ T damage_at(T strength, T softening, T failureStrain, T plasticStrain) {
     const T sf = strength;
     if (sf <= T(0)) return T(0);
-    const T v = -softening * (plasticStrain - failureStrain) / sf;
+    const T v = Fn<T>::div(-softening * (plasticStrain - failureStrain), sf);
     return v <= T(0) ? T(0) : (v >= T(1) ? T(1) : v);
 }
 
