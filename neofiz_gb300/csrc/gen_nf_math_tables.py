@@ -13,10 +13,14 @@ definitions:
   -log(invc) as hi + lo, so that log z = -log(invc) + log1p(z invc - 1) holds exactly for the
   stored invc.
   exp table, 128 entries: 2^(j/128) as hi + lo.
+  integer log table, 128 entries for nf_ilog.h: invc 2^53 (two words) and
+  (-log(invc) hi + lo) 2^84 - 1088 LN2 (three words, modulo 2^96), LN2 the integer nearest
+  (NF_LN2_HI + NF_LN2_LO) 2^84, so that a biased exponent k + 1088 >= 0 multiplies LN2.
 
 Run it from this directory: python gen_nf_math_tables.py > nf_math_tables.h
 """
 import struct
+from fractions import Fraction
 
 import mpmath
 
@@ -62,6 +66,28 @@ def exp_entries():
     return [split(mpmath.power(2, mpmath.mpf(j) / ENTRIES)) for j in range(ENTRIES)]
 
 
+LN2_PAIR = (float.fromhex("0x1.62e42fee00000p-1"), float.fromhex("0x1.a39ef35793c76p-33"))
+LOG_BIAS = 1088
+
+
+def fixed84(*parts) -> int:
+    """The integer nearest the exact sum of the parts times 2^84."""
+    v = sum(Fraction(p) for p in parts) * 2 ** 84
+    return (2 * v.numerator + v.denominator) // (2 * v.denominator)
+
+
+def log_words():
+    ln2 = fixed84(*LN2_PAIR)
+    rows = []
+    for invc, hi, lo in log_entries():
+        ic = Fraction(invc) * 2 ** 53
+        assert ic.denominator == 1
+        c = (fixed84(hi, lo) - LOG_BIAS * ln2) % (1 << 96)
+        ic = int(ic)
+        rows.append([ic & 0xffffffff, ic >> 32, c & 0xffffffff, (c >> 32) & 0xffffffff, c >> 64])
+    return ln2, rows
+
+
 def main():
     ln2 = mpmath.log(2)
     step = ln2 / ENTRIES
@@ -81,6 +107,13 @@ def main():
     out += ["", "/* 2^(j/128) hi, lo */", "#define NF_EXP_TABLE \\"]
     for hi, lo in exp_entries():
         out.append(f"    {hi.hex()}, {lo.hex()}, \\")
+    fixed, rows = log_words()
+    out += ["", "/* ln 2 in units of 2^-84, and the integer log table: invc 2^53 (lo, hi), then",
+            " * -log(invc) - 1088 ln 2 in those units (lo, mid, hi); padded to 32 bytes */",
+            *(f"#define NF_LN2_FIX{i} 0x{(fixed >> 32 * i) & 0xffffffff:08x}u" for i in range(3)),
+            "#define NF_LOG_BIAS 1088", "#define NF_LOG_WORDS \\"]
+    for row in rows:
+        out.append("    " + ", ".join(f"0x{w:08x}u" for w in row) + ", 0u, 0u, 0u, \\")
     out += ["", "#endif /* NF_MATH_TABLES_H */"]
     print("\n".join(out))
 

@@ -15,6 +15,7 @@
 #include <cstdint>
 #include "nf_math.h"
 #include "nf_ifp.h"
+#include "nf_ilog.h"
 
 namespace nf {
 
@@ -41,8 +42,8 @@ using MatF = MatT<float>;
 // Elementary functions per real type.
 template <typename T> struct Fn;
 template <> struct Fn<double> {
-    static __device__ __forceinline__ double pow(double a, double b) { return nf_pow(a, b); }
-    static __device__ __forceinline__ double log(double a) { return nf_log(a); }
+    static __device__ __forceinline__ double pow(double a, double b) { return nf_pow_fast(a, b); }
+    static __device__ __forceinline__ double log(double a) { return nf_log_fast(a); }
     // IEEE quotient and root, in integer arithmetic (nf_ifp.h)
     static __device__ __forceinline__ double sqrt(double a) { return nf_sqrt(a); }
     static __device__ __forceinline__ double div(double a, double b) { return nf_div(a, b); }

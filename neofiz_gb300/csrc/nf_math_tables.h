@@ -269,4 +269,140 @@
     0x1.fa7c1819e90d8p+0, 0x1.74853f3a5931ep-55, \
     0x1.fd3c22b8f71f1p+0, 0x1.2eb74966579e7p-57, \
 
+/* ln 2 in units of 2^-84, and the integer log table: invc 2^53 (lo, hi), then
+ * -log(invc) - 1088 ln 2 in those units (lo, mid, hi); padded to 32 bytes */
+#define NF_LN2_FIX0 0x9abc9e3bu
+#define NF_LN2_FIX1 0x7f7d1cf7u
+#define NF_LN2_FIX2 0x000b1721u
+#define NF_LOG_BIAS 1088
+#define NF_LOG_WORDS \
+    0xa2a6e520u, 0x002d4279u, 0x3f7ebecdu, 0x6976389cu, 0xd0d825a1u, 0u, 0u, 0u, \
+    0x2d02d02eu, 0x002d02d0u, 0x1ab39689u, 0xb46e8be2u, 0xd0d83c32u, 0u, 0u, 0u, \
+    0xd4a245f2u, 0x002cc3d8u, 0xa7a7cbcbu, 0x5752af2fu, 0xd0d852a4u, 0u, 0u, 0u, \
+    0xb21642c8u, 0x002c8590u, 0x8adb7a1au, 0xaa76bab8u, 0xd0d868f6u, 0u, 0u, 0u, \
+    0xee02c480u, 0x002c47f4u, 0x22a85d97u, 0x04bf189fu, 0xd0d87f2au, 0u, 0u, 0u, \
+    0xc0b02c0cu, 0x002c0b02u, 0x40cfd07fu, 0xbba872a7u, 0xd0d8953eu, 0u, 0u, 0u, \
+    0x71a02bceu, 0x002bceb7u, 0xd8f1ac1eu, 0x234f697cu, 0xd0d8ab35u, 0u, 0u, 0u, \
+    0x572620aeu, 0x002b9310u, 0x8d0cad25u, 0x8e78174du, 0xd0d8c10du, 0u, 0u, 0u, \
+    0xd602b580u, 0x002b580au, 0xe328c17au, 0x4e955f68u, 0xd0d8d6c8u, 0u, 0u, 0u, \
+    0x6102b1dau, 0x002b1da4u, 0x8c361e4au, 0xb3d00c75u, 0xd0d8ec65u, 0u, 0u, 0u, \
+    0x78a0d674u, 0x002ae3dau, 0x308d32c0u, 0x0d0dbed9u, 0xd0d901e6u, 0u, 0u, 0u, \
+    0xaaaaaaaau, 0x002aaaaau, 0x00508a62u, 0xa7f7accau, 0xd0d91749u, 0u, 0u, 0u, \
+    0x91e81fd6u, 0x002a7212u, 0x23a210b3u, 0xd1013579u, 0xd0d92c90u, 0u, 0u, 0u, \
+    0xd5c5f02au, 0x002a3a0fu, 0x3cf4fb02u, 0xd36e48c9u, 0xd0d941bbu, 0u, 0u, 0u, \
+    0x2a02a02au, 0x002a02a0u, 0x88efc817u, 0xf959a4d1u, 0xd0d956cau, 0u, 0u, 0u, \
+    0x4e5e0a72u, 0x0029cbc1u, 0xc2d2a270u, 0x8bbaea8fu, 0xd0d96bbeu, 0u, 0u, 0u, \
+    0x0e4b5edcu, 0x00299571u, 0xf406d359u, 0xd26c8af5u, 0xd0d98096u, 0u, 0u, 0u, \
+    0x40a57eb6u, 0x00295fadu, 0x5f846e53u, 0x14318d95u, 0xd0d99554u, 0u, 0u, 0u, \
+    0xc765a0ceu, 0x00292a73u, 0x0f8fd758u, 0x96bb320au, 0xd0d9a9f6u, 0u, 0u, 0u, \
+    0x8f5c28f6u, 0x0028f5c2u, 0x16ac5d0du, 0x9eae6d3fu, 0xd0d9be7eu, 0u, 0u, 0u, \
+    0x8feb9f34u, 0x0028c197u, 0xb88231f7u, 0x6fa943b1u, 0xd0d9d2ecu, 0u, 0u, 0u, \
+    0xcac5b3f6u, 0x00288df0u, 0x0e1a9938u, 0x4c4801acu, 0xd0d9e740u, 0u, 0u, 0u, \
+    0x4baa3f0eu, 0x00285accu, 0x4ab73deeu, 0x762a5286u, 0xd0d9fb7au, 0u, 0u, 0u, \
+    0x28282828u, 0x00282828u, 0x035c70aeu, 0x2df837dfu, 0xd0da0f9bu, 0u, 0u, 0u, \
+    0x7f6027f6u, 0x0027f602u, 0x4bd24ad6u, 0xb366e1c0u, 0xd0da23a2u, 0u, 0u, 0u, \
+    0x79c95204u, 0x0027c459u, 0x20824fe1u, 0x453d6899u, 0xd0da3791u, 0u, 0u, 0u, \
+    0x48f757ceu, 0x0027932bu, 0x007a229au, 0x215969e7u, 0xd0da4b67u, 0u, 0u, 0u, \
+    0x27627628u, 0x00276276u, 0xb07a07f1u, 0x84b38871u, 0xd0da5f24u, 0u, 0u, 0u, \
+    0x5830fec6u, 0x00273238u, 0x08f44214u, 0xab63d0e2u, 0xd0da72c9u, 0u, 0u, 0u, \
+    0x27027028u, 0x00270270u, 0x120ed3feu, 0xd0a6037eu, 0xd0da8656u, 0u, 0u, 0u, \
+    0xe7bc0e90u, 0x0026d31bu, 0x8108db12u, 0x2eddc3dcu, 0xd0da99ccu, 0u, 0u, 0u, \
+    0xf656f182u, 0x0026a439u, 0x52f11bb4u, 0xff9aaf36u, 0xd0daad29u, 0u, 0u, 0u, \
+    0xb6af7964u, 0x002675c8u, 0xdca14785u, 0x7b9c5a1fu, 0xd0dac070u, 0u, 0u, 0u, \
+    0x9456217eu, 0x002647c6u, 0x40ceb221u, 0xdad63657u, 0xd0dad39fu, 0u, 0u, 0u, \
+    0x0261a320u, 0x00261a32u, 0x3032d44fu, 0x54736147u, 0xd0dae6b8u, 0u, 0u, 0u, \
+    0x7b425ed0u, 0x0025ed09u, 0x5eef32e2u, 0x1eda5bf8u, 0xd0daf9bau, 0u, 0u, 0u, \
+    0x8097012eu, 0x0025c04bu, 0xc01859f4u, 0x6fb0acfcu, 0xd0db0ca5u, 0u, 0u, 0u, \
+    0x9b025940u, 0x002593f6u, 0x0294dd52u, 0x7bde6d02u, 0xd0db1f7au, 0u, 0u, 0u, \
+    0x5a025680u, 0x00256809u, 0x2d237892u, 0x7791be95u, 0xd0db3239u, 0u, 0u, 0u, \
+    0x53c8253cu, 0x00253c82u, 0xd06a80d7u, 0x964231abu, 0xd0db44e2u, 0u, 0u, 0u, \
+    0x25116026u, 0x00251160u, 0xbc85ee3du, 0x0ab41386u, 0xd0db5776u, 0u, 0u, 0u, \
+    0x71024e6au, 0x0024e6a1u, 0x33d145f1u, 0x06fbab6eu, 0xd0db69f4u, 0u, 0u, 0u, \
+    0xe10125e2u, 0x0024bc44u, 0x32ed637bu, 0xbc8064c9u, 0xd0db7c5cu, 0u, 0u, 0u, \
+    0x24924924u, 0x00249249u, 0x229913d8u, 0x5bffe71fu, 0xd0db8eb0u, 0u, 0u, 0u, \
+    0xf13579beu, 0x002468acu, 0x8e4b058du, 0x15911c6du, 0xd0dba0efu, 0u, 0u, 0u, \
+    0x0243f6f0u, 0x00243f6fu, 0x15120248u, 0x18a72658u, 0xd0dbb319u, 0u, 0u, 0u, \
+    0x18cf81b2u, 0x0024168eu, 0xf6a50472u, 0x9414429bu, 0xd0dbc52eu, 0u, 0u, 0u, \
+    0xfb823ee0u, 0x0023ee08u, 0x795f06a4u, 0xb60c9f44u, 0xd0dbd72fu, 0u, 0u, 0u, \
+    0x767f70e8u, 0x0023c5deu, 0x63d1526bu, 0xac291efcu, 0xd0dbe91cu, 0u, 0u, 0u, \
+    0x5b45023au, 0x00239e0du, 0x9260351eu, 0xa36a0dfcu, 0xd0dbfaf5u, 0u, 0u, 0u, \
+    0x808dda52u, 0x00237694u, 0xe4ccf7c8u, 0xc839c7eau, 0xd0dc0cbau, 0u, 0u, 0u, \
+    0xc234f72cu, 0x00234f72u, 0xe37daf56u, 0x466f4f15u, 0xd0dc1e6cu, 0u, 0u, 0u, \
+    0x01194538u, 0x002328a7u, 0x60a59260u, 0x4950d56fu, 0xd0dc300au, 0u, 0u, 0u, \
+    0x23023024u, 0x00230230u, 0xdb18b071u, 0xfb96379fu, 0xd0dc4194u, 0u, 0u, 0u, \
+    0x1284e6f2u, 0x0022dc0du, 0x93916829u, 0x876b6a91u, 0xd0dc530cu, 0u, 0u, 0u, \
+    0xbeea4e1au, 0x0022b63cu, 0x9c850835u, 0x1672dbc3u, 0xd0dc6471u, 0u, 0u, 0u, \
+    0x1c159a76u, 0x002290beu, 0x7c6a5666u, 0xd1c7c4c8u, 0xd0dc75c2u, 0u, 0u, 0u, \
+    0x226b9022u, 0x00226b90u, 0x47a4fa23u, 0xe2007234u, 0xd0dc8701u, 0u, 0u, 0u, \
+    0xceba6066u, 0x002246b1u, 0x544a35adu, 0x6f307e58u, 0xd0dc982eu, 0u, 0u, 0u, \
+    0x22222222u, 0x00222222u, 0x05d54566u, 0xa0eb000eu, 0xd0dca948u, 0u, 0u, 0u, \
+    0x21fde022u, 0x0021fde0u, 0x7fdc24d2u, 0x9e44adeau, 0xd0dcba50u, 0u, 0u, 0u, \
+    0xd7cd3920u, 0x0021d9eau, 0xe228a4a1u, 0x8dd5f617u, 0xd0dccb46u, 0u, 0u, 0u, \
+    0x511e8d2cu, 0x0021b641u, 0x1b8ddb62u, 0x95bd0b26u, 0xd0dcdc2au, 0u, 0u, 0u, \
+    0x9f79b476u, 0x002192e2u, 0x08b6c6a9u, 0xdb9fe614u, 0xd0dcecfcu, 0u, 0u, 0u, \
+    0xd84b3b90u, 0x00216fcdu, 0x34575d73u, 0x84ae3dd3u, 0xd0dcfdbdu, 0u, 0u, 0u, \
+    0x14d0214eu, 0x00214d02u, 0x97fb3330u, 0xb5a3748eu, 0xd0dd0e6cu, 0u, 0u, 0u, \
+    0x720212a8u, 0x00212a7eu, 0x5d888432u, 0x92c87aecu, 0xd0dd1f0au, 0u, 0u, 0u, \
+    0x10842108u, 0x00210842u, 0x5adecb5cu, 0x3ff5a98cu, 0xd0dd2f97u, 0u, 0u, 0u, \
+    0x148fef8cu, 0x0020e64cu, 0x022d884au, 0xe0949103u, 0xd0dd4012u, 0u, 0u, 0u, \
+    0xa5e353f8u, 0x0020c49bu, 0x4c311810u, 0x97a1c083u, 0xd0dd507du, 0u, 0u, 0u, \
+    0xefae6808u, 0x0020a32fu, 0x6fec6034u, 0x87ae837bu, 0xd0dd60d7u, 0u, 0u, 0u, \
+    0x20820820u, 0x00208208u, 0x8137bc58u, 0xd2e2964du, 0xd0dd7120u, 0u, 0u, 0u, \
+    0x6a3ebc34u, 0x00206123u, 0x581e58e8u, 0x9afdd269u, 0xd0dd8159u, 0u, 0u, 0u, \
+    0x02040810u, 0x00204081u, 0x8c0debb5u, 0x0159d1f1u, 0xd0dd9182u, 0u, 0u, 0u, \
+    0x20202020u, 0x00202020u, 0x38e12bb2u, 0x26eb8b23u, 0xd0dda19au, 0u, 0u, 0u, \
+    0x00000000u, 0x00200000u, 0x5e5f8540u, 0x2c44e3aeu, 0xd0ddb1a2u, 0u, 0u, 0u, \
+    0x01fc07f0u, 0x001fc07fu, 0xf75bbca9u, 0x56aff415u, 0xd0ddd182u, 0u, 0u, 0u, \
+    0x1f81f820u, 0x001f81f8u, 0xe5fec2f5u, 0x7da6dbb5u, 0xd0ddf123u, 0u, 0u, 0u, \
+    0x9e4a4271u, 0x001f4465u, 0xf6042515u, 0x98643a72u, 0xd0de1086u, 0u, 0u, 0u, \
+    0xf07c1f08u, 0x001f07c1u, 0x3f936930u, 0x987ec47au, 0xd0de2facu, 0u, 0u, 0u, \
+    0xb301ecc0u, 0x001ecc07u, 0x9ba79019u, 0x6a14d999u, 0xd0de4e96u, 0u, 0u, 0u, \
+    0xabf0b767u, 0x001e9131u, 0x56912cd5u, 0xf3f67a96u, 0xd0de6d44u, 0u, 0u, 0u, \
+    0xc901e574u, 0x001e573au, 0x2873ede6u, 0x17cdaf3cu, 0xd0de8bb9u, 0u, 0u, 0u, \
+    0x1e1e1e1eu, 0x001e1e1eu, 0xa16b6b8cu, 0xb2456ec3u, 0xd0dea9f3u, 0u, 0u, 0u, \
+    0xe3f8868au, 0x001de5d6u, 0x92e5ab01u, 0x9b2f1b5cu, 0xd0dec7f5u, 0u, 0u, 0u, \
+    0x76b981dbu, 0x001dae60u, 0x59891d77u, 0xa5a6a0cbu, 0xd0dee5bfu, 0u, 0u, 0u, \
+    0x54b82c34u, 0x001d77b6u, 0x18f1fe27u, 0xa0354532u, 0xd0df0352u, 0u, 0u, 0u, \
+    0x1d41d41du, 0x001d41d4u, 0x3c1dcedcu, 0x54f33a63u, 0xd0df20afu, 0u, 0u, 0u, \
+    0x8f6ec074u, 0x001d0cb5u, 0x89ba5083u, 0x89a7fd60u, 0xd0df3dd6u, 0u, 0u, 0u, \
+    0x89039b0bu, 0x001cd856u, 0x7ab04263u, 0xffe99104u, 0xd0df5ac8u, 0u, 0u, 0u, \
+    0x055ee191u, 0x001ca4b3u, 0x90bce6bfu, 0x753aa022u, 0xd0df7787u, 0u, 0u, 0u, \
+    0x1c71c71cu, 0x001c71c7u, 0xfcfe2dc0u, 0xa32792dcu, 0xd0df9412u, 0u, 0u, 0u, \
+    0x01c3f8f0u, 0x001c3f8fu, 0x19026a5au, 0x3f62a25au, 0xd0dfb06bu, 0u, 0u, 0u, \
+    0x0381c0e0u, 0x001c0e07u, 0xcb32736fu, 0xfbdef579u, 0xd0dfcc91u, 0u, 0u, 0u, \
+    0x899406f7u, 0x001bdd2bu, 0x8e8045cdu, 0x86ead0a2u, 0xd0dfe887u, 0u, 0u, 0u, \
+    0x14c1bad0u, 0x001bacf9u, 0x87e040ceu, 0x8b48e252u, 0xd0e0044cu, 0u, 0u, 0u, \
+    0x3dda338bu, 0x001b7d6cu, 0xfed93819u, 0xb048b59cu, 0xd0e01fe1u, 0u, 0u, 0u, \
+    0xb4e81b4fu, 0x001b4e81u, 0xe15a006au, 0x99de5351u, 0xd0e03b47u, 0u, 0u, 0u, \
+    0x406c80d9u, 0x001b2036u, 0x53bc057bu, 0xe8b91a35u, 0xd0e0567eu, 0u, 0u, 0u, \
+    0xbca1af28u, 0x001af286u, 0x176e0181u, 0x3a59d629u, 0xd0e07188u, 0u, 0u, 0u, \
+    0x1ac5701bu, 0x001ac570u, 0xcd0a140cu, 0x29281df1u, 0xd0e08c64u, 0u, 0u, 0u, \
+    0x606a63beu, 0x001a98efu, 0x35dbf2a6u, 0x4c86fecfu, 0xd0e0a713u, 0u, 0u, 0u, \
+    0xa6d01a6du, 0x001a6d01u, 0x71638660u, 0x38e8fcd0u, 0xd0e0c196u, 0u, 0u, 0u, \
+    0x1a41a41au, 0x001a41a4u, 0x1527ab4fu, 0x7fe36e85u, 0xd0e0dbedu, 0u, 0u, 0u, \
+    0xf97a4b02u, 0x001a16d3u, 0x87866776u, 0xb0413a5au, 0xd0e0f619u, 0u, 0u, 0u, \
+    0x951033d9u, 0x0019ec8eu, 0xcb795143u, 0x5614fbacu, 0xd0e1101bu, 0u, 0u, 0u, \
+    0x4ee4a102u, 0x0019c2d1u, 0xe59ebf11u, 0xfaca9548u, 0xd0e129f2u, 0u, 0u, 0u, \
+    0x9999999au, 0x00199999u, 0x53e44044u, 0x253836f2u, 0xd0e143a1u, 0u, 0u, 0u, \
+    0xf80cb872u, 0x001970e4u, 0xd7d1a6edu, 0x59aedb20u, 0xd0e15d26u, 0u, 0u, 0u, \
+    0xfcd6e9e0u, 0x001948b0u, 0x5b9cd640u, 0x1a0a420bu, 0xd0e17683u, 0u, 0u, 0u, \
+    0x49d0e229u, 0x001920fbu, 0x0da2a10bu, 0xe5c06ed5u, 0xd0e18fb7u, 0u, 0u, 0u, \
+    0x8f9c18fau, 0x0018f9c1u, 0x880a2e0eu, 0x39f0ab73u, 0xd0e1a8c5u, 0u, 0u, 0u, \
+    0x8d3018d3u, 0x0018d301u, 0x96182434u, 0x917217beu, 0xd0e1c1abu, 0u, 0u, 0u, \
+    0x0f6bf3aau, 0x0018acb9u, 0xfa3c8328u, 0x64e1c7e6u, 0xd0e1da6bu, 0u, 0u, 0u, \
+    0xf0abb04au, 0x001886e5u, 0x5e876d6bu, 0x2ab07663u, 0xd0e1f305u, 0u, 0u, 0u, \
+    0x18618618u, 0x00186186u, 0x1f46b735u, 0x572fcd32u, 0xd0e20b79u, 0u, 0u, 0u, \
+    0x7ab2beddu, 0x00183c97u, 0x385128ddu, 0x5c9f4a2du, 0xd0e223c8u, 0u, 0u, 0u, \
+    0x18181818u, 0x00181818u, 0xd6f0268fu, 0xab38c207u, 0xd0e23bf2u, 0u, 0u, 0u, \
+    0xfd017f40u, 0x0017f405u, 0x760caa01u, 0xb13c8557u, 0xd0e253f8u, 0u, 0u, 0u, \
+    0x417d05f4u, 0x0017d05fu, 0x956ab787u, 0xdafd2afau, 0xd0e26bdau, 0u, 0u, 0u, \
+    0x08e0ecc3u, 0x0017ad22u, 0xccf0df14u, 0x92eb0303u, 0xd0e28399u, 0u, 0u, 0u, \
+    0x8178a4c8u, 0x00178a4cu, 0xe02b52b3u, 0x419f3528u, 0xd0e29b35u, 0u, 0u, 0u, \
+    0xe434a9b1u, 0x001767dcu, 0x4ea289dfu, 0x4de68da7u, 0xd0e2b2aeu, 0u, 0u, 0u, \
+    0x745d1746u, 0x001745d1u, 0xdda2640eu, 0x1ccbfb5eu, 0xd0e2ca05u, 0u, 0u, 0u, \
+    0x7f46debcu, 0x00172428u, 0x9932ab92u, 0x11a2c1d6u, 0xd0e2e13au, 0u, 0u, 0u, \
+    0x5c0b8170u, 0x001702e0u, 0xc0d1d498u, 0x8e1061b9u, 0xd0e2f84du, 0u, 0u, 0u, \
+    0x6b4337c7u, 0x0016e1f7u, 0x4e8632f3u, 0xf2163a49u, 0xd0e30f3fu, 0u, 0u, 0u, \
+    0x16c16c17u, 0x0016c16cu, 0xc682e8c4u, 0x9c1ae620u, 0xd0e32611u, 0u, 0u, 0u, \
+
 #endif /* NF_MATH_TABLES_H */

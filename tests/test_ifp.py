@@ -1,5 +1,6 @@
 """The integer division and square root of the FP64 kernels (neofiz_gb300/csrc/nf_ifp.h) against
-the machine's, bit for bit: every result must be the correctly rounded one.
+the machine's, and the logarithm and power that use integer arithmetic (nf_ilog.h) against
+nf_math.h's, bit for bit.
 
 One check compiles from the header for the host, where the FP32 approximation the methods start
 from is moved through its whole documented error range (and past it), and for the device, where
@@ -22,7 +23,7 @@ CHECK = r"""
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
-#include "nf_ifp.h"
+#include "nf_ilog.h"
 #ifdef __CUDACC__
 #define FN static __host__ __device__
 #else
@@ -64,6 +65,34 @@ FN double number(Rng &r) {
     default: return dval(sign | ((1023 - 40 + r.next() % 80) << 52) | significand(r));
     }
 }
+// bad logarithms in the low word, bad powers in the high word
+FN uint64_t check_log(uint64_t seed, int n) {
+    Rng r{seed};
+    uint64_t bad = 0;
+    for (int i = 0; i < n; i++) {
+        double x;
+        switch (r.next() & 15) {
+        case 0: x = number(r); break;
+        case 1: x = 1.0 + (double)(int64_t)r.next() * 0x1p-70; break;    // near log 1 = 0
+        // a table interval's end, and its neighbours
+        case 2: x = dval(NF_LOG_OFF + ((r.next() % 128) << 45) + (r.next() % 5) - 2); break;
+        // the ends of the fixed-point sum's range
+        case 3: x = dval((r.next() & 1 ? 0x3bf0000000000000ULL : 0x43f0000000000000ULL)
+                         + (r.next() % 5) - 2); break;
+        default: x = dval(((1023 - 66 + r.next() % 132) << 52) | significand(r));
+        }
+        if (!same(nf_log_fast(x), nf_log(x))) bad++;
+        double y = (double)(r.next() >> 11) * 0x1p-53;
+        switch (r.next() & 7) {
+        case 0: y = number(r); break;
+        case 1: y = 1.0; break;
+        case 2: y = dval(((1013 + r.next() % 13) << 52) | significand(r)); break;
+        case 3: y = 1.0 + 0.2 * y; break;
+        }
+        if (!same(nf_pow_fast(x, y), nf_pow(x, y))) bad += 1ULL << 32;
+    }
+    return bad;
+}
 // bad divisions in the low word, bad roots in the high word
 FN uint64_t check(uint64_t seed, int n) {
     Rng r{seed};
@@ -90,7 +119,8 @@ FN uint64_t check(uint64_t seed, int n) {
 #ifdef __CUDACC__
 __global__ void k_check(uint64_t seed, int n, unsigned long long *bad) {
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    const uint64_t b = check(seed + t * 0xD1B54A32D192ED03ULL, n);
+    const uint64_t at = seed + t * 0xD1B54A32D192ED03ULL;
+    const uint64_t b = check(at, n) + check_log(at, n);
     if (b) atomicAdd(bad, (unsigned long long)b);
 }
 int main() {
@@ -105,6 +135,17 @@ int main() {
 int main() {
     uint64_t bad = 0;
     for (nf_ifp_off = -2; nf_ifp_off <= 2; nf_ifp_off++) bad += check(7 + nf_ifp_off, 6000000);
+    bad += check_log(11, 6000000);
+    // the integer forms are what ran: few of the path's arguments take nf_math.h's sequence
+    nf_ilog_slow_count = 0;
+    Rng r{5};
+    for (int i = 0; i < 1000000; i++) {
+        const double x = dval(((1003 + r.next() % 40) << 52) | (r.next() & 0xfffffffffffffULL));
+        if (fabs(nf_log(x)) < 0.004) continue;
+        nf_log_fast(x);
+        nf_pow_fast(x, 0.1 + 1.0 * (double)(r.next() >> 11) * 0x1p-53);
+    }
+    if (nf_ilog_slow_count > 4000) bad++;
     printf("bad %llu\n", (unsigned long long)bad);
     return bad != 0;
 }
