@@ -187,6 +187,98 @@ __device__ __forceinline__ bool near_yield(double norm, double radius) {
 }
 __device__ __forceinline__ bool near_yield(float norm, float radius) { return norm > 0.81f * radius; }
 
+// One iteration of J2.solve (J2.java:343-372): the residual g, the strain term and g / slope.
+template <typename T>
+struct NewtonStep {
+    T g, strain, quotient;
+};
+template <typename T>
+__device__ __forceinline__ NewtonStep<T> newton_step(T norm, T stiffness, T plasticStrain,
+                                                     T thermal, T dt, const MatT<T> &jc,
+                                                     T dGamma) {
+    const T dEps = T(SQRT_2_3) * dGamma;
+    const T eps = plasticStrain + dEps;
+    const T rate = dt > T(0) ? Fn<T>::div(dEps, dt) : T(0);
+    const T strain = jc_strainTerm(jc, eps);
+    const T rateFactor = jc_rateTerm(jc, rate);
+    const T g = norm - stiffness * dGamma - T(SQRT_2_3) * strain * rateFactor * thermal;
+    T slope = -stiffness
+              - T(TWO_THIRDS) * Fn<T>::div(jc.n * (strain - jc.a), eps) * rateFactor * thermal;
+    if (!(rate <= jc.refRate)) {
+        slope -= Fn<T>::div(T(SQRT_2_3) * strain * jc.c * thermal, dGamma);
+    }
+    return NewtonStep<T>{g, strain, Fn<T>::div(g, slope)};
+}
+static __device__ __noinline__ NewtonStep<double> newton_slow(double norm, double stiffness,
+                                                              double plasticStrain, double thermal,
+                                                              double dt, const MatDev &jc,
+                                                              double dGamma) {
+    return newton_step(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
+}
+
+// The iteration per real type: what it keeps over a solve, and the step. In FP64 a solve is one
+// long dependent chain, so the step is straight-line code: the power and the logarithm, and the
+// two quotients of the slope, run beside each other, every quotient, power and logarithm by its
+// branch-free form, and one test at the end sends the point through newton_step when any of
+// them was not settled (about one point-iteration in a thousand).
+template <typename T>
+struct Newton {
+    __device__ __forceinline__ Newton(T, const MatT<T> &) {}
+    __device__ __forceinline__ NewtonStep<T> step(T norm, T stiffness, T plasticStrain, T thermal,
+                                                  T dt, const MatT<T> &jc, T dGamma) const {
+        return newton_step(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
+    }
+    static __device__ __forceinline__ bool positive(T x) { return x > T(0); }
+    static __device__ __forceinline__ bool within(T x, T bound) { return Fn<T>::abs(x) <= bound; }
+    static __device__ __forceinline__ bool between(T x, T lo, T hi) { return x > lo && x < hi; }
+};
+template <>
+struct Newton<double> {
+    nf_divisor byDt;
+    int plain;                   // dt > 0 and the reference rate is 1/s (no second division)
+    __device__ __forceinline__ Newton(double dt, const MatDev &jc)
+        : byDt(nf_divisor_of(dt)), plain(dt > 0.0 && jc.refRate == 1.0) {}
+    __device__ __forceinline__ NewtonStep<double> step(double norm, double stiffness,
+                                                       double plasticStrain, double thermal,
+                                                       double dt, const MatDev &jc,
+                                                       double dGamma) const {
+        int okRate, okPow, okLog, ok1, ok2, okStep;
+        const double dEps = SQRT_2_3 * dGamma;
+        const double eps = plasticStrain + dEps;
+        const double rate = nf_div_try(dEps, byDt, &okRate);
+        const double lg = nf_log_try(rate, &okLog);
+        const double pw = nf_pow_try(eps, jc.n, &okPow);
+        const double strain = jc.a + jc.b * pw;
+        // rate <= 1 by bits: a sure quotient of dEps >= 0 by dt > 0 is no NaN
+        const bool slow = __double_as_longlong(rate) <= __double_as_longlong(1.0);
+        const bool flat = slow || jc.c == 0.0;             // 1 + 0 log is 1
+        const double rateFactor = flat ? 1.0 : 1.0 + jc.c * lg;
+        const double flow = SQRT_2_3 * strain;
+        const double g = norm - stiffness * dGamma - flow * rateFactor * thermal;
+        const double q1 = nf_div_try(jc.n * (strain - jc.a), nf_divisor_of(eps), &ok1);
+        const double q2 = nf_div_try(flow * jc.c * thermal, nf_divisor_of(dGamma), &ok2);
+        const double base = -stiffness - TWO_THIRDS * q1 * rateFactor * thermal;
+        const double slope = slow ? base : base - q2;
+        const double q = nf_div_try(g, nf_divisor_of(slope), &okStep);
+        if (plain & okRate & okPow & (okLog | flat) & ok1 & (ok2 | slow) & okStep)
+            return NewtonStep<double>{g, strain, q};
+        return newton_slow(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
+    }
+    // x > 0, |x| <= bound (bound >= 0), and lo < x < hi (0 <= lo, hi), by the integer order of
+    // the bits: off the FP64 pipe. A NaN is above every number or below every positive one.
+    static __device__ __forceinline__ bool positive(double x) {
+        const long long u = __double_as_longlong(x);
+        return u > 0 && u <= 0x7ff0000000000000LL;
+    }
+    static __device__ __forceinline__ bool within(double x, double bound) {
+        return (__double_as_longlong(x) & 0x7fffffffffffffffLL) <= __double_as_longlong(bound);
+    }
+    static __device__ __forceinline__ bool between(double x, double lo, double hi) {
+        const long long u = __double_as_longlong(x);
+        return u > __double_as_longlong(lo) && u < __double_as_longlong(hi);
+    }
+};
+
 // J2.solve, J2.java:332-375, given the thermal term jc_thermalTerm(jc, temperature) of the
 // point's temperature (the reference evaluates it first thing, from the same argument).
 template <typename T>
@@ -196,23 +288,15 @@ static __device__ __noinline__ SolveOut<T> j2_solve(T norm, T stiffness, T plast
     T lo = T(0);
     T hi = Fn<T>::div(norm, stiffness);
     T dGamma = hi;
-    const typename Fn<T>::Divisor byDt = Fn<T>::divisor(dt);     // shared by the iterations
+    const Newton<T> newton(dt, jc);
+#pragma unroll 1
     for (int iteration = 0; iteration < SOLVE_ITERATIONS; iteration++) {
-        const T dEps = T(SQRT_2_3) * dGamma;
-        const T eps = plasticStrain + dEps;
-        const T rate = dt > T(0) ? Fn<T>::div_by(dEps, dt, byDt) : T(0);
-        const T strain = jc_strainTerm(jc, eps);
-        const T rateFactor = jc_rateTerm(jc, rate);
-        const T g = norm - stiffness * dGamma - T(SQRT_2_3) * strain * rateFactor * thermal;
-        if (g > T(0)) lo = dGamma; else hi = dGamma;
-        if (Fn<T>::abs(g) <= tolerance) return SolveOut<T>{dGamma, strain, iteration + 1, 1};
-        T slope = -stiffness
-                  - T(TWO_THIRDS) * Fn<T>::div(jc.n * (strain - jc.a), eps) * rateFactor * thermal;
-        if (!(rate <= jc.refRate)) {
-            slope -= Fn<T>::div(T(SQRT_2_3) * strain * jc.c * thermal, dGamma);
-        }
-        T next = dGamma - Fn<T>::div(g, slope);
-        if (!(next > lo && next < hi)) next = T(0.5) * (lo + hi);
+        const NewtonStep<T> n = newton.step(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
+        if (Newton<T>::positive(n.g)) lo = dGamma; else hi = dGamma;
+        if (Newton<T>::within(n.g, tolerance))
+            return SolveOut<T>{dGamma, n.strain, iteration + 1, 1};
+        T next = dGamma - n.quotient;
+        if (!Newton<T>::between(next, lo, hi)) next = T(0.5) * (lo + hi);
         dGamma = next;
     }
     return SolveOut<T>{dGamma, T(0), SOLVE_ITERATIONS, 0};

@@ -162,6 +162,16 @@ NF_IFP double nf_div_digits(double a, nf_divisor b, int *unsure) {
     return nf_ifp_make((uint32_t)(r >> 32), (uint32_t)r);
 }
 
+/* a / b where *sure, without a branch (a may be a zero). */
+NF_IFP double nf_div_try(double a, nf_divisor b, int *sure) {
+    int unsure;
+    const double q = nf_div_digits(a, b, &unsure);
+    const uint32_t ha = nf_ifp_hi(a);
+    const int zero = ((ha << 1) | nf_ifp_lo(a)) == 0u;
+    *sure = nf_ifp_moderate(b.h) & ((nf_ifp_moderate(ha) & (unsure ^ 1)) | zero);
+    return zero ? nf_ifp_make((ha ^ b.h) & 0x80000000u, 0u) : q;
+}
+
 /* a / b, rounded as the machine division rounds. */
 NF_IFP double nf_div_by(double a, double b, nf_divisor v) {
     int unsure;

@@ -168,27 +168,33 @@ NF_IFP double nf_ilog_round(nf_ilog v, uint32_t *below) {
                        + ((uint64_t)((uint32_t)(1033 - v.n) << 20 | v.neg) << 32);
     return nf_ifp_make((uint32_t)(m >> 32), (uint32_t)m);
 }
-/* The slack in units of *below, rounded up: 2^(84 - 75 + n - 11) <= 2^17 (|log x| >= 2^-8). */
-NF_IFP int nf_ilog_near_half(uint32_t below) { return below - 0x7ffc0000u < 0x80000u; }
+/* The slack in units of below is 2^(84 - 75 + n - 11), n <= 19: whether half lies within it. */
+NF_IFP int nf_ilog_near_half(uint32_t below, int n) {
+    return below - 0x80000000u + (1u << n) < (2u << n);
+}
 
-/* nf_log(x). */
-NF_IFP double nf_log_fast(double x) {
+/* nf_log(x) where *sure, without a branch. */
+NF_IFP double nf_log_try(double x, int *sure) {
     nf_ilog v;
     uint32_t below;
     const int ok = nf_ilog_of(x, &v);
-    if (!ok) return nf_log_slow(x);
     const double r = nf_ilog_round(v, &below);
-    return nf_ilog_near_half(below) ? nf_log_slow(x) : r;
+    *sure = ok & !nf_ilog_near_half(below, v.n);
+    return r;
+}
+NF_IFP double nf_log_fast(double x) {
+    int sure;
+    const double r = nf_log_try(x, &sure);
+    return sure ? r : nf_log_slow(x);
 }
 
-/* nf_pow(x, y). */
-NF_IFP double nf_pow_fast(double x, double y) {
+/* nf_pow(x, y) where *sure, without a branch. */
+NF_IFP double nf_pow_try(double x, double y, int *sure) {
     nf_ilog v;
     uint32_t below;
     const uint32_t yh = nf_ifp_hi(y);
-    /* 2^-9 <= y < 2: the slack of y log x is below 2^(ey + 1 - 75) */
-    int ok = nf_ilog_of(x, &v) & (yh - 0x3f600000u < 0x00a00000u);
-    if (!ok) return nf_pow_slow(x, y);
+    /* 2^-9 <= y < 2 */
+    const int ok = nf_ilog_of(x, &v) & (yh - 0x3f600000u < 0x00a00000u);
     const double lh = nf_ilog_round(v, &below);
     /* lo = log x - lh: 43 bits and a sign */
     const uint64_t rest = ((uint64_t)(v.w1 & 0x7ffu) << 32) | v.w0;
@@ -209,12 +215,13 @@ NF_IFP double nf_pow_fast(double x, double y) {
     const int n = (int)kd;
     const double al = fma(-kd, NF_EXP_L_LO, fma(-kd, NF_EXP_L_HI, p));
     const double r = al + plo;
-    /* the sum's error and how far it stays from half an ulp of r (all exact), against the slack */
+    /* the sum's error and how far it stays from half an ulp of r (all exact), against y times
+     * the slack (the high words of two doubles order as they do) */
     const double e = plo - (r - al);
     const uint32_t rx = nf_ifp_hi(r) & 0x7ff00000u;
     const double gap = nf_ifp_make(rx - (53u << 20), 0u) - fabs(e);
-    const int sure = ((int32_t)nf_ifp_hi(gap) >= (int32_t)((yh & 0x7ff00000u) - (74u << 20)))
-                     & (rx > (60u << 20)) & !nf_ilog_near_half(below);
+    *sure = ok & ((int32_t)nf_ifp_hi(gap) > (int32_t)(yh - ((uint32_t)(-NF_LOG_SLACK_EXP) << 20)))
+            & (rx > (60u << 20)) & !nf_ilog_near_half(below, v.n);
     const int j = n & 127, m = (n - j) / 128;
     const double thi = nf_exp_tab(2 * j), tlo = nf_exp_tab(2 * j + 1);
     double t = fma(r, 0x1.1111111111111p-7, 0x1.5555555555555p-5);
@@ -222,8 +229,12 @@ NF_IFP double nf_pow_fast(double x, double y) {
     t = fma(r, t, 0.5);
     const double q = fma(r * r, t, r);
     const double er = thi + fma(thi, q, tlo);          /* in [0.99, 2): |p| < 90 scales by bits */
-    const double res = nf_ifp_make(nf_ifp_hi(er) + ((uint32_t)m << 20), nf_ifp_lo(er));
-    return sure ? res : nf_pow_slow(x, y);
+    return nf_ifp_make(nf_ifp_hi(er) + ((uint32_t)m << 20), nf_ifp_lo(er));
+}
+NF_IFP double nf_pow_fast(double x, double y) {
+    int sure;
+    const double r = nf_pow_try(x, y, &sure);
+    return sure ? r : nf_pow_slow(x, y);
 }
 
 #endif /* NF_ILOG_H */
