@@ -117,7 +117,7 @@ bool shape_valid(const Batch &B, const BatchShape &s) {
     if (s.threads != 32 && s.threads != 128 && s.threads != 256) return false;
     if (s.stage && !B.mixed) return false;
     if (s.chunk < 1 || s.blocksPerSm < 1) return false;
-    return batch_max_blocks_per_sm(B.mode, s, B.b.maxNodes) >= s.blocksPerSm;
+    return batch_max_blocks_per_sm(B.mode, s, B.b.maxNodes, B.b.maxElems) >= s.blocksPerSm;
 }
 
 // The run's launches: reset the queue, launch one chunk; GRAPH_CHUNKS times.
@@ -337,13 +337,14 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
     std::vector<BatchScalars> sc(count);
     std::vector<double> cost(count);
     B->inst.resize(count);
-    int maxNodes = 1;
+    int maxNodes = 1, maxElems = 1;
     for (int k = 0; k < count; k++) {
         const nf_batch_instance &p = instances[k];
         const int n0 = mesh->node_offset[k], n1 = mesh->node_offset[k + 1];
         const int e0 = mesh->element_offset[k], e1 = mesh->element_offset[k + 1];
         const int nn = n1 - n0, ne = e1 - e0;
         maxNodes = std::max(maxNodes, nn);
+        maxElems = std::max(maxElems, ne);
         const double *r = mesh->r + n0, *z = mesh->z + n0;
         const int32_t *lc = mesh->conn + 4LL * e0;
         const int k0 = mesh->pressure_offset ? mesh->pressure_offset[k] : 0;
@@ -469,6 +470,7 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
     b.order = dOrder;
     b.count = count;
     b.maxNodes = maxNodes;
+    b.maxElems = maxElems;
     e_ = cudaSuccess;
 #define U(dst, src, n) if (e_ == cudaSuccess) e_ = bupload(*B, dst, src, n)
     U(d.X0, X0.data(), N); U(d.V, V.data(), N); U(d.mass, mass.data(), N);
@@ -507,7 +509,7 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
     }
     // default shape: the most resident blocks of 256 threads, capped at 8 per SM
     BatchShape s{256, 0, 1, 256};
-    const int occ = batch_max_blocks_per_sm(B->mode, s, maxNodes);
+    const int occ = batch_max_blocks_per_sm(B->mode, s, maxNodes, maxElems);
     s.blocksPerSm = std::max(1, std::min(occ, 8));
     B->shape = s;
     nf_status st = bsync(*B);
@@ -603,7 +605,7 @@ nf_status nf_batch_tune(nf_batch *h, int32_t trial_steps, nf_batch_config *chose
     for (int threads : {32, 128, 256})
         for (int stage = 0; stage <= (B.mixed ? 1 : 0); stage++) {
             BatchShape s{threads, stage, 1, trial_steps};
-            const int occ = batch_max_blocks_per_sm(B.mode, s, B.b.maxNodes);
+            const int occ = batch_max_blocks_per_sm(B.mode, s, B.b.maxNodes, B.b.maxElems);
             bool atOcc = false;
             for (int bps : {1, 2, 4, 8, 16, 32}) {
                 if (bps > occ) break;

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(256) k_batch_initial(Dev d, BatchDev b) {
     } else {
         double m = DMAX;
         for (int e = in.e0 + threadIdx.x; e < in.e1; e += 256)
-            element_reduced(d, e, 0.0, in.hourglass, m);
+            element_reduced<false>(d, e, 0.0, in.hourglass, m);
         me = block_min_edge<256>(m, shMin);
     }
     const double t0 = b.sc[blockIdx.x].time;
@@ -113,28 +113,24 @@ __global__ void __launch_bounds__(MEASURE_BLOCK) k_batch_measure(Dev d, BatchDev
 
 // ------------------------------------------------------------------------------------ launch
 
-template <bool MIXED, bool STAGE, int T, bool COMP>
-static const void *steps_kernel() {
-    return (const void *)k_batch_steps<MIXED, STAGE, T>;
-}
-
-template <bool MIXED, bool STAGE, bool COMP>
+template <bool MIXED, bool STAGE, bool INT>
 static const void *by_threads(int threads) {
-    if (threads == 32) return steps_kernel<MIXED, STAGE, 32, COMP>();
-    return threads == 128 ? steps_kernel<MIXED, STAGE, 128, COMP>()
-                          : steps_kernel<MIXED, STAGE, 256, COMP>();
+    if (threads == 32) return (const void *)k_batch_steps<MIXED, STAGE, 32, INT>;
+    return threads == 128 ? (const void *)k_batch_steps<MIXED, STAGE, 128, INT>
+                          : (const void *)k_batch_steps<MIXED, STAGE, 256, INT>;
 }
 
-template <bool MIXED, bool COMP>
-static const void *by_shape(const BatchShape &s) {
-    if (MIXED && s.stage) return by_threads<MIXED, true, COMP>(s.threads);
-    return by_threads<MIXED, false, COMP>(s.threads);
-}
-
-static const void *select_kernel(int mode, const BatchShape &s) {
+// The kernel of a shape; lone: its blocks give no quarter SM more than one warp of elements.
+static const void *select_kernel(int mode, const BatchShape &s, bool lone) {
     if (mode == NF_PRECISION_COMPENSATED) return comp_steps_kernel(s);
-    if (mode == NF_PRECISION_MIXED) return by_shape<true, false>(s);
-    return by_shape<false, false>(s);
+    if (mode == NF_PRECISION_MIXED)
+        return s.stage ? by_threads<true, true, false>(s.threads) : by_threads<true, false, false>(s.threads);
+    return lone ? by_threads<false, false, false>(s.threads) : by_threads<false, false, true>(s.threads);
+}
+// Warps with elements that a shape keeps on one SM.
+static bool lone_warps(const BatchShape &s, int maxElems) {
+    const int lanes = maxElems < s.threads ? maxElems : s.threads;
+    return !int_products((long long)s.blocksPerSm * ((lanes + 31) / 32), 1);
 }
 
 size_t batch_shared_bytes(int mode, const BatchShape &s, int maxNodes) {
@@ -143,8 +139,8 @@ size_t batch_shared_bytes(int mode, const BatchShape &s, int maxNodes) {
 }
 
 // Resident blocks per SM of a shape (0 when it cannot launch, e.g. too much shared memory).
-int batch_max_blocks_per_sm(int mode, const BatchShape &s, int maxNodes) {
-    const void *k = select_kernel(mode, s);
+int batch_max_blocks_per_sm(int mode, const BatchShape &s, int maxNodes, int maxElems) {
+    const void *k = select_kernel(mode, s, lone_warps(s, maxElems));
     const size_t smem = batch_shared_bytes(mode, s, maxNodes);
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
@@ -161,7 +157,7 @@ int batch_max_blocks_per_sm(int mode, const BatchShape &s, int maxNodes) {
 
 cudaError_t launch_batch_steps(const Dev &d, const BatchDev &b, int mode, const BatchShape &s,
                                int sms, cudaStream_t st) {
-    const void *k = select_kernel(mode, s);
+    const void *k = select_kernel(mode, s, lone_warps(s, b.maxElems));
     const size_t smem = batch_shared_bytes(mode, s, b.maxNodes);
     int blocks = sms * s.blocksPerSm;
     if (blocks > b.count) blocks = b.count;

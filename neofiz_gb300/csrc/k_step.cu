@@ -257,12 +257,13 @@ __device__ __forceinline__ void min_edge_commit(Dev &d, double minEdge) {
 }
 
 // reducedIntegration, ExplicitSolver.java:1373-1504
+template <bool INT>
 __global__ void __launch_bounds__(BLOCK) k_element_reduced(Dev d, int zeroStrain) {
     if (!d.s->active) return;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     double minEdge = DMAX;
     if (e < d.E) {
-        element_reduced(d, e, zeroStrain ? 0.0 : d.s->dt, d.hourglass, minEdge);
+        element_reduced<INT>(d, e, zeroStrain ? 0.0 : d.s->dt, d.hourglass, minEdge);
     }
     min_edge_commit(d, minEdge);
 }
@@ -275,6 +276,7 @@ __global__ void __launch_bounds__(BLOCK) k_element_reduced(Dev d, int zeroStrain
 // decides each element's erosion (erode_element): an element's erosion reads only its own point
 // and nodes, which no other element's update writes, so deciding it just before the element's
 // own update is the same as a pass over all elements before any update.
+template <bool INT>
 __global__ void __launch_bounds__(BLOCK) k_element_reduced_listed(Dev d, int zeroStrain, int erode) {
     __shared__ double sh[BLOCK / 32];
     if (!d.s->active) return;
@@ -294,7 +296,7 @@ __global__ void __launch_bounds__(BLOCK) k_element_reduced_listed(Dev d, int zer
         double2 cur[4];                  // x + u of the nodes, for the erosion test and cr/cz
         element_current(d, e, cur);
         if (erode) erode_element(d, e, energy, cur);
-        element_reduced(d, e, zeroStrain ? 0.0 : d.s->dt, d.hourglass, minEdge, &cost, cur);
+        element_reduced<INT>(d, e, zeroStrain ? 0.0 : d.s->dt, d.hourglass, minEdge, &cost, cur);
     }
     const unsigned want = __ballot_sync(0xffffffffu, cost > 0);
     if (want) {
@@ -340,9 +342,10 @@ int listed_pass_smem(int device) {
         return 0;
     const int smem = perSm / 3 + 2048;
     if (smem > optin || 2 * (smem + 1024) > perSm) return 0;
-    if (cudaFuncSetAttribute(k_element_reduced_listed, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem) != cudaSuccess)
-        return 0;
+    for (const void *k : {(const void *)k_element_reduced_listed<false>,
+                          (const void *)k_element_reduced_listed<true>})
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+            return 0;
     return smem;
 }
 
@@ -746,11 +749,17 @@ static int assemble(Solver &S, int zeroStrain, bool prepared = false, bool erode
             k_element_full<<<grid_for(d.E, BLOCK), BLOCK, 0, st>>>(d, zeroStrain);
             n++;
         } else if (d.hot) {
-            k_element_reduced_listed<<<grid_for((long long)d.E + d.hotCap, BLOCK), BLOCK,
-                                       d.hotSmem, st>>>(d, zeroStrain, erode ? 1 : 0);
+            const int grid = grid_for((long long)d.E + d.hotCap, BLOCK);
+            if (int_products(d.E / 32, d.sms))
+                k_element_reduced_listed<true><<<grid, BLOCK, d.hotSmem, st>>>(d, zeroStrain, erode ? 1 : 0);
+            else
+                k_element_reduced_listed<false><<<grid, BLOCK, d.hotSmem, st>>>(d, zeroStrain, erode ? 1 : 0);
             n++;
         } else {
-            k_element_reduced<<<grid_for(d.E, BLOCK), BLOCK, 0, st>>>(d, zeroStrain);
+            if (int_products(d.E / 32, d.sms))
+                k_element_reduced<true><<<grid_for(d.E, BLOCK), BLOCK, 0, st>>>(d, zeroStrain);
+            else
+                k_element_reduced<false><<<grid_for(d.E, BLOCK), BLOCK, 0, st>>>(d, zeroStrain);
             n++;
         }
     }

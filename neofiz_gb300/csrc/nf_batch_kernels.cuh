@@ -116,7 +116,7 @@ __device__ bool burst_sample(const Dev &d, const BatchDev &b, const BatchInst &i
     return out;
 }
 
-template <bool MIXED, bool STAGE, int T, bool COMP>
+template <bool MIXED, bool STAGE, int T, bool COMP, bool INT>
 __device__ void run_instance(const Dev &d, const BatchDev &b, int k, int chunk, float4 *sPMid,
                              float2 *sVdt, double *shMin, int (*wallCount)[2], BlockStep *bs) {
     const BatchInst in = b.inst[k];
@@ -154,7 +154,7 @@ __device__ void run_instance(const Dev &d, const BatchDev &b, int k, int chunk, 
             wallCount[par ^ 1][0] = 0;
             wallCount[par ^ 1][1] = 0;
         }
-        minEdge = batch_step<MIXED, T, COMP>(d, in, dt, dtPrev, time, steps, geo, pMid, vdt,
+        minEdge = batch_step<MIXED, T, COMP, INT>(d, in, dt, dtPrev, time, steps, geo, pMid, vdt,
                                              base, &scp->status, &wallCount[par][0],
                                              &wallCount[par][1], impulse, loss, fric, shMin,
                                              bs);
@@ -189,7 +189,7 @@ __device__ void run_instance(const Dev &d, const BatchDev &b, int k, int chunk, 
 
 // The queue loop of the persistent kernel: each block takes the next instance (most
 // expensive first) for a chunk of steps until none is left.
-template <bool MIXED, bool STAGE, int T, bool COMP>
+template <bool MIXED, bool STAGE, int T, bool COMP, bool INT>
 __device__ __forceinline__ void batch_queue(const Dev &d, const BatchDev &b, int chunk) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ double shMin[T / 32 + 1];
@@ -204,22 +204,23 @@ __device__ __forceinline__ void batch_queue(const Dev &d, const BatchDev &b, int
         const int q = next;
         __syncthreads();
         if (q >= b.count) return;
-        run_instance<MIXED, STAGE, T, COMP>(d, b, b.order[q], chunk, sPMid, sVdt, shMin,
-                                            wallCount, &bs);
+        run_instance<MIXED, STAGE, T, COMP, INT>(d, b, b.order[q], chunk, sPMid, sVdt, shMin,
+                                                 wallCount, &bs);
     }
 }
 
 // The FP64 and mixed forms (the compiler's register choice).
-template <bool MIXED, bool STAGE, int T>
+// INT: the FP64 element's products on the integer units (int_products).
+template <bool MIXED, bool STAGE, int T, bool INT>
 __global__ void __launch_bounds__(T) k_batch_steps(Dev d, BatchDev b, int chunk) {
-    batch_queue<MIXED, STAGE, T, false>(d, b, chunk);
+    batch_queue<MIXED, STAGE, T, false, INT>(d, b, chunk);
 }
 
 // The compensated form keeps few values live across its FP32 phases: capped at 64 registers
 // (1024 resident threads per SM) it hides more memory latency than with the compiler's choice.
 template <bool STAGE, int T>
 __global__ void __launch_bounds__(T, 1024 / T) k_batch_steps_comp(Dev d, BatchDev b, int chunk) {
-    batch_queue<true, STAGE, T, true>(d, b, chunk);
+    batch_queue<true, STAGE, T, true, false>(d, b, chunk);
 }
 
 }  // namespace nf

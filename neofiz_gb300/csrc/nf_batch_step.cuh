@@ -137,7 +137,7 @@ __device__ double block_min_edge_next_f(float v, double *sh, BlockStep *bs, cons
 // compensated form's FP32 nodal update and gather (nf_bodies.cuh). With bs (a block-shared
 // BlockStep prepared for this step), the step's coefficients and the next step size come from
 // thread 0 through it; without, every thread evaluates them.
-template <bool MIXED, int T, bool COMP = false>
+template <bool MIXED, int T, bool COMP = false, bool INT = false>
 __device__ __forceinline__ double batch_step(const Dev &d, const BatchInst &in, double &dt,
                                              double &dtPrev, double &time, long long &steps,
                                              const MixedGeo &geo, const float4 *pMid,
@@ -185,7 +185,8 @@ __device__ __forceinline__ double batch_step(const Dev &d, const BatchInst &in, 
         }
     } else {
         double m = DMAX;
-        for (int e = in.e0 + threadIdx.x; e < in.e1; e += T) element_reduced(d, e, dt, in.hourglass, m);
+        for (int e = in.e0 + threadIdx.x; e < in.e1; e += T)
+            element_reduced<INT>(d, e, dt, in.hourglass, m);
         for (int k = in.k0 + threadIdx.x; k < in.k1; k += T)
             pressure_edge(d, k, time, in.pressure, in.ramp);
         me = bs ? block_min_edge_next<T>(m, shMin, bs, in, dt, dtPrev, d.finite)

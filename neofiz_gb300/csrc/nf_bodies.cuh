@@ -142,10 +142,6 @@ static __device__ __forceinline__ void prepare_node(const Dev &d, int i, double 
     geo.vdt[geo.base + i] = make_float2(nf_narrow(v.x * sdt), nf_narrow(v.y * sdt));
 }
 
-// reducedIntegration, ExplicitSolver.java:1373-1504, for element e: B at the centroid, strain
-// increments, Cayley co-rotation, J2/Johnson-Cook return, FB hourglass, the eight force
-// terms into the element's contribution slots; folds its shortest edge into minEdge.
-// *cost (when given) receives the point's Johnson-Cook cost class (j2_update).
 // The current positions x + u of element e's four nodes (the sums cr/cz and currentArea both
 // start from).
 static __device__ __forceinline__ void element_current(const Dev &d, int e, double2 *cur) {
@@ -158,7 +154,158 @@ static __device__ __forceinline__ void element_current(const Dev &d, int e, doub
     }
 }
 
-// cur (when given) holds element_current(d, e), already formed for the erosion test.
+// The element's kinematics of one assembly in the machine's arithmetic: mid-step coordinates,
+// displacement increments, shape derivatives (d2 = -d0, d3 = -d1), Jacobian and radius.
+struct ElementKin {
+    double r[4], z[4], a[4], c[4];
+    double d0r, d1r, d0z, d1z, det, rg;
+};
+static __device__ void kinematics_machine(const Dev &d, int e, double strainDt, ElementKin &k) {
+    const int4 c = d.conn[e];
+    const int n[4] = {c.x, c.y, c.z, c.w};
+    const double mid = -0.5 * strainDt;
+    for (int i = 0; i < 4; i++) {
+        const double2 v = d.V[n[i]], x = d.X0[n[i]];
+        if (d.finite) {                                  // cr/cz, :1176-1182
+            const double2 u = d.U[n[i]];
+            k.r[i] = x.x + u.x + mid * v.x;
+            k.z[i] = x.y + u.y + mid * v.y;
+        } else {
+            k.r[i] = x.x;
+            k.z[i] = x.y;
+        }
+        k.a[i] = v.x * strainDt;
+        k.c[i] = v.y * strainDt;
+    }
+    const double *r = k.r, *z = k.z;
+    const double J00 = 0.25 * (-r[0] + r[1] + r[2] - r[3]);
+    const double J01 = 0.25 * (-z[0] + z[1] + z[2] - z[3]);
+    const double J10 = 0.25 * (-r[0] - r[1] + r[2] + r[3]);
+    const double J11 = 0.25 * (-z[0] - z[1] + z[2] + z[3]);
+    k.det = J00 * J11 - J01 * J10;
+    const double inv = 1.0 / k.det;
+    k.d0r = 0.25 * (J01 - J11) * inv;
+    k.d1r = 0.25 * (J01 + J11) * inv;
+    k.d0z = 0.25 * (J10 - J00) * inv;
+    k.d1z = -0.25 * (J10 + J00) * inv;
+    k.rg = d.axi ? 0.25 * (r[0] + r[1] + r[2] + r[3]) : 0.0;
+}
+
+// What the return map starts from: strain increments, rotated stress and back stress, and the
+// element's shortest squared edge folded into minEdge. The machine's arithmetic, for the
+// elements whose integer forms were not settled.
+static __device__ __noinline__ void strain_machine(const Dev &d, int e, double strainDt,
+                                                   double *strain, double *sg, double *bk,
+                                                   double *minEdge) {
+    ElementKin k;
+    kinematics_machine(d, e, strainDt, k);
+    const double *r = k.r, *z = k.z, *a = k.a, *c = k.c;
+    if (d.finite)
+        *minEdge = shortestEdge(*minEdge, r[0], r[1], r[2], r[3], z[0], z[1], z[2], z[3]);
+    const double d2r = -k.d0r, d3r = -k.d1r, d2z = -k.d0z, d3z = -k.d1z;
+    const double dRdZ = k.d0z * a[0] + k.d1z * a[1] + d2z * a[2] + d3z * a[3];
+    const double dZdR = k.d0r * c[0] + k.d1r * c[1] + d2r * c[2] + d3r * c[3];
+    strain[0] = k.d0r * a[0] + k.d1r * a[1] + d2r * a[2] + d3r * a[3];
+    strain[1] = k.d0z * c[0] + k.d1z * c[1] + d2z * c[2] + d3z * c[3];
+    strain[2] = d.axi ? 0.25 * (a[0] + a[1] + a[2] + a[3]) / k.rg : 0.0;
+    strain[3] = dRdZ + dZdR;
+    for (int i = 0; i < 4; i++) {
+        sg[i] = d.sig[4 * (size_t)e + i];
+        bk[i] = d.back[4 * (size_t)e + i];
+    }
+    if (d.finite) {
+        const double spinDt = 0.5 * (dZdR - dRdZ);
+        if (!is_zero(spinDt)) {
+            const double h = 0.5 * spinDt;
+            const double cs = (1.0 - h * h) / (1.0 + h * h), sn = 2.0 * h / (1.0 + h * h);
+            corot_rotate(sg, cs, sn);
+            corot_rotate(bk, cs, sn);
+        }
+    }
+}
+
+// The force terms and the hourglass update from the new stress sg, in the machine's arithmetic.
+static __device__ __noinline__ void forces_machine(const Dev &d, int e, double strainDt,
+                                                   double hourglass, const double *sg) {
+    ElementKin k;
+    kinematics_machine(d, e, strainDt, k);
+    const double *r = k.r, *z = k.z, *a = k.a, *c = k.c;
+    const double dr[4] = {k.d0r, k.d1r, -k.d0r, -k.d1r}, dz[4] = {k.d0z, k.d1z, -k.d0z, -k.d1z};
+    const double sR = sg[0], sZ = sg[1], sT = sg[2], sRZ = sg[3];
+    const double dV = 4.0 * (d.axi ? 2.0 * NF_PI * k.rg * k.det : d.thickness * k.det);
+    const double hh = d.axi ? sT / k.rg * dV * 0.25 : 0.0;
+    double gr[4], gz[4];
+    for (int i = 0; i < 4; i++) {
+        gr[i] = d.axi ? -((dr[i] * sR + dz[i] * sRZ) * dV + hh) : -(dr[i] * sR + dz[i] * sRZ) * dV;
+        gz[i] = -(dz[i] * sZ + dr[i] * sRZ) * dV;
+    }
+    if (hourglass > 0.0) {
+        const double hr = r[0] - r[1] + r[2] - r[3];
+        const double hz = z[0] - z[1] + z[2] - z[3];
+        const double one[4] = {1.0, -1.0, 1.0, -1.0};
+        double y[4];
+        for (int i = 0; i < 4; i++) y[i] = one[i] - hr * dr[i] - hz * dz[i];
+        const double kk = hourglass * d.mats[d.emat[e]].mu * dV
+                          * (dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2] + dr[3] * dr[3]
+                             + dz[0] * dz[0] + dz[1] * dz[1] + dz[2] * dz[2] + dz[3] * dz[3]);
+        double2 hg = d.hg[e];
+        hg.x += kk * (y[0] * a[0] + y[1] * a[1] + y[2] * a[2] + y[3] * a[3]);
+        hg.y += kk * (y[0] * c[0] + y[1] * c[1] + y[2] * c[2] + y[3] * c[3]);
+        d.hg[e] = hg;
+        for (int i = 0; i < 4; i++) {
+            gr[i] -= y[i] * hg.x;
+            gz[i] -= y[i] * hg.y;
+        }
+        d.hgK[e] = kk;
+    }
+    double *ef = d.contribution + 8 * (size_t)e;
+    for (int i = 0; i < 4; i++) {
+        ef[i] = gr[i];
+        ef[4 + i] = gz[i];
+    }
+}
+
+// -(t + f) dV and its opposite corner's -(-t - f) dV, given the rounded products t and f of the
+// corner (the opposite corner's are their negatives), s = t + f and g = s dV. Negating both
+// terms negates the sum unless it is a zero: equal opposite terms give +0 both times.
+static __device__ __forceinline__ double opposite_force(double t, double f, double s, double g,
+                                                        double dV) {
+    const bool mirrored = !is_zero(s) || __double_as_longlong(t) == __double_as_longlong(f);
+    return mirrored ? g : copysign(0.0, -dV);
+}
+
+// A product on the integer units or on the FP64 pipe.
+template <bool INT> struct Product;
+template <> struct Product<true> {
+    static __device__ __forceinline__ double of(double a, double b, uint32_t *bad) {
+        return nf_mul_try(a, b, bad);
+    }
+};
+template <> struct Product<false> {
+    static __device__ __forceinline__ double of(double a, double b, uint32_t *) { return a * b; }
+};
+
+// reducedIntegration, ExplicitSolver.java:1373-1504, for element e: B at the centroid, strain
+// increments, Cayley co-rotation, J2/Johnson-Cook return, FB hourglass, the eight force
+// terms into the element's contribution slots; folds its shortest edge into minEdge.
+// *cost (when given) receives the point's Johnson-Cook cost class (j2_update). cur (when given)
+// holds element_current(d, e), already formed for the erosion test.
+//
+// The FP64 pipe issues one warp instruction per 64 to 76 cycles on a quarter SM, whatever the
+// operation, and bounds this code. So the quotients, the scalings by powers of two and, with INT,
+// the products run on the integer units (nf_ifp.h) beside the additions on the FP64 pipe, in
+// straight-line code. A product is 53 integer instructions: with two warps or more on a quarter
+// SM they fill the time between its FP64 instructions, but a lone warp issues them in between
+// and is faster without (int_products). An element with any operand outside their ranges (one
+// test at the end of each half) is redone by strain_machine and forces_machine. Every value has
+// the bits of the reference's sequence:
+//  * -0.5 dt v is -(dt v) / 2 exactly, and 2 (0.5 spin) is spin;
+//  * J = S / 4 with S the corner sums and det = D / 16 with D = S00 S11 - S01 S10, so
+//    0.25 (J01 - J11) / det = (S01 - S11) / D: powers of two cancel while every scaled value
+//    stays normal, which bounding the S and D exponents guarantees;
+//  * the derivatives of opposite corners are negatives, so are their products, and 1 - hr d2r -
+//    hz d2z is (1 + hr d0r) + hz d0z with the products of corner 0.
+template <bool INT>
 static __device__ __forceinline__ void element_reduced(const Dev &d, int e, double strainDt,
                                                        double hourglass, double &minEdge,
                                                        int *cost = nullptr,
@@ -166,172 +313,203 @@ static __device__ __forceinline__ void element_reduced(const Dev &d, int e, doub
     double *ef = d.contribution + 8 * (size_t)e;
     if (d.gone != nullptr && d.gone[e]) {
         for (int k = 0; k < 8; k++) ef[k] = 0.0;
-    } else {
-        const MatDev &fl = d.mats[d.emat[e]];
-        const double lambda = fl.lambda, mu = fl.mu;
-        const int4 c = d.conn[e];
-        const double mid = -0.5 * strainDt;
-        const double2 v0 = d.V[c.x], v1 = d.V[c.y], v2 = d.V[c.z], v3 = d.V[c.w];
-        double r0, r1, r2, r3, z0, z1, z2, z3;
-        if (d.finite) {                                  // cr/cz, :1176-1182
-            double2 p[4];
-            if (cur) {
-                for (int k = 0; k < 4; k++) p[k] = cur[k];
-            } else {
-                element_current(d, e, p);
-            }
-            r0 = p[0].x + mid * v0.x; r1 = p[1].x + mid * v1.x;
-            r2 = p[2].x + mid * v2.x; r3 = p[3].x + mid * v3.x;
-            z0 = p[0].y + mid * v0.y; z1 = p[1].y + mid * v1.y;
-            z2 = p[2].y + mid * v2.y; z3 = p[3].y + mid * v3.y;
-        } else {
-            const double2 x0 = d.X0[c.x], x1 = d.X0[c.y], x2 = d.X0[c.z], x3 = d.X0[c.w];
-            r0 = x0.x; r1 = x1.x; r2 = x2.x; r3 = x3.x;
-            z0 = x0.y; z1 = x1.y; z2 = x2.y; z3 = x3.y;
-        }
-        const double a0 = v0.x * strainDt, a1 = v1.x * strainDt;
-        const double a2 = v2.x * strainDt, a3 = v3.x * strainDt;
-        const double c0 = v0.y * strainDt, c1 = v1.y * strainDt;
-        const double c2 = v2.y * strainDt, c3 = v3.y * strainDt;
-
-        if (d.finite) minEdge = shortestEdge(minEdge, r0, r1, r2, r3, z0, z1, z2, z3);
-
-        // J = S / 4 with S the corner sums, det = D / 16 with D = S00 S11 - S01 S10, and so
-        // 0.25 (J01 - J11) / det = (S01 - S11) / D: the powers of two cancel exactly (rounding
-        // commutes with them) as long as every scaled value stays normal, which bounding the
-        // S and D exponents guarantees; otherwise the reference's own sequence runs
-        const double S00 = -r0 + r1 + r2 - r3;
-        const double S01 = -z0 + z1 + z2 - z3;
-        const double S10 = -r0 - r1 + r2 + r3;
-        const double S11 = -z0 - z1 + z2 + z3;
-        const double D = S00 * S11 - S01 * S10;
-        double det, d0r, d1r, d0z, d1z;
-        if (moderate_or_zero(S00) && moderate_or_zero(S01) && moderate_or_zero(S10) &&
-            moderate_or_zero(S11) && moderate_or_zero(D)) {
-            const double invD = nf_div(1.0, D);
-            det = 0.0625 * D;
-            d0r = (S01 - S11) * invD;
-            d1r = (S01 + S11) * invD;
-            d0z = (S10 - S00) * invD;
-            d1z = -((S10 + S00) * invD);
-        } else {
-            const double J00 = 0.25 * S00, J01 = 0.25 * S01, J10 = 0.25 * S10, J11 = 0.25 * S11;
-            det = J00 * J11 - J01 * J10;
-            const double inv = nf_div(1.0, det);
-            d0r = 0.25 * (J01 - J11) * inv;
-            d1r = 0.25 * (J01 + J11) * inv;
-            d0z = 0.25 * (J10 - J00) * inv;
-            d1z = -0.25 * (J10 + J00) * inv;
-        }
-        const double d2r = -d0r;
-        const double d3r = -d1r;
-        const double d2z = -d0z;
-        const double d3z = -d1z;
-
-        const double dEpsR = d0r * a0 + d1r * a1 + d2r * a2 + d3r * a3;
-        const double dEpsZ = d0z * c0 + d1z * c1 + d2z * c2 + d3z * c3;
-        const double dRdZ = d0z * a0 + d1z * a1 + d2z * a2 + d3z * a3;
-        const double dZdR = d0r * c0 + d1r * c1 + d2r * c2 + d3r * c3;
-        const double dGamRZ = dRdZ + dZdR;
-
-        double rg = 0.0, dEpsT = 0.0;
-        nf_divisor byRg{};
-        if (d.axi) {
-            rg = 0.25 * (r0 + r1 + r2 + r3);
-            byRg = nf_divisor_of(rg);
-            dEpsT = nf_div_by(0.25 * (a0 + a1 + a2 + a3), rg, byRg);
-        }
-        double sg[4], bk[4];
-        {
-            const double2 *ps = reinterpret_cast<const double2 *>(d.sig + 4 * (size_t)e);
-            const double2 *pb = reinterpret_cast<const double2 *>(d.back + 4 * (size_t)e);
-            const double2 s01 = ps[0], s23 = ps[1], b01 = pb[0], b23 = pb[1];
-            sg[0] = s01.x; sg[1] = s01.y; sg[2] = s23.x; sg[3] = s23.y;
-            bk[0] = b01.x; bk[1] = b01.y; bk[2] = b23.x; bk[3] = b23.y;
-        }
-        if (d.finite) {
-            const double spinDt = 0.5 * (dZdR - dRdZ);
-            if (!is_zero(spinDt)) {
-                double cs, sn;
-                corot_angles(spinDt, cs, sn);
-                corot_rotate(sg, cs, sn);
-                // a back stress of +0s (no kinematic hardening) rotates to itself
-                if (!(all_plus_zero(bk[0], bk[1], bk[2], bk[3]) && corot_keeps_zero(cs, sn)))
-                    corot_rotate(bk, cs, sn);
-            }
-        }
-        double epsP = d.epsP[e], work = d.wP[e];
-        double2 *const jcYield = d.jcYield && fl.jc ? d.jcYield + e : nullptr;
-        if (d.hasDamage) {
-            DamageRef dr;
-            dr.failureStrain = d.dFail[e];
-            dr.strength = d.dStrength + e;
-            dr.softening = d.dSoft + e;
-            dr.width = d.dWidth + e;
-            dr.geometry = d.dGeom + 5 * (size_t)e;
-            dr.fractureEnergy = d.dGf[e];
-            dr.youngs = fl.youngs;
-            j2_update(sg, bk, epsP, work, dEpsR, dEpsZ, dEpsT, dGamRZ, lambda, mu, fl,
-                      strainDt, &dr, d.dStrength[e], d.dSoft[e], cost, jcYield);
-        } else {
-            j2_update(sg, bk, epsP, work, dEpsR, dEpsZ, dEpsT, dGamRZ, lambda, mu, fl,
-                      strainDt, (const DamageRef *)nullptr, 0.0, 0.0, cost, jcYield);
-        }
-        {
-            double2 *ps = reinterpret_cast<double2 *>(d.sig + 4 * (size_t)e);
-            double2 *pb = reinterpret_cast<double2 *>(d.back + 4 * (size_t)e);
-            ps[0] = make_double2(sg[0], sg[1]); ps[1] = make_double2(sg[2], sg[3]);
-            pb[0] = make_double2(bk[0], bk[1]); pb[1] = make_double2(bk[2], bk[3]);
-            d.epsP[e] = epsP;
-            d.wP[e] = work;
-        }
-        const double sR = sg[0], sZ = sg[1], sT = sg[2], sRZ = sg[3];
-        const double dV = 4.0 * (d.axi ? 2.0 * NF_PI * rg * det : d.thickness * det);
-
-        double g0r, g1r, g2r, g3r;
-        if (d.axi) {
-            const double hh = nf_div_by(sT, rg, byRg) * dV * 0.25;
-            g0r = -((d0r * sR + d0z * sRZ) * dV + hh);
-            g1r = -((d1r * sR + d1z * sRZ) * dV + hh);
-            g2r = -((d2r * sR + d2z * sRZ) * dV + hh);
-            g3r = -((d3r * sR + d3z * sRZ) * dV + hh);
-        } else {
-            g0r = -(d0r * sR + d0z * sRZ) * dV;
-            g1r = -(d1r * sR + d1z * sRZ) * dV;
-            g2r = -(d2r * sR + d2z * sRZ) * dV;
-            g3r = -(d3r * sR + d3z * sRZ) * dV;
-        }
-        double g0z = -(d0z * sZ + d0r * sRZ) * dV;
-        double g1z = -(d1z * sZ + d1r * sRZ) * dV;
-        double g2z = -(d2z * sZ + d2r * sRZ) * dV;
-        double g3z = -(d3z * sZ + d3r * sRZ) * dV;
-
-        const double qhg = hourglass;
-        if (qhg > 0.0) {
-            const double hr = r0 - r1 + r2 - r3;
-            const double hz = z0 - z1 + z2 - z3;
-            const double y0 = 1.0 - hr * d0r - hz * d0z;
-            const double y1 = -1.0 - hr * d1r - hz * d1z;
-            const double y2 = 1.0 - hr * d2r - hz * d2z;
-            const double y3 = -1.0 - hr * d3r - hz * d3z;
-            const double k = qhg * mu * dV
-                             * (d0r * d0r + d1r * d1r + d2r * d2r + d3r * d3r
-                                + d0z * d0z + d1z * d1z + d2z * d2z + d3z * d3z);
-            double2 hg = d.hg[e];
-            hg.x += k * (y0 * a0 + y1 * a1 + y2 * a2 + y3 * a3);
-            hg.y += k * (y0 * c0 + y1 * c1 + y2 * c2 + y3 * c3);
-            d.hg[e] = hg;
-            const double qr = hg.x, qz = hg.y;
-            g0r -= y0 * qr; g1r -= y1 * qr; g2r -= y2 * qr; g3r -= y3 * qr;
-            g0z -= y0 * qz; g1z -= y1 * qz; g2z -= y2 * qz; g3z -= y3 * qz;
-            d.hgK[e] = k;
-        }
-        double2 *ef2 = reinterpret_cast<double2 *>(ef);
-        ef2[0] = make_double2(g0r, g1r);
-        ef2[1] = make_double2(g2r, g3r);
-        ef2[2] = make_double2(g0z, g1z);
-        ef2[3] = make_double2(g2z, g3z);
+        return;
     }
+    const MatDev &fl = d.mats[d.emat[e]];
+    const double lambda = fl.lambda, mu = fl.mu;
+    const int4 c = d.conn[e];
+    const double2 v0 = d.V[c.x], v1 = d.V[c.y], v2 = d.V[c.z], v3 = d.V[c.w];
+    uint32_t bad = 0;
+    const double a0 = Product<INT>::of(v0.x, strainDt, &bad), a1 = Product<INT>::of(v1.x, strainDt, &bad);
+    const double a2 = Product<INT>::of(v2.x, strainDt, &bad), a3 = Product<INT>::of(v3.x, strainDt, &bad);
+    const double c0 = Product<INT>::of(v0.y, strainDt, &bad), c1 = Product<INT>::of(v1.y, strainDt, &bad);
+    const double c2 = Product<INT>::of(v2.y, strainDt, &bad), c3 = Product<INT>::of(v3.y, strainDt, &bad);
+    double r0, r1, r2, r3, z0, z1, z2, z3;
+    if (d.finite) {                                  // cr/cz, :1176-1182
+        double2 p[4];
+        if (cur) {
+            for (int k = 0; k < 4; k++) p[k] = cur[k];
+        } else {
+            element_current(d, e, p);
+        }
+        r0 = p[0].x - nf_scale_try(a0, -1, &bad); r1 = p[1].x - nf_scale_try(a1, -1, &bad);
+        r2 = p[2].x - nf_scale_try(a2, -1, &bad); r3 = p[3].x - nf_scale_try(a3, -1, &bad);
+        z0 = p[0].y - nf_scale_try(c0, -1, &bad); z1 = p[1].y - nf_scale_try(c1, -1, &bad);
+        z2 = p[2].y - nf_scale_try(c2, -1, &bad); z3 = p[3].y - nf_scale_try(c3, -1, &bad);
+    } else {
+        const double2 x0 = d.X0[c.x], x1 = d.X0[c.y], x2 = d.X0[c.z], x3 = d.X0[c.w];
+        r0 = x0.x; r1 = x1.x; r2 = x2.x; r3 = x3.x;
+        z0 = x0.y; z1 = x1.y; z2 = x2.y; z3 = x3.y;
+    }
+    const double r10 = r1 - r0, z10 = z1 - z0;
+    double edge = minEdge;
+    if (d.finite) {                                  // shortestEdge, :1191-1197
+        const double r21 = r2 - r1, z21 = z2 - z1, r32 = r3 - r2, z32 = z3 - z2;
+        const double r03 = r0 - r3, z03 = z0 - z3;
+        const double e0 = Product<INT>::of(r10, r10, &bad) + Product<INT>::of(z10, z10, &bad);
+        const double e1 = Product<INT>::of(r21, r21, &bad) + Product<INT>::of(z21, z21, &bad);
+        const double e2 = Product<INT>::of(r32, r32, &bad) + Product<INT>::of(z32, z32, &bad);
+        const double e3 = Product<INT>::of(r03, r03, &bad) + Product<INT>::of(z03, z03, &bad);
+        edge = jmin_nonneg(edge, jmin_nonneg(jmin_nonneg(e0, e1), jmin_nonneg(e2, e3)));
+    }
+    const double S00 = r10 + r2 - r3;
+    const double S01 = z10 + z2 - z3;
+    const double S10 = -r0 - r1 + r2 + r3;
+    const double S11 = -z0 - z1 + z2 + z3;
+    const double D = Product<INT>::of(S00, S11, &bad) - Product<INT>::of(S01, S10, &bad);
+    bad |= !(moderate_or_zero(S00) & moderate_or_zero(S01) & moderate_or_zero(S10) &
+             moderate_or_zero(S11) & moderate_or_zero(D));
+    const double invD = nf_quot_try(1.0, nf_divisor_of(D), &bad);
+    const double det = nf_scale_try(D, -4, &bad);
+    const double d0r = Product<INT>::of(S01 - S11, invD, &bad);
+    const double d1r = Product<INT>::of(S01 + S11, invD, &bad);
+    const double d0z = Product<INT>::of(S10 - S00, invD, &bad);
+    const double d1z = -Product<INT>::of(S10 + S00, invD, &bad);
+
+    double strain[4];
+    strain[0] = Product<INT>::of(d0r, a0, &bad) + Product<INT>::of(d1r, a1, &bad)
+                - Product<INT>::of(d0r, a2, &bad) - Product<INT>::of(d1r, a3, &bad);
+    strain[1] = Product<INT>::of(d0z, c0, &bad) + Product<INT>::of(d1z, c1, &bad)
+                - Product<INT>::of(d0z, c2, &bad) - Product<INT>::of(d1z, c3, &bad);
+    const double dRdZ = Product<INT>::of(d0z, a0, &bad) + Product<INT>::of(d1z, a1, &bad)
+                        - Product<INT>::of(d0z, a2, &bad) - Product<INT>::of(d1z, a3, &bad);
+    const double dZdR = Product<INT>::of(d0r, c0, &bad) + Product<INT>::of(d1r, c1, &bad)
+                        - Product<INT>::of(d0r, c2, &bad) - Product<INT>::of(d1r, c3, &bad);
+    strain[3] = dRdZ + dZdR;
+
+    double rg = 0.0;
+    nf_divisor byRg{};
+    strain[2] = 0.0;
+    if (d.axi) {
+        rg = nf_scale_try(r0 + r1 + r2 + r3, -2, &bad);
+        byRg = nf_divisor_of(rg);
+        strain[2] = nf_quot_try(nf_scale_try(a0 + a1 + a2 + a3, -2, &bad), byRg, &bad);
+    }
+    double sg[4], bk[4];
+    {
+        const double2 *ps = reinterpret_cast<const double2 *>(d.sig + 4 * (size_t)e);
+        const double2 *pb = reinterpret_cast<const double2 *>(d.back + 4 * (size_t)e);
+        const double2 s01 = ps[0], s23 = ps[1], b01 = pb[0], b23 = pb[1];
+        sg[0] = s01.x; sg[1] = s01.y; sg[2] = s23.x; sg[3] = s23.y;
+        bk[0] = b01.x; bk[1] = b01.y; bk[2] = b23.x; bk[3] = b23.y;
+    }
+    if (d.finite) {
+        const double w = dZdR - dRdZ;
+        const double spinDt = nf_scale_try(w, -1, &bad);
+        if (!is_zero(spinDt)) {
+            const double h = nf_scale_try(w, -2, &bad);
+            const double hh = Product<INT>::of(h, h, &bad);
+            const nf_divisor by = nf_divisor_of(1.0 + hh);
+            const double cs = nf_quot_try(1.0 - hh, by, &bad), sn = nf_quot_try(spinDt, by, &bad);
+            // a back stress of +0s (no kinematic hardening) rotates to itself
+            const bool still = all_plus_zero(bk[0], bk[1], bk[2], bk[3]) && corot_keeps_zero(cs, sn);
+            const double ccc = Product<INT>::of(cs, cs, &bad), sss = Product<INT>::of(sn, sn, &bad);
+            const double csn = Product<INT>::of(cs, sn, &bad), csn2 = nf_scale_try(csn, 1, &bad);
+            const double diff = ccc - sss;
+            auto rotate = [&](double *t) {           // corot_rotate
+                const double rr = t[0], zz = t[1], rz = t[3];
+                const double shear = Product<INT>::of(csn2, rz, &bad);
+                t[0] = Product<INT>::of(ccc, rr, &bad) - shear + Product<INT>::of(sss, zz, &bad);
+                t[1] = Product<INT>::of(sss, rr, &bad) + shear + Product<INT>::of(ccc, zz, &bad);
+                t[3] = Product<INT>::of(csn, rr - zz, &bad) + Product<INT>::of(diff, rz, &bad);
+            };
+            rotate(sg);
+            if (!still) rotate(bk);
+        }
+    }
+    if (bad) strain_machine(d, e, strainDt, strain, sg, bk, &minEdge);
+    else minEdge = edge;
+
+    double epsP = d.epsP[e], work = d.wP[e];
+    double2 *const jcYield = d.jcYield && fl.jc ? d.jcYield + e : nullptr;
+    if (d.hasDamage) {
+        DamageRef dr;
+        dr.failureStrain = d.dFail[e];
+        dr.strength = d.dStrength + e;
+        dr.softening = d.dSoft + e;
+        dr.width = d.dWidth + e;
+        dr.geometry = d.dGeom + 5 * (size_t)e;
+        dr.fractureEnergy = d.dGf[e];
+        dr.youngs = fl.youngs;
+        j2_update(sg, bk, epsP, work, strain[0], strain[1], strain[2], strain[3], lambda, mu, fl,
+                  strainDt, &dr, d.dStrength[e], d.dSoft[e], cost, jcYield);
+    } else {
+        j2_update(sg, bk, epsP, work, strain[0], strain[1], strain[2], strain[3], lambda, mu, fl,
+                  strainDt, (const DamageRef *)nullptr, 0.0, 0.0, cost, jcYield);
+    }
+    {
+        double2 *ps = reinterpret_cast<double2 *>(d.sig + 4 * (size_t)e);
+        double2 *pb = reinterpret_cast<double2 *>(d.back + 4 * (size_t)e);
+        ps[0] = make_double2(sg[0], sg[1]); ps[1] = make_double2(sg[2], sg[3]);
+        pb[0] = make_double2(bk[0], bk[1]); pb[1] = make_double2(bk[2], bk[3]);
+        d.epsP[e] = epsP;
+        d.wP[e] = work;
+    }
+    const double sR = sg[0], sZ = sg[1], sT = sg[2], sRZ = sg[3];
+    const double dV = nf_scale_try(d.axi ? Product<INT>::of(Product<INT>::of(2.0 * NF_PI, rg, &bad), det, &bad)
+                                         : Product<INT>::of(d.thickness, det, &bad), 2, &bad);
+    double g0r, g1r, g2r, g3r, g0z, g1z, g2z, g3z;
+    {
+        const double t0 = Product<INT>::of(d0r, sR, &bad), f0 = Product<INT>::of(d0z, sRZ, &bad);
+        const double t1 = Product<INT>::of(d1r, sR, &bad), f1 = Product<INT>::of(d1z, sRZ, &bad);
+        const double w0 = t0 + f0, w1 = t1 + f1;
+        const double G0 = Product<INT>::of(w0, dV, &bad), G1 = Product<INT>::of(w1, dV, &bad);
+        const double H0 = opposite_force(t0, f0, w0, G0, dV);
+        const double H1 = opposite_force(t1, f1, w1, G1, dV);
+        if (d.axi) {
+            const double hh = nf_scale_try(Product<INT>::of(nf_quot_try(sT, byRg, &bad), dV, &bad), -2, &bad);
+            g0r = -(G0 + hh);
+            g1r = -(G1 + hh);
+            g2r = -(hh - H0);                        // -(-G0 + hh)
+            g3r = -(hh - H1);
+        } else {
+            g0r = -G0; g1r = -G1; g2r = H0; g3r = H1;
+        }
+        const double p0 = Product<INT>::of(d0z, sZ, &bad), q0 = Product<INT>::of(d0r, sRZ, &bad);
+        const double p1 = Product<INT>::of(d1z, sZ, &bad), q1 = Product<INT>::of(d1r, sRZ, &bad);
+        const double s0 = p0 + q0, s1 = p1 + q1;
+        const double K0 = Product<INT>::of(s0, dV, &bad), K1 = Product<INT>::of(s1, dV, &bad);
+        g0z = -K0; g1z = -K1;
+        g2z = opposite_force(p0, q0, s0, K0, dV);
+        g3z = opposite_force(p1, q1, s1, K1, dV);
+    }
+    double2 hg;
+    double kh = 0.0;
+    if (hourglass > 0.0) {
+        const double hr = -r10 + r2 - r3;
+        const double hz = -z10 + z2 - z3;
+        const double m0 = Product<INT>::of(hr, d0r, &bad), n0 = Product<INT>::of(hz, d0z, &bad);
+        const double m1 = Product<INT>::of(hr, d1r, &bad), n1 = Product<INT>::of(hz, d1z, &bad);
+        const double y0 = 1.0 - m0 - n0, y2 = 1.0 + m0 + n0;
+        const double y1 = -1.0 - m1 - n1, y3 = -1.0 + m1 + n1;
+        const double q0 = Product<INT>::of(d0r, d0r, &bad), q1 = Product<INT>::of(d1r, d1r, &bad);
+        const double q2 = Product<INT>::of(d0z, d0z, &bad), q3 = Product<INT>::of(d1z, d1z, &bad);
+        kh = Product<INT>::of(Product<INT>::of(Product<INT>::of(hourglass, mu, &bad), dV, &bad),
+                        q0 + q1 + q0 + q1 + q2 + q3 + q2 + q3, &bad);
+        hg = d.hg[e];
+        hg.x += Product<INT>::of(kh, Product<INT>::of(y0, a0, &bad) + Product<INT>::of(y1, a1, &bad)
+                               + Product<INT>::of(y2, a2, &bad) + Product<INT>::of(y3, a3, &bad), &bad);
+        hg.y += Product<INT>::of(kh, Product<INT>::of(y0, c0, &bad) + Product<INT>::of(y1, c1, &bad)
+                               + Product<INT>::of(y2, c2, &bad) + Product<INT>::of(y3, c3, &bad), &bad);
+        const double qr = hg.x, qz = hg.y;
+        g0r -= Product<INT>::of(y0, qr, &bad); g1r -= Product<INT>::of(y1, qr, &bad);
+        g2r -= Product<INT>::of(y2, qr, &bad); g3r -= Product<INT>::of(y3, qr, &bad);
+        g0z -= Product<INT>::of(y0, qz, &bad); g1z -= Product<INT>::of(y1, qz, &bad);
+        g2z -= Product<INT>::of(y2, qz, &bad); g3z -= Product<INT>::of(y3, qz, &bad);
+    }
+    if (bad) {
+        forces_machine(d, e, strainDt, hourglass, sg);
+        return;
+    }
+    if (hourglass > 0.0) {
+        d.hg[e] = hg;
+        d.hgK[e] = kh;
+    }
+    double2 *ef2 = reinterpret_cast<double2 *>(ef);
+    ef2[0] = make_double2(g0r, g1r);
+    ef2[1] = make_double2(g2r, g3r);
+    ef2[2] = make_double2(g0z, g1z);
+    ef2[3] = make_double2(g2z, g3z);
 }
 
 static __device__ __forceinline__ float diff_hl(float4 a, float4 b, int comp) {

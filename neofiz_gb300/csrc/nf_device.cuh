@@ -16,6 +16,7 @@
 #include "nf_math.h"
 #include "nf_ifp.h"
 #include "nf_ilog.h"
+#include "nf_fpconv.h"
 
 namespace nf {
 
@@ -171,8 +172,8 @@ __device__ __forceinline__ T jc_quasiStatic(const MatT<T> &f, T eps, T temperatu
     return jc_strainTerm(f, eps) * jc_thermalTerm(f, temperature);
 }
 
-// What J2.solve returns, and what it knew of its answer: the iterations taken and, when it
-// converged, the strain term at the returned increment (the new state's, which the caller
+// What J2.solve returns, and what it knew of its answer: the iterations computed in full (its
+// cost) and, when it converged, the strain term at the returned increment (the new state's, which the caller
 // would otherwise evaluate again).
 template <typename T>
 struct SolveOut {
@@ -223,11 +224,13 @@ static __device__ __noinline__ NewtonStep<double> newton_slow(double norm, doubl
 // them was not settled (about one point-iteration in a thousand).
 template <typename T>
 struct Newton {
-    __device__ __forceinline__ Newton(T, const MatT<T> &) {}
+    __device__ __forceinline__ Newton(T, T, T, T, T, const MatT<T> &) {}
     __device__ __forceinline__ NewtonStep<T> step(T norm, T stiffness, T plasticStrain, T thermal,
                                                   T dt, const MatT<T> &jc, T dGamma) const {
         return newton_step(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
     }
+    __device__ __forceinline__ bool bisects(T, T, T, bool &) const { return false; }
+    static __device__ __forceinline__ T middle(T lo, T hi) { return T(0.5) * (lo + hi); }
     static __device__ __forceinline__ bool positive(T x) { return x > T(0); }
     static __device__ __forceinline__ bool within(T x, T bound) { return Fn<T>::abs(x) <= bound; }
     static __device__ __forceinline__ bool between(T x, T lo, T hi) { return x > lo && x < hi; }
@@ -236,8 +239,67 @@ template <>
 struct Newton<double> {
     nf_divisor byDt;
     int plain;                   // dt > 0 and the reference rate is 1/s (no second division)
-    __device__ __forceinline__ Newton(double dt, const MatDev &jc)
-        : byDt(nf_divisor_of(dt)), plain(dt > 0.0 && jc.refRate == 1.0) {}
+    float norm, stiffness, plasticStrain, thermal, perDt, a, b, n, c;
+    __device__ __forceinline__ Newton(double norm_, double stiffness_, double plasticStrain_,
+                                      double thermal_, double dt, const MatDev &jc)
+        : byDt(nf_divisor_of(dt)), plain(dt > 0.0 && jc.refRate == 1.0), norm(nf_narrow(norm_)),
+          stiffness(nf_narrow(stiffness_)), plasticStrain(nf_narrow(plasticStrain_)),
+          thermal(nf_narrow(thermal_)), perDt(1.0f / nf_narrow(dt)), a(nf_narrow(jc.a)),
+          b(nf_narrow(jc.b)), n(nf_narrow(jc.n)), c(nf_narrow(jc.c)) {}
+
+    // Whether the iteration at dGamma is certain to bisect, and the sign of its residual: decided
+    // in FP32 where the answer is clear. In a long solve two iterations of three bisect (the
+    // power law is steep near zero and Newton's step leaves the bracket), and such an iteration
+    // needs only its residual's sign and that the step is too long. The approximations' bounds
+    // are PTX's: rcp 2^-23, lg2 2^-22 (absolute near 1, relative elsewhere), ex2 2^-22. eps^n is
+    // then good to 2^-17 for |n log2 eps| < 32, the residual g, a difference of positive terms
+    // whose sum is m, to 2^-16 m, and the slope, a sum of positive terms, to 2^-16 of itself.
+    // With |g| above 2^-8 m the step is good to 2^-7; one longer than the bracket by 2^-5 leaves
+    // it in FP64 too, and |g| is far above the solve's tolerance. Anything else (a NaN, a rate
+    // within 2^-8 of the reference rate, where the slope jumps, a bracket too narrow for FP32)
+    // is not decided here.
+    __device__ __forceinline__ bool bisects(double dGamma, double lo, double hi, bool &up) const {
+        const float dg = cut(dGamma), gapUp = cut(hi) - dg, gapDown = dg - cut(lo);
+        const float dEps = 0.8164966f * dg, eps = plasticStrain + dEps, rate = dEps * perDt;
+        const float power = n * lg2(eps), pw = ex2(power), strain = a + b * pw;
+        const bool fast = rate > 1.0f;
+        const float rateFactor = fast ? 1.0f + c * (0.6931472f * lg2(rate)) : 1.0f;
+        const float flow = 0.8164966f * strain * thermal, taken = stiffness * dg;
+        const float pull = flow * rateFactor;
+        const float g = norm - taken - pull, size = fabsf(g);
+        float slope = stiffness + 0.6666667f * (n * b * pw * rcp(eps)) * rateFactor * thermal;
+        if (fast) slope += flow * c * rcp(dg);
+        up = g > 0.0f;
+        const float gap = up ? gapUp : gapDown;
+        return plain && size > 0x1p-8f * (norm + taken + pull) && size > 1.0e-9f * a
+               && fabsf(rate - 1.0f) > 0x1p-8f && power > -32.0f && gap > 0x1p-12f * dg
+               && dg > 1.0e-30f && size > slope * gap * (1.0f + 0x1p-5f) && size < 1.0e30f
+               && slope < 1.0e30f;
+    }
+    static __device__ __forceinline__ float rcp(float x) {
+        float y;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+        return y;
+    }
+    static __device__ __forceinline__ float lg2(float x) {
+        float y;
+        asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+        return y;
+    }
+    static __device__ __forceinline__ float ex2(float x) {
+        float y;
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+        return y;
+    }
+    // x >= 0 cut to FP32's 24 bits (relative error 2^-23); 0 outside FP32's normal range
+    static __device__ __forceinline__ float cut(double x) {
+        const uint32_t h = nf_ifp_hi(x) - (896u << 20);
+        return h - 0x00100000u < 0x0fd00000u ? __uint_as_float(nf_ifp_shl(h, nf_ifp_lo(x), 3)) : 0.0f;
+    }
+    // (lo + hi) / 2 of a bracket 0 <= lo <= hi; lo is 0 until a residual is positive
+    static __device__ __forceinline__ double middle(double lo, double hi) {
+        return nf_scale2(is_zero(lo) ? hi : lo + hi, -1);
+    }
     __device__ __forceinline__ NewtonStep<double> step(double norm, double stiffness,
                                                        double plasticStrain, double thermal,
                                                        double dt, const MatDev &jc,
@@ -247,21 +309,26 @@ struct Newton<double> {
         const double eps = plasticStrain + dEps;
         const double rate = nf_div_try(dEps, byDt, &okRate);
         const double lg = nf_log_try(rate, &okLog);
-        const double pw = nf_pow_try(eps, jc.n, &okPow);
+        nf_pow_tail tail;
+        const double pw = nf_pow_try(eps, jc.n, &okPow, &tail);
         const double strain = jc.a + jc.b * pw;
         // rate <= 1 by bits: a sure quotient of dEps >= 0 by dt > 0 is no NaN
         const bool slow = __double_as_longlong(rate) <= __double_as_longlong(1.0);
         const bool flat = slow || jc.c == 0.0;             // 1 + 0 log is 1
-        const double rateFactor = flat ? 1.0 : 1.0 + jc.c * lg;
+        // the products off the chain through the power run on the integer units
+        uint32_t bad = 0;
+        const double clg = nf_mul_try(jc.c, flat ? 1.0 : lg, &bad);
+        const double rateFactor = flat ? 1.0 : 1.0 + clg;
         const double flow = SQRT_2_3 * strain;
-        const double g = norm - stiffness * dGamma - flow * rateFactor * thermal;
+        const double g = norm - nf_mul_try(stiffness, dGamma, &bad) - flow * rateFactor * thermal;
         const double q1 = nf_div_try(jc.n * (strain - jc.a), nf_divisor_of(eps), &ok1);
-        const double q2 = nf_div_try(flow * jc.c * thermal, nf_divisor_of(dGamma), &ok2);
+        const double fct = nf_mul_try(nf_mul_try(flow, jc.c, &bad), thermal, &bad);
+        const double q2 = nf_div_try(fct, nf_divisor_of(dGamma), &ok2);
         const double base = -stiffness - TWO_THIRDS * q1 * rateFactor * thermal;
         const double slope = slow ? base : base - q2;
         const double q = nf_div_try(g, nf_divisor_of(slope), &okStep);
-        if (plain & okRate & okPow & (okLog | flat) & ok1 & (ok2 | slow) & okStep)
-            return NewtonStep<double>{g, strain, q};
+        if (plain & okRate & (okLog | flat) & ok1 & (ok2 | slow) & okStep & (bad ^ 1u))
+            if (okPow || nf_pow_settled(&tail)) return NewtonStep<double>{g, strain, q};
         return newton_slow(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
     }
     // x > 0, |x| <= bound (bound >= 0), and lo < x < hi (0 <= lo, hi), by the integer order of
@@ -288,18 +355,34 @@ static __device__ __noinline__ SolveOut<T> j2_solve(T norm, T stiffness, T plast
     T lo = T(0);
     T hi = Fn<T>::div(norm, stiffness);
     T dGamma = hi;
-    const Newton<T> newton(dt, jc);
+    const Newton<T> newton(norm, stiffness, plasticStrain, thermal, dt, jc);
+    // iterations so far and those computed in full; one loop exit, so that a warp's lanes bisect
+    // as far as they can and then step together
+    int iteration = 0, steps = 0, converged = 0;
+    T strain = T(0);
 #pragma unroll 1
-    for (int iteration = 0; iteration < SOLVE_ITERATIONS; iteration++) {
-        const NewtonStep<T> n = newton.step(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
-        if (Newton<T>::positive(n.g)) lo = dGamma; else hi = dGamma;
-        if (Newton<T>::within(n.g, tolerance))
-            return SolveOut<T>{dGamma, n.strain, iteration + 1, 1};
-        T next = dGamma - n.quotient;
-        if (!Newton<T>::between(next, lo, hi)) next = T(0.5) * (lo + hi);
-        dGamma = next;
+    while (!converged && iteration < SOLVE_ITERATIONS) {
+        bool up;
+#pragma unroll 1
+        while (iteration < SOLVE_ITERATIONS && newton.bisects(dGamma, lo, hi, up)) {
+            if (up) lo = dGamma; else hi = dGamma;
+            dGamma = Newton<T>::middle(lo, hi);
+            iteration++;
+        }
+        if (iteration < SOLVE_ITERATIONS) {
+            const NewtonStep<T> n =
+                newton.step(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
+            if (Newton<T>::positive(n.g)) lo = dGamma; else hi = dGamma;
+            converged = Newton<T>::within(n.g, tolerance);
+            T next = dGamma - n.quotient;
+            if (!Newton<T>::between(next, lo, hi)) next = Newton<T>::middle(lo, hi);
+            if (!converged) dGamma = next;
+            strain = n.strain;
+            iteration++;
+            steps++;
+        }
     }
-    return SolveOut<T>{dGamma, T(0), SOLVE_ITERATIONS, 0};
+    return SolveOut<T>{dGamma, strain, steps, converged};
 }
 
 // Damage.begin, Damage.java:306-336

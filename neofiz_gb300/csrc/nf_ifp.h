@@ -219,4 +219,62 @@ NF_IFP double nf_sqrt(double a) {
     return sqrt(a);
 }
 
+/* Products and scalings in integer arithmetic for straight-line code: each returns the machine's
+ * bits or sets *bad, which the caller tests once at the end to take the machine path instead.
+ * A product costs about as much on the integer units as on the FP64 pipe; code that spreads its
+ * products over both runs them side by side. */
+
+/* x is +-0. */
+NF_IFP int nf_ifp_zero(uint32_t h, uint32_t l) { return ((h << 1) | l) == 0u; }
+
+/* a b: both moderate, or one a zero and the other moderate or a zero. */
+NF_IFP double nf_mul_try(double a, double b, uint32_t *bad) {
+    const uint32_t ha = nf_ifp_hi(a), la = nf_ifp_lo(a), hb = nf_ifp_hi(b), lb = nf_ifp_lo(b);
+    const uint32_t ma = (ha & 0xfffffu) | 0x100000u, mb = (hb & 0xfffffu) | 0x100000u;
+    const int za = nf_ifp_zero(ha, la), zb = nf_ifp_zero(hb, lb);
+    /* the 106-bit product of the significands, in [2^104, 2^106); its top 64 bits in t (above
+     * 2^106 2^-64 a leading zero at most), the rest only as zero or not */
+    const uint64_t p = (uint64_t)la * lb;
+    const uint64_t q = (uint64_t)la * mb + ((uint64_t)ma * lb + (p >> 32));
+    const uint64_t r = (uint64_t)ma * mb + (q >> 32);
+    const uint32_t th = nf_ifp_shr((uint32_t)(r >> 32), (uint32_t)r, 10);
+    const uint32_t rest = ((uint32_t)q & 0x3ffu) | (uint32_t)p;
+    const uint32_t tl = nf_ifp_shr((uint32_t)r, (uint32_t)q, 10) | (rest < 1u ? rest : 1u);
+    const uint32_t n = th >> 31;                       /* 0: normalise by one place */
+    const uint64_t t = (((uint64_t)th << 32) | tl) << (n ^ 1u);
+    const uint32_t e = (ha & 0x7ff00000u) + (hb & 0x7ff00000u) - 0x3ff00000u + (n << 20);
+    const uint32_t sign = (ha ^ hb) & 0x80000000u;
+    *bad |= ((uint32_t)((nf_ifp_moderate(ha) | za) & (nf_ifp_moderate(hb) | zb)) ^ 1u)
+            | ((e >= 0x7fe00000u) & (uint32_t)((za | zb) ^ 1));
+    /* round to nearest even at bit 11 */
+    const uint32_t up = (((uint32_t)t & 0x7ffu) + 0x3ffu + ((uint32_t)(t >> 11) & 1u)) >> 11;
+    const uint64_t v = (t >> 11) + up + ((uint64_t)(e + sign - 0x100000u) << 32);
+    const int zero = za | zb;
+    return nf_ifp_make(zero ? sign : (uint32_t)(v >> 32), zero ? 0u : (uint32_t)v);
+}
+
+/* x 2^k, |k| <= 8: a zero or a number in 2^+-1000. */
+NF_IFP double nf_scale_try(double x, int k, uint32_t *bad) {
+    const uint32_t h = nf_ifp_hi(x), l = nf_ifp_lo(x);
+    const int normal = (h & 0x7fffffffu) - 0x01700000u < 0x7d000000u;
+    const int zero = nf_ifp_zero(h, l);
+    *bad |= (uint32_t)(normal | zero) ^ 1u;
+    return nf_ifp_make(zero ? h : h + ((uint32_t)k << 20), l);
+}
+
+/* x 2^k, |k| <= 8, by the machine's product outside nf_scale_try's range. */
+NF_IFP double nf_scale2(double x, int k) {
+    uint32_t bad = 0;
+    const double r = nf_scale_try(x, k, &bad);
+    return bad ? x * nf_ifp_make((uint32_t)(1023 + k) << 20, 0u) : r;
+}
+
+/* a / b (nf_div_try) with the same convention. */
+NF_IFP double nf_quot_try(double a, nf_divisor b, uint32_t *bad) {
+    int sure;
+    const double q = nf_div_try(a, b, &sure);
+    *bad |= (uint32_t)sure ^ 1u;
+    return q;
+}
+
 #endif /* NF_IFP_H */

@@ -9,8 +9,9 @@
  *
  * with r = z invc - 1 = rh + rl exact, rh the part nf_log_dd's rounded product gives. nf_log_dd
  * rounds inside: its cubic term (|rh^3 / 3| < 2^-25.5) five times and the sum of its small
- * terms, together less than 2^-76 for |k| <= 64; the fixed-point terms are truncated by less
- * than 2^-77. So the two sums lie within NF_LOG_SLACK = 2^-75 of each other, and where no
+ * terms, together less than 240 units for |k| <= 64; the fixed-point terms are off by less than
+ * 115 (the -rh^3/6 term 77, k ln2 32). So the two sums lie within 384 units of each other (207
+ * is the most that 60 million arguments showed), and where no
  * rounding boundary lies that close to the fixed-point sum, both round to the same double
  * (Ziv's test: A. Ziv, "Fast evaluation of elementary mathematical functions with correctly
  * rounded last bit", ACM TOMS 17, 1991). Where one does, and outside 2^-64 <= x < 2^64 or for
@@ -26,7 +27,10 @@
 #include "nf_math.h"
 #include "nf_ifp.h"
 
-#define NF_LOG_SLACK_EXP (-75)
+/* (NF_EXP_L_HI + NF_EXP_L_LO) 2^96, exact */
+#define NF_LN2_128_0 0x5793c767u
+#define NF_LN2_128_1 0xefa39ef3u
+#define NF_LN2_128_2 0x0162e42fu
 
 #if defined(__CUDACC__)
 #define NF_ILOG_SLOW static __host__ __device__ __noinline__
@@ -168,7 +172,7 @@ NF_IFP double nf_ilog_round(nf_ilog v, uint32_t *below) {
                        + ((uint64_t)((uint32_t)(1033 - v.n) << 20 | v.neg) << 32);
     return nf_ifp_make((uint32_t)(m >> 32), (uint32_t)m);
 }
-/* The slack in units of below is 2^(84 - 75 + n - 11), n <= 19: whether half lies within it. */
+/* Whether half lies within the slack (384 2^n units, below 2^(n - 2) of below's; n <= 19). */
 NF_IFP int nf_ilog_near_half(uint32_t below, int n) {
     return below - 0x80000000u + (1u << n) < (2u << n);
 }
@@ -188,53 +192,119 @@ NF_IFP double nf_log_fast(double x) {
     return sure ? r : nf_log_slow(x);
 }
 
-/* nf_pow(x, y) where *sure, without a branch. */
-NF_IFP double nf_pow_try(double x, double y, int *sure) {
+/* The last sum of a power whose r the slack may move by a unit: er = RN(thi + w). inRange: only
+ * r's rounding is open, |r| in [2^(-1 - z), 2^-z). */
+typedef struct { double thi, w, er; int inRange, z; } nf_pow_tail;
+
+/* nf_pow(x, y) where *sure, without a branch. The product p = y lh, its error, the reduced
+ * argument a = p - n ln2/128 and the sum r = a + plo are nf_exp_dd's, each rounded as its FP64
+ * operation rounds: products and differences are exact in fixed point (n ln2/128 is a multiple
+ * of 2^-96), so every rounding is known but the last, which has the slack in it and is sure
+ * where the sum's tail stays that far from half a unit. */
+NF_IFP double nf_pow_try(double x, double y, int *sure, nf_pow_tail *tail) {
     nf_ilog v;
     uint32_t below;
-    const uint32_t yh = nf_ifp_hi(y);
+    const uint32_t yh = nf_ifp_hi(y), yl = nf_ifp_lo(y);
     /* 2^-9 <= y < 2 */
-    const int ok = nf_ilog_of(x, &v) & (yh - 0x3f600000u < 0x00a00000u);
-    const double lh = nf_ilog_round(v, &below);
-    /* lo = log x - lh: 43 bits and a sign */
-    const uint64_t rest = ((uint64_t)(v.w1 & 0x7ffu) << 32) | v.w0;
-    const int roundedUp = (int)(below >> 31);
-    uint64_t g = roundedUp ? ((uint64_t)0x800 << 32) - rest : rest;
-    g |= 1u;
-    const uint32_t gh = (uint32_t)(g >> 32);
-    const int sh = gh ? nf_ilog_clz(gh) : 32 + nf_ilog_clz((uint32_t)g);     /* >= 20 */
-    g <<= sh;                                                                /* top bit set */
-    /* value g 2^(-84 - n - sh): field 1023 + 63 - 84 - n - sh, the leading bit adds one to it */
-    const uint64_t gb = (g >> 11) + ((uint64_t)((uint32_t)(1001 - v.n - sh) << 20) << 32);
-    const double ll = nf_ifp_make((uint32_t)(gb >> 32) | (v.neg ^ (roundedUp ? 0x80000000u : 0u)),
-                                  (uint32_t)gb);
-    const double p = y * lh;
-    const double plo = fma(y, ll, fma(y, lh, -p));
-    /* nf_exp_dd(p, plo) */
-    const double kd = rint(p * NF_EXP_N_OVER_LN2);
-    const int n = (int)kd;
-    const double al = fma(-kd, NF_EXP_L_LO, fma(-kd, NF_EXP_L_HI, p));
-    const double r = al + plo;
-    /* the sum's error and how far it stays from half an ulp of r (all exact), against y times
-     * the slack (the high words of two doubles order as they do) */
-    const double e = plo - (r - al);
-    const uint32_t rx = nf_ifp_hi(r) & 0x7ff00000u;
-    const double gap = nf_ifp_make(rx - (53u << 20), 0u) - fabs(e);
-    *sure = ok & ((int32_t)nf_ifp_hi(gap) > (int32_t)(yh - ((uint32_t)(-NF_LOG_SLACK_EXP) << 20)))
-            & (rx > (60u << 20)) & !nf_ilog_near_half(below, v.n);
-    const int j = n & 127, m = (n - j) / 128;
+    int ok = nf_ilog_of(x, &v) & (yh - 0x3f600000u < 0x00a00000u);
+    below = nf_ifp_shl(v.w1, v.w0, 21);
+    ok &= !nf_ilog_near_half(below, v.n);
+    /* |lh| = lm 2^(-41 - n) (lm up to 2^53), |log x| - |lh| = g 2^(-84 - n) */
+    const uint32_t up = below >> 31;
+    const uint64_t lm = ((((uint64_t)v.w2 << 32) | v.w1) >> 11) + up;
+    const int64_t g = (int64_t)(((uint64_t)(v.w1 & 0x7ffu) << 32) | v.w0) - ((int64_t)up << 43);
+    /* P = y's significand times lm, in units 2^(ey - n - 93); p its 53-bit rounding */
+    const int ey = (int)(yh >> 20) - 1023;
+    const uint32_t myh = (yh & 0xfffffu) | 0x100000u;
+    const uint32_t ll = (uint32_t)lm, lh = (uint32_t)(lm >> 32);
+    const uint64_t b0 = (uint64_t)yl * ll;
+    const uint64_t b1 = (uint64_t)yl * lh + ((uint64_t)myh * ll + (b0 >> 32));
+    const uint64_t b2 = (uint64_t)myh * lh + (b1 >> 32);       /* P = b2 : lo b1 : lo b0 */
+    const uint32_t P0 = (uint32_t)b0, P1 = (uint32_t)b1, P2 = (uint32_t)b2, P3 = (uint32_t)(b2 >> 32);
+    const int top = (int)(P3 >> 9);                            /* P >= 2^105 */
+    /* shifted so that 53 bits are dropped */
+    const uint32_t s0 = P0 << (top ^ 1), s1 = nf_ilog_up(P1, P0, top ^ 1);
+    const uint32_t s2 = nf_ilog_up(P2, P1, top ^ 1), s3 = nf_ilog_up(P3, P2, top ^ 1);
+    const uint32_t half = (s1 >> 20) & 1u;
+    const uint64_t pm = ((((uint64_t)s3 << 32) | s2) << 11 | (s1 >> 21)) + half;
+    const int64_t pr = (int64_t)(((uint64_t)(s1 & 0x1fffffu) << 32) | s0) - ((int64_t)half << 53);
+    ok &= ((s1 & 0x1fffffu) != 0x100000u);                     /* a halfway case, or near one */
+    /* |p| in [2^k, 2^(k+1)): p = pm 2^(k - 52) */
+    const int k = ey - v.n + 11 + top;
+    /* n = rint(p 128 / ln2) from its integer and 20 fraction bits, at most 4 units off */
+    const uint32_t v20 = nf_ifp_mulhi((uint32_t)(pm >> 21), 0xb8aa3b29u) >> ((3 - k) & 31);
+    const uint32_t n = (v20 + 0x80000u) >> 20;
+    ok &= (((v20 + 4u - 0x80000u) & 0xfffffu) >= 8u) & (k <= 3);
+    /* a = RN(p - n ln2/128) in units of 2^-96: |p| is below 2^4 and the difference below 2^-8 */
+    const int sp = 44 + k;
+    const uint32_t q0 = (uint32_t)pm << (sp & 31), q1 = nf_ilog_up((uint32_t)(pm >> 32), (uint32_t)pm, sp & 31);
+    const uint32_t q2 = nf_ilog_up(0u, (uint32_t)(pm >> 32), sp & 31);
+    const int wide = sp >= 32;
+    const uint32_t t0 = wide ? 0u : q0, t1 = wide ? q0 : q1, t2 = wide ? q1 : q2;
+    const uint64_t m0 = (uint64_t)n * NF_LN2_128_0;
+    const uint64_t m1 = (uint64_t)n * NF_LN2_128_1 + (m0 >> 32);
+    const uint32_t m2 = n * NF_LN2_128_2 + (uint32_t)(m1 >> 32);
+    const uint64_t tl = ((uint64_t)t1 << 32) | t0, ml = ((uint64_t)(uint32_t)m1 << 32) | (uint32_t)m0;
+    const uint64_t dl = tl - ml;
+    const uint32_t dh = t2 - m2 - (tl < ml);
+    const uint32_t neg = (uint32_t)((int32_t)dh >> 31);
+    /* |difference|, exactly */
+    const uint64_t al = (dl ^ (((uint64_t)neg << 32) | neg)) + (neg & 1u);
+    const uint32_t ah = (dh ^ neg) + (uint32_t)((neg & 1u) & (al == 0u));
+    ok &= (ah >= 0x10u) & (sp >= 0);
+    const int z = nf_ilog_clz(ah | 1u);
+    const uint32_t u2 = nf_ilog_up(ah, (uint32_t)(al >> 32), z);
+    const uint32_t u1 = nf_ilog_up((uint32_t)(al >> 32), (uint32_t)al, z), u0 = (uint32_t)al << z;
+    /* rounded to 53 bits: a = am 2^43 in units 2^(-96 - z); a halfway case is not settled */
+    const uint32_t au = (u1 >> 10) & 1u;
+    const uint64_t am = ((((uint64_t)u2 << 32) | u1) >> 11) + au;
+    ok &= !(((u1 & 0x7ffu) == 0x400u) & (u0 == 0u));
+    /* plo = perr + y ll in units 2^(ey - n - 93), then in a's */
+    const uint64_t gm = nf_ilog_mulhi64((((uint64_t)myh << 32) | yl) << 11,
+                                        (uint64_t)(g < 0 ? -g : g) << 19) >> 9;
+    const int64_t pl = (pr >> (top ^ 1)) + (g < 0 ? -(int64_t)gm : (int64_t)gm);
+    const int sh = ey - v.n + 3 + z;
+    const int64_t ps = neg ? -pl : pl;
+    ok &= (sh <= 40) & (sh >= -20);
+    /* r = RN(a + plo): a ends above the lower 43 bits; 32 bits of the fraction below */
+    const uint64_t low = sh >= 0 ? (uint64_t)ps << (sh & 63) : (uint64_t)(ps >> (-sh & 63));
+    const uint32_t f32 = (uint32_t)(low >> 11);
+    const uint64_t rm = am + (uint64_t)(ps >> ((43 - sh) & 63)) + (f32 >> 31);
+    /* the slack of y ll in units of that fraction: 384 2^n y / 2^43 2^(sh - 11) */
+    const int ts = ey + z - 10;
+    const uint32_t w3 = (3u * myh) >> 2;
+    const uint32_t ws = (ts >= 0 ? w3 << (ts & 31) : w3 >> (-ts & 31)) + 4u;
+    ok &= (uint32_t)(rm >> 52) == 1u;
+    *sure = ok & (ts <= 9) & (f32 - 0x80000000u + ws >= 2u * ws);
+    const uint64_t rb = rm + ((uint64_t)((uint32_t)(1021 - z) << 20 | ((neg << 31) ^ v.neg)) << 32);
+    const double r = nf_ifp_make((uint32_t)(rb >> 32), (uint32_t)rb);
+    /* nf_exp_dd from r on */
+    const int ni = v.neg ? -(int)n : (int)n;
+    const int j = ni & 127, m = (ni - j) / 128;
     const double thi = nf_exp_tab(2 * j), tlo = nf_exp_tab(2 * j + 1);
     double t = fma(r, 0x1.1111111111111p-7, 0x1.5555555555555p-5);
     t = fma(r, t, 0x1.5555555555555p-3);
     t = fma(r, t, 0.5);
     const double q = fma(r * r, t, r);
-    const double er = thi + fma(thi, q, tlo);          /* in [0.99, 2): |p| < 90 scales by bits */
+    const double w = fma(thi, q, tlo);
+    const double er = thi + w;                         /* in [0.99, 2): |p| < 16 scales by bits */
+    tail->thi = thi; tail->w = w; tail->er = er; tail->inRange = ok; tail->z = z;
     return nf_ifp_make(nf_ifp_hi(er) + ((uint32_t)m << 20), nf_ifp_lo(er));
+}
+/* Whether the power's last sum is sure although r's rounding is not: r one unit, 2^(-53 - z),
+ * off moves q by less than two units and one of its own rounding, and w, with thi below 2 and
+ * its own rounding, by less than sixteen; the sum's error must stay that far from half a unit. */
+NF_IFP int nf_pow_settled(const nf_pow_tail *t) {
+    const double e = (t->thi - t->er) + t->w;          /* exact: |w| < thi */
+    const uint32_t unit = nf_ifp_hi(t->er) & 0x7ff00000u;
+    const double gap = nf_ifp_make(unit - (53u << 20), 0u) - fabs(e);
+    return t->inRange & ((int32_t)nf_ifp_hi(gap) > (int32_t)((uint32_t)(1023 - 49 - t->z) << 20));
 }
 NF_IFP double nf_pow_fast(double x, double y) {
     int sure;
-    const double r = nf_pow_try(x, y, &sure);
-    return sure ? r : nf_pow_slow(x, y);
+    nf_pow_tail tail;
+    const double r = nf_pow_try(x, y, &sure, &tail);
+    return sure || nf_pow_settled(&tail) ? r : nf_pow_slow(x, y);
 }
 
 #endif /* NF_ILOG_H */

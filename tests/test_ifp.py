@@ -1,6 +1,6 @@
-"""The integer division and square root of the FP64 kernels (neofiz_gb300/csrc/nf_ifp.h) against
-the machine's, and the logarithm and power that use integer arithmetic (nf_ilog.h) against
-nf_math.h's, bit for bit.
+"""The integer division, square root and product of the FP64 kernels (neofiz_gb300/csrc/nf_ifp.h)
+against the machine's, and the logarithm and power that use integer arithmetic (nf_ilog.h)
+against nf_math.h's, bit for bit.
 
 One check compiles from the header for the host, where the FP32 approximation the methods start
 from is moved through its whole documented error range (and past it), and for the device, where
@@ -113,6 +113,15 @@ FN uint64_t check(uint64_t seed, int n) {
         case 2: x = -x; break;
         }
         if (!same(nf_sqrt(x), sqrt(x))) bad += 1ULL << 32;
+        // products and scalings: the machine's bits, or refused; the path's range is not refused
+        uint32_t no = 0;
+        const double p = nf_mul_try(a, b, &no);
+        const bool near1 = fabs(a) > 0x1p-200 && fabs(a) < 0x1p200 && fabs(b) > 0x1p-200 && fabs(b) < 0x1p200;
+        if (no ? near1 : !same(p, a * b)) bad++;
+        no = 0;
+        const int k = (int)(r.next() % 17) - 8;
+        const double q = nf_scale_try(a, k, &no);
+        if (no ? near1 : !same(q, a * dval((uint64_t)(1023 + k) << 52))) bad++;
     }
     return bad;
 }
