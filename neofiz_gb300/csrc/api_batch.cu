@@ -994,7 +994,7 @@ nf_status nf_batch_adjoint_forward(nf_batch *h, int32_t checkpoint_every, int32_
     a.barPlane = ba;
     B.adjBarOff = barOff;
     BCK(&B, cudaEventRecord(B.ev0, B.stream));
-    launch_adjoint_forward(B.d, B.b, a, B.stream);
+    launch_adjoint_forward(B.d, B.b, a, B.sms, B.stream);
     B.launches += 1;
     BCK(&B, cudaEventRecord(B.ev1, B.stream));
     st = bsync(B);
@@ -1157,7 +1157,7 @@ nf_status nf_batch_adjoint_backward_many(nf_batch *h, const int32_t *objectives,
     BCK(&B, cudaMemsetAsync(a.bar, 0, (size_t)B.adjBarBytes * count, B.stream));
     a.width = count;
     BCK(&B, cudaEventRecord(B.ev0, B.stream));
-    launch_adjoint_backward(B.d, B.b, a, B.stream);
+    launch_adjoint_backward(B.d, B.b, a, B.sms, B.stream);
     B.launches += 1;
     BCK(&B, cudaEventRecord(B.ev1, B.stream));
     nf_status st = bsync(B);

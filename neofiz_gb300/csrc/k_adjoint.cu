@@ -83,10 +83,12 @@ __device__ BarBlock bar_at(char *p, int n, int e, int k) {
 
 // Copies the instance's evolving state between the solver arrays and a block (save: to the
 // block). Each node is copied by the thread that owns it in the step's node loops.
-template <int T>
-__device__ void copy_state(const Dev &d, const BatchInst &in, StateBlock s, bool save) {
+template <int T, bool TEAM>
+__device__ void copy_state(const Team<TEAM> &team, const Dev &d, const BatchInst &in, StateBlock s,
+                           bool save) {
     const int n = in.n1 - in.n0, e = in.e1 - in.e0;
-    for (int i = threadIdx.x; i < n; i += T) {
+    const int tid = team.tid(), stride = TEAM ? team.size * T : T;
+    for (int i = tid; i < n; i += stride) {
         const int g = in.n0 + i;
         if (save) {
             s.U[i] = d.U[g]; s.V[i] = d.V[g]; s.F[i] = d.F[g]; s.flags[i] = d.flags[g];
@@ -94,7 +96,7 @@ __device__ void copy_state(const Dev &d, const BatchInst &in, StateBlock s, bool
             d.U[g] = s.U[i]; d.V[g] = s.V[i]; d.F[g] = s.F[i]; d.flags[g] = s.flags[i];
         }
     }
-    for (int j = threadIdx.x; j < e; j += T) {
+    for (int j = tid; j < e; j += stride) {
         const int g = in.e0 + j;
         double2 *a = reinterpret_cast<double2 *>(d.sig + 4 * (size_t)g);
         double2 *b = reinterpret_cast<double2 *>(d.back + 4 * (size_t)g);
@@ -158,11 +160,14 @@ __device__ void elem_in(const Dev &d, const BatchInst &in, const StateBlock &pre
 // BurstCase.loadCapacity (BurstCase.java:533-553) of the instance's current state: the hoop
 // stress times the current element area summed by a fixed tree, over the bore radius and the
 // height (exact extrema). Valid in every thread.
-template <int T>
-__device__ double capacity_of(const Dev &d, const BatchInst &in, double *shRed) {
-    __shared__ double shExt[3];
+template <int T, bool TEAM>
+__device__ double capacity_of(const Team<TEAM> &team, const Dev &d, const BatchInst &in,
+                              double *shRed) {
+    __shared__ double parts[TEAM ? TEAM_MAX : 1][4];     // hoop, bore, low, high of each block
+    __shared__ double result;
+    const int tid = team.tid(), stride = TEAM ? team.size * T : T;
     double hoop = 0.0;
-    for (int e = in.e0 + threadIdx.x; e < in.e1; e += T) {
+    for (int e = in.e0 + tid; e < in.e1; e += stride) {
         const int4 c = d.conn[e];
         const int nn[4] = {c.x, c.y, c.z, c.w};
         double sum = 0.0;
@@ -180,7 +185,7 @@ __device__ double capacity_of(const Dev &d, const BatchInst &in, double *shRed) 
     }
     const double total = block_total<T>(hoop, shRed);
     double bore = DMAX, low = DMAX, high = -DMAX;
-    for (int i = in.n0 + threadIdx.x; i < in.n1; i += T) {
+    for (int i = in.n0 + tid; i < in.n1; i += stride) {
         const double2 x = d.X0[i];
         double r = x.x, z = x.y;
         if (d.finite) {
@@ -197,52 +202,55 @@ __device__ double capacity_of(const Dev &d, const BatchInst &in, double *shRed) 
         low = fmin(low, __shfl_down_sync(0xffffffffu, low, o));
         high = fmax(high, __shfl_down_sync(0xffffffffu, high, o));
     }
-    if (threadIdx.x == 0) {
-        shExt[0] = DMAX; shExt[1] = DMAX; shExt[2] = -DMAX;
+    // exact extrema in any order: each block's thread 0 folds its warps', then the blocks'
+    double ext[3] = {bore, low, -high};
+    for (int q = 0; q < 3; q++) {
+        if ((threadIdx.x & 31) == 0) shRed[threadIdx.x >> 5] = ext[q];
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 0; w < T / 32; w++) ext[q] = fmin(ext[q], shRed[w]);
+        __syncthreads();
     }
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) {
-        // order-free extrema of finite values: a lock-free min over warps through shared
-        // memory would need atomics on doubles; the first thread folds the warps instead
-        shRed[threadIdx.x >> 5] = bore;
-    }
-    __syncthreads();
     if (threadIdx.x == 0)
-        for (int w = 0; w < T / 32; w++) shExt[0] = fmin(shExt[0], shRed[w]);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) shRed[threadIdx.x >> 5] = low;
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int w = 0; w < T / 32; w++) shExt[1] = fmin(shExt[1], shRed[w]);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) shRed[threadIdx.x >> 5] = high;
-    __syncthreads();
+        for (int r = 0; r < team.size; r++) {
+            double *o = team.at(parts, r)[team.rank];
+            o[0] = total; o[1] = ext[0]; o[2] = ext[1]; o[3] = ext[2];
+        }
+    team.sync();
     if (threadIdx.x == 0) {
-        for (int w = 0; w < T / 32; w++) shExt[2] = fmax(shExt[2], shRed[w]);
-        shRed[T / 32] = total / (shExt[0] * (shExt[2] - shExt[1]));
+        double sum = 0.0;
+        for (int r = 0; r < team.size; r++) {
+            sum += parts[r][0];
+            for (int q = 0; q < 3; q++) ext[q] = fmin(ext[q], parts[r][1 + q]);
+        }
+        result = sum / (ext[0] * (-ext[2] - ext[1]));
     }
-    __syncthreads();
-    const double cap = shRed[T / 32];
-    __syncthreads();
-    return cap;
+    team.sync();
+    return result;
 }
 
 // Forward: every instance to its t_end, a checkpoint every `every` steps, the final state.
+template <bool INT, bool TEAM>
 __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev a) {
     __shared__ double shMin[ADJ_T / 32 + 1];
     __shared__ int wallCount[2][2];
-    const int k = blockIdx.x;
+    __shared__ double slots[TEAM ? TEAM_MAX : 1][3];
+    __shared__ BlockStep bs;
+    const Team<TEAM> team;
+    const int k = blockIdx.x / team.size;
     const BatchInst in = b.inst[k];
     BatchScalars *scp = b.sc + k;
     const int n = in.n1 - in.n0, e = in.e1 - in.e0;
     double dt = scp->dt, dtPrev = scp->dtPrevious, time = scp->time;
     double minEdge = scp->minEdgeSquared;
     long long steps = scp->steps;
-    double impulse = 0.0, loss = 0.0, fric = 0.0;
+    double wall[3] = {0.0, 0.0, 0.0};        // impulse, energy loss, friction work
     if (threadIdx.x == 0) {
         wallCount[0][0] = wallCount[0][1] = wallCount[1][0] = wallCount[1][1] = 0;
+        block_step_init(bs, d, in, dt, dtPrev);
     }
-    __syncthreads();
+    team.sync();
+    int(*counts)[2] = TEAM ? team.at(&wallCount[0], 0) : wallCount;   // the first block's
     const MixedGeo none{nullptr, nullptr, nullptr, 0};
     char *ckpt = a.ckpt + a.ckptOff[k];
     const size_t bytes = a.stateBytes[k];
@@ -254,12 +262,12 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev
         if (steps % a.every == 0) {
             const long long c = steps / a.every;
             if (c >= a.ckptCap[k]) {
-                if (threadIdx.x == 0) atomicOr(a.overflow, 1);
+                if (team.first()) atomicOr(a.overflow, 1);
                 break;
             }
             StateBlock s = state_at(ckpt + c * bytes, n, e);
-            copy_state<ADJ_T>(d, in, s, true);
-            if (threadIdx.x == 0) {
+            copy_state<ADJ_T>(team, d, in, s, true);
+            if (team.first()) {
                 s.scal[0] = dt; s.scal[1] = dtPrev; s.scal[2] = time;
                 s.scal[3] = (double)steps; s.scal[4] = minEdge;
             }
@@ -269,37 +277,35 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev
             wallCount[par ^ 1][0] = 0;
             wallCount[par ^ 1][1] = 0;
         }
-        minEdge = batch_step<false, ADJ_T>(d, in, dt, dtPrev, time, steps, none, nullptr, nullptr,
-                                           0, &scp->status, &wallCount[par][0],
-                                           &wallCount[par][1], impulse, loss, fric, shMin);
+        minEdge = batch_step<false, ADJ_T, false, INT, TEAM>(
+            team, d, in, dt, dtPrev, time, steps, none, nullptr, nullptr, 0, &scp->status,
+            &counts[par][0], &counts[par][1], wall[0], wall[1], wall[2], shMin, &bs);
         if (a.sampleEvery > 0 && steps % a.sampleEvery == 0) {
-            __syncthreads();
-            const double cap = capacity_of<ADJ_T>(d, in, shMin);
+            team.sync();
+            const double cap = capacity_of<ADJ_T>(team, d, in, shMin);
             if (cap > peak) {                  // the same decision in every thread
                 peak = cap;
                 peakStep = steps;
                 StateBlock pk = state_at(a.peak + a.peakOff[k], n, e);
-                copy_state<ADJ_T>(d, in, pk, true);
-                if (threadIdx.x == 0) {
+                copy_state<ADJ_T>(team, d, in, pk, true);
+                if (team.first()) {
                     pk.scal[0] = dt; pk.scal[1] = dtPrev; pk.scal[2] = time;
                     pk.scal[3] = (double)steps; pk.scal[4] = minEdge;
                 }
             }
         }
     }
-    const double ti = block_total<ADJ_T>(impulse, shMin);
-    const double tl = block_total<ADJ_T>(loss, shMin);
-    const double tf = block_total<ADJ_T>(fric, shMin);
+    team_totals<TEAM, ADJ_T, 3>(team, wall, shMin, slots);
     StateBlock fin = state_at(a.fin + a.finOff[k], n, e);
-    copy_state<ADJ_T>(d, in, fin, true);
-    if (threadIdx.x == 0) {
+    copy_state<ADJ_T>(team, d, in, fin, true);
+    if (team.first()) {
         scp->dt = dt; scp->dtPrevious = dtPrev; scp->time = time; scp->steps = steps;
         scp->minEdgeSquared = minEdge;
         if (taken > 0) {
             scp->wContact = wallCount[(taken - 1) & 1][0];
             scp->wStuck = wallCount[(taken - 1) & 1][1];
         }
-        scp->wImpulse += ti; scp->wEnergyLoss += tl; scp->wFriction += tf;
+        scp->wImpulse += wall[0]; scp->wEnergyLoss += wall[1]; scp->wFriction += wall[2];
         scp->done = 1;
         a.steps[k] = steps;
         a.peakStep[k] = peakStep;
@@ -307,48 +313,56 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev
         fin.scal[0] = dt; fin.scal[1] = dtPrev; fin.scal[2] = time; fin.scal[3] = (double)steps;
         fin.scal[4] = minEdge;
     }
+    team.sync();                             // the first block's counts stay until all are done
 }
 
 // The reverse of one step whose pre-step state is `pre`.
 // The wall counters and status word of the recomputed nodal update go to `scratch` (shared
 // memory: atomics need a shared or global address).
-__device__ void reverse_step(const Dev &d, const BatchInst &in, const MatDev &mat, StateBlock pre,
-                             BarBlock bar, double *pacc, double *shRed, int *shOwner,
-                             double *shDtb, double *shDtPrevb, double *shTimeb, int *scratch) {
+// owner0 is the first block's shared word; shDtb, shDtPrevb and shTimeb are each block's own and
+// equal in all of them.
+template <bool TEAM>
+__device__ void reverse_step(const Team<TEAM> &team, const Dev &d, const BatchInst &in,
+                             const MatDev &mat, StateBlock pre, BarBlock bar, double *pacc,
+                             double *shRed, double (*slots)[4], int *owner0, double *shDtb,
+                             double *shDtPrevb, double *shTimeb, int *scratch) {
     const int n = in.n1 - in.n0, e = in.e1 - in.e0;
+    const int tid = team.tid(), stride = TEAM ? team.size * ADJ_T : ADJ_T;
     const double dt = pre.scal[0], dtPrev = pre.scal[1], minEdge = pre.scal[4];
     const double dtAvg = 0.5 * (dtPrev + dt);
     const double half = 0.5 * in.damping * dtAvg;
-    const double decay = (1.0 - half) / (1.0 + half), gain = dtAvg / (1.0 + half);
+    const nf_divisor by = nf_divisor_of(1.0 + half);
+    const double decay = nf_div_by(1.0 - half, 1.0 + half, by);
+    const double gain = nf_div_by(dtAvg, 1.0 + half, by);
     // u', v' of this step, from the tape
     {
         double i0 = 0.0, l0 = 0.0, f0 = 0.0;
         const NodalCoef co{decay, gain, dtAvg, dt};
         const WallRef w{in.hasWall, in.wallPlane, in.wallFriction, scratch, scratch + 1};
         const MixedGeo none{nullptr, nullptr, nullptr, 0};
-        for (int i = threadIdx.x; i < n; i += ADJ_T) {
+        for (int i = tid; i < n; i += stride) {
             const int g = in.n0 + i;
             d.U[g] = pre.U[i]; d.V[g] = pre.V[i]; d.F[g] = pre.F[i]; d.flags[g] = pre.flags[i];
             nodal_node(d, g, co, w, none, reinterpret_cast<uint32_t *>(scratch + 2), i0, l0, f0);
         }
     }
-    if (threadIdx.x == 0) *shOwner = 0x7fffffff;
-    __syncthreads();
+    if (team.first()) *owner0 = 0x7fffffff;
+    team.sync();
     const int finite = d.finite;
     double edgeb = 0.0;
     if (finite && minEdge > 0.0 && minEdge < DMAX) {
         edgeb = *shDtb * in.cfl * sqrt(in.massScale) / in.wave * 0.5 / sqrt(minEdge);
-        for (int le = threadIdx.x; le < e; le += ADJ_T) {
+        for (int le = tid; le < e; le += stride) {
             nf_adj_elem_in x;
             elem_in(d, in, pre, le, &x);
-            if (nf_adj_edge_owner(&x, dt, finite, minEdge) >= 0) atomicMin(shOwner, le);
+            if (nf_adj_edge_owner(&x, dt, finite, minEdge) >= 0) atomicMin(owner0, le);
         }
     }
-    __syncthreads();
-    const int owner = *shOwner;
+    team.sync();
+    const int owner = *owner0;
     const nf_adj_mat m = adj_mat_of(mat);
     double dtb = 0.0;
-    for (int le = threadIdx.x; le < e; le += ADJ_T) {
+    for (int le = tid; le < e; le += stride) {
         nf_adj_elem_in x;
         elem_in(d, in, pre, le, &x);
         nf_adj_elem_bar ab;
@@ -387,7 +401,7 @@ __device__ void reverse_step(const Dev &d, const BatchInst &in, const MatDev &ma
     // pressure edges, loaded at this step's end time (:1203-1207, :1511-1556)
     double tpress = 0.0;
     const double tnow = pre.scal[2] + dt;
-    for (int j = threadIdx.x; j < in.k1 - in.k0; j += ADJ_T) {
+    for (int j = tid; j < in.k1 - in.k0; j += stride) {
         const int2 ed = d.pedges[in.k0 + j];
         const int la = ed.x - in.n0, lb = ed.y - in.n0;
         const double cb[4] = {bar.F[la].x, bar.F[lb].x, bar.F[la].y, bar.F[lb].y};
@@ -396,9 +410,9 @@ __device__ void reverse_step(const Dev &d, const BatchInst &in, const MatDev &ma
                              in.ramp, d.axi, finite, d.thickness, cb, bar.edge + 4 * (size_t)j,
                              bar.edge + 4 * (size_t)j + 2, &tpress);
     }
-    __syncthreads();
+    team.sync();
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int i = threadIdx.x; i < n; i += ADJ_T) {
+    for (int i = tid; i < n; i += stride) {
         const int g = in.n0 + i;
         double ub[2] = {bar.U[i].x, bar.U[i].y}, vb[2] = {bar.V[i].x, bar.V[i].y}, fb[2];
         for (int s = d.nodeSlotStart[g]; s < d.nodeSlotStart[g + 1]; s++) {
@@ -421,20 +435,20 @@ __device__ void reverse_step(const Dev &d, const BatchInst &in, const MatDev &ma
         bar.F[i] = make_double2(fb[0], fb[1]);
     }
     pacc[NF_ADJ_P_MU] += acc[3];
-    const double tDt = block_total<ADJ_T>(dtb + acc[2], shRed);
-    const double tDecay = block_total<ADJ_T>(acc[0], shRed);
-    const double tGain = block_total<ADJ_T>(acc[1], shRed);
-    const double tTime = block_total<ADJ_T>(tpress, shRed);
+    double sums[4] = {dtb + acc[2], acc[0], acc[1], tpress};
+    team_totals<TEAM, ADJ_T, 4>(team, sums, shRed, slots);
     if (threadIdx.x == 0) {
+        const double tDt = sums[0], tDecay = sums[1], tGain = sums[2], tTime = sums[3];
         const double dtAvgb = nf_adj_dtavg(tDecay, tGain, dtAvg, in.damping);
         *shTimeb += tTime;                      // time' = time + dt
         *shDtb = *shDtPrevb + tDt + 0.5 * dtAvgb + *shTimeb;
         *shDtPrevb = 0.5 * dtAvgb;
     }
-    __syncthreads();
+    team.sync();
 }
 
 // Backward: the reverse sweep over all steps of every instance, segment by segment.
+template <bool INT, bool TEAM>
 __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDev a) {
     __shared__ double shMin[ADJ_T / 32 + 1];
     __shared__ double shRed[ADJ_T / 32 + 1];
@@ -442,7 +456,11 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDe
     __shared__ int scratch[3];                   // wall counts and status of recomputed steps
     __shared__ double shDtb[NF_ADJ_MAX_WIDTH], shDtPrevb[NF_ADJ_MAX_WIDTH];
     __shared__ double shTimeb[NF_ADJ_MAX_WIDTH];
-    const int k = blockIdx.x;
+    __shared__ double slots[TEAM ? TEAM_MAX : 1][4], gradSlots[TEAM ? TEAM_MAX : 1][NF_ADJ_P_COUNT];
+    __shared__ BlockStep bs;
+    const Team<TEAM> team;
+    const int k = blockIdx.x / team.size;
+    const int tid = team.tid(), stride = TEAM ? team.size * ADJ_T : ADJ_T;
     const int W = a.width;
     const BatchInst in = b.inst[k];
     const MatDev mat = d.mats[k];
@@ -460,32 +478,33 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDe
         for (int w = 0; w < NF_ADJ_MAX_WIDTH; w++) shDtb[w] = shDtPrevb[w] = shTimeb[w] = 0.0;
         scratch[0] = scratch[1] = scratch[2] = 0;
     }
-    __syncthreads();
+    team.sync();
+    int *owner0 = team.at(&shOwner, 0);
     const MixedGeo none{nullptr, nullptr, nullptr, 0};
     uint32_t *scratchStatus = reinterpret_cast<uint32_t *>(scratch + 2);
     const long long segments = (N + a.every - 1) / a.every;
     for (long long sgi = segments - 1; sgi >= 0; sgi--) {
         StateBlock c = state_at(ckpt + sgi * bytes, n, e);
-        copy_state<ADJ_T>(d, in, c, false);
+        copy_state<ADJ_T>(team, d, in, c, false);
         double dt = c.scal[0], dtPrev = c.scal[1], time = c.scal[2];
         long long steps = (long long)c.scal[3];
-        __syncthreads();
+        if (threadIdx.x == 0) block_step_init(bs, d, in, dt, dtPrev);
+        team.sync();
         const long long start = sgi * a.every;
         const long long end = start + a.every < N ? start + a.every : N;
         double i0 = 0.0, l0 = 0.0, f0 = 0.0;
         for (long long j = start; j < end; j++) {
             StateBlock t = state_at(tape + (j - start) * bytes, n, e);
-            copy_state<ADJ_T>(d, in, t, true);
-            if (threadIdx.x == 0) {
+            copy_state<ADJ_T>(team, d, in, t, true);
+            if (team.first()) {
                 t.scal[0] = dt; t.scal[1] = dtPrev; t.scal[2] = time; t.scal[3] = (double)steps;
             }
-            const double me = batch_step<false, ADJ_T>(d, in, dt, dtPrev, time, steps, none,
-                                                       nullptr, nullptr, 0, scratchStatus,
-                                                       &scratch[0], &scratch[1], i0, l0, f0,
-                                                       shMin);
-            if (threadIdx.x == 0) t.scal[4] = me;
+            const double me = batch_step<false, ADJ_T, false, INT, TEAM>(
+                team, d, in, dt, dtPrev, time, steps, none, nullptr, nullptr, 0, scratchStatus,
+                &scratch[0], &scratch[1], i0, l0, f0, shMin, &bs);
+            if (team.first()) t.scal[4] = me;
         }
-        __syncthreads();
+        team.sync();
         for (long long j = end - 1; j >= start; j--) {
             const StateBlock pre = state_at(tape + (j - start) * bytes, n, e);
             for (int w = 0; w < W; w++) {
@@ -496,29 +515,40 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDe
                     const double2 *seedU = reinterpret_cast<const double2 *>(sd);
                     const double *seedSig =
                         reinterpret_cast<const double *>(sd + al16(16 * (size_t)n));
-                    for (int i = threadIdx.x; i < n; i += ADJ_T) {
+                    for (int i = tid; i < n; i += stride) {
                         bar.U[i].x += seedU[i].x;
                         bar.U[i].y += seedU[i].y;
                     }
-                    for (int q = threadIdx.x; q < 4 * e; q += ADJ_T) bar.sig[q] += seedSig[q];
-                    __syncthreads();
+                    for (int q = tid; q < 4 * e; q += stride) bar.sig[q] += seedSig[q];
+                    team.sync();
                 }
                 // the forward values each objective's reverse reads are recomputed from the
                 // same tape entry, so every objective sees the same bits
-                reverse_step(d, in, mat, pre, bar, pacc[w], shRed, &shOwner, &shDtb[w],
+                reverse_step(team, d, in, mat, pre, bar, pacc[w], shRed, slots, owner0, &shDtb[w],
                              &shDtPrevb[w], &shTimeb[w], scratch);
             }
         }
     }
-    for (int w = 0; w < W; w++)
-        for (int p = 0; p < NF_ADJ_P_COUNT; p++) {
-            const double t = block_total<ADJ_T>(pacc[w][p], shRed);
-            if (threadIdx.x == 0)
-                a.grad[((size_t)w * b.count + k) * NF_ADJ_P_COUNT + p] = t;
-        }
+    for (int w = 0; w < W; w++) {
+        team_totals<TEAM, ADJ_T, NF_ADJ_P_COUNT>(team, pacc[w], shRed, gradSlots);
+        if (team.first())
+            for (int p = 0; p < NF_ADJ_P_COUNT; p++)
+                a.grad[((size_t)w * b.count + k) * NF_ADJ_P_COUNT + p] = pacc[w][p];
+        team.sync();
+    }
     // the solver arrays back to the forward's final state
     StateBlock fin = state_at(a.fin + a.finOff[k], n, e);
-    copy_state<ADJ_T>(d, in, fin, false);
+    copy_state<ADJ_T>(team, d, in, fin, false);
+    team.sync();
+}
+
+static const void *forward_kernel(bool ints, bool team) {
+    if (team) return ints ? (const void *)k_adj_forward<true, true> : (const void *)k_adj_forward<false, true>;
+    return ints ? (const void *)k_adj_forward<true, false> : (const void *)k_adj_forward<false, false>;
+}
+static const void *backward_kernel(bool ints, bool team) {
+    if (team) return ints ? (const void *)k_adj_backward<true, true> : (const void *)k_adj_backward<false, true>;
+    return ints ? (const void *)k_adj_backward<true, false> : (const void *)k_adj_backward<false, false>;
 }
 
 // Raises the context's per-thread stack limit to what the adjoint kernels' frames need (the
@@ -526,7 +556,10 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDe
 // lower. The device call graph has no cycles, so the frames are fixed at compile time.
 cudaError_t adjoint_reserve_stack() {
     size_t need = 0;
-    const void *kernels[2] = {(const void *)k_adj_forward, (const void *)k_adj_backward};
+    const void *kernels[] = {
+        forward_kernel(false, false), forward_kernel(true, false), forward_kernel(false, true),
+        forward_kernel(true, true), backward_kernel(false, false), backward_kernel(true, false),
+        backward_kernel(false, true), backward_kernel(true, true)};
     for (const void *f : kernels) {
         cudaFuncAttributes at;
         const cudaError_t e = cudaFuncGetAttributes(&at, f);
@@ -540,12 +573,30 @@ cudaError_t adjoint_reserve_stack() {
     return need > cur ? cudaDeviceSetLimit(cudaLimitStackSize, need) : cudaSuccess;
 }
 
-void launch_adjoint_forward(const Dev &d, const BatchDev &b, const AdjDev &a, cudaStream_t st) {
-    if (b.count > 0) k_adj_forward<<<b.count, ADJ_T, 0, st>>>(d, b, a);
+// One team of blocks per instance (batch_team), its products on the integer units where its
+// quarter SMs have more than one warp of elements (int_products).
+static void launch_adjoint(const void *(*kernel)(bool, bool), const Dev &d, const BatchDev &b,
+                           const AdjDev &a, int sms, cudaStream_t st) {
+    if (b.count <= 0) return;
+    Dev dd = d;
+    BatchDev bb = b;
+    AdjDev aa = a;
+    void *args[] = {&dd, &bb, &aa};
+    const int team = batch_team(kernel(false, true), ADJ_T, b.count, b.maxElems, sms);
+    const int warps = (b.maxElems + 31) / 32 < ADJ_T / 32 * team ? (b.maxElems + 31) / 32 : ADJ_T / 32 * team;
+    const bool ints = int_products((warps + team - 1) / team, 1);
+    if (team > 1) launch_team(kernel(ints, true), b.count, team, ADJ_T, args, st);
+    else cudaLaunchKernel(kernel(ints, false), dim3(b.count), dim3(ADJ_T), args, 0, st);
 }
 
-void launch_adjoint_backward(const Dev &d, const BatchDev &b, const AdjDev &a, cudaStream_t st) {
-    if (b.count > 0) k_adj_backward<<<b.count, ADJ_T, 0, st>>>(d, b, a);
+void launch_adjoint_forward(const Dev &d, const BatchDev &b, const AdjDev &a, int sms,
+                            cudaStream_t st) {
+    launch_adjoint(forward_kernel, d, b, a, sms, st);
+}
+
+void launch_adjoint_backward(const Dev &d, const BatchDev &b, const AdjDev &a, int sms,
+                             cudaStream_t st) {
+    launch_adjoint(backward_kernel, d, b, a, sms, st);
 }
 
 }  // namespace nf

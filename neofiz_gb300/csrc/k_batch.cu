@@ -115,22 +115,27 @@ __global__ void __launch_bounds__(MEASURE_BLOCK) k_batch_measure(Dev d, BatchDev
 
 template <bool MIXED, bool STAGE, bool INT>
 static const void *by_threads(int threads) {
-    if (threads == 32) return (const void *)k_batch_steps<MIXED, STAGE, 32, INT>;
-    return threads == 128 ? (const void *)k_batch_steps<MIXED, STAGE, 128, INT>
-                          : (const void *)k_batch_steps<MIXED, STAGE, 256, INT>;
+    if (threads == 32) return (const void *)k_batch_steps<MIXED, STAGE, 32, INT, false>;
+    return threads == 128 ? (const void *)k_batch_steps<MIXED, STAGE, 128, INT, false>
+                          : (const void *)k_batch_steps<MIXED, STAGE, TEAM_THREADS, INT, false>;
 }
 
 // The kernel of a shape; lone: its blocks give no quarter SM more than one warp of elements.
-static const void *select_kernel(int mode, const BatchShape &s, bool lone) {
-    if (mode == NF_PRECISION_COMPENSATED) return comp_steps_kernel(s);
-    if (mode == NF_PRECISION_MIXED)
+static const void *select_kernel(int mode, const BatchShape &s, bool lone, bool team) {
+    if (mode == NF_PRECISION_COMPENSATED) return comp_steps_kernel(s, team);
+    if (mode == NF_PRECISION_MIXED) {
+        if (team) return (const void *)k_batch_steps<true, false, TEAM_THREADS, false, true>;
         return s.stage ? by_threads<true, true, false>(s.threads) : by_threads<true, false, false>(s.threads);
+    }
+    if (team) return lone ? (const void *)k_batch_steps<false, false, TEAM_THREADS, false, true>
+                          : (const void *)k_batch_steps<false, false, TEAM_THREADS, true, true>;
     return lone ? by_threads<false, false, false>(s.threads) : by_threads<false, false, true>(s.threads);
 }
-// Warps with elements that a shape keeps on one SM.
-static bool lone_warps(const BatchShape &s, int maxElems) {
-    const int lanes = maxElems < s.threads ? maxElems : s.threads;
-    return !int_products((long long)s.blocksPerSm * ((lanes + 31) / 32), 1);
+// Whether a shape keeps no more than one warp with elements on a quarter SM.
+static bool lone_warps(const BatchShape &s, int maxElems, int team) {
+    const int warps = (maxElems + 31) / 32 < s.threads / 32 * team ? (maxElems + 31) / 32
+                                                                   : s.threads / 32 * team;
+    return !int_products((long long)s.blocksPerSm * ((warps + team - 1) / team), 1);
 }
 
 size_t batch_shared_bytes(int mode, const BatchShape &s, int maxNodes) {
@@ -138,9 +143,52 @@ size_t batch_shared_bytes(int mode, const BatchShape &s, int maxNodes) {
                                                 : 0;
 }
 
+// Blocks that step one instance together, for `count` instances of up to maxElems elements on
+// sms SMs: a power of two, with a block per SM for every instance, and no more than shortens the
+// longest queue of element warps on a quarter SM (one with four warps or fewer has none). Kernel
+// `k` with `threads` threads a block must fit as that many clusters at once.
+int batch_team(const void *k, int threads, int count, int maxElems, int sms) {
+    const int warps = (maxElems + 31) / 32;
+    auto depth = [&](int team) { return (warps + 4 * team - 1) / (4 * team); };
+    int best = 1;
+    for (int team = 2; team <= TEAM_MAX && (long long)count * team <= sms; team *= 2) {
+        if (depth(team) >= depth(best)) continue;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = team;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(count * team);
+        cfg.blockDim = dim3(threads);
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess) {
+            (void)cudaGetLastError();
+            break;
+        }
+        if (clusters >= count) best = team;
+    }
+    return best;
+}
+cudaError_t launch_team(const void *k, int teams, int team, int threads, void **args,
+                        cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = team;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(teams * team);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, k, args);
+}
+
 // Resident blocks per SM of a shape (0 when it cannot launch, e.g. too much shared memory).
 int batch_max_blocks_per_sm(int mode, const BatchShape &s, int maxNodes, int maxElems) {
-    const void *k = select_kernel(mode, s, lone_warps(s, maxElems));
+    const void *k = select_kernel(mode, s, lone_warps(s, maxElems, 1), false);
     const size_t smem = batch_shared_bytes(mode, s, maxNodes);
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
@@ -155,17 +203,26 @@ int batch_max_blocks_per_sm(int mode, const BatchShape &s, int maxNodes, int max
     return n;
 }
 
+// A batch with fewer instances than SMs steps each by a team of blocks (batch_team) where the
+// shape allows it: one 64-rod FP64 sweep fills 128 SMs instead of 64.
 cudaError_t launch_batch_steps(const Dev &d, const BatchDev &b, int mode, const BatchShape &s,
                                int sms, cudaStream_t st) {
-    const void *k = select_kernel(mode, s, lone_warps(s, b.maxElems));
-    const size_t smem = batch_shared_bytes(mode, s, b.maxNodes);
-    int blocks = sms * s.blocksPerSm;
-    if (blocks > b.count) blocks = b.count;
-    if (blocks < 1) blocks = 1;
     Dev dd = d;
     BatchDev bb = b;
     int chunk = s.chunk;
     void *args[] = {&dd, &bb, &chunk};
+    if (s.threads == TEAM_THREADS && !s.stage) {
+        const int team = batch_team(select_kernel(mode, s, false, true), TEAM_THREADS, b.count,
+                                    b.maxElems, sms);
+        if (team > 1)
+            return launch_team(select_kernel(mode, s, lone_warps(s, b.maxElems, team), true),
+                               b.count, team, TEAM_THREADS, args, st);
+    }
+    const void *k = select_kernel(mode, s, lone_warps(s, b.maxElems, 1), false);
+    const size_t smem = batch_shared_bytes(mode, s, b.maxNodes);
+    int blocks = sms * s.blocksPerSm;
+    if (blocks > b.count) blocks = b.count;
+    if (blocks < 1) blocks = 1;
     return cudaLaunchKernel(k, dim3(blocks), dim3(s.threads), args, smem, st);
 }
 

@@ -31,15 +31,16 @@ __global__ void k_batch_comp_sync(Dev d) {
     d.F[i] = make_double2((double)f.x, (double)f.y);
 }
 
-const void *comp_steps_kernel(const BatchShape &s) {
+const void *comp_steps_kernel(const BatchShape &s, bool team) {
+    if (team) return (const void *)k_batch_steps_comp<false, TEAM_THREADS, true>;
     if (s.stage) {
-        if (s.threads == 32) return (const void *)k_batch_steps_comp<true, 32>;
-        return s.threads == 128 ? (const void *)k_batch_steps_comp<true, 128>
-                                : (const void *)k_batch_steps_comp<true, 256>;
+        if (s.threads == 32) return (const void *)k_batch_steps_comp<true, 32, false>;
+        return s.threads == 128 ? (const void *)k_batch_steps_comp<true, 128, false>
+                                : (const void *)k_batch_steps_comp<true, TEAM_THREADS, false>;
     }
-    if (s.threads == 32) return (const void *)k_batch_steps_comp<false, 32>;
-    return s.threads == 128 ? (const void *)k_batch_steps_comp<false, 128>
-                            : (const void *)k_batch_steps_comp<false, 256>;
+    if (s.threads == 32) return (const void *)k_batch_steps_comp<false, 32, false>;
+    return s.threads == 128 ? (const void *)k_batch_steps_comp<false, 128, false>
+                            : (const void *)k_batch_steps_comp<false, TEAM_THREADS, false>;
 }
 
 void launch_batch_comp(const Dev &d, bool toFloat, cudaStream_t st) {

@@ -24,6 +24,23 @@
 
 #include "nf_math.h"
 
+/* The device runs quotients, roots, logarithms and powers in integer arithmetic (nf_ifp.h,
+ * nf_ilog.h: the same bits as the operations and as nf_math.h) and the return map's solve by the
+ * forward kernels' own (j2_solve_to: the same iterates); the host compiles the operations. */
+#if defined(__CUDA_ARCH__)
+#define NF_ADJ_DIV(a, b) nf_div((a), (b))
+#define NF_ADJ_SQRT(a) nf_sqrt(a)
+#define NF_ADJ_LOG(a) nf_adj_log_device(a)
+#define NF_ADJ_POW(a, b) nf_adj_pow_device((a), (b))
+static __device__ __noinline__ double nf_adj_log_device(double a) { return nf_log_fast(a); }
+static __device__ __noinline__ double nf_adj_pow_device(double a, double b) { return nf_pow_fast(a, b); }
+#else
+#define NF_ADJ_DIV(a, b) ((a) / (b))
+#define NF_ADJ_SQRT(a) sqrt(a)
+#define NF_ADJ_LOG(a) nf_log(a)
+#define NF_ADJ_POW(a, b) nf_pow((a), (b))
+#endif
+
 enum { NF_ADJ_P_A = 0, NF_ADJ_P_B, NF_ADJ_P_N, NF_ADJ_P_C, NF_ADJ_P_M, NF_ADJ_P_HKIN,
        NF_ADJ_P_MU, NF_ADJ_P_GF, NF_ADJ_P_SY0, NF_ADJ_P_HISO, NF_ADJ_P_COUNT };
 
@@ -50,17 +67,17 @@ typedef struct {
 /* ------------------------------------------------------------------ Johnson-Cook */
 
 NF_HD double nf_adj_strain_term(const nf_adj_mat *f, double eps) {
-    return eps <= 0.0 ? f->a : f->a + f->b * nf_pow(eps, f->n);
+    return eps <= 0.0 ? f->a : f->a + f->b * NF_ADJ_POW(eps, f->n);
 }
 NF_HD double nf_adj_rate_term(const nf_adj_mat *f, double rate) {
     if (rate <= f->refRate) return 1.0;
-    return 1.0 + f->c * nf_log(rate / f->refRate);
+    return 1.0 + f->c * NF_ADJ_LOG(NF_ADJ_DIV(rate, f->refRate));
 }
 NF_HD double nf_adj_thermal_term(const nf_adj_mat *f, double temperature) {
-    const double homologous = (temperature - f->room) / (f->melt - f->room);
+    const double homologous = NF_ADJ_DIV(temperature - f->room, f->melt - f->room);
     if (homologous <= 0.0) return 1.0;
     if (homologous >= 1.0) return 0.0;
-    return 1.0 - nf_pow(homologous, f->m);
+    return 1.0 - NF_ADJ_POW(homologous, f->m);
 }
 
 /* J2.solve, J2.java:332-375, in the forward kernels' order, to the reverse's tolerance. */
@@ -68,6 +85,12 @@ NF_HD double nf_adj_solve(double norm, double stiffness, double plasticStrain,
                           double temperature, double dt, const nf_adj_mat *jc) {
     const double thermal = nf_adj_thermal_term(jc, temperature);
     const double tolerance = NF_ADJ_TOLERANCE * jc->a;
+#if defined(__CUDA_ARCH__)
+    nf::MatDev m;
+    m.a = jc->a; m.b = jc->b; m.n = jc->n; m.c = jc->c; m.refRate = jc->refRate;
+    return nf::j2_solve_to(norm, stiffness, plasticStrain, thermal, dt, m, tolerance,
+                           NF_ADJ_ITERATIONS).dGamma;
+#else
     double lo = 0.0, hi = norm / stiffness, dGamma = hi;
     for (int iteration = 0; iteration < NF_ADJ_ITERATIONS; iteration++) {
         const double dEps = NF_ADJ_SQRT_2_3 * dGamma;
@@ -86,6 +109,7 @@ NF_HD double nf_adj_solve(double norm, double stiffness, double plasticStrain,
         dGamma = next;
     }
     return dGamma;
+#endif
 }
 
 /* ------------------------------------------------------------------ J2 return map */
@@ -120,13 +144,13 @@ NF_HD void nf_adj_j2_forward(const double *s, const double *bk, double epsP, dou
     tp->t[1] = s[1] + lt + 2.0 * mu * dZZ;
     tp->t[2] = s[2] + lt + 2.0 * mu * dTT;
     tp->t[3] = s[3] + mu * dGamRZ;
-    const double p = (tp->t[0] + tp->t[1] + tp->t[2]) / 3.0;
+    const double p = NF_ADJ_DIV(tp->t[0] + tp->t[1] + tp->t[2], 3.0);
     tp->x[0] = tp->t[0] - p - bk[0];
     tp->x[1] = tp->t[1] - p - bk[1];
     tp->x[2] = tp->t[2] - p - bk[2];
     tp->x[3] = tp->t[3] - bk[3];
     const double *x = tp->x;
-    tp->norm = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + 2.0 * x[3] * x[3]);
+    tp->norm = NF_ADJ_SQRT(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + 2.0 * x[3] * x[3]);
     const int jc = f->jc != 0;
     tp->temperature = !jc ? 0.0 : f->room + f->thermalCoefficient * work;
     tp->softening = dm != 0 && dm->strength > 0.0;
@@ -163,16 +187,16 @@ NF_HD void nf_adj_j2_forward(const double *s, const double *bk, double epsP, dou
     tp->stiffness = 2.0 * mu + NF_ADJ_TWO_THIRDS * f->hKin;
     double dGamma;
     if (!jc || tp->softening) {
-        dGamma = (tp->norm - tp->radius) / (tp->stiffness + NF_ADJ_TWO_THIRDS * tp->hardening);
+        dGamma = NF_ADJ_DIV(tp->norm - tp->radius, tp->stiffness + NF_ADJ_TWO_THIRDS * tp->hardening);
         if (tp->softening && fs + tp->hardening * NF_ADJ_SQRT_2_3 * dGamma < 0.0) {
-            dGamma = tp->norm / tp->stiffness;
+            dGamma = NF_ADJ_DIV(tp->norm, tp->stiffness);
             tp->fallback = 1;
         }
     } else {
         dGamma = nf_adj_solve(tp->norm, tp->stiffness, epsP, tp->temperature, strainDt, f);
     }
     tp->dGamma = dGamma;
-    const double inv = 1.0 / tp->norm;
+    const double inv = NF_ADJ_DIV(1.0, tp->norm);
     for (int k = 0; k < 4; k++) tp->n[k] = x[k] * inv;
     const double *n = tp->n;
     tp->pull = 2.0 * mu * dGamma;
@@ -223,7 +247,7 @@ NF_HD void nf_adj_j2_reverse(const nf_adj_j2_tape *tp, const double *bk, double 
         /* bb, epsPb, workb and the damage state pass through */
     } else {
         const double *n = tp->n, *x = tp->x;
-        const double norm = tp->norm, dGamma = tp->dGamma, inv = 1.0 / norm;
+        const double norm = tp->norm, dGamma = tp->dGamma, inv = NF_ADJ_DIV(1.0, norm);
         double nb[4] = {0.0, 0.0, 0.0, 0.0};
         double epsP1b = *epsPb;
         double tempb = 0.0;
@@ -314,14 +338,14 @@ NF_HD void nf_adj_j2_reverse(const nf_adj_j2_tape *tp, const double *bk, double 
         double stiffb = 0.0, epsPbIn = epsP1b;             /* epsP' = epsP + ... */
         if (!jc || tp->softening) {
             if (tp->fallback) {
-                normb += dGammab / tp->stiffness;
-                stiffb -= dGammab * dGamma / tp->stiffness;
+                normb += NF_ADJ_DIV(dGammab, tp->stiffness);
+                stiffb -= NF_ADJ_DIV(dGammab * dGamma, tp->stiffness);
             } else {
                 const double den = tp->stiffness + NF_ADJ_TWO_THIRDS * tp->hardening;
-                normb += dGammab / den;
-                const double radiusb = -dGammab / den;
-                stiffb -= dGammab * dGamma / den;
-                const double hardb = -dGammab * dGamma / den * NF_ADJ_TWO_THIRDS;
+                normb += NF_ADJ_DIV(dGammab, den);
+                const double radiusb = NF_ADJ_DIV(-dGammab, den);
+                stiffb -= NF_ADJ_DIV(dGammab * dGamma, den);
+                const double hardb = NF_ADJ_DIV(-dGammab * dGamma, den) * NF_ADJ_TWO_THIRDS;
                 const double fsb = NF_ADJ_SQRT_2_3 * radiusb;
                 if (tp->softening) {
                     if (!tp->clamped) {
@@ -339,36 +363,39 @@ NF_HD void nf_adj_j2_reverse(const nf_adj_j2_tape *tp, const double *bk, double 
         } else {
             const double dEps = NF_ADJ_SQRT_2_3 * dGamma;
             const double eps = epsP + dEps;
-            const double rate = strainDt > 0.0 ? dEps / strainDt : 0.0;
-            const double S = nf_adj_strain_term(f, eps);
-            const double R = nf_adj_rate_term(f, rate);
-            const double Th = nf_adj_thermal_term(f, tp->temperature);
-            const double en = eps > 0.0 ? nf_pow(eps, f->n) : 0.0;
-            const double Sp = eps > 0.0 ? f->b * f->n * en / eps : 0.0;
+            const double rate = strainDt > 0.0 ? NF_ADJ_DIV(dEps, strainDt) : 0.0;
+            /* the strain, rate and thermal terms and the powers and logarithms in them, once */
+            const double en = eps > 0.0 ? NF_ADJ_POW(eps, f->n) : 0.0;
+            const double S = eps <= 0.0 ? f->a : f->a + f->b * en;
             const int rated = !(rate <= f->refRate);
-            const double Rp = rated ? f->c / rate : 0.0;
-            const double h = (tp->temperature - f->room) / (f->melt - f->room);
+            const double lr = rated ? NF_ADJ_LOG(NF_ADJ_DIV(rate, f->refRate)) : 0.0;
+            const double R = rated ? 1.0 + f->c * lr : 1.0;
+            const double span = f->melt - f->room;
+            const double h = NF_ADJ_DIV(tp->temperature - f->room, span);
             const int heated = h > 0.0 && h < 1.0;
-            const double hm = heated ? nf_pow(h, f->m) : 0.0;
+            const double hm = heated ? NF_ADJ_POW(h, f->m) : 0.0;
+            const double Th = h <= 0.0 ? 1.0 : h >= 1.0 ? 0.0 : 1.0 - (heated ? hm : NF_ADJ_POW(h, f->m));
+            const double Sp = eps > 0.0 ? NF_ADJ_DIV(f->b * f->n * en, eps) : 0.0;
+            const double Rp = rated ? NF_ADJ_DIV(f->c, rate) : 0.0;
             const double gdg = -tp->stiffness
                                - NF_ADJ_SQRT_2_3 * (Sp * NF_ADJ_SQRT_2_3 * R * Th
-                                                    + S * Rp * (strainDt > 0.0 ? NF_ADJ_SQRT_2_3 / strainDt : 0.0) * Th);
-            const double w = -dGammab / gdg;
+                                                    + S * Rp * (strainDt > 0.0 ? NF_ADJ_DIV(NF_ADJ_SQRT_2_3, strainDt) : 0.0) * Th);
+            const double w = NF_ADJ_DIV(-dGammab, gdg);
             normb += w;
             stiffb += w * (-dGamma);
             epsPbIn += w * (-NF_ADJ_SQRT_2_3 * Sp * R * Th);
             if (heated) {
-                tempb += w * (-NF_ADJ_SQRT_2_3 * S * R * (-f->m * hm / h / (f->melt - f->room)));
-                pb[NF_ADJ_P_M] += w * (-NF_ADJ_SQRT_2_3 * S * R * (-hm * nf_log(h)));
+                tempb += w * (-NF_ADJ_SQRT_2_3 * S * R * NF_ADJ_DIV(NF_ADJ_DIV(-f->m * hm, h), span));
+                pb[NF_ADJ_P_M] += w * (-NF_ADJ_SQRT_2_3 * S * R * (-hm * NF_ADJ_LOG(h)));
             }
             if (rated && strainDt > 0.0) {
-                if (dtb) *dtb += w * (NF_ADJ_SQRT_2_3 * S * Th * f->c / strainDt);
-                pb[NF_ADJ_P_C] += w * (-NF_ADJ_SQRT_2_3 * S * Th * nf_log(rate / f->refRate));
+                if (dtb) *dtb += w * NF_ADJ_DIV(NF_ADJ_SQRT_2_3 * S * Th * f->c, strainDt);
+                pb[NF_ADJ_P_C] += w * (-NF_ADJ_SQRT_2_3 * S * Th * lr);
             }
             pb[NF_ADJ_P_A] += w * (-NF_ADJ_SQRT_2_3 * R * Th);
             if (eps > 0.0) {
                 pb[NF_ADJ_P_B] += w * (-NF_ADJ_SQRT_2_3 * R * Th * en);
-                pb[NF_ADJ_P_N] += w * (-NF_ADJ_SQRT_2_3 * R * Th * f->b * en * nf_log(eps));
+                pb[NF_ADJ_P_N] += w * (-NF_ADJ_SQRT_2_3 * R * Th * f->b * en * NF_ADJ_LOG(eps));
             }
         }
         pb[NF_ADJ_P_HKIN] += NF_ADJ_TWO_THIRDS * stiffb;
@@ -386,7 +413,8 @@ NF_HD void nf_adj_j2_reverse(const nf_adj_j2_tape *tp, const double *bk, double 
         }
         tb[3] += xb[3];
         bkb[3] -= xb[3];
-        for (int k = 0; k < 3; k++) tb[k] += pbar / 3.0;
+        const double third = NF_ADJ_DIV(pbar, 3.0);
+        for (int k = 0; k < 3; k++) tb[k] += third;
         for (int k = 0; k < 4; k++) bb[k] = bkb[k];
     }
     /* trial = s + lt I + 2 mu d (normal), s_rz + mu dGamRZ */
@@ -476,7 +504,7 @@ NF_HD void nf_adj_element_reduced(const nf_adj_elem_in *in, const nf_adj_mat *f,
     const double J10 = 0.25 * (-r[0] - r[1] + r[2] + r[3]);
     const double J11 = 0.25 * (-z[0] - z[1] + z[2] + z[3]);
     const double det = J00 * J11 - J01 * J10;
-    const double inv = 1.0 / det;
+    const double inv = NF_ADJ_DIV(1.0, det);
     double dr[4], dz[4];
     dr[0] = 0.25 * (J01 - J11) * inv;
     dr[1] = 0.25 * (J01 + J11) * inv;
@@ -494,7 +522,7 @@ NF_HD void nf_adj_element_reduced(const nf_adj_elem_in *in, const nf_adj_mat *f,
     double rg = 0.0, dEpsT = 0.0;
     if (axi) {
         rg = 0.25 * (r[0] + r[1] + r[2] + r[3]);
-        dEpsT = 0.25 * (a[0] + a[1] + a[2] + a[3]) / rg;
+        dEpsT = NF_ADJ_DIV(0.25 * (a[0] + a[1] + a[2] + a[3]), rg);
     }
     /* co-rotation (the forward skips it at zero spin; the derivative is taken there too) */
     double s1[4], b1[4];
@@ -504,7 +532,7 @@ NF_HD void nf_adj_element_reduced(const nf_adj_elem_in *in, const nf_adj_mat *f,
     }
     const double spinDt = finite ? 0.5 * (dZdR - dRdZ) : 0.0;
     const double hh = 0.5 * spinDt, q1 = 1.0 + hh * hh;
-    const double cs = (1.0 - hh * hh) / q1, sn = 2.0 * hh / q1;
+    const double cs = NF_ADJ_DIV(1.0 - hh * hh, q1), sn = NF_ADJ_DIV(2.0 * hh, q1);
     if (finite && spinDt != 0.0) {
         nf_adj_rotate_forward(s1, cs, sn);
         nf_adj_rotate_forward(b1, cs, sn);
@@ -594,9 +622,9 @@ NF_HD void nf_adj_element_reduced(const nf_adj_elem_in *in, const nf_adj_mat *f,
         sRZb += tzb * dr[j];
     }
     if (axi) {
-        sTb += hqb * dV * 0.25 / rg;
-        rgb -= hqb * sT * dV * 0.25 / (rg * rg);
-        dVb += hqb * sT / rg * 0.25;
+        sTb += NF_ADJ_DIV(hqb * dV * 0.25, rg);
+        rgb -= NF_ADJ_DIV(hqb * sT * dV * 0.25, rg * rg);
+        dVb += NF_ADJ_DIV(hqb * sT, rg) * 0.25;
         rgb += dVb * 4.0 * 2.0 * NF_PI * det;
         detb += dVb * 4.0 * 2.0 * NF_PI * rg;
     } else {
@@ -620,8 +648,8 @@ NF_HD void nf_adj_element_reduced(const nf_adj_elem_in *in, const nf_adj_mat *f,
         nf_adj_rotate(in->back, bb4, cs, sn, &ccb, &ssb, &csb);
         const double cb_ = 2.0 * cs * ccb + sn * csb;
         const double snb = 2.0 * sn * ssb + cs * csb;
-        const double dcdh = -4.0 * hh / (q1 * q1);
-        const double dsdh = 2.0 * (1.0 - hh * hh) / (q1 * q1);
+        const double dcdh = NF_ADJ_DIV(-4.0 * hh, q1 * q1);
+        const double dsdh = NF_ADJ_DIV(2.0 * (1.0 - hh * hh), q1 * q1);
         spinb = 0.5 * (cb_ * dcdh + snb * dsdh);
     }
     for (int k = 0; k < 4; k++) {
@@ -632,8 +660,9 @@ NF_HD void nf_adj_element_reduced(const nf_adj_elem_in *in, const nf_adj_mat *f,
     const double dRdZb = dGamRZb - 0.5 * spinb;
     /* rg, dEpsT */
     if (axi) {
-        for (int k = 0; k < 4; k++) ab_[k] += 0.25 * dEpsTb / rg;
-        rgb -= dEpsTb * dEpsT / rg;
+        const double dab = NF_ADJ_DIV(0.25 * dEpsTb, rg);
+        for (int k = 0; k < 4; k++) ab_[k] += dab;
+        rgb -= NF_ADJ_DIV(dEpsTb * dEpsT, rg);
         for (int k = 0; k < 4; k++) rb[k] += 0.25 * rgb;
     }
     /* strain increments */
@@ -785,21 +814,21 @@ NF_HD void nf_adj_node(double x0z, double ur, double uz, double vr, double vz, d
         vrb = 0.0;
     } else if (resting && friction > 0.0) {
         const double normal = -fz;
-        const double trial = -m * decay * vr / gain - fr;
+        const double trial = NF_ADJ_DIV(-m * decay * vr, gain) - fr;
         const double limit = isinf(friction) ? INFINITY : friction * normal;
         if (fabs(trial) <= limit) {
             vrb = 0.0;                           /* stuck: v = 0, u unchanged */
         } else {
             const double sgn = trial < 0.0 ? -1.0 : 1.0;
             const double tangential = copysign(limit, trial);
-            const double slid = decay * vr + gain * (fr + tangential) / m;
+            const double slid = decay * vr + NF_ADJ_DIV(gain * (fr + tangential), m);
             const double slidb = vrb + dt * urb;
             acc[2] += slid * urb;
             acc[0] += vr * slidb;
-            acc[1] += (fr + tangential) / m * slidb;
+            acc[1] += NF_ADJ_DIV(fr + tangential, m) * slidb;
             vrb = decay * slidb;
-            frb += gain / m * slidb;
-            const double tb = gain / m * slidb;
+            const double tb = NF_ADJ_DIV(gain, m) * slidb;
+            frb += tb;
             acc[3] += sgn * normal * tb;
             fzb += -sgn * friction * tb;
         }

@@ -7,8 +7,6 @@
 
 namespace nf {
 
-// Up to `chunk` steps of instance k by the whole block: ExplicitSolver.step, :940-991, with the
-// loop condition of TaylorImpactCase.java:250-253 (step while time < t_end).
 // An instance's displacement and centroid hoop stress in the batch's precision.
 template <bool MIXED, bool COMP>
 __device__ __forceinline__ double2 inst_u(const Dev &d, int i) {
@@ -24,19 +22,21 @@ __device__ __forceinline__ double inst_hoop(const Dev &d, int e) {
     return MIXED ? (double)d.sigF[4 * (size_t)e + 2] : d.sig[4 * (size_t)e + 2];
 }
 
-// One sample of BurstCase.run (BurstCase.java:449-490) for instance k by the whole block:
-// loadCapacity (:533-553, the hoop stress times the element area summed in element order by
-// thread 0), hoopStrain (:560-569), the applied pressure (borePressure, pressureAt
+// One sample of BurstCase.run (BurstCase.java:449-490) for instance k by its team of blocks:
+// loadCapacity (:533-553, the hoop stress times the element area summed in element order by the
+// first thread), hoopStrain (:560-569), the applied pressure (borePressure, pressureAt
 // :1203-1207), the running peak and the turnover test. Returns whether the peak was
 // traversed (the same answer in every thread).
-template <bool MIXED, bool COMP, int T>
-__device__ bool burst_sample(const Dev &d, const BatchDev &b, const BatchInst &in, int k,
+template <bool MIXED, bool COMP, int T, bool TEAM>
+__device__ bool burst_sample(const Team<TEAM> &team, const Dev &d, const BatchDev &b,
+                             const BatchInst &in, int k,
                              double time, double *sh) {
-    __shared__ double ext[5][T / 32];
+    __shared__ double ext[TEAM ? TEAM_MAX : 1][5][T / 32];
     __shared__ int verdict;
     const BurstDev &bd = b.burst;
     const bool finite = d.finite != 0;
-    for (int e = in.e0 + threadIdx.x; e < in.e1; e += T) {
+    const int tid = team.tid(), stride = TEAM ? team.size * T : T;
+    for (int e = in.e0 + tid; e < in.e1; e += stride) {
         const int4 c = d.conn[e];
         const int nn[4] = {c.x, c.y, c.z, c.w};
         double sum = 0.0;
@@ -54,7 +54,7 @@ __device__ bool burst_sample(const Dev &d, const BatchDev &b, const BatchInst &i
     }
     // extrema, exact in any order: loadCapacity's bore, low, high; hoopStrain's bore, rim
     double bore = DMAX, low = DMAX, high = -DMAX, boreH = DMAX, rimH = -DMAX;
-    for (int i = in.n0 + threadIdx.x; i < in.n1; i += T) {
+    for (int i = in.n0 + tid; i < in.n1; i += stride) {
         const double2 x = d.X0[i], u = inst_u<MIXED, COMP>(d, i);
         const double r = finite ? x.x + u.x : x.x, z = finite ? x.y + u.y : x.y;
         bore = fmin(bore, r);
@@ -72,16 +72,19 @@ __device__ bool burst_sample(const Dev &d, const BatchDev &b, const BatchInst &i
     }
     if ((threadIdx.x & 31) == 0) {
         const int w = threadIdx.x >> 5;
-        ext[0][w] = bore; ext[1][w] = low; ext[2][w] = high; ext[3][w] = boreH; ext[4][w] = rimH;
+        double(*o)[T / 32] = team.at(&ext[0], 0)[team.rank];   // in the first block
+        o[0][w] = bore; o[1][w] = low; o[2][w] = high; o[3][w] = boreH; o[4][w] = rimH;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < T / 32; w++) {
-            bore = fmin(bore, ext[0][w]);
-            low = fmin(low, ext[1][w]);
-            high = fmax(high, ext[2][w]);
-            boreH = fmin(boreH, ext[3][w]);
-            rimH = fmax(rimH, ext[4][w]);
+    team.sync();
+    if (team.first()) {
+        for (int w = 0; w < team.size * (T / 32); w++) {
+            const double(*o)[T / 32] = ext[w / (T / 32)];
+            const int q = w % (T / 32);
+            bore = fmin(bore, o[0][q]);
+            low = fmin(low, o[1][q]);
+            high = fmax(high, o[2][q]);
+            boreH = fmin(boreH, o[3][q]);
+            rimH = fmax(rimH, o[4][q]);
         }
         double hoopArea = 0.0;
         for (int e = in.e0; e < in.e1; e++) hoopArea += bd.scratch[e];
@@ -110,30 +113,34 @@ __device__ bool burst_sample(const Dev &d, const BatchDev &b, const BatchInst &i
         }
         verdict = st.traversed;
     }
-    __syncthreads();
-    const bool out = verdict != 0;
-    __syncthreads();
+    team.sync();
+    const bool out = *team.at(&verdict, 0) != 0;
+    team.sync();
     return out;
 }
 
-template <bool MIXED, bool STAGE, int T, bool COMP, bool INT>
-__device__ void run_instance(const Dev &d, const BatchDev &b, int k, int chunk, float4 *sPMid,
-                             float2 *sVdt, double *shMin, int (*wallCount)[2], BlockStep *bs) {
+// Up to `chunk` steps of instance k by its team of blocks: ExplicitSolver.step, :940-991, with
+// the loop condition of TaylorImpactCase.java:250-253 (step while time < t_end). Every block
+// takes the same decisions from the same values; the first block's first thread writes them.
+template <bool MIXED, bool STAGE, int T, bool COMP, bool INT, bool TEAM>
+__device__ void run_instance(const Team<TEAM> &team, const Dev &d, const BatchDev &b, int k,
+                             int chunk, float4 *sPMid, float2 *sVdt, double *shMin,
+                             int (*wallCount)[2], double (*slots)[3], BlockStep *bs) {
     const BatchInst in = b.inst[k];
     BatchScalars *scp = b.sc + k;
     if (scp->done) return;
-    const int tid = threadIdx.x;
     double dt = scp->dt, dtPrev = scp->dtPrevious, time = scp->time;
     double minEdge = scp->minEdgeSquared;
     long long steps = scp->steps;
     const long long limit = scp->stepLimit;
-    double impulse = 0.0, loss = 0.0, fric = 0.0;
-    if (tid == 0) {
+    double wall[3] = {0.0, 0.0, 0.0};        // impulse, energy loss, friction work
+    int(*counts)[2] = TEAM ? team.at(&wallCount[0], 0) : wallCount;   // the first block's
+    if (threadIdx.x == 0) {
         wallCount[0][0] = wallCount[0][1] = 0;
         wallCount[1][0] = wallCount[1][1] = 0;
         block_step_init(*bs, d, in, dt, dtPrev);
     }
-    __syncthreads();
+    team.sync();
     float4 *pMid = STAGE ? sPMid : d.pMid;
     float2 *vdt = STAGE ? sVdt : d.vdt;
     const int base = STAGE ? in.n0 : 0;
@@ -150,21 +157,18 @@ __device__ void run_instance(const Dev &d, const BatchDev &b, int k, int chunk, 
         // RigidWall.beginStep: this step's counts go to buffer `par`; the other is cleared for
         // the next step (its last users passed this step's first barrier already)
         const int par = taken & 1;
-        if (tid == 0) {
+        if (threadIdx.x == 0) {
             wallCount[par ^ 1][0] = 0;
             wallCount[par ^ 1][1] = 0;
         }
-        minEdge = batch_step<MIXED, T, COMP, INT>(d, in, dt, dtPrev, time, steps, geo, pMid, vdt,
-                                             base, &scp->status, &wallCount[par][0],
-                                             &wallCount[par][1], impulse, loss, fric, shMin,
-                                             bs);
+        minEdge = batch_step<MIXED, T, COMP, INT, TEAM>(
+            team, d, in, dt, dtPrev, time, steps, geo, pMid, vdt, base, &scp->status,
+            &counts[par][0], &counts[par][1], wall[0], wall[1], wall[2], shMin, bs);
         if (every > 0 && steps % every == 0)
-            traversed = burst_sample<MIXED, COMP, T>(d, b, in, k, time, shMin);
+            traversed = burst_sample<MIXED, COMP, T, TEAM>(team, d, b, in, k, time, shMin);
     }
-    const double ti = block_total<T>(impulse, shMin);
-    const double tl = block_total<T>(loss, shMin);
-    const double tf = block_total<T>(fric, shMin);
-    if (tid == 0) {
+    team_totals<TEAM, T, 3>(team, wall, shMin, slots);
+    if (team.first()) {
         scp->dt = dt;
         scp->dtPrevious = dtPrev;
         scp->time = time;
@@ -174,9 +178,9 @@ __device__ void run_instance(const Dev &d, const BatchDev &b, int k, int chunk, 
             scp->wContact = wallCount[(taken - 1) & 1][0];
             scp->wStuck = wallCount[(taken - 1) & 1][1];
         }
-        scp->wImpulse += ti;
-        scp->wEnergyLoss += tl;
-        scp->wFriction += tf;
+        scp->wImpulse += wall[0];
+        scp->wEnergyLoss += wall[1];
+        scp->wFriction += wall[2];
         const bool ended = every > 0 ? (steps % every == 0 && !(time < in.tEnd))
                                      : !(time < in.tEnd);
         if (ended || traversed || steps >= limit) {
@@ -184,43 +188,45 @@ __device__ void run_instance(const Dev &d, const BatchDev &b, int k, int chunk, 
             atomicSub(b.remaining, 1);
         }
     }
-    __syncthreads();
+    team.sync();
 }
 
-// The queue loop of the persistent kernel: each block takes the next instance (most
-// expensive first) for a chunk of steps until none is left.
-template <bool MIXED, bool STAGE, int T, bool COMP, bool INT>
+// The queue loop of the persistent kernel: each team takes the next instance (most expensive
+// first) for a chunk of steps until none is left.
+template <bool MIXED, bool STAGE, int T, bool COMP, bool INT, bool TEAM>
 __device__ __forceinline__ void batch_queue(const Dev &d, const BatchDev &b, int chunk) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ double shMin[T / 32 + 1];
     __shared__ int wallCount[2][2];
+    __shared__ double slots[TEAM ? TEAM_MAX : 1][3];
     __shared__ int next;
     __shared__ BlockStep bs;
+    const Team<TEAM> team;
     float4 *sPMid = reinterpret_cast<float4 *>(dyn);
     float2 *sVdt = reinterpret_cast<float2 *>(dyn + sizeof(float4) * (size_t)b.maxNodes);
     for (;;) {
-        if (threadIdx.x == 0) next = atomicAdd(b.queue, 1);
-        __syncthreads();
-        const int q = next;
-        __syncthreads();
+        if (team.first()) next = atomicAdd(b.queue, 1);
+        team.sync();
+        const int q = *team.at(&next, 0);
+        team.sync();
         if (q >= b.count) return;
-        run_instance<MIXED, STAGE, T, COMP, INT>(d, b, b.order[q], chunk, sPMid, sVdt, shMin,
-                                                 wallCount, &bs);
+        run_instance<MIXED, STAGE, T, COMP, INT, TEAM>(team, d, b, b.order[q], chunk, sPMid, sVdt,
+                                                       shMin, wallCount, slots, &bs);
     }
 }
 
 // The FP64 and mixed forms (the compiler's register choice).
 // INT: the FP64 element's products on the integer units (int_products).
-template <bool MIXED, bool STAGE, int T, bool INT>
+template <bool MIXED, bool STAGE, int T, bool INT, bool TEAM>
 __global__ void __launch_bounds__(T) k_batch_steps(Dev d, BatchDev b, int chunk) {
-    batch_queue<MIXED, STAGE, T, false, INT>(d, b, chunk);
+    batch_queue<MIXED, STAGE, T, false, INT, TEAM>(d, b, chunk);
 }
 
 // The compensated form keeps few values live across its FP32 phases: capped at 64 registers
 // (1024 resident threads per SM) it hides more memory latency than with the compiler's choice.
-template <bool STAGE, int T>
+template <bool STAGE, int T, bool TEAM>
 __global__ void __launch_bounds__(T, 1024 / T) k_batch_steps_comp(Dev d, BatchDev b, int chunk) {
-    batch_queue<true, STAGE, T, true, false>(d, b, chunk);
+    batch_queue<true, STAGE, T, true, false, TEAM>(d, b, chunk);
 }
 
 }  // namespace nf

@@ -4,7 +4,44 @@
 
 #include "nf_bodies.cuh"
 
+#include <cooperative_groups.h>
+
 namespace nf {
+
+// The blocks that step one instance together: one block, or (TEAM) a thread-block cluster, for
+// batches with fewer instances than SMs. Warps are dealt round-robin over the blocks, so an
+// instance with few warps of elements spreads over every block's quarter SMs; a cluster barrier
+// orders global memory and the blocks' shared memory as a block barrier does within a block.
+template <bool TEAM>
+struct Team {
+    int rank, size;
+    __device__ __forceinline__ Team() {
+        if (TEAM) {
+            const auto c = cooperative_groups::this_cluster();
+            rank = (int)c.block_rank();
+            size = (int)c.num_blocks();
+        } else {
+            rank = 0;
+            size = 1;
+        }
+    }
+    // this thread's place among the team's threads, of which each block has T
+    __device__ __forceinline__ int tid() const {
+        return TEAM ? (((int)threadIdx.x >> 5) * size + rank) * 32 + ((int)threadIdx.x & 31)
+                    : (int)threadIdx.x;
+    }
+    __device__ __forceinline__ bool first() const { return threadIdx.x == 0 && rank == 0; }
+    __device__ __forceinline__ void sync() const {
+        if (TEAM) cooperative_groups::this_cluster().sync();
+        else __syncthreads();
+    }
+    // block r's copy of a shared variable
+    template <typename V>
+    __device__ __forceinline__ V *at(V *p, int r) const {
+        return TEAM ? cooperative_groups::this_cluster().map_shared_rank(p, r) : p;
+    }
+};
+constexpr int TEAM_MAX = 8;                  // blocks of a team (the portable cluster size)
 
 __device__ __forceinline__ unsigned long long bbits(double x) {
     return (unsigned long long)__double_as_longlong(x);
@@ -52,6 +89,28 @@ __device__ double block_total(double v, double *sh) {
     return t;
 }
 
+// COUNT block sums added over the team in rank order, in v[] of every block's thread 0.
+// `slots` is block-shared; a team barrier separates one use of it from the next.
+template <bool TEAM, int T, int COUNT>
+__device__ __forceinline__ void team_totals(const Team<TEAM> &team, double (&v)[COUNT], double *sh,
+                                            double (*slots)[COUNT]) {
+    double t[COUNT];
+    for (int i = 0; i < COUNT; i++) t[i] = block_total<T>(v[i], sh);
+    if (!TEAM) {
+        for (int i = 0; i < COUNT; i++) v[i] = t[i];
+        return;
+    }
+    if (threadIdx.x == 0)
+        for (int r = 0; r < team.size; r++)
+            for (int i = 0; i < COUNT; i++) team.at(slots, r)[team.rank][i] = t[i];
+    team.sync();
+    for (int i = 0; i < COUNT; i++) {
+        double sum = 0.0;
+        for (int r = 0; r < team.size; r++) sum += slots[r][i];
+        v[i] = sum;
+    }
+}
+
 // The coming step's size and nodal coefficients (:947-956, :985-990), computed once per block
 // by thread 0 and read by every thread: the same formulas as each thread would evaluate, so
 // the same bits, without every thread spending FP64 divisions and a square root on them.
@@ -87,120 +146,120 @@ __device__ __forceinline__ void block_step_init(BlockStep &bs, const Dev &d, con
     bs.hourglass = (float)in.hourglass;
 }
 
-// Thread 0's part of a step's end: the block minimum of the warps' minima (exact, by the order
-// of the bits), the CFL step (:985-990) and the next step's coefficients. Out of line: one
-// thread runs it once a step, and its FP64 division and square root stay out of the
-// registers of the element and node loops.
-static __device__ __noinline__ void block_step_advance(double *sh, int warps, BlockStep *bs,
-                                                const BatchInst &in, double dt, double dtPrev,
-                                                int finite) {
-    unsigned long long m = bbits(sh[0]);
-    for (int w = 1; w < warps; w++) m = min(m, bbits(sh[w]));
-    const double me = bdouble(m);
-    sh[warps] = me;
+// Thread 0's part of a step's end: the minimum of `count` minima (exact, by the order of the
+// bits), the CFL step (:985-990) and the next step's coefficients. Out of line: one thread runs
+// it once a step, and its division and square root stay out of the registers of the element and
+// node loops.
+__device__ __forceinline__ double min_of(const double *v, int count) {
+    unsigned long long m = bbits(v[0]);
+    for (int w = 1; w < count; w++) m = min(m, bbits(v[w]));
+    return bdouble(m);
+}
+static __device__ __noinline__ double block_step_advance(const double *v, int count, BlockStep *bs,
+                                                         const BatchInst &in, double dt,
+                                                         double dtPrev, int finite) {
+    const double me = min_of(v, count);
     if (finite) block_step_coef(*bs, in, nf_div(in.cfl * nf_sqrt(me * in.massScale), in.wave), dt);
     else block_step_coef(*bs, in, dt, dtPrev);
+    return me;
 }
 
-// The common end of block_min_edge_next(_f): each warp's minimum is in sh[warp].
-template <int T>
-__device__ __forceinline__ double block_min_tail(double *sh, BlockStep *bs, const BatchInst &in,
-                                                 double dt, double dtPrev, int finite) {
+// The team's exact minimum of the warps' minima (each warp's in sh[warp]), returned to every
+// thread, with each block's thread 0 preparing the next step in its bs between the barriers.
+template <bool TEAM, int T>
+__device__ __forceinline__ double team_min_tail(const Team<TEAM> &team, double *sh, BlockStep *bs,
+                                                const BatchInst &in, double dt, double dtPrev,
+                                                int finite) {
+    __shared__ double ranks[TEAM_MAX];
     __syncthreads();
-    if (threadIdx.x == 0) block_step_advance(sh, T / 32, bs, in, dt, dtPrev, finite);
+    if (TEAM) {
+        if (threadIdx.x == 0) {
+            const double mine = min_of(sh, T / 32);
+            for (int r = 0; r < team.size; r++) team.at(ranks, r)[team.rank] = mine;
+        }
+        team.sync();
+        if (threadIdx.x == 0)
+            sh[T / 32] = block_step_advance(ranks, team.size, bs, in, dt, dtPrev, finite);
+    } else if (threadIdx.x == 0) {
+        sh[T / 32] = block_step_advance(sh, T / 32, bs, in, dt, dtPrev, finite);
+    }
     __syncthreads();
     return sh[T / 32];
 }
 
-// block_min_edge, with thread 0 also preparing the next step in bs between the barriers.
-template <int T>
-__device__ double block_min_edge_next(double v, double *sh, BlockStep *bs, const BatchInst &in,
-                                      double dt, double dtPrev, int finite) {
+template <bool TEAM, int T>
+__device__ double team_min_edge_next(const Team<TEAM> &team, double v, double *sh, BlockStep *bs,
+                                     const BatchInst &in, double dt, double dtPrev, int finite) {
     for (int o = 16; o > 0; o >>= 1) v = jmin(v, __shfl_down_sync(0xffffffffu, v, o));
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-    return block_min_tail<T>(sh, bs, in, dt, dtPrev, finite);
+    return team_min_tail<TEAM, T>(team, sh, bs, in, dt, dtPrev, finite);
 }
 
 // The same for FP32 edges: the warps reduce in FP32 (exact), lane 0 widens its minimum.
-template <int T>
-__device__ double block_min_edge_next_f(float v, double *sh, BlockStep *bs, const BatchInst &in,
-                                        double dt, double dtPrev, int finite) {
+template <bool TEAM, int T>
+__device__ double team_min_edge_next_f(const Team<TEAM> &team, float v, double *sh, BlockStep *bs,
+                                       const BatchInst &in, double dt, double dtPrev, int finite) {
     for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_down_sync(0xffffffffu, v, o));
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = (double)v;
-    return block_min_tail<T>(sh, bs, in, dt, dtPrev, finite);
+    return team_min_tail<TEAM, T>(team, sh, bs, in, dt, dtPrev, finite);
 }
 
-// One step of instance `in` by the whole block, ExplicitSolver.step :940-991: the nodal update
-// (with the mixed form's float geometry when geo.pMid is set), the assembly with the block's
-// exact shortest squared edge, the per-node gather, the next CFL step. dt, dtPrev, time and
-// steps advance in place; returns the shortest squared edge. COMP (with MIXED): the
-// compensated form's FP32 nodal update and gather (nf_bodies.cuh). With bs (a block-shared
-// BlockStep prepared for this step), the step's coefficients and the next step size come from
-// thread 0 through it; without, every thread evaluates them.
-template <bool MIXED, int T, bool COMP = false, bool INT = false>
-__device__ __forceinline__ double batch_step(const Dev &d, const BatchInst &in, double &dt,
-                                             double &dtPrev, double &time, long long &steps,
-                                             const MixedGeo &geo, const float4 *pMid,
-                                             const float2 *vdt, int base, uint32_t *status,
-                                             int *wallContact, int *wallStuck, double &impulse,
-                                             double &loss, double &fric, double *shMin,
-                                             BlockStep *bs = nullptr) {
+// One step of instance `in` by its team of blocks, ExplicitSolver.step :940-991: the nodal update
+// (with the mixed form's float geometry when geo.pMid is set), the assembly with the exact
+// shortest squared edge, the per-node gather, the next CFL step. dt, dtPrev, time and steps
+// advance in place; returns the shortest squared edge. COMP (with MIXED): the compensated form's
+// FP32 nodal update and gather (nf_bodies.cuh). INT: int_products. The step's coefficients and
+// the next step size come from bs, which each block's thread 0 keeps prepared.
+template <bool MIXED, int T, bool COMP, bool INT, bool TEAM>
+__device__ __forceinline__ double batch_step(const Team<TEAM> &team, const Dev &d,
+                                             const BatchInst &in, double &dt, double &dtPrev,
+                                             double &time, long long &steps, const MixedGeo &geo,
+                                             const float4 *pMid, const float2 *vdt, int base,
+                                             uint32_t *status, int *wallContact, int *wallStuck,
+                                             double &impulse, double &loss, double &fric,
+                                             double *shMin, BlockStep *bs) {
     static_assert(!COMP || MIXED, "the compensated form assembles in FP32");
-    NodalCoef co;
-    if (bs) {
-        co = NodalCoef{bs->decay, bs->gain, bs->dtAvg, dt};
-    } else {
-        const double dtAvg = 0.5 * (dtPrev + dt);                   // :947-956
-        const double half = 0.5 * in.damping * dtAvg;
-        const nf_divisor by = nf_divisor_of(1.0 + half);
-        co = NodalCoef{nf_div_by(1.0 - half, 1.0 + half, by), nf_div_by(dtAvg, 1.0 + half, by),
-                       dtAvg, dt};
-    }
+    const NodalCoef co{bs->decay, bs->gain, bs->dtAvg, dt};
     const WallRef w{in.hasWall, in.wallPlane, in.wallFriction, wallContact, wallStuck};
-    if (COMP) {                                                  // requires bs
-        for (int i = in.n0 + threadIdx.x; i < in.n1; i += T)
+    const int tid = team.tid(), stride = TEAM ? team.size * T : T;
+    if (COMP) {
+        for (int i = in.n0 + tid; i < in.n1; i += stride)
             nodal_node_comp(d, i, bs->fdecay, bs->fgain, bs->fdtAvg, bs->fdt, bs->plane,
                             bs->friction, w, geo, status, impulse, loss, fric);
     } else {
-        for (int i = in.n0 + threadIdx.x; i < in.n1; i += T)
+        for (int i = in.n0 + tid; i < in.n1; i += stride)
             nodal_node(d, i, co, w, geo, status, impulse, loss, fric);
     }
-    __syncthreads();
+    team.sync();
     time += dt;                                                       // :973-974
     steps += 1;
     double me;
     if (MIXED) {
         float m = 3.4028235e38f;
-        const float sdt = bs ? bs->fdt : (float)dt, qhg = bs ? bs->hourglass : (float)in.hourglass;
-        for (int e = in.e0 + threadIdx.x; e < in.e1; e += T)
-            element_reduced_f32(d, e, sdt, qhg, pMid, vdt, base, m);
-        for (int k = in.k0 + threadIdx.x; k < in.k1; k += T) {   // applyPressure, :1203-1207
+        for (int e = in.e0 + tid; e < in.e1; e += stride)
+            element_reduced_f32(d, e, bs->fdt, bs->hourglass, pMid, vdt, base, m);
+        for (int k = in.k0 + tid; k < in.k1; k += stride) {   // applyPressure, :1203-1207
             if (COMP) pressure_edge_comp(d, k, time, in.pressure, in.ramp);
             else pressure_edge_f32(d, k, time, in.pressure, in.ramp);
         }
-        if (bs) {
-            me = block_min_edge_next_f<T>(m, shMin, bs, in, dt, dtPrev, d.finite);
-        } else {
-            me = block_min_edge_f<T>(m, shMin);
-        }
+        me = team_min_edge_next_f<TEAM, T>(team, m, shMin, bs, in, dt, dtPrev, d.finite);
     } else {
         double m = DMAX;
-        for (int e = in.e0 + threadIdx.x; e < in.e1; e += T)
+        for (int e = in.e0 + tid; e < in.e1; e += stride)
             element_reduced<INT>(d, e, dt, in.hourglass, m);
-        for (int k = in.k0 + threadIdx.x; k < in.k1; k += T)
+        for (int k = in.k0 + tid; k < in.k1; k += stride)
             pressure_edge(d, k, time, in.pressure, in.ramp);
-        me = bs ? block_min_edge_next<T>(m, shMin, bs, in, dt, dtPrev, d.finite)
-                : block_min_edge<T>(m, shMin);
+        me = team_min_edge_next<TEAM, T>(team, m, shMin, bs, in, dt, dtPrev, d.finite);
     }
     // the gather keeps the nodal loop's node-to-thread map, so the next nodal update reads
     // only forces its own thread wrote
-    for (int i = in.n0 + threadIdx.x; i < in.n1; i += T) {
+    for (int i = in.n0 + tid; i < in.n1; i += stride) {
         if (COMP) d.fC[i] = gather_node_comp(d, i, bs->gravR, bs->gravZ);
         else d.F[i] = MIXED ? gather_node_f32(d, i) : gather_node(d, i);
     }
     if (d.finite) {                                                   // :985-990
         dtPrev = dt;
-        dt = bs ? bs->dt : nf_div(in.cfl * nf_sqrt(me * in.massScale), in.wave);
+        dt = bs->dt;
     }
     return me;
 }

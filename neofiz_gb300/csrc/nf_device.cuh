@@ -348,10 +348,11 @@ struct Newton<double> {
 
 // J2.solve, J2.java:332-375, given the thermal term jc_thermalTerm(jc, temperature) of the
 // point's temperature (the reference evaluates it first thing, from the same argument).
+// To |g| <= tolerance or `limit` iterations.
 template <typename T>
-static __device__ __noinline__ SolveOut<T> j2_solve(T norm, T stiffness, T plasticStrain,
-                                                    T thermal, T dt, const MatT<T> &jc) {
-    const T tolerance = Fn<T>::tolerance * jc.a;
+static __device__ __noinline__ SolveOut<T> j2_solve_to(T norm, T stiffness, T plasticStrain,
+                                                       T thermal, T dt, const MatT<T> &jc,
+                                                       T tolerance, int limit) {
     T lo = T(0);
     T hi = Fn<T>::div(norm, stiffness);
     T dGamma = hi;
@@ -361,15 +362,15 @@ static __device__ __noinline__ SolveOut<T> j2_solve(T norm, T stiffness, T plast
     int iteration = 0, steps = 0, converged = 0;
     T strain = T(0);
 #pragma unroll 1
-    while (!converged && iteration < SOLVE_ITERATIONS) {
+    while (!converged && iteration < limit) {
         bool up;
 #pragma unroll 1
-        while (iteration < SOLVE_ITERATIONS && newton.bisects(dGamma, lo, hi, up)) {
+        while (iteration < limit && newton.bisects(dGamma, lo, hi, up)) {
             if (up) lo = dGamma; else hi = dGamma;
             dGamma = Newton<T>::middle(lo, hi);
             iteration++;
         }
-        if (iteration < SOLVE_ITERATIONS) {
+        if (iteration < limit) {
             const NewtonStep<T> n =
                 newton.step(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
             if (Newton<T>::positive(n.g)) lo = dGamma; else hi = dGamma;
@@ -383,6 +384,13 @@ static __device__ __noinline__ SolveOut<T> j2_solve(T norm, T stiffness, T plast
         }
     }
     return SolveOut<T>{dGamma, strain, steps, converged};
+}
+
+template <typename T>
+__device__ __forceinline__ SolveOut<T> j2_solve(T norm, T stiffness, T plasticStrain, T thermal,
+                                                T dt, const MatT<T> &jc) {
+    return j2_solve_to(norm, stiffness, plasticStrain, thermal, dt, jc, Fn<T>::tolerance * jc.a,
+                       SOLVE_ITERATIONS);
 }
 
 // Damage.begin, Damage.java:306-336
