@@ -507,10 +507,15 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
         launch_batch_comp(d, true, B->stream);
         B->launches += 1;
     }
-    // default shape: the most resident blocks of 256 threads, capped at 8 per SM
+    // default shape: blocks of 256 threads, or no wider than the largest instance needs (a block's
+    // idle warps hold the registers of other instances' blocks: 512 wall slices of 16 elements
+    // take 220 ms in blocks of 256 and 87 in blocks of 32), and the most of them resident, up
+    // to 2048 threads per SM. The compensated one-warp kernels round differently from the wider
+    // ones, so that form stops at 128.
     BatchShape s{256, 0, 1, 256};
+    if (maxElems <= 128) s.threads = maxElems <= 32 && !B->comp ? 32 : 128;
     const int occ = batch_max_blocks_per_sm(B->mode, s, maxNodes, maxElems);
-    s.blocksPerSm = std::max(1, std::min(occ, 8));
+    s.blocksPerSm = std::max(1, std::min(occ, 2048 / s.threads));
     B->shape = s;
     nf_status st = bsync(*B);
     if (st) {

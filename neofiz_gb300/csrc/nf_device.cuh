@@ -59,7 +59,6 @@ template <> struct Fn<double> {
     static __device__ __forceinline__ double cos(double a) { return nf_cos(a); }
     static __device__ __forceinline__ double abs(double a) { return ::fabs(a); }
     static __device__ __forceinline__ double div3(double a);
-    static constexpr double tolerance = SOLVE_TOLERANCE;
 };
 // The FP32 forms run well inside their error budget with CUDA's fast pow and log (a few ulp
 // instead of correctly rounded): the Johnson-Cook solve of a plastic point calls them in
@@ -189,54 +188,31 @@ __device__ __forceinline__ bool near_yield(double norm, double radius) {
 __device__ __forceinline__ bool near_yield(float norm, float radius) { return norm > 0.81f * radius; }
 
 // One iteration of J2.solve (J2.java:343-372): the residual g, the strain term and g / slope.
-template <typename T>
 struct NewtonStep {
-    T g, strain, quotient;
+    double g, strain, quotient;
 };
-template <typename T>
-__device__ __forceinline__ NewtonStep<T> newton_step(T norm, T stiffness, T plasticStrain,
-                                                     T thermal, T dt, const MatT<T> &jc,
-                                                     T dGamma) {
-    const T dEps = T(SQRT_2_3) * dGamma;
-    const T eps = plasticStrain + dEps;
-    const T rate = dt > T(0) ? Fn<T>::div(dEps, dt) : T(0);
-    const T strain = jc_strainTerm(jc, eps);
-    const T rateFactor = jc_rateTerm(jc, rate);
-    const T g = norm - stiffness * dGamma - T(SQRT_2_3) * strain * rateFactor * thermal;
-    T slope = -stiffness
-              - T(TWO_THIRDS) * Fn<T>::div(jc.n * (strain - jc.a), eps) * rateFactor * thermal;
-    if (!(rate <= jc.refRate)) {
-        slope -= Fn<T>::div(T(SQRT_2_3) * strain * jc.c * thermal, dGamma);
-    }
-    return NewtonStep<T>{g, strain, Fn<T>::div(g, slope)};
-}
-static __device__ __noinline__ NewtonStep<double> newton_slow(double norm, double stiffness,
-                                                              double plasticStrain, double thermal,
-                                                              double dt, const MatDev &jc,
-                                                              double dGamma) {
-    return newton_step(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
+// The iteration as the reference writes it, for the points whose step was not settled.
+static __device__ __noinline__ NewtonStep newton_slow(double norm, double stiffness,
+                                                      double plasticStrain, double thermal,
+                                                      double dt, const MatDev &jc, double dGamma) {
+    const double dEps = SQRT_2_3 * dGamma;
+    const double eps = plasticStrain + dEps;
+    const double rate = dt > 0.0 ? nf_div(dEps, dt) : 0.0;
+    const double strain = jc_strainTerm(jc, eps);
+    const double rateFactor = jc_rateTerm(jc, rate);
+    const double g = norm - stiffness * dGamma - SQRT_2_3 * strain * rateFactor * thermal;
+    double slope = -stiffness
+                   - TWO_THIRDS * nf_div(jc.n * (strain - jc.a), eps) * rateFactor * thermal;
+    if (!(rate <= jc.refRate)) slope -= nf_div(SQRT_2_3 * strain * jc.c * thermal, dGamma);
+    return NewtonStep{g, strain, nf_div(g, slope)};
 }
 
-// The iteration per real type: what it keeps over a solve, and the step. In FP64 a solve is one
-// long dependent chain, so the step is straight-line code: the power and the logarithm, and the
-// two quotients of the slope, run beside each other, every quotient, power and logarithm by its
-// branch-free form, and one test at the end sends the point through newton_step when any of
-// them was not settled (about one point-iteration in a thousand).
-template <typename T>
+// What an FP64 solve keeps, and its iteration. A solve is one long dependent chain, so the step
+// is straight-line code: the power and the logarithm, and the two quotients of the slope, run
+// beside each other, every quotient, power and logarithm by its branch-free form, and one test
+// at the end sends the point through newton_slow when any of them was not settled (about one
+// point-iteration in a hundred thousand).
 struct Newton {
-    __device__ __forceinline__ Newton(T, T, T, T, T, const MatT<T> &) {}
-    __device__ __forceinline__ NewtonStep<T> step(T norm, T stiffness, T plasticStrain, T thermal,
-                                                  T dt, const MatT<T> &jc, T dGamma) const {
-        return newton_step(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
-    }
-    __device__ __forceinline__ bool bisects(T, T, T, bool &) const { return false; }
-    static __device__ __forceinline__ T middle(T lo, T hi) { return T(0.5) * (lo + hi); }
-    static __device__ __forceinline__ bool positive(T x) { return x > T(0); }
-    static __device__ __forceinline__ bool within(T x, T bound) { return Fn<T>::abs(x) <= bound; }
-    static __device__ __forceinline__ bool between(T x, T lo, T hi) { return x > lo && x < hi; }
-};
-template <>
-struct Newton<double> {
     nf_divisor byDt;
     int plain;                   // dt > 0 and the reference rate is 1/s (no second division)
     float norm, stiffness, plasticStrain, thermal, perDt, a, b, n, c;
@@ -300,7 +276,7 @@ struct Newton<double> {
     static __device__ __forceinline__ double middle(double lo, double hi) {
         return nf_scale2(is_zero(lo) ? hi : lo + hi, -1);
     }
-    __device__ __forceinline__ NewtonStep<double> step(double norm, double stiffness,
+    __device__ __forceinline__ NewtonStep step(double norm, double stiffness,
                                                        double plasticStrain, double thermal,
                                                        double dt, const MatDev &jc,
                                                        double dGamma) const {
@@ -328,7 +304,7 @@ struct Newton<double> {
         const double slope = slow ? base : base - q2;
         const double q = nf_div_try(g, nf_divisor_of(slope), &okStep);
         if (plain & okRate & (okLog | flat) & ok1 & (ok2 | slow) & okStep & (bad ^ 1u))
-            if (okPow || nf_pow_settled(&tail)) return NewtonStep<double>{g, strain, q};
+            if (okPow || nf_pow_settled(&tail)) return NewtonStep{g, strain, q};
         return newton_slow(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
     }
     // x > 0, |x| <= bound (bound >= 0), and lo < x < hi (0 <= lo, hi), by the integer order of
@@ -347,50 +323,76 @@ struct Newton<double> {
 };
 
 // J2.solve, J2.java:332-375, given the thermal term jc_thermalTerm(jc, temperature) of the
-// point's temperature (the reference evaluates it first thing, from the same argument).
-// To |g| <= tolerance or `limit` iterations.
-template <typename T>
-static __device__ __noinline__ SolveOut<T> j2_solve_to(T norm, T stiffness, T plasticStrain,
-                                                       T thermal, T dt, const MatT<T> &jc,
-                                                       T tolerance, int limit) {
-    T lo = T(0);
-    T hi = Fn<T>::div(norm, stiffness);
-    T dGamma = hi;
-    const Newton<T> newton(norm, stiffness, plasticStrain, thermal, dt, jc);
+// point's temperature (the reference evaluates it first thing, from the same argument), to
+// |g| <= tolerance or `limit` iterations.
+static __device__ __noinline__ SolveOut<double> j2_solve_to(double norm, double stiffness,
+                                                            double plasticStrain, double thermal,
+                                                            double dt, const MatDev &jc,
+                                                            double tolerance, int limit) {
+    double lo = 0.0;
+    double hi = nf_div(norm, stiffness);
+    double dGamma = hi, strain = 0.0;
+    const Newton newton(norm, stiffness, plasticStrain, thermal, dt, jc);
     // iterations so far and those computed in full; one loop exit, so that a warp's lanes bisect
     // as far as they can and then step together
     int iteration = 0, steps = 0, converged = 0;
-    T strain = T(0);
 #pragma unroll 1
     while (!converged && iteration < limit) {
         bool up;
 #pragma unroll 1
         while (iteration < limit && newton.bisects(dGamma, lo, hi, up)) {
             if (up) lo = dGamma; else hi = dGamma;
-            dGamma = Newton<T>::middle(lo, hi);
+            dGamma = Newton::middle(lo, hi);
             iteration++;
         }
         if (iteration < limit) {
-            const NewtonStep<T> n =
+            const NewtonStep n =
                 newton.step(norm, stiffness, plasticStrain, thermal, dt, jc, dGamma);
-            if (Newton<T>::positive(n.g)) lo = dGamma; else hi = dGamma;
-            converged = Newton<T>::within(n.g, tolerance);
-            T next = dGamma - n.quotient;
-            if (!Newton<T>::between(next, lo, hi)) next = Newton<T>::middle(lo, hi);
+            if (Newton::positive(n.g)) lo = dGamma; else hi = dGamma;
+            converged = Newton::within(n.g, tolerance);
+            double next = dGamma - n.quotient;
+            if (!Newton::between(next, lo, hi)) next = Newton::middle(lo, hi);
             if (!converged) dGamma = next;
             strain = n.strain;
             iteration++;
             steps++;
         }
     }
-    return SolveOut<T>{dGamma, strain, steps, converged};
+    return SolveOut<double>{dGamma, strain, steps, converged};
 }
-
-template <typename T>
-__device__ __forceinline__ SolveOut<T> j2_solve(T norm, T stiffness, T plasticStrain, T thermal,
-                                                T dt, const MatT<T> &jc) {
-    return j2_solve_to(norm, stiffness, plasticStrain, thermal, dt, jc, Fn<T>::tolerance * jc.a,
+__device__ __forceinline__ SolveOut<double> j2_solve(double norm, double stiffness,
+                                                     double plasticStrain, double thermal,
+                                                     double dt, const MatDev &jc) {
+    return j2_solve_to(norm, stiffness, plasticStrain, thermal, dt, jc, SOLVE_TOLERANCE * jc.a,
                        SOLVE_ITERATIONS);
+}
+// The FP32 forms' solve: a few tens of instructions an iteration, so it is written plainly.
+static __device__ __noinline__ SolveOut<float> j2_solve(float norm, float stiffness,
+                                                        float plasticStrain, float thermal,
+                                                        float dt, const MatF &jc) {
+    const float tolerance = Fn<float>::tolerance * jc.a;
+    float lo = 0.0f;
+    float hi = norm / stiffness;
+    float dGamma = hi;
+    for (int iteration = 0; iteration < SOLVE_ITERATIONS; iteration++) {
+        const float dEps = float(SQRT_2_3) * dGamma;
+        const float eps = plasticStrain + dEps;
+        const float rate = dt > 0.0f ? dEps / dt : 0.0f;
+        const float strain = jc_strainTerm(jc, eps);
+        const float rateFactor = jc_rateTerm(jc, rate);
+        const float g = norm - stiffness * dGamma - float(SQRT_2_3) * strain * rateFactor * thermal;
+        if (g > 0.0f) lo = dGamma; else hi = dGamma;
+        if (fabsf(g) <= tolerance) return SolveOut<float>{dGamma, strain, iteration + 1, 1};
+        float slope = -stiffness
+                      - float(TWO_THIRDS) * (jc.n * (strain - jc.a) / eps) * rateFactor * thermal;
+        if (!(rate <= jc.refRate)) {
+            slope -= float(SQRT_2_3) * strain * jc.c * thermal / dGamma;
+        }
+        float next = dGamma - g / slope;
+        if (!(next > lo && next < hi)) next = 0.5f * (lo + hi);
+        dGamma = next;
+    }
+    return SolveOut<float>{dGamma, 0.0f, SOLVE_ITERATIONS, 0};
 }
 
 // Damage.begin, Damage.java:306-336
