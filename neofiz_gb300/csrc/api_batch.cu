@@ -35,6 +35,8 @@ struct Batch {
     BatchShape shape{256, 0, 1, 256};
     cudaGraphExec_t graph = nullptr;
     BatchShape graphShape{};
+    int graphTeam = 0, graphLeft = -1;
+    std::vector<int> elems;                  // the instances' element counts, most expensive first
     int32_t *hostRemaining = nullptr;        // pinned
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double lastMs = 0.0;
@@ -120,24 +122,39 @@ bool shape_valid(const Batch &B, const BatchShape &s) {
     return batch_max_blocks_per_sm(B.mode, s, B.b.maxNodes, B.b.maxElems) >= s.blocksPerSm;
 }
 
+// Blocks per instance while the `left` most expensive instances run (the cheap ones finish
+// first, and those left spread over more blocks), and the teams resident.
+int team_of(const Batch &B, int left, int *teams) {
+    int n[4];
+    batch_teams(B.mode, B.shape, B.sms, n);
+    const int team = choose_team(B.elems.data(), std::max(1, std::min(left, B.count)), n);
+    *teams = team == 1 ? n[0] : team == 2 ? n[1] : team == 4 ? n[2] : n[3];
+    return team;
+}
+
 // The run's launches: reset the queue, launch one chunk; GRAPH_CHUNKS times.
-cudaError_t enqueue_chunks(Batch &B, int chunks) {
+cudaError_t enqueue_chunks(Batch &B, int chunks, int team, int teams) {
     for (int c = 0; c < chunks; c++) {
         cudaError_t e = cudaMemsetAsync(B.b.queue, 0, sizeof(int32_t), B.stream);
         if (e != cudaSuccess) return e;
-        e = launch_batch_steps(B.d, B.b, B.mode, B.shape, B.sms, B.stream);
+        e = launch_batch_steps(B.d, B.b, B.mode, B.shape, team, teams, B.stream);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
-nf_status ensure_graph(Batch &B) {
-    if (B.graph && memcmp(&B.graphShape, &B.shape, sizeof(BatchShape)) == 0) return NF_OK;
+nf_status ensure_graph(Batch &B, int left) {
+    const bool sameShape = B.graph && memcmp(&B.graphShape, &B.shape, sizeof(BatchShape)) == 0;
+    if (sameShape && B.graphLeft == left) return NF_OK;
+    int teams = 1;
+    const int team = team_of(B, left, &teams);
+    B.graphLeft = left;
+    if (sameShape && B.graphTeam == team) return NF_OK;
     if (B.graph) cudaGraphExecDestroy(B.graph);
     B.graph = nullptr;
     cudaGraph_t g = nullptr;
     BCK(&B, cudaStreamBeginCapture(B.stream, cudaStreamCaptureModeThreadLocal));
-    const cudaError_t launched = enqueue_chunks(B, GRAPH_CHUNKS);
+    const cudaError_t launched = enqueue_chunks(B, GRAPH_CHUNKS, team, teams);
     const cudaError_t ended = cudaStreamEndCapture(B.stream, &g);
     if (launched != cudaSuccess || ended != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -149,6 +166,7 @@ nf_status ensure_graph(Batch &B) {
     cudaGraphDestroy(g);
     if (inst != cudaSuccess) return bfail(&B, NF_EDEVICE, "graph instantiate: %s", cudaGetErrorString(inst));
     B.graphShape = B.shape;
+    B.graphTeam = team;
     return NF_OK;
 }
 
@@ -412,6 +430,7 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
     std::vector<int32_t> order(count);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return cost[a] > cost[c]; });
+    for (int k : order) B->elems.push_back(B->inst[k].e1 - B->inst[k].e0);
 
     d.N = N; d.E = E; d.K = K; d.ppe = 1;
     d.hasDamage = damage ? 1 : 0;
@@ -556,16 +575,16 @@ nf_status nf_batch_run(nf_batch *h, int64_t max_steps) {
     Batch &B = *reinterpret_cast<Batch *>(h);
     B.lastMs = 0.0;
     if (max_steps <= 0) return NF_OK;
-    nf_status st = ensure_graph(B);
-    if (st) return st;
     BCK(&B, cudaEventRecord(B.ev0, B.stream));
     launch_batch_arm(B.b, (long long)max_steps, B.stream);
     B.launches += 1;
     BCK(&B, cudaMemcpyAsync(B.hostRemaining, B.b.remaining, sizeof(int32_t),
                             cudaMemcpyDeviceToHost, B.stream));
-    st = bsync(B);
+    nf_status st = bsync(B);
     if (st) return st;
     while (*B.hostRemaining > 0) {
+        st = ensure_graph(B, *B.hostRemaining);
+        if (st) return st;
         BCK(&B, cudaGraphLaunch(B.graph, B.stream));
         B.launches += GRAPH_CHUNKS;
         BCK(&B, cudaMemcpyAsync(B.hostRemaining, B.b.remaining, sizeof(int32_t),
@@ -634,7 +653,9 @@ nf_status nf_batch_tune(nf_batch *h, int32_t trial_steps, nf_batch_config *chose
             B.shape = cands[i];
             cudaEventRecord(B.ev0, B.stream);
             launch_batch_arm(B.b, trial_steps, B.stream);
-            cudaError_t e = enqueue_chunks(B, 1);
+            int teams = 1;
+            const int team = team_of(B, B.count, &teams);
+            cudaError_t e = enqueue_chunks(B, 1, team, teams);
             cudaEventRecord(B.ev1, B.stream);
             B.launches += 2;
             if (e == cudaSuccess) e = cudaStreamSynchronize(B.stream);
@@ -999,7 +1020,7 @@ nf_status nf_batch_adjoint_forward(nf_batch *h, int32_t checkpoint_every, int32_
     a.barPlane = ba;
     B.adjBarOff = barOff;
     BCK(&B, cudaEventRecord(B.ev0, B.stream));
-    launch_adjoint_forward(B.d, B.b, a, B.sms, B.stream);
+    launch_adjoint_forward(B.d, B.b, a, B.elems.data(), B.sms, B.stream);
     B.launches += 1;
     BCK(&B, cudaEventRecord(B.ev1, B.stream));
     st = bsync(B);
@@ -1162,7 +1183,7 @@ nf_status nf_batch_adjoint_backward_many(nf_batch *h, const int32_t *objectives,
     BCK(&B, cudaMemsetAsync(a.bar, 0, (size_t)B.adjBarBytes * count, B.stream));
     a.width = count;
     BCK(&B, cudaEventRecord(B.ev0, B.stream));
-    launch_adjoint_backward(B.d, B.b, a, B.sms, B.stream);
+    launch_adjoint_backward(B.d, B.b, a, B.elems.data(), B.sms, B.stream);
     B.launches += 1;
     BCK(&B, cudaEventRecord(B.ev1, B.stream));
     nf_status st = bsync(B);

@@ -573,30 +573,32 @@ cudaError_t adjoint_reserve_stack() {
     return need > cur ? cudaDeviceSetLimit(cudaLimitStackSize, need) : cudaSuccess;
 }
 
-// One team of blocks per instance (batch_team), its products on the integer units where its
-// quarter SMs have more than one warp of elements (int_products).
+// One team of blocks per instance (choose_team), its products on the integer units where its
+// quarter SMs have more than one warp of elements (int_products). One block fits on an SM.
 static void launch_adjoint(const void *(*kernel)(bool, bool), const Dev &d, const BatchDev &b,
-                           const AdjDev &a, int sms, cudaStream_t st) {
+                           const AdjDev &a, const int *elems, int sms, cudaStream_t st) {
     if (b.count <= 0) return;
     Dev dd = d;
     BatchDev bb = b;
     AdjDev aa = a;
     void *args[] = {&dd, &bb, &aa};
-    const int team = batch_team(kernel(false, true), ADJ_T, b.count, b.maxElems, sms);
+    int teams[4] = {sms, 0, 0, 0};
+    for (int q = 1; q < 4; q++) teams[q] = max_teams(kernel(true, true), 1 << q, ADJ_T);
+    const int team = choose_team(elems, b.count, teams);
     const int warps = (b.maxElems + 31) / 32 < ADJ_T / 32 * team ? (b.maxElems + 31) / 32 : ADJ_T / 32 * team;
     const bool ints = int_products((warps + team - 1) / team, 1);
     if (team > 1) launch_team(kernel(ints, true), b.count, team, ADJ_T, args, st);
     else cudaLaunchKernel(kernel(ints, false), dim3(b.count), dim3(ADJ_T), args, 0, st);
 }
 
-void launch_adjoint_forward(const Dev &d, const BatchDev &b, const AdjDev &a, int sms,
-                            cudaStream_t st) {
-    launch_adjoint(forward_kernel, d, b, a, sms, st);
+void launch_adjoint_forward(const Dev &d, const BatchDev &b, const AdjDev &a, const int *elems,
+                            int sms, cudaStream_t st) {
+    launch_adjoint(forward_kernel, d, b, a, elems, sms, st);
 }
 
-void launch_adjoint_backward(const Dev &d, const BatchDev &b, const AdjDev &a, int sms,
-                             cudaStream_t st) {
-    launch_adjoint(backward_kernel, d, b, a, sms, st);
+void launch_adjoint_backward(const Dev &d, const BatchDev &b, const AdjDev &a, const int *elems,
+                             int sms, cudaStream_t st) {
+    launch_adjoint(backward_kernel, d, b, a, elems, sms, st);
 }
 
 }  // namespace nf

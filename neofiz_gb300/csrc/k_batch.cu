@@ -17,6 +17,9 @@
 // autotuner (api_batch.cu); none of them changes the trajectory.
 #include "nf_batch_kernels.cuh"
 
+#include <algorithm>
+#include <functional>
+
 namespace nf {
 
 constexpr int MEASURE_BLOCK = 256;
@@ -143,38 +146,9 @@ size_t batch_shared_bytes(int mode, const BatchShape &s, int maxNodes) {
                                                 : 0;
 }
 
-// Blocks that step one instance together, for `count` instances of up to maxElems elements on
-// sms SMs: a power of two, with a block per SM for every instance, and no more than shortens the
-// longest queue of element warps on a quarter SM (one with four warps or fewer has none). Kernel
-// `k` with `threads` threads a block must fit as that many clusters at once.
-int batch_team(const void *k, int threads, int count, int maxElems, int sms) {
-    const int warps = (maxElems + 31) / 32;
-    auto depth = [&](int team) { return (warps + 4 * team - 1) / (4 * team); };
-    int best = 1;
-    for (int team = 2; team <= TEAM_MAX && (long long)count * team <= sms; team *= 2) {
-        if (depth(team) >= depth(best)) continue;
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = team;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.gridDim = dim3(count * team);
-        cfg.blockDim = dim3(threads);
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess) {
-            (void)cudaGetLastError();
-            break;
-        }
-        if (clusters >= count) best = team;
-    }
-    return best;
-}
-cudaError_t launch_team(const void *k, int teams, int team, int threads, void **args,
-                        cudaStream_t st) {
+static cudaLaunchConfig_t team_config(cudaLaunchAttribute &at, int teams, int team, int threads,
+                                      cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = team;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
@@ -183,7 +157,72 @@ cudaError_t launch_team(const void *k, int teams, int team, int threads, void **
     cfg.stream = st;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
+    return cfg;
+}
+// Teams of `team` blocks that kernel k keeps resident (0: none).
+int max_teams(const void *k, int team, int threads) {
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = team_config(at, 1, team, threads, nullptr);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+// Blocks per instance for the `count` most expensive instances (their element counts in `elems`),
+// given the teams of 1, 2, 4 and 8 blocks that can be resident. A step costs an instance a fixed
+// part and its elements' rounds over the team's threads, half a round at least (below four warps
+// a block its quarter SMs have one warp each already): 0.6 + elements / (256 team). Teams take
+// the instances in this order, each the next when it is free; the time until the last is done,
+// plus half the longest instance's (which goes on when most have ended), is compared. On 60
+// timings (10 to 600 ragged rods in three forms and 16 equal ones, 1 to 8 blocks each; e.g. 64
+// FP64 rods 65, 44 and 59 ms with 2, 4 and 8 blocks, 256 mixed rods 328, 197 and 173 with 1, 2
+// and 4) this picks the fastest, or one within 2 % of it, of every group.
+int choose_team(const int *elems, int count, const int (&teams)[4]) {
+    if (count >= 8 * teams[0]) return 1;     // long queues: nothing to share out
+    int best = 1;
+    double least = 0.0;
+    std::vector<double> busy;                // a heap: the team free first on top
+    for (int q = 0; q < 4; q++) {
+        const int team = 1 << q, n = teams[q] < count ? teams[q] : count;
+        if (n < 1) continue;
+        busy.assign(n, 0.0);
+        double longest = 0.0, last = 0.0;
+        for (int k = 0; k < count; k++) {
+            const double rounds = elems[k] / (256.0 * team);
+            const double t = 0.6 + (rounds > 0.5 ? rounds : 0.5);
+            if (t > longest) longest = t;
+            std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
+            busy.back() += t;
+            if (busy.back() > last) last = busy.back();
+            std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+        }
+        const double cost = last + 0.5 * longest;
+        if (q == 0 || cost < 0.98 * least) {
+            best = team;
+            least = cost;
+        }
+    }
+    return best;
+}
+cudaError_t launch_team(const void *k, int teams, int team, int threads, void **args,
+                        cudaStream_t st) {
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = team_config(at, teams, team, threads, st);
     return cudaLaunchKernelExC(&cfg, k, args);
+}
+
+// Teams of 1, 2, 4 and 8 blocks that a shape keeps resident; only the 256-thread kernels without
+// staged nodes come as teams.
+void batch_teams(int mode, const BatchShape &s, int sms, int (&teams)[4]) {
+    teams[0] = sms * s.blocksPerSm;
+    for (int q = 1; q < 4; q++) {
+        teams[q] = 0;
+        if (s.threads != TEAM_THREADS || s.stage) continue;
+        const int n = max_teams(select_kernel(mode, s, false, true), 1 << q, TEAM_THREADS);
+        teams[q] = n < teams[0] >> q ? n : teams[0] >> q;
+    }
 }
 
 // Resident blocks per SM of a shape (0 when it cannot launch, e.g. too much shared memory).
@@ -203,27 +242,21 @@ int batch_max_blocks_per_sm(int mode, const BatchShape &s, int maxNodes, int max
     return n;
 }
 
-// A batch with fewer instances than SMs steps each by a team of blocks (batch_team) where the
-// shape allows it: one 64-rod FP64 sweep fills 128 SMs instead of 64.
+// team: blocks per instance (choose_team); teams: how many of them.
 cudaError_t launch_batch_steps(const Dev &d, const BatchDev &b, int mode, const BatchShape &s,
-                               int sms, cudaStream_t st) {
+                               int team, int teams, cudaStream_t st) {
     Dev dd = d;
     BatchDev bb = b;
     int chunk = s.chunk;
     void *args[] = {&dd, &bb, &chunk};
-    if (s.threads == TEAM_THREADS && !s.stage) {
-        const int team = batch_team(select_kernel(mode, s, false, true), TEAM_THREADS, b.count,
-                                    b.maxElems, sms);
-        if (team > 1)
-            return launch_team(select_kernel(mode, s, lone_warps(s, b.maxElems, team), true),
-                               b.count, team, TEAM_THREADS, args, st);
-    }
-    const void *k = select_kernel(mode, s, lone_warps(s, b.maxElems, 1), false);
+    const bool lone = lone_warps(s, b.maxElems, team);
+    if (teams > b.count) teams = b.count;
+    if (teams < 1) teams = 1;
+    if (team > 1)
+        return launch_team(select_kernel(mode, s, lone, true), teams, team, TEAM_THREADS, args, st);
     const size_t smem = batch_shared_bytes(mode, s, b.maxNodes);
-    int blocks = sms * s.blocksPerSm;
-    if (blocks > b.count) blocks = b.count;
-    if (blocks < 1) blocks = 1;
-    return cudaLaunchKernel(k, dim3(blocks), dim3(s.threads), args, smem, st);
+    return cudaLaunchKernel(select_kernel(mode, s, lone, false), dim3(teams), dim3(s.threads), args,
+                            smem, st);
 }
 
 void launch_batch_initial(const Dev &d, const BatchDev &b, bool mixed, cudaStream_t st) {

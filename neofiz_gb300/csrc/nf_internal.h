@@ -360,10 +360,11 @@ size_t adj_state_bytes(int n, int e);
 size_t adj_bar_bytes(int n, int e, int k);
 size_t adj_seed_bytes(int n, int e);
 cudaError_t adjoint_reserve_stack();
-void launch_adjoint_forward(const Dev &d, const BatchDev &b, const AdjDev &a, int sms,
-                            cudaStream_t st);
-void launch_adjoint_backward(const Dev &d, const BatchDev &b, const AdjDev &a, int sms,
-                             cudaStream_t st);
+// elems: the instances' element counts, most expensive first.
+void launch_adjoint_forward(const Dev &d, const BatchDev &b, const AdjDev &a, const int *elems,
+                            int sms, cudaStream_t st);
+void launch_adjoint_backward(const Dev &d, const BatchDev &b, const AdjDev &a, const int *elems,
+                             int sms, cudaStream_t st);
 
 // A launch configuration of the batched step (chosen by the autotuner).
 struct BatchShape {
@@ -382,11 +383,13 @@ void launch_batch_arm(const BatchDev &b, long long maxSteps, cudaStream_t st);
 void launch_batch_comp(const Dev &d, bool toFloat, cudaStream_t st);
 const void *comp_steps_kernel(const BatchShape &shape, bool team);      // k_batch_comp.cu
 constexpr int TEAM_THREADS = 256;            // threads of a block of a team, and of the widest shape
-int batch_team(const void *k, int threads, int count, int maxElems, int sms);
+int max_teams(const void *k, int team, int threads);
+int choose_team(const int *elems, int count, const int (&teams)[4]);
+void batch_teams(int mode, const BatchShape &shape, int sms, int (&teams)[4]);
 cudaError_t launch_team(const void *k, int teams, int team, int threads, void **args,
                         cudaStream_t st);
 cudaError_t launch_batch_steps(const Dev &d, const BatchDev &b, int mode,
-                               const BatchShape &shape, int sms, cudaStream_t st);
+                               const BatchShape &shape, int team, int teams, cudaStream_t st);
 void launch_batch_measure(const Dev &d, const BatchDev &b, cudaStream_t st);
 
 // Set-up helpers of api.cu shared with api_batch.cu.
