@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev
 // memory: atomics need a shared or global address).
 // owner0 is the first block's shared word; shDtb, shDtPrevb and shTimeb are each block's own and
 // equal in all of them.
-template <bool TEAM>
+template <bool INT, bool TEAM>
 __device__ void reverse_step(const Team<TEAM> &team, const Dev &d, const BatchInst &in,
                              const MatDev &mat, StateBlock pre, BarBlock bar, double *pacc,
                              double *shRed, double (*slots)[4], int *owner0, double *shDtb,
@@ -343,7 +343,7 @@ __device__ void reverse_step(const Team<TEAM> &team, const Dev &d, const BatchIn
         for (int i = tid; i < n; i += stride) {
             const int g = in.n0 + i;
             d.U[g] = pre.U[i]; d.V[g] = pre.V[i]; d.F[g] = pre.F[i]; d.flags[g] = pre.flags[i];
-            nodal_node(d, g, co, w, none, reinterpret_cast<uint32_t *>(scratch + 2), i0, l0, f0);
+            nodal_node<INT>(d, g, co, w, none, reinterpret_cast<uint32_t *>(scratch + 2), i0, l0, f0);
         }
     }
     if (team.first()) *owner0 = 0x7fffffff;
@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDe
                 }
                 // the forward values each objective's reverse reads are recomputed from the
                 // same tape entry, so every objective sees the same bits
-                reverse_step(team, d, in, mat, pre, bar, pacc[w], shRed, slots, owner0, &shDtb[w],
+                reverse_step<INT>(team, d, in, mat, pre, bar, pacc[w], shRed, slots, owner0, &shDtb[w],
                              &shDtPrevb[w], &shTimeb[w], scratch);
             }
         }

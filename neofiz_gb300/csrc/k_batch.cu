@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(256) k_batch_initial(Dev d, BatchDev b) {
     }
     __syncthreads();
     for (int i = in.n0 + threadIdx.x; i < in.n1; i += 256)
-        d.F[i] = MIXED ? gather_node_f32(d, i) : gather_node(d, i);
+        d.F[i] = MIXED ? gather_node_f32<false>(d, i) : gather_node<false>(d, i);
     if (threadIdx.x == 0) b.sc[blockIdx.x].minEdgeSquared = me;
 }
 
@@ -127,8 +127,11 @@ static const void *by_threads(int threads) {
 static const void *select_kernel(int mode, const BatchShape &s, bool lone, bool team) {
     if (mode == NF_PRECISION_COMPENSATED) return comp_steps_kernel(s, team);
     if (mode == NF_PRECISION_MIXED) {
-        if (team) return (const void *)k_batch_steps<true, false, TEAM_THREADS, false, true>;
-        return s.stage ? by_threads<true, true, false>(s.threads) : by_threads<true, false, false>(s.threads);
+        if (team) return lone ? (const void *)k_batch_steps<true, false, TEAM_THREADS, false, true>
+                              : (const void *)k_batch_steps<true, false, TEAM_THREADS, true, true>;
+        if (lone) return s.stage ? by_threads<true, true, false>(s.threads)
+                                 : by_threads<true, false, false>(s.threads);
+        return s.stage ? by_threads<true, true, true>(s.threads) : by_threads<true, false, true>(s.threads);
     }
     if (team) return lone ? (const void *)k_batch_steps<false, false, TEAM_THREADS, false, true>
                           : (const void *)k_batch_steps<false, false, TEAM_THREADS, true, true>;

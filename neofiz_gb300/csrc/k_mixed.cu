@@ -99,8 +99,10 @@ __global__ void __launch_bounds__(MB) k_erode_mixed(Dev d) {
 }
 
 __device__ __forceinline__ void min_edge_commit_f(Dev &d, float minEdge) {
-    for (int o = 16; o > 0; o >>= 1) minEdge = fminf(minEdge, __shfl_down_sync(0xffffffffu, minEdge, o));
-    if ((threadIdx.x & 31) == 0) atomicMin(&d.s->minEdgeBits, dbits_m((double)minEdge));
+    // fminf passes over a NaN: its bits lie above every number's
+    const float m = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(minEdge)));
+    const unsigned long long bits = dbits_m(nf_widen(m));
+    if ((threadIdx.x & 31) == 0 && bits < __ldcg(&d.s->minEdgeBits)) atomicMin(&d.s->minEdgeBits, bits);
 }
 
 // reducedIntegration (ExplicitSolver.java:1373-1504) in FP32. With `erode` each element first
@@ -219,11 +221,12 @@ __global__ void k_pressure_mixed(Dev d) {
 }
 
 // The per-node gather (:1147-1165) of float contributions into FP64 forces, same order.
+template <bool INT>
 __global__ void __launch_bounds__(MB) k_gather_mixed(Dev d) {
     if (!d.s->active) return;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= d.N) return;
-    d.F[n] = gather_node_f32(d, n);
+    d.F[n] = gather_node_f32<INT>(d, n);
     if (d.hasContact) d.contactState[n] = 0;
 }
 
@@ -302,7 +305,8 @@ int launch_pressure_mixed(Solver &S) {
     return 1;
 }
 int launch_gather_mixed(Solver &S) {
-    k_gather_mixed<<<grid_for(S.d.N, MB), MB, 0, S.stream>>>(S.d);
+    if (int_products(S.d.N / 32, S.d.sms)) k_gather_mixed<true><<<grid_for(S.d.N, MB), MB, 0, S.stream>>>(S.d);
+    else k_gather_mixed<false><<<grid_for(S.d.N, MB), MB, 0, S.stream>>>(S.d);
     return 1;
 }
 void launch_convert_state(Solver &S, bool toFloat, int what) {

@@ -228,7 +228,7 @@ __device__ __forceinline__ double batch_step(const Team<TEAM> &team, const Dev &
                             bs->friction, w, geo, status, impulse, loss, fric);
     } else {
         for (int i = in.n0 + tid; i < in.n1; i += stride)
-            nodal_node(d, i, co, w, geo, status, impulse, loss, fric);
+            nodal_node<INT>(d, i, co, w, geo, status, impulse, loss, fric);
     }
     team.sync();
     time += dt;                                                       // :973-974
@@ -255,7 +255,7 @@ __device__ __forceinline__ double batch_step(const Team<TEAM> &team, const Dev &
     // only forces its own thread wrote
     for (int i = in.n0 + tid; i < in.n1; i += stride) {
         if (COMP) d.fC[i] = gather_node_comp(d, i, bs->gravR, bs->gravZ);
-        else d.F[i] = MIXED ? gather_node_f32(d, i) : gather_node(d, i);
+        else d.F[i] = MIXED ? gather_node_f32<INT>(d, i) : gather_node<INT>(d, i);
     }
     if (d.finite) {                                                   // :985-990
         dtPrev = dt;

@@ -8,6 +8,19 @@
 
 namespace nf {
 
+// A product on the integer units or on the FP64 pipe (with `bad`: nf_mul_try's convention).
+template <bool INT> struct Product;
+template <> struct Product<true> {
+    static __device__ __forceinline__ double of(double a, double b, uint32_t *bad) {
+        return nf_mul_try(a, b, bad);
+    }
+    static __device__ __forceinline__ double of(double a, double b) { return nf_mul(a, b); }
+};
+template <> struct Product<false> {
+    static __device__ __forceinline__ double of(double a, double b, uint32_t *) { return a * b; }
+    static __device__ __forceinline__ double of(double a, double b) { return a * b; }
+};
+
 // One node of nodalUpdate, ExplicitSolver.java:998-1062, with RigidWall.hold/crosses/arrive/
 // slide (RigidWall.java:163-259): shared by the single-scene kernel and the batched one. Adds
 // the node's wall terms to impulse/loss/fric. When geo.pMid is set (the mixed form) it also
@@ -27,11 +40,19 @@ struct MixedGeo {
     int base;
 };
 
+// With INT (int_products) the products run on the integer units: the update is two dozen FP64
+// instructions a node otherwise, which bound it. 1M nodes of the mixed form: 71 us with all of
+// them on the FP64 pipe, 54 us so (76 and 59 us between events), bound by the dozen additions
+// left and by the loads. A product by a decay of 1 (no damping) is its factor, and -0.5 dt v is
+// -(v dt) / 2 exactly.
+template <bool INT>
 static __device__ __forceinline__ void nodal_node(const Dev &d, int i, const NodalCoef &co,
                                                   const WallRef &w, const MixedGeo &geo,
                                                   uint32_t *status, double &impulse,
                                                   double &loss, double &fric) {
+    using P = Product<INT>;
     const double decay = co.decay, gain = co.gain, dtAvg = co.dtAvg, dt = co.dt;
+    const bool undamped = __double_as_longlong(decay) == __double_as_longlong(1.0);
     uint8_t fl = d.flags[i];
     const bool fixedR = fl & 1, fixedZ = fl & 2;
     bool onWall = fl & 4;
@@ -41,6 +62,7 @@ static __device__ __forceinline__ void nodal_node(const Dev &d, int i, const Nod
     const double invM = d.invMass[i];
     const bool resting = w.present && onWall && f.y <= 0.0;
     uint8_t ws = 0;
+    double stepR = 0.0, stepZ = 0.0;                     // v dt, where it moved the node
     if (fixedR) {
         v.x = 0.0;
     } else if (resting && w.friction > 0.0) {
@@ -60,10 +82,12 @@ static __device__ __forceinline__ void nodal_node(const Dev &d, int i, const Nod
             ws |= NF_WALL_SLID;
             v.x = slid;
         }
-        u.x += v.x * dt;
+        stepR = v.x * dt;
+        u.x += stepR;
     } else {
-        v.x = decay * v.x + gain * f.x * invM;
-        u.x += v.x * dt;
+        v.x = (undamped ? v.x : P::of(decay, v.x)) + P::of(P::of(gain, f.x), invM);
+        stepR = P::of(v.x, dt);
+        u.x += stepR;
     }
     const double2 x0 = d.X0[i];
     if (fixedZ) {
@@ -72,20 +96,22 @@ static __device__ __forceinline__ void nodal_node(const Dev &d, int i, const Nod
         impulse += -f.y * dtAvg;                         // RigidWall.hold :178-181
         atomicAdd(w.contact, 1);
         ws |= NF_WALL_HELD;
+        stepZ = v.y * dt;                                // the geometry's v dt only
     } else {
-        const double trial = decay * v.y + gain * f.y * invM;
-        const double zc = x0.y + u.y;
-        if (w.present && zc + trial * dt < w.plane) {
+        const double trial = (undamped ? v.y : P::of(decay, v.y)) + P::of(P::of(gain, f.y), invM);
+        stepZ = P::of(trial, dt);
+        if (w.present && less_bits(x0.y + u.y + stepZ, w.plane)) {
             impulse += -m * trial;                       // RigidWall.arrive :205-209
             loss += 0.5 * m * trial * trial;
             atomicAdd(w.contact, 1);
-            u.y += w.plane - zc;
+            u.y += w.plane - (x0.y + u.y);
             v.y = 0.0;
+            stepZ = 0.0;
             onWall = true;
             ws |= NF_WALL_ARRIVED;
         } else {
             v.y = trial;
-            u.y += v.y * dt;
+            u.y += stepZ;
             if (w.present) onWall = false;
         }
     }
@@ -100,22 +126,19 @@ static __device__ __forceinline__ void nodal_node(const Dev &d, int i, const Nod
     if (geo.pMid) {
         // the geometry of the coming assembly: mid-step and current positions as float
         // pairs, and v dt (see k_prepare_mixed)
-        const double mid = -0.5 * dt;
-        double pr, pz;
+        const double xr = x0.x + u.x, xz = x0.y + u.y;
+        double pr = x0.x, pz = x0.y;
         if (d.finite) {
-            pr = x0.x + u.x + mid * v.x;
-            pz = x0.y + u.y + mid * v.y;
-        } else {
-            pr = x0.x;
-            pz = x0.y;
+            pr = xr - nf_scale2(stepR, -1);
+            pz = xz - nf_scale2(stepZ, -1);
         }
         const float2 sr = nf_split(pr), sz = nf_split(pz);
         geo.pMid[geo.base + i] = make_float4(sr.x, sr.y, sz.x, sz.y);
         if (geo.pCur) {
-            const float2 qr = nf_split(x0.x + u.x), qz = nf_split(x0.y + u.y);
+            const float2 qr = nf_split(xr), qz = nf_split(xz);
             geo.pCur[geo.base + i] = make_float4(qr.x, qr.y, qz.x, qz.y);
         }
-        geo.vdt[geo.base + i] = make_float2(nf_narrow(v.x * dt), nf_narrow(v.y * dt));
+        geo.vdt[geo.base + i] = make_float2(nf_narrow(stepR), nf_narrow(stepZ));
     }
 }
 
@@ -273,17 +296,6 @@ static __device__ __forceinline__ double opposite_force(double t, double f, doub
     const bool mirrored = !is_zero(s) || __double_as_longlong(t) == __double_as_longlong(f);
     return mirrored ? g : copysign(0.0, -dV);
 }
-
-// A product on the integer units or on the FP64 pipe.
-template <bool INT> struct Product;
-template <> struct Product<true> {
-    static __device__ __forceinline__ double of(double a, double b, uint32_t *bad) {
-        return nf_mul_try(a, b, bad);
-    }
-};
-template <> struct Product<false> {
-    static __device__ __forceinline__ double of(double a, double b, uint32_t *) { return a * b; }
-};
 
 // reducedIntegration, ExplicitSolver.java:1373-1504, for element e: B at the centroid, strain
 // increments, Cayley co-rotation, J2/Johnson-Cook return, FB hourglass, the eight force
@@ -923,62 +935,100 @@ static __device__ __forceinline__ float2 gather_node_comp(const Dev &d, int n, f
     return make_float2(sr + m * gR, sz + m * gZ);
 }
 
+// The last addition of a gather, s + m g: s is never -0 (a sum that starts at +0 is not), so
+// adding the +-0 that a zero g gives with a finite mass changes nothing.
+template <bool INT>
+static __device__ __forceinline__ double add_weight(double s, double m, double g) {
+    const bool finite = (__double2hiint(m) & 0x7ff00000) != 0x7ff00000;
+    if (!is_zero(g) || !finite) s += Product<INT>::of(m, g);
+    return s;
+}
+// 0 + x: x, but +0 for -0.
+static __device__ __forceinline__ double first_term(double x) {
+    return is_zero(x) ? 0.0 : x;
+}
+
 // gather, ExplicitSolver.java:1147-1165: node n's sources in ascending order, then m g.
-// Four slots at a time: their indices, then their values, are loaded before any is added, so
-// the loads overlap; the sums still take the slots in order.
+// The first slot, then three at a time (an interior node has four): their indices, then their
+// values, are loaded before any is added, so the loads overlap; the sums still take the slots in
+// order. The first sum, with 0, and the weight where there is no gravity are not formed: six FP64
+// additions an interior node instead of ten and two products.
+template <bool INT>
 static __device__ __forceinline__ double2 gather_node(const Dev &d, int n) {
     double sr = 0.0, sz = 0.0;
-    const int end = d.nodeSlotStart[n + 1];
+    const int begin = d.nodeSlotStart[n], end = d.nodeSlotStart[n + 1];
     const double m = d.mass[n];
-    for (int k = d.nodeSlotStart[n]; k < end; k += 4) {
-        const int cnt = end - k < 4 ? end - k : 4;
-        int slot[4];
-        double vr[4], vz[4];
+    if (begin < end) {
+        const int slot = d.nodeSlot[begin];
+        sr = first_term(d.contribution[slot]);
+        sz = first_term(d.contribution[slot + 4]);
+    }
+    for (int k = begin + 1; k < end; k += 3) {
+        const int cnt = end - k < 3 ? end - k : 3;
+        int slot[3];
+        double vr[3], vz[3];
 #pragma unroll
-        for (int j = 0; j < 4; j++) slot[j] = j < cnt ? d.nodeSlot[k + j] : 0;
+        for (int j = 0; j < 3; j++) slot[j] = j < cnt ? d.nodeSlot[k + j] : 0;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
+        for (int j = 0; j < 3; j++) {
             vr[j] = j < cnt ? d.contribution[slot[j]] : 0.0;
             vz[j] = j < cnt ? d.contribution[slot[j] + 4] : 0.0;
         }
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
+        for (int j = 0; j < 3; j++) {
             if (j < cnt) {
                 sr += vr[j];
                 sz += vz[j];
             }
         }
     }
-    return make_double2(sr + m * d.gravR, sz + m * d.gravZ);
+    return make_double2(add_weight<INT>(sr, m, d.gravR), add_weight<INT>(sz, m, d.gravZ));
 }
 
-// The same gather of float contributions into FP64 sums (the mixed form), four slots at a
-// time like gather_node. Each float is widened to double by integer arithmetic (exact, the
-// value the conversion gives): only the sums use the FP64 pipe.
+// The warp's smallest non-negative bit pattern into *best by the integer minimum of its halves
+// (all 32 lanes call it). One address takes every warp's minimum, and most do not lower it any
+// more, so a warp looks before it adds its atomic to the queue there.
+__device__ __forceinline__ void commit_min_bits(unsigned long long bits, unsigned long long *best) {
+    const unsigned hi = (unsigned)(bits >> 32);
+    const unsigned h = __reduce_min_sync(0xffffffffu, hi);
+    const unsigned l = __reduce_min_sync(0xffffffffu, hi == h ? (unsigned)bits : 0xffffffffu);
+    const unsigned long long m = ((unsigned long long)h << 32) | l;
+    if ((threadIdx.x & 31) == 0 && m < __ldcg(best)) atomicMin(best, m);
+}
+
+// The same gather of float contributions into FP64 sums (the mixed form). Each float is widened
+// to double by integer arithmetic (exact, the value the conversion gives): only the sums use the
+// FP64 pipe. 200k elements: 10.5 us in a profile, waiting for the contributions' loads.
+template <bool INT>
 static __device__ __forceinline__ double2 gather_node_f32(const Dev &d, int n) {
     double sr = 0.0, sz = 0.0;
-    const int end = d.nodeSlotStart[n + 1];
+    const int begin = d.nodeSlotStart[n], end = d.nodeSlotStart[n + 1];
     const double m = d.mass[n];
-    for (int k = d.nodeSlotStart[n]; k < end; k += 4) {
-        const int cnt = end - k < 4 ? end - k : 4;
-        int slot[4];
-        float vr[4], vz[4];
+    if (begin < end) {
+        const int slot = d.nodeSlot[begin];
+        sr = first_term(nf_widen(d.contribF[slot]));
+        sz = first_term(nf_widen(d.contribF[slot + 4]));
+    }
+    for (int k = begin + 1; k < end; k += 3) {
+        const int cnt = end - k < 3 ? end - k : 3;
+        int slot[3];
+        float vr[3], vz[3];
 #pragma unroll
-        for (int j = 0; j < 4; j++) slot[j] = j < cnt ? d.nodeSlot[k + j] : 0;
+        for (int j = 0; j < 3; j++) slot[j] = j < cnt ? d.nodeSlot[k + j] : 0;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
+        for (int j = 0; j < 3; j++) {
             vr[j] = j < cnt ? d.contribF[slot[j]] : 0.0f;
             vz[j] = j < cnt ? d.contribF[slot[j] + 4] : 0.0f;
         }
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
+        for (int j = 0; j < 3; j++) {
             if (j < cnt) {
                 sr += nf_widen(vr[j]);
                 sz += nf_widen(vz[j]);
             }
         }
     }
-    return make_double2(sr + m * d.gravR, sz + m * d.gravZ);
+    return make_double2(add_weight<INT>(sr, m, d.gravR), add_weight<INT>(sz, m, d.gravZ));
 }
 
 }  // namespace nf

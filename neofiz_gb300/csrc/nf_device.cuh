@@ -155,6 +155,17 @@ __device__ __forceinline__ bool is_zero(double x) {
 }
 __device__ __forceinline__ bool is_zero(float x) { return x == 0.0f; }
 
+// a < b off the FP64 pipe: bit patterns order as their values do once negative ones are
+// mirrored, a zero's sign aside; false for a NaN.
+__device__ __forceinline__ bool less_bits(double a, double b) {
+    long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    const bool number = (unsigned long long)(x << 1) <= 0xffe0000000000000ULL &&
+                        (unsigned long long)(y << 1) <= 0xffe0000000000000ULL;
+    x = x < 0 ? (long long)(0x8000000000000000ULL - (unsigned long long)x) : x;   // -0 is 0
+    y = y < 0 ? (long long)(0x8000000000000000ULL - (unsigned long long)y) : y;
+    return number && x < y;
+}
+
 template <typename T>
 __device__ __forceinline__ T jc_thermalTerm(const MatT<T> &f, T temperature) {
     const T above = temperature - f.room, span = f.melt - f.room;

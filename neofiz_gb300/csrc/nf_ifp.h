@@ -265,8 +265,32 @@ NF_IFP double nf_scale_try(double x, int k, uint32_t *bad) {
 /* x 2^k, |k| <= 8, by the machine's product outside nf_scale_try's range. */
 NF_IFP double nf_scale2(double x, int k) {
     uint32_t bad = 0;
-    const double r = nf_scale_try(x, k, &bad);
-    return bad ? x * nf_ifp_make((uint32_t)(1023 + k) << 20, 0u) : r;
+    double r = nf_scale_try(x, k, &bad);
+    if (bad) {
+        const double f = nf_ifp_make((uint32_t)(1023 + k) << 20, 0u);
+#if defined(__CUDA_ARCH__)
+        asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(x), "d"(f));
+#else
+        r = x * f;
+#endif
+    }
+    return r;
+}
+
+/* a b. */
+NF_IFP double nf_mul(double a, double b) {
+    uint32_t bad = 0;
+    double r = nf_mul_try(a, b, &bad);
+    if (bad) {
+#if defined(__CUDA_ARCH__)
+        /* volatile: a branch around the instruction, which the compiler would otherwise issue
+         * for every product and select from */
+        asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+#else
+        r = a * b;
+#endif
+    }
+    return r;
 }
 
 /* a / b (nf_div_try) with the same convention. */

@@ -446,14 +446,14 @@ int listed_pass_smem(int device);
 size_t scan_tmp_ints(int n);
 
 int grid_for(long long n, int block);
-// Whether `warps` warps of elements give the quarter SMs more than one each at a time, where the
-// element's products go to the integer units (element_reduced): on a 200k-quad scene 143 us a
+// Whether `warps` warps of elements or nodes give the quarter SMs more than one each at a time,
+// where their products go to the integer units (element_reduced, nodal_node): on a 200k-quad scene 143 us a
 // pass against 163 without, on 16-element batch instances alone on their quarter SM 99 us a step
 // against 74.
 inline bool int_products(long long warps, int sms) { return warps > 4LL * sms; }
 // Fixed grids of the node and element kernels that reduce per block, striding over the items.
-// The nodal update takes one node per thread up to sixteen blocks per SM (every block resident
-// at once, no second pass over the nodes); the element kernels stop at eight.
+// The nodal update takes one node per thread up to sixteen blocks per SM (two rounds of the
+// eight that fit); the element kernels stop at eight.
 inline int nodal_grid(const Solver &S) {
     const int g = grid_for(S.d.N, 128), cap = 16 * S.d.sms;
     return g < cap ? g : cap;
