@@ -12,6 +12,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <utility>
 
 using namespace nf;
@@ -56,22 +57,21 @@ cudaError_t dalloc(Solver &S, T **p, size_t count) {
     return e;
 }
 
-// The set-up arrays of nf_create carved from one allocation: one cudaMalloc and one memset
-// instead of one each per array (the allocations dominated creating a 200k-element scene).
+// Set-up arrays carved from one allocation: one cudaMalloc and one memset instead of one each
+// per array (the allocations dominated creating a 200k-element scene).
 struct Arena {
     std::vector<std::pair<void **, size_t>> items;
     template <typename T>
     void add(T **p, size_t count) {
         items.push_back({reinterpret_cast<void **>(p), sizeof(T) * (count ? count : 1)});
     }
-    cudaError_t commit(Solver &S) {
+    cudaError_t commit(Solver &S, Solver::Block &block) {
         size_t total = 0;
         for (auto &it : items) total += (it.second + 255) & ~(size_t)255;
         void *base = nullptr;
         cudaError_t e = cudaMalloc(&base, total);
         if (e != cudaSuccess) return e;
-        S.arena = base;
-        S.arenaBytes = total;
+        block = {base, total};
         char *p = static_cast<char *>(base);
         for (auto &it : items) {
             *it.first = p;
@@ -344,11 +344,20 @@ nf_status nf_create(const nf_mesh *mesh, const nf_material *materials, int32_t m
         for (int e = 0; e < E; e++)
             if (element_material[e] < 0 || element_material[e] >= material_count)
                 return fail(nullptr, NF_EINVAL, "element %d has no material", e);
-    for (int e = 0; e < E; e++)                                    // QuadMesh.java:228-237
-        if (signed_area(mesh->r, mesh->z, mesh->conn, e) <= 0.0)
+    int noArea = E;                                                // the first without (NaN)
+    double noAreaValue = 0.0;
+    for (int e = 0; e < E; e++) {                                  // QuadMesh.java:228-237
+        const double area = signed_area(mesh->r, mesh->z, mesh->conn, e);
+        if (area > 0.0) continue;
+        if (noArea == E) {
+            noArea = e;
+            noAreaValue = fabs(area);
+        }
+        if (area <= 0.0)
             return fail(nullptr, NF_ESTATE,
                         "element %d has non-positive area; node ordering must be "
                         "counter-clockwise in (r, z)", e);
+    }
     int dev_count = 0;
     if (cudaGetDeviceCount(&dev_count) != cudaSuccess || dev_count < 1)
         return fail(nullptr, NF_EDEVICE, "no CUDA device is visible");
@@ -365,15 +374,13 @@ nf_status nf_create(const nf_mesh *mesh, const nf_material *materials, int32_t m
         S->d.coopBlocks = contact_coop_blocks(S->d.sms);
     }
     S->N = N; S->E = E; S->K = K;
+    S->noArea = noArea;
+    S->noAreaValue = noAreaValue;
     S->formulation = formulation; S->integration = integration; S->kinematics = kinematics;
     S->ppe = integration == NF_FULL ? 4 : 1;
     S->materials.assign(materials, materials + material_count);
     S->emat.assign(E, 0);
     if (element_material) std::copy(element_material, element_material + E, S->emat.begin());
-    S->hostR.assign(mesh->r, mesh->r + N);
-    S->hostZ.assign(mesh->z, mesh->z + N);
-    S->hostConn.assign(mesh->conn, mesh->conn + 4LL * E);
-
     d.N = N; d.E = E; d.K = K; d.ppe = S->ppe;
     d.axi = formulation == NF_AXISYMMETRIC;
     d.finite = kinematics == NF_FINITE_STRAIN;
@@ -393,81 +400,15 @@ nf_status nf_create(const nf_mesh *mesh, const nf_material *materials, int32_t m
     if (!element_material || material_count == 1) {
         d.fastestWave = mat_wave(materials[0]);
     } else {
+        std::vector<double> waves(material_count);
+        for (int m = 0; m < material_count; m++) waves[m] = mat_wave(materials[m]);
         double fastest = 0.0;
-        for (int e = 0; e < E; e++) {
-            const double c = mat_wave(materials[S->emat[e]]);
-            if (c > fastest) fastest = c;
-        }
+        for (int e = 0; e < E; e++) fastest = std::max(fastest, waves[element_material[e]]);
         d.fastestWave = fastest;
     }
 
-    // lumped mass, ExplicitSolver.java:1559-1597
-    std::vector<double> mass(N, 0.0);
-    lumped_mass(mesh->r, mesh->z, mesh->conn, E, materials, S->emat.data(), d.axi != 0, thickness,
-                mass.data());
-
-    // node slots, ExplicitSolver.java:347-366
-    std::vector<int32_t> slotStart(N + 1, 0), slots(4LL * E + 2LL * K);
-    node_slots(mesh->conn, N, E, mesh->pressure_edges, K, slotStart.data(), slots.data());
-
-    // initial step, QuadMesh.minimumEdgeLength + ExplicitSolver.java:333-338
-    const double edge = min_edge_length(mesh->r, mesh->z, mesh->conn, E);
-    DevScalars s0{};
-    s0.minEdgeSquared = edge * edge;
-    s0.dt = cfl_safety * edge / d.fastestWave;
-    s0.dtPrevious = s0.dt;
-    s0.minEdgeBits = 0x7fefffffffffffffULL;   // Double.MAX_VALUE
-    s0.tEnd = INFINITY;
-    d.dt0 = s0.dt;
-
-    // edge groups for the free surface: element-edges with the same undirected node pair, in
-    // (lower node, higher node, element-edge) order -- a counting sort by the lower node (stable
-    // in element-edge order) and an insertion sort by the higher node within each node's few
-    // edges, linear in the mesh where a comparison sort of the 4E keys is not
-    std::vector<std::pair<long long, int>> keys(4LL * E);
-    {
-        std::vector<int32_t> start(N + 1, 0);
-        for (long long q = 0; q < 4LL * E; q++) {
-            const int a = mesh->conn[q], b = mesh->conn[(q & ~3LL) + ((q + 1) & 3)];
-            start[std::min(a, b) + 1]++;
-        }
-        for (int i = 0; i < N; i++) start[i + 1] += start[i];
-        std::vector<int32_t> cursor(start.begin(), start.end() - 1);
-        for (long long q = 0; q < 4LL * E; q++) {
-            const int a = mesh->conn[q], b = mesh->conn[(q & ~3LL) + ((q + 1) & 3)];
-            const long long lo = std::min(a, b), hi = std::max(a, b);
-            keys[cursor[lo]++] = std::make_pair((lo << 32) | hi, (int)q);
-        }
-        for (int i = 0; i < N; i++)
-            for (int j = start[i] + 1; j < start[i + 1]; j++)
-                for (int m = j; m > start[i] && keys[m] < keys[m - 1]; m--)
-                    std::swap(keys[m], keys[m - 1]);
-    }
-    std::vector<int32_t> edgeGroup(4LL * E), groupStart, groupMember(4LL * E);
-    for (size_t i = 0; i < keys.size();) {
-        size_t j = i;
-        const int g = (int)groupStart.size();
-        groupStart.push_back((int)i);
-        while (j < keys.size() && keys[j].first == keys[i].first) {
-            edgeGroup[keys[j].second] = g;
-            groupMember[j] = keys[j].second;
-            j++;
-        }
-        i = j;
-    }
-    groupStart.push_back((int)keys.size());
-
     // device allocations
     const size_t P = (size_t)E * S->ppe;
-    std::vector<double2> X0(N), zero2(N);
-    for (int i = 0; i < N; i++) X0[i] = make_double2(mesh->r[i], mesh->z[i]);
-    std::vector<int4> conn4(E);
-    for (int e = 0; e < E; e++)
-        conn4[e] = make_int4(mesh->conn[4 * e], mesh->conn[4 * e + 1], mesh->conn[4 * e + 2],
-                             mesh->conn[4 * e + 3]);
-    std::vector<int2> pe(K);
-    for (int k = 0; k < K; k++)
-        pe[k] = make_int2(mesh->pressure_edges[2 * k], mesh->pressure_edges[2 * k + 1]);
     // the Johnson-Cook work list of the FP64 one-point element pass
     bool anyJC = false;
     for (int m = 0; m < material_count; m++) anyJC = anyJC || mats[m].jc != 0;
@@ -491,7 +432,10 @@ nf_status nf_create(const nf_mesh *mesh, const nf_material *materials, int32_t m
     A(d.nodeSlotStart, N + 1); A(d.nodeSlot, 4LL * E + 2LL * K);
     A(d.pedges, K);
     A(d.partials, (size_t)PARTIAL_SLOTS * d.maxBlocks);
-    A(d.edgeGroup, 4LL * E); A(d.groupStart, groupStart.size()); A(d.groupMember, 4LL * E);
+    A(d.edgeGroup, 4LL * E); A(d.groupStart, 4LL * E + 1); A(d.groupMember, 4LL * E);
+    A(S->stage, std::max(N, E));
+    int32_t *scratch = nullptr;
+    A(scratch, setup_scratch_ints(N, E));
     A(d.s, 1);
     if (listed) {
         d.hotSmem = listed_pass_smem(S->device);
@@ -499,26 +443,44 @@ nf_status nf_create(const nf_mesh *mesh, const nf_material *materials, int32_t m
         A(d.jcYield, E);
     }
 #undef A
-    const cudaError_t e_ = arena.commit(*S);
+    const cudaError_t e_ = arena.commit(*S, S->arena);
     if (e_ != cudaSuccess) {
         nf_status st = fail(nullptr, NF_ENOMEM, "device allocation failed: %s", cudaGetErrorString(e_));
         nf_destroy(reinterpret_cast<nf_solver *>(S));
         return st;
     }
-    upload(*S, d.X0, X0.data(), N);
-    upload(*S, d.mass, mass.data(), N);
-    std::vector<double> invMass(N);
-    for (int i = 0; i < N; i++) invMass[i] = 1.0 / mass[i];     // nodalUpdate's 1/m, once
-    upload(*S, d.invMass, invMass.data(), N);
-    upload(*S, d.conn, conn4.data(), E);
-    upload(*S, d.emat, S->emat.data(), E);
+    double *rz = reinterpret_cast<double *>(d.U);               // see launch_setup
+    upload(*S, rz, mesh->r, N);
+    upload(*S, rz + N, mesh->z, N);
+    upload(*S, reinterpret_cast<int32_t *>(d.conn), mesh->conn, 4LL * E);
+    if (element_material) upload(*S, d.emat, element_material, E);
     upload(*S, d.mats, mats.data(), material_count);
-    upload(*S, d.nodeSlotStart, slotStart.data(), N + 1);
-    upload(*S, d.nodeSlot, slots.data(), slots.size());
-    upload(*S, d.pedges, pe.data(), K);
-    upload(*S, d.edgeGroup, edgeGroup.data(), edgeGroup.size());
-    upload(*S, d.groupStart, groupStart.data(), groupStart.size());
-    upload(*S, d.groupMember, groupMember.data(), groupMember.size());
+    upload(*S, reinterpret_cast<int32_t *>(d.pedges), mesh->pressure_edges, 2LL * K);
+    DevScalars s0{};
+    s0.minEdgeBits = 0x7ff0000000000000ULL;   // none yet
+    upload(*S, d.s, &s0, 1);
+    const int *most = launch_setup(*S, scratch);
+    CK(nullptr, cudaMemcpyAsync(&S->maxCorners, most, sizeof(int), cudaMemcpyDeviceToHost, S->stream));
+    nf_status st = read_scalars(*S, &s0);
+    if (st) {
+        g_err = S->err;
+        nf_destroy(reinterpret_cast<nf_solver *>(S));
+        return st;
+    }
+
+    // initial step, QuadMesh.minimumEdgeLength + ExplicitSolver.java:333-338: the root of the
+    // least square is the least root
+    double edge = DBL_MAX;
+    if (s0.minEdgeBits < 0x7ff0000000000000ULL) {
+        memcpy(&edge, &s0.minEdgeBits, sizeof edge);
+        edge = sqrt(edge);
+    }
+    s0.minEdgeSquared = edge * edge;
+    s0.dt = cfl_safety * edge / d.fastestWave;
+    s0.dtPrevious = s0.dt;
+    s0.minEdgeBits = 0x7fefffffffffffffULL;   // Double.MAX_VALUE
+    s0.tEnd = INFINITY;
+    d.dt0 = s0.dt;
     upload(*S, d.s, &s0, 1);
     if (d.hot) {
         HotList h0{};                          // listing stamps start at 0: nothing listed
@@ -528,7 +490,7 @@ nf_status nf_create(const nf_mesh *mesh, const nf_material *materials, int32_t m
     if (d.jcYield) launch_jc_yield(d, S->stream);
     d.scanTmpSize = (int)scanInts;
     d.scanTmp = nullptr;
-    nf_status st = sync_check(*S);
+    st = sync_check(*S);
     if (st) {
         g_err = S->err;
         nf_destroy(reinterpret_cast<nf_solver *>(S));
@@ -565,12 +527,10 @@ nf_status nf_destroy(nf_solver *h) {
                     d.fastCount, d.fastEntry, d.fastF, d.fastFL, d.fastAB, d.fastA, d.fastN,
                     d.fastL, d.nodeCell,
                     d.hot, d.hotList, d.hotNext, d.hotStamp, d.jcYield};
-    const char *a0 = static_cast<const char *>(S->arena), *a1 = a0 + S->arenaBytes;
-    for (void *p : ptrs) {
-        const char *c = static_cast<const char *>(p);
-        if (p && !(S->arena && c >= a0 && c < a1)) cudaFree(p);      // arena arrays go below
-    }
-    if (S->arena) cudaFree(S->arena);
+    for (void *p : ptrs)                     // the arenas' arrays go with them
+        if (p && !S->arena.holds(p) && !S->contactArena.holds(p)) cudaFree(p);
+    if (S->arena.base) cudaFree(S->arena.base);
+    if (S->contactArena.base) cudaFree(S->contactArena.base);
     if (S->ownStream) cudaStreamDestroy(S->ownStream);
     delete S;
     return NF_OK;
@@ -719,13 +679,10 @@ nf_status nf_set_contact(nf_solver *h, double friction, double damping, double s
     Dev &d = S.d;
     const int N = S.N, E = S.E;
     // a node's free edges are at most two per element around it
-    std::vector<int32_t> valence(N, 0);
-    for (long long k = 0; k < 4LL * E; k++) valence[S.hostConn[k]]++;
-    int segCap = 2;
-    for (int n = 0; n < N; n++) segCap = std::max(segCap, 2 * valence[n]);
+    const int segCap = std::max(2, 2 * S.maxCorners);
     if (!d.dead) {
-        cudaError_t e_ = cudaSuccess;
-#define A(ptr, n) if (e_ == cudaSuccess) e_ = dalloc(S, &(ptr), (n))
+        Arena arena;
+#define A(ptr, n) arena.add(&(ptr), (n))
         A(d.dead, E);
         A(d.surfFlag, 4LL * E);
         A(d.segA, 4LL * E); A(d.segB, 4LL * E);
@@ -760,20 +717,11 @@ nf_status nf_set_contact(nf_solver *h, double friction, double damping, double s
         A(d.scanTmp, (size_t)d.scanTmpSize);
         A(d.coopSums, (size_t)d.coopBlocks);
 #undef A
+        const cudaError_t e_ = arena.commit(S, S.contactArena);
         if (e_ != cudaSuccess)
             return fail(&S, NF_ENOMEM, "contact allocation failed: %s", cudaGetErrorString(e_));
         d.segCap = segCap;
-        // the end nodes of every element edge (QuadMesh.surface's edge k of element e runs
-        // from corner k to corner k + 1)
-        std::vector<int32_t> a(4LL * E), b(4LL * E);
-        for (long long q = 0; q < 4LL * E; q++) {
-            a[q] = S.hostConn[q];
-            b[q] = S.hostConn[(q & ~3LL) + ((q + 1) & 3)];
-        }
-        CK(&S, upload(S, d.segA, a.data(), a.size()));
-        CK(&S, upload(S, d.segB, b.data(), b.size()));
-        const nf_status up = sync_check(S);             // a and b are about to go
-        if (up) return up;
+        launch_segments(S);
     } else {
         CK(&S, cudaMemsetAsync(d.dead, 0, E, S.stream));
     }
@@ -858,32 +806,23 @@ nf_status nf_set_damage(nf_solver *h, const double *gf, const double *eps) {
                         "2mu + (2/3)(H_kin - E) = %.17g <= 0", worst);
     }
     const int E = S.E, ppe = S.ppe;
-    std::vector<double> geom(5LL * E);
-    for (int e = 0; e < E; e++) {                              // ExplicitSolver.java:767-789
-        const int b = e * 4;
-        const double *r = S.hostR.data(), *z = S.hostZ.data();
-        const int32_t *c = S.hostConn.data();
-        const int n0 = c[b], n1 = c[b + 1], n2 = c[b + 2], n3 = c[b + 3];
-        geom[5 * e + 1] = 0.5 * (r[n1] - r[n0] + r[n2] - r[n3]);
-        geom[5 * e + 2] = 0.5 * (z[n1] - z[n0] + z[n2] - z[n3]);
-        geom[5 * e + 3] = 0.5 * (r[n3] - r[n0] + r[n2] - r[n1]);
-        geom[5 * e + 4] = 0.5 * (z[n3] - z[n0] + z[n2] - z[n1]);
-        geom[5 * e] = fabs(signed_area(r, z, c, e));
-    }
-    for (int e = 0; e < E; e++)                                // Damage.java:232-243
-        for (int g = 0; g < ppe; g++) {
+    bool clean = S.noArea == E;
+    for (const nf_material &m : S.materials) clean = clean && m.youngs_modulus > 0.0;
+    for (int e = 0; e < E && clean; e++) clean = gf[e] > 0.0 && eps[e] > 0.0;
+    if (!clean) {                                              // which, in the reference's order
+        for (int e = 0; e < E; e++) {                          // Damage.java:232-243
             if (!(gf[e] > 0.0)) return fail(&S, NF_EINVAL, "fracture energy must be positive, was %.17g", gf[e]);
             const double youngs = S.materials[S.emat[e]].youngs_modulus;
             if (!(youngs > 0.0)) return fail(&S, NF_EINVAL, "Young's modulus must be positive, was %.17g", youngs);
         }
-    for (int e = 0; e < E; e++)                                // Damage.java:249-260
-        for (int g = 0; g < ppe; g++) {
-            const int p = e * ppe + g;
+        for (int e = 0; e < E; e++) {                          // Damage.java:249-260
+            const int p = e * ppe;
             if (!(eps[e] > 0.0))
                 return fail(&S, NF_EINVAL, "failure strain must be positive; point %d has %.17g", p, eps[e]);
-            if (!(geom[5 * e] > 0.0))
-                return fail(&S, NF_EINVAL, "area must be positive; point %d has %.17g", p, geom[5 * e]);
+            if (e == S.noArea)
+                return fail(&S, NF_EINVAL, "area must be positive; point %d has %.17g", p, S.noAreaValue);
         }
+    }
     Dev &d = S.d;
     const size_t P = (size_t)E * ppe;
     if (!d.dFail) {
@@ -901,7 +840,7 @@ nf_status nf_set_damage(nf_solver *h, const double *gf, const double *eps) {
     }
     CK(&S, upload(S, d.dFail, eps, E));
     CK(&S, upload(S, d.dGf, gf, E));
-    CK(&S, upload(S, d.dGeom, geom.data(), geom.size()));
+    launch_damage_geometry(S);
     d.hasDamage = 1;
     S.damageSet = true;
     if (d.mixed) {
@@ -1180,16 +1119,16 @@ nf_status nf_read_field(nf_solver *h, int32_t field, void *dst, size_t nbytes) {
     mixed_to_double(S);
     st = sync_check(S);
     if (st) return st;
-    auto pair = [&](const double2 *src, int comp) -> nf_status {
-        std::vector<double2> tmp(count);
-        CK(&S, cudaMemcpy(tmp.data(), src, sizeof(double2) * count, cudaMemcpyDeviceToHost));
-        double *o = (double *)dst;
-        for (size_t i = 0; i < count; i++) o[i] = comp ? tmp[i].y : tmp[i].x;
-        return NF_OK;
-    };
     auto copy = [&](const void *src) -> nf_status {
-        CK(&S, cudaMemcpy(dst, src, nbytes, cudaMemcpyDeviceToHost));
-        return NF_OK;
+        // the destination's pages first: a copy of 32 MB into pages not mapped yet took 13.6 ms
+        // (the device faults them in one by one), with them touched it takes 1.3 ms
+        for (size_t i = 0; i < nbytes; i += 4096) ((volatile char *)dst)[i] = 0;
+        CK(&S, cudaMemcpyAsync(dst, src, nbytes, cudaMemcpyDeviceToHost, S.stream));
+        return sync_check(S);
+    };
+    auto pair = [&](const double2 *src, int comp) -> nf_status {
+        launch_component(S, src, S.stage, count, comp);
+        return copy(S.stage);
     };
     switch (field) {
         case NF_FIELD_UR: return pair(d.U, 0);
@@ -1250,14 +1189,15 @@ nf_status nf_read_field(nf_solver *h, int32_t field, void *dst, size_t nbytes) {
             return NF_OK;
         }
         case NF_FIELD_SURFACE_EDGES: {              // the free edges in element order
-            std::vector<int32_t> flag(4LL * S.E);
+            std::vector<int32_t> flag(4LL * S.E), conn(flag.size());
             CK(&S, cudaMemcpy(flag.data(), d.surfFlag, 4 * flag.size(), cudaMemcpyDeviceToHost));
+            CK(&S, cudaMemcpy(conn.data(), d.conn, 4 * conn.size(), cudaMemcpyDeviceToHost));
             int32_t *o = (int32_t *)dst;
             size_t k = 0;
             for (size_t q = 0; q < flag.size() && k + 1 < count + 1; q++) {
                 if (!flag[q]) continue;
-                o[k++] = S.hostConn[q];
-                o[k++] = S.hostConn[(q & ~(size_t)3) + ((q + 1) & 3)];
+                o[k++] = conn[q];
+                o[k++] = conn[(q & ~(size_t)3) + ((q + 1) & 3)];
             }
             return NF_OK;
         }

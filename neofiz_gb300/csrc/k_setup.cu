@@ -1,0 +1,281 @@
+// k_setup.cu -- the arrays a scene derives from its mesh: node positions, shortest edge, the
+// sources of every node, the edge groups of the free surface, lumped masses, the damage model's
+// element geometry and the surface's edge ends. Every value is the host expression's (no
+// contraction, sums in the same order), so the results are those of the serial loops.
+//
+// One core took 64 ms over these for 1M quads, half as long as the 400 steps that followed;
+// here they are 1 ms of kernels (each a pass or two over the mesh, bound by its gathers) behind
+// the upload of the mesh. Below about a thousand elements the launches cost what the host loops
+// did (50 us). The orderings are counting sorts: an entry's place in its node's list is the
+// number of smaller entries there, which each entry counts for itself, so no list is walked by
+// one thread alone whatever the mesh's valences.
+#include "nf_bodies.cuh"
+#include "nf_internal.h"
+
+namespace nf {
+
+constexpr int SB = 256;
+
+__device__ __forceinline__ int conn_at(const Dev &d, long long q) {
+    return reinterpret_cast<const int *>(d.conn)[q];
+}
+__device__ __forceinline__ int edge_end(const Dev &d, long long q) {
+    return conn_at(d, (q & ~3LL) + ((q + 1) & 3));
+}
+
+__global__ void __launch_bounds__(SB) k_positions(Dev d, const double *r, const double *z) {
+    const int n = blockIdx.x * SB + threadIdx.x;
+    if (n < d.N) d.X0[n] = make_double2(r[n], z[n]);
+}
+
+// QuadMesh.minimumEdgeLength squared, as bits (a NaN is passed over).
+__global__ void __launch_bounds__(SB) k_shortest_edge(Dev d) {
+    const int e = blockIdx.x * SB + threadIdx.x;
+    unsigned long long best = 0x7ff0000000000000ULL;
+    if (e < d.E) {
+        const int4 c = d.conn[e];
+        const int nn[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const double2 a = d.X0[nn[k]], b = d.X0[nn[(k + 1) & 3]];
+            const double dr = b.x - a.x, dz = b.y - a.y;
+            const unsigned long long q = __double_as_longlong(dr * dr + dz * dz);
+            best = q < best ? q : best;
+        }
+    }
+    commit_min_bits(best, &d.s->minEdgeBits);
+}
+
+// The sources of every node: element corner q (slot 8 e + corner), pressure-edge end k.
+__device__ __forceinline__ int source_node(const Dev &d, long long q) {
+    const long long n4 = 4LL * d.E;
+    return q < n4 ? conn_at(d, q) : reinterpret_cast<const int *>(d.pedges)[q - n4];
+}
+__device__ __forceinline__ int source_slot(const Dev &d, long long q) {
+    const long long n4 = 4LL * d.E;
+    if (q < n4) return (int)((q >> 2) * 8 + (q & 3));
+    const long long k = q - n4;
+    return (int)((d.E + (k >> 1)) * 8 + (k & 1));
+}
+
+__global__ void __launch_bounds__(SB) k_count(Dev d, int *sources, int *edges) {
+    const long long q = (long long)blockIdx.x * SB + threadIdx.x;
+    if (q >= 4LL * d.E + 2LL * d.K) return;
+    atomicAdd(&sources[source_node(d, q)], 1);
+    if (q < 4LL * d.E) atomicAdd(&edges[min(conn_at(d, q), edge_end(d, q))], 1);
+}
+// The most elements around a node (its corners, counted once each).
+__global__ void __launch_bounds__(SB) k_corners(Dev d, int *corners) {
+    const long long q = (long long)blockIdx.x * SB + threadIdx.x;
+    if (q < 4LL * d.E) atomicAdd(&corners[conn_at(d, q)], 1);
+}
+__global__ void __launch_bounds__(SB) k_most(int n, const int *corners, int *most) {
+    const int i = blockIdx.x * SB + threadIdx.x;
+    const int m = __reduce_max_sync(0xffffffffu, i < n ? corners[i] : 0);
+    if ((threadIdx.x & 31) == 0 && m > __ldcg(most)) atomicMax(most, m);
+}
+// Into the nodes' ranges in any order; the counts run down to zero.
+__global__ void __launch_bounds__(SB) k_file(Dev d, int *sources, int *edges, const int *edgeStart,
+                                             int *sourceBin, int *edgeBin) {
+    const long long q = (long long)blockIdx.x * SB + threadIdx.x;
+    if (q >= 4LL * d.E + 2LL * d.K) return;
+    const int n = source_node(d, q);
+    sourceBin[d.nodeSlotStart[n] + atomicSub(&sources[n], 1) - 1] = source_slot(d, q);
+    if (q < 4LL * d.E) {
+        const int lo = min(conn_at(d, q), edge_end(d, q));
+        edgeBin[edgeStart[lo] + atomicSub(&edges[lo], 1) - 1] = (int)q;
+    }
+}
+// buildNodeSlots (ExplicitSolver.java:347-366): a node's sources ascending; and the edges of one
+// lower node by higher node, then by element edge.
+__global__ void __launch_bounds__(SB) k_rank(Dev d, const int *edgeStart, const int *sourceBin,
+                                             const int *edgeBin) {
+    const long long q = (long long)blockIdx.x * SB + threadIdx.x;
+    if (q >= 4LL * d.E + 2LL * d.K) return;
+    {
+        const int n = source_node(d, q), slot = source_slot(d, q);
+        const int begin = d.nodeSlotStart[n], end = d.nodeSlotStart[n + 1];
+        int rank = 0;
+        for (int j = begin; j < end; j++) rank += sourceBin[j] < slot;
+        d.nodeSlot[begin + rank] = slot;
+    }
+    if (q < 4LL * d.E) {
+        const int a = conn_at(d, q), b = edge_end(d, q);
+        const int lo = min(a, b), hi = max(a, b);
+        const int begin = edgeStart[lo], end = edgeStart[lo + 1];
+        int rank = 0;
+        for (int j = begin; j < end; j++) {
+            const int p = edgeBin[j], h = max(conn_at(d, p), edge_end(d, p));
+            rank += h < hi || (h == hi && p < (int)q);
+        }
+        d.groupMember[begin + rank] = (int)q;
+    }
+}
+// Equal undirected node pairs are neighbours now: a group starts where the pair changes.
+__global__ void __launch_bounds__(SB) k_heads(Dev d, int *head) {
+    const long long i = (long long)blockIdx.x * SB + threadIdx.x;
+    if (i >= 4LL * d.E) return;
+    int first = 1;
+    if (i > 0) {
+        const int q = d.groupMember[i], p = d.groupMember[i - 1];
+        const int a = conn_at(d, q), b = edge_end(d, q), f = conn_at(d, p), g = edge_end(d, p);
+        first = min(a, b) != min(f, g) || max(a, b) != max(f, g);
+    }
+    head[i] = first;
+}
+__global__ void __launch_bounds__(SB) k_groups(Dev d, const int *head, const int *before) {
+    const long long i = (long long)blockIdx.x * SB + threadIdx.x;
+    if (i >= 4LL * d.E) return;
+    const int g = before[i] + head[i] - 1;
+    d.edgeGroup[d.groupMember[i]] = g;
+    if (head[i]) d.groupStart[g] = (int)i;
+    if (i == 4LL * d.E - 1) d.groupStart[g + 1] = 4 * d.E;
+}
+
+// lumpMass, ExplicitSolver.java:1559-1597: 2x2 Gauss lumping. The four points' volumes by
+// element, then each node adds its corners' shares: in element order, for each element point by
+// point, and where an element has the node at several corners, those in turn within the point.
+__global__ void __launch_bounds__(SB) k_lump_volumes(Dev d, double4 *volumes) {
+    const int e = blockIdx.x * SB + threadIdx.x;
+    if (e >= d.E) return;
+    const double G = 0.5773502691896258;
+    const double gx[4] = {-G, G, G, -G}, ge[4] = {-G, -G, G, G};
+    const int4 c = d.conn[e];
+    const double2 p0 = d.X0[c.x], p1 = d.X0[c.y], p2 = d.X0[c.z], p3 = d.X0[c.w];
+    double v[4];
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+        const double xi = gx[g], eta = ge[g];
+        const double xm = 1.0 - xi, xp = 1.0 + xi;
+        const double em = 1.0 - eta, ep = 1.0 + eta;
+        const double N0 = 0.25 * xm * em, N1 = 0.25 * xp * em;
+        const double N2 = 0.25 * xp * ep, N3 = 0.25 * xm * ep;
+        const double dN0x = -0.25 * em, dN1x = 0.25 * em, dN2x = 0.25 * ep, dN3x = -0.25 * ep;
+        const double dN0e = -0.25 * xm, dN1e = -0.25 * xp, dN2e = 0.25 * xp, dN3e = 0.25 * xm;
+        const double J00 = dN0x * p0.x + dN1x * p1.x + dN2x * p2.x + dN3x * p3.x;
+        const double J01 = dN0x * p0.y + dN1x * p1.y + dN2x * p2.y + dN3x * p3.y;
+        const double J10 = dN0e * p0.x + dN1e * p1.x + dN2e * p2.x + dN3e * p3.x;
+        const double J11 = dN0e * p0.y + dN1e * p1.y + dN2e * p2.y + dN3e * p3.y;
+        const double det = J00 * J11 - J01 * J10;
+        const double rg = N0 * p0.x + N1 * p1.x + N2 * p2.x + N3 * p3.x;
+        v[g] = d.axi ? 2.0 * NF_PI * rg * det : d.thickness * det;
+    }
+    volumes[e] = make_double4(v[0], v[1], v[2], v[3]);
+}
+__global__ void __launch_bounds__(SB) k_lump(Dev d, const double4 *volumes) {
+    const int n = blockIdx.x * SB + threadIdx.x;
+    if (n >= d.N) return;
+    const double G = 0.5773502691896258;
+    const double gx[4] = {-G, G, G, -G}, ge[4] = {-G, -G, G, G};
+    double m = 0.0;
+    const int end = d.nodeSlotStart[n + 1];
+    for (int k = d.nodeSlotStart[n]; k < end;) {
+        const int e = d.nodeSlot[k] >> 3;
+        if (e >= d.E) break;                              // pressure edges come last
+        int corners = 0;
+        for (; k < end && (d.nodeSlot[k] >> 3) == e; k++) corners |= 1 << (d.nodeSlot[k] & 7);
+        const double rho = d.mats[d.emat[e]].density;
+        const double4 v4 = volumes[e];
+        const double v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+            const double xm = 1.0 - gx[g], xp = 1.0 + gx[g];
+            const double em = 1.0 - ge[g], ep = 1.0 + ge[g];
+            const double shape[4] = {0.25 * xm * em, 0.25 * xp * em, 0.25 * xp * ep,
+                                     0.25 * xm * ep};
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                if (corners >> c & 1) m += rho * shape[c] * v[g];
+        }
+    }
+    d.mass[n] = m;
+    d.invMass[n] = 1.0 / m;                               // nodalUpdate's 1/m, once
+}
+
+// The damage model's element geometry, ExplicitSolver.java:767-789.
+__global__ void __launch_bounds__(SB) k_damage_geometry(Dev d) {
+    const int e = blockIdx.x * SB + threadIdx.x;
+    if (e >= d.E) return;
+    const int4 c = d.conn[e];
+    const double2 p[4] = {d.X0[c.x], d.X0[c.y], d.X0[c.z], d.X0[c.w]};
+    double a = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const double2 i = p[k], j = p[(k + 1) & 3];
+        a += i.x * j.y - j.x * i.y;
+    }
+    double *o = d.dGeom + 5 * (size_t)e;
+    o[0] = fabs(0.5 * a);
+    o[1] = 0.5 * (p[1].x - p[0].x + p[2].x - p[3].x);
+    o[2] = 0.5 * (p[1].y - p[0].y + p[2].y - p[3].y);
+    o[3] = 0.5 * (p[3].x - p[0].x + p[2].x - p[1].x);
+    o[4] = 0.5 * (p[3].y - p[0].y + p[2].y - p[1].y);
+}
+
+// The end nodes of every element edge (QuadMesh.surface's edge k of element e runs from corner
+// k to corner k + 1).
+__global__ void __launch_bounds__(SB) k_segments(Dev d) {
+    const long long q = (long long)blockIdx.x * SB + threadIdx.x;
+    if (q >= 4LL * d.E) return;
+    d.segA[q] = conn_at(d, q);
+    d.segB[q] = edge_end(d, q);
+}
+
+__global__ void __launch_bounds__(SB) k_component(const double2 *src, double *dst, int n, int y) {
+    const int i = blockIdx.x * SB + threadIdx.x;
+    if (i < n) dst[i] = y ? src[i].y : src[i].x;
+}
+
+size_t setup_scratch_ints(int N, int E) {
+    return scan_tmp_ints(std::max(4 * E, N + 1)) + 4 * ((size_t)N + 1) + 1;
+}
+
+// conn, emat, mats, pedges and s are uploaded, and r and z into U. The lists in between use
+// `contribution`, which like U is zeroed again, and `scratch` (setup_scratch_ints, zeroed).
+// Returns where the greatest number of elements around a node will be.
+int *launch_setup(Solver &S, int *scratch) {
+    Dev &d = S.d;
+    cudaStream_t st = S.stream;
+    const int N = d.N, E = d.E;
+    const long long entries = 4LL * E + 2LL * d.K;
+    int *sources = scratch, *edges = sources + N + 1, *edgeStart = edges + N + 1;
+    int *corners = edgeStart + N + 1, *most = corners + N + 1, *tmp = most + 1;
+    int *sourceBin = reinterpret_cast<int *>(d.contribution), *edgeBin = sourceBin + entries;
+    int *head = edgeBin + 4LL * E, *before = head + 4LL * E;   // 16 E + 2 K of 16 (E + K)
+    const double *r = reinterpret_cast<const double *>(d.U);
+    if (N > 0) k_positions<<<grid_for(N, SB), SB, 0, st>>>(d, r, r + N);
+    cudaMemsetAsync(d.U, 0, sizeof(double2) * (size_t)N, st);
+    if (entries > 0) {
+        const int grid = grid_for(entries, SB);
+        if (E > 0) k_shortest_edge<<<grid_for(E, SB), SB, 0, st>>>(d);
+        k_count<<<grid, SB, 0, st>>>(d, sources, edges);
+        if (E > 0) k_corners<<<grid_for(4LL * E, SB), SB, 0, st>>>(d, corners);
+        k_most<<<grid_for(N, SB), SB, 0, st>>>(N, corners, most);
+        scan_exclusive(sources, d.nodeSlotStart, N + 1, nullptr, tmp, st, nullptr, nullptr);
+        scan_exclusive(edges, edgeStart, N + 1, nullptr, tmp, st, nullptr, nullptr);
+        k_file<<<grid, SB, 0, st>>>(d, sources, edges, edgeStart, sourceBin, edgeBin);
+        k_rank<<<grid, SB, 0, st>>>(d, edgeStart, sourceBin, edgeBin);
+    }
+    if (E > 0) {
+        const int grid = grid_for(4LL * E, SB);
+        k_heads<<<grid, SB, 0, st>>>(d, head);
+        scan_exclusive(head, before, 4 * E, nullptr, tmp, st, nullptr, nullptr);
+        k_groups<<<grid, SB, 0, st>>>(d, head, before);
+        k_lump_volumes<<<grid_for(E, SB), SB, 0, st>>>(d, reinterpret_cast<double4 *>(d.contribution));
+    }
+    if (N > 0)
+        k_lump<<<grid_for(N, SB), SB, 0, st>>>(d, reinterpret_cast<const double4 *>(d.contribution));
+    cudaMemsetAsync(d.contribution, 0, sizeof(double) * 8 * ((size_t)E + d.K), st);
+    return most;
+}
+void launch_damage_geometry(Solver &S) {
+    if (S.d.E > 0) k_damage_geometry<<<grid_for(S.d.E, SB), SB, 0, S.stream>>>(S.d);
+}
+void launch_segments(Solver &S) {
+    if (S.d.E > 0) k_segments<<<grid_for(4LL * S.d.E, SB), SB, 0, S.stream>>>(S.d);
+}
+void launch_component(Solver &S, const double2 *src, double *dst, size_t count, int y) {
+    k_component<<<grid_for((long long)count, SB), SB, 0, S.stream>>>(src, dst, (int)count, y);
+}
+
+}  // namespace nf

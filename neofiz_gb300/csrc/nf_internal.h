@@ -254,8 +254,6 @@ struct Solver {
     size_t hostScratchBytes = 0;
     std::vector<nf_material> materials;
     std::vector<int32_t> emat;
-    std::vector<double> hostR, hostZ;
-    std::vector<int32_t> hostConn;
     double massScale = 1.0;
     double hourglass = 0.05;
     bool contactSet = false, damageSet = false, erosionSet = false;
@@ -272,8 +270,19 @@ struct Solver {
     bool noGraphs = false;       // capture failed once: steps are enqueued directly
     // a device-side wait that ran out leaves the state invalid: later run calls refuse
     nf_status failed = NF_OK;
-    void *arena = nullptr;       // nf_create's set-up arrays, one allocation
-    size_t arenaBytes = 0;
+    struct Block {
+        void *base = nullptr;
+        size_t bytes = 0;
+        bool holds(const void *p) const {
+            const char *c = static_cast<const char *>(p), *b = static_cast<const char *>(base);
+            return b && c >= b && c < b + bytes;
+        }
+    };
+    Block arena, contactArena;   // nf_create's arrays and nf_set_contact's, an allocation each
+    double *stage = nullptr;     // one component of a field on its way to the host
+    int maxCorners = 0;          // the most elements around a node
+    int noArea = 0;              // the first element whose area is not a positive number
+    double noAreaValue = 0.0;
     // per-group event profiling
     bool profiling = false;
     struct Rec { int group; cudaEvent_t a, b; };
@@ -405,6 +414,13 @@ void setup_node_slots(const int32_t *conn, int N, int E, const int32_t *pedges, 
                       int32_t *slotStart, int32_t *slots);
 double setup_min_edge(const double *r, const double *z, const int32_t *conn, int E);
 void set_thread_error(const char *message);
+
+// Launchers (k_setup.cu)
+size_t setup_scratch_ints(int N, int E);
+int *launch_setup(Solver &S, int *scratch);
+void launch_damage_geometry(Solver &S);
+void launch_segments(Solver &S);
+void launch_component(Solver &S, const double2 *src, double *dst, size_t count, int y);
 
 // Launchers (k_step.cu). Each returns the number of kernels it enqueued.
 int launch_initial_assembly(Solver &S);
