@@ -242,6 +242,7 @@ __device__ bool grid_scan(const Dev &d, int32_t *in, int32_t *out, int32_t *out2
 struct Grid {
     double cellSize, r0, z0;
     int cols, rows, hashed, bucketN;
+    int direct, mask;            // the direct-indexed layout, and a cell's bits in its index
     long long cells;
     float screen;                // the FP32 screen's margin (search_group)
 };
@@ -254,6 +255,8 @@ __device__ void grid_from_box(const Dev &d, int nodes, Grid &g) {
         g.cols = g.rows = 1;
         g.cells = 1;
         g.hashed = 0;
+        g.direct = 1;
+        g.mask = d.fastCells - 1;
         g.bucketN = 2;
         g.screen = 0.0f;
         return;
@@ -272,7 +275,9 @@ __device__ void grid_from_box(const Dev &d, int nodes, Grid &g) {
     g.rows = b > 1 ? b : 1;
     g.cells = (long long)g.cols * (long long)g.rows;
     g.hashed = g.cells > d.bucketCap;
-    g.bucketN = (int)((g.hashed ? (long long)d.bucketCap : g.cells) + 1);
+    g.direct = !g.hashed;
+    g.mask = g.direct ? d.fastCells - 1 : -1;
+    g.bucketN = 1 + (g.hashed ? d.bucketCap : (int)min(g.cells, (long long)d.fastCells));
     // every surface node lies within W = max(rhi - rlo, zhi - zlo) of the origin in each
     // coordinate; 2^-18 W bounds the FP32 screen's error twice over
     const double w = rhi - rlo > zhi - zlo ? rhi - rlo : zhi - zlo;
@@ -282,7 +287,7 @@ __device__ void grid_from_box(const Dev &d, int nodes, Grid &g) {
 __device__ __forceinline__ int iclamp(int v, int n) { return v < 0 ? 0 : v >= n ? n - 1 : v; }
 
 __device__ __forceinline__ int bucket_of(const Dev &d, const Grid &g, long long cell) {
-    return g.hashed ? (int)(cell % d.bucketCap) : (int)cell;
+    return g.hashed ? (int)(cell % d.bucketCap) : (int)cell & g.mask;
 }
 
 // Contact.depth, Contact.java:642-652
@@ -301,12 +306,19 @@ __device__ __forceinline__ double depth_of(const Dev &d, int n, int q) {
     return gap < 0.0 ? -gap : 0.0;
 }
 
-// Files one incident term (the pair of slave node m, role r, as m << 2 | r) in node j's fixed
-// list; a list that overflows switches the step to the general path (a scan over the counts).
-__device__ __forceinline__ void inc_push(const Dev &d, int j, int entry) {
-    const int pos = atomicAdd(&d.incCount[j], 1);
-    if (pos < INC_CAP) d.incSlots[(size_t)j * INC_CAP + pos] = entry;
-    else d.s->incOverflow = 1;
+// Files the pair's three incident terms (slave node m, role r, as m << 2 | r) in its nodes' fixed
+// lists; a list that overflows switches the step to the general path (a scan over the counts).
+// The three places are claimed before any is written, so the atomics' round trips overlap.
+__device__ __forceinline__ void inc_push(const Dev &d, int n, int a, int b) {
+    const int node[3] = {n, a, b};
+    int pos[3];
+#pragma unroll
+    for (int r = 0; r < 3; r++) pos[r] = atomicAdd(&d.incCount[node[r]], 1);
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        if (pos[r] < INC_CAP) d.incSlots[(size_t)node[r] * INC_CAP + pos[r]] = (n << 2) | r;
+        else d.s->incOverflow = 1;
+    }
 }
 
 // x is a normal number below 2^1000 in size (the exponent field alone).
@@ -388,9 +400,7 @@ __device__ void resolve_pair(const Dev &d, int n, int q) {
     d.pairDiss[n] = dthis;
     d.contactState[n] = state;
     d.pairNodes[n] = make_int4(n, a, b, 1);
-    inc_push(d, n, (n << 2) | 0);
-    inc_push(d, a, (n << 2) | 1);
-    inc_push(d, b, (n << 2) | 2);
+    inc_push(d, n, a, b);
 }
 
 // Contact.nearestPenetrated (Contact.java:570-606) for 32 / SG slaves per warp, SG lanes (a
@@ -407,11 +417,11 @@ __device__ void resolve_pair(const Dev &d, int n, int q) {
 // than 2^-19 W, and a candidate is dropped only when its FP32 value clears the bound by
 // 2^-18 W (g.screen). The few that pass take the exact FP64 test, each lane its own. The
 // grid's buckets as the search reads them: the counting-sort layout (bucket b's entries at
-// [start[b], start[b + 1]), each with its cell) or the direct-indexed one (cell c's entries at
-// [c cap, c cap + count[c]), every entry in its own cell).
+// [start[b], start[b + 1]), each with its cell) or the direct-indexed one (bucket b's entries at
+// [b cap, b cap + count[b]), with their cells where cells share buckets).
 struct BucketView {
     const int32_t *start, *count;
-    const long long *cell;                     // null in the direct-indexed layout
+    const long long *cell;                     // null where a bucket holds one cell only
     const int32_t *entry;
     const float4 *f;                           // first node - grid origin, normal (FP32)
     const float *fl;                           // length (FP32)
@@ -432,9 +442,11 @@ __device__ __forceinline__ void bucket_range(const BucketView &v, int b, int &lo
 
 constexpr int SG = 8;                          // lanes per slave
 constexpr int KEPT = 4;                        // screened candidates a lane keeps for later
+constexpr int NO_PAIR = -1;                    // what a search without a pair returns,
+constexpr int FELL = -2;                       // and one that saw the last master too deep
 constexpr int OWN_KEPT = 4;                    // a slave's own segments held in registers
-__device__ void search_group(const Dev &d, const Grid &g, const BucketView &v, int idx,
-                             int listLen, double &bestOut, int &segOut, bool &fellOut) {
+__device__ int search_group(const Dev &d, const Grid &g, const BucketView &v, int idx,
+                            int listLen) {
     const int lane = threadIdx.x & 31, gl = lane & (SG - 1);
     int n = idx < listLen ? d.nodeList[idx] : -1;
     const bool live = n >= 0;
@@ -536,7 +548,7 @@ __device__ void search_group(const Dev &d, const Grid &g, const BucketView &v, i
         int c, k;
         long long cc;
         locate(t, c, k, cc);
-        if (v.cell && v.cell[k] != cc) return;          // a hashed bucket shares cells
+        if (v.cell && v.cell[k] != cc) return;          // cells may share a bucket
         const int entry = v.entry[k];
         const int sg = entry >> 1;
         const double2 pa = v.a[k], nq = v.n[k];
@@ -614,23 +626,21 @@ __device__ void search_group(const Dev &d, const Grid &g, const BucketView &v, i
         }
     }
     const unsigned fellBits = __ballot_sync(0xffffffffu, fell);
-    fellOut = ((fellBits >> (lane & ~(SG - 1))) & ((1u << SG) - 1u)) != 0u;
-    bestOut = __shfl_sync(0xffffffffu, best, 0, SG);
-    segOut = __shfl_sync(0xffffffffu, bestSeg, 0, SG);
+    const bool anyFell = ((fellBits >> (lane & ~(SG - 1))) & ((1u << SG) - 1u)) != 0u;
+    return __shfl_sync(0xffffffffu, bestSeg >= 0 ? bestSeg : anyFell ? FELL : NO_PAIR, 0, SG);
 }
 
 // The pair of slave node n from its search (Contact.java:446-462): master, last master, the
 // escape count and the pair forces; one lane.
-__device__ void finish_slave(const Dev &d, int n, double best, int bestSeg, bool anyFell) {
-    const int last = d.lastMaster[n];
-    d.master[n] = best > 0.0 ? bestSeg : -1;
-    if (!(best > 0.0)) {                      // no pair: Contact.java:446-452
-        if (last >= 0 && anyFell) atomicAdd(&d.s->escaped, 1);
+__device__ void finish_slave(const Dev &d, int n, int found) {
+    d.master[n] = found >= 0 ? found : -1;
+    if (found < 0) {                          // no pair: Contact.java:446-452
+        if (found == FELL && d.lastMaster[n] >= 0) atomicAdd(&d.s->escaped, 1);
         d.lastMaster[n] = -1;
         return;
     }
-    d.lastMaster[n] = bestSeg;
-    resolve_pair(d, n, bestSeg);
+    d.lastMaster[n] = found;
+    resolve_pair(d, n, found);
 }
 
 // ---------------------------------------------------------------------------- the pass
@@ -822,12 +832,15 @@ __global__ void __launch_bounds__(CB, 2) k_contact_pass(Dev d) {
     const Grid g = grid;
     // Per surface node: its normal from its segments in ascending order; its grid cell, once
     // (the search reads it for the node as a slave); and the filing of every segment end at the
-    // node under that cell. A grid of at most fastCells - 1 cells is indexed directly: each
-    // entry takes the next of its cell's slots (fastLimit of the fastCap reserved) and is filed
-    // there at once, with the FP32 values the search's screen reads. A larger (or hashed) grid,
-    // or a cell that outgrows its slots, takes the counting sort: the counts, an exclusive
-    // scan, the filing.
-    const bool fast = !g.hashed && g.cells < d.fastCells;
+    // node under that cell. The cell's low bits index buckets of fixed size: each entry takes the
+    // next of its bucket's slots (fastLimit of the fastCap reserved) and is filed there at once,
+    // with the FP32 values the search's screen reads. In a grid of more than fastCells cells,
+    // bodies apart or a fine mesh, cells share buckets, and an entry keeps its cell for the
+    // search to tell them by: the surface is a line through the grid, so few do. 1M quads, 75k
+    // to 430k cells for 65,536 buckets: 58 us from the filing to the end of the search through
+    // the counting sort, which such a grid took, and 44 us so. A hashed grid, or a bucket that
+    // outgrows its slots, takes the counting sort: the counts, an exclusive scan, the filing.
+    const bool fast = g.direct, folded = g.cells > d.fastCells;
     FOR_GRID(i, nodeLen) {
         const int n = d.nodeList[i];
         if (n < 0) continue;
@@ -848,6 +861,7 @@ __global__ void __launch_bounds__(CB, 2) k_contact_pass(Dev d) {
         const int cj = iclamp(jd2i(nf_div_by(d.cz[n] - g.z0, g.cellSize, byCell)), g.rows);
         d.nodeCell[n] = make_int2(ci, cj);
         const long long cell = (long long)cj * g.cols + ci;
+        const int bucket = bucket_of(d, g, cell);
         // the node's ends, two at a time: both slots are claimed before either is written, so
         // the atomics' round trips overlap
         for (int k0 = 0; k0 < count; k0 += 2) {
@@ -856,7 +870,7 @@ __global__ void __launch_bounds__(CB, 2) k_contact_pass(Dev d) {
             for (int j = 0; j < 2; j++) {
                 qs[j] = k0 + j < count ? own[k0 + j] : -1;
                 as[j] = qs[j] >= 0 ? d.segA[qs[j]] : -1;
-                pos[j] = fast && qs[j] >= 0 ? atomicAdd(&d.fastCount[cell], 1) : 0;
+                pos[j] = fast && qs[j] >= 0 ? atomicAdd(&d.fastCount[bucket], 1) : 0;
             }
 #pragma unroll
             for (int j = 0; j < 2; j++) {
@@ -866,11 +880,12 @@ __global__ void __launch_bounds__(CB, 2) k_contact_pass(Dev d) {
                 d.entryCell[entry] = cell;
                 if (fast) {
                     if (pos[j] < d.fastLimit) {
-                        const size_t slot = (size_t)cell * d.fastCap + pos[j];
+                        const size_t slot = (size_t)bucket * d.fastCap + pos[j];
                         const double2 pa = make_double2(d.cr[a], d.cz[a]);
                         const double2 nq = make_double2(d.snr[q], d.snz[q]);
                         const double lq = d.slen[q];
                         d.fastEntry[slot] = entry;
+                        if (folded) d.fastCell[slot] = cell;
                         d.fastF[slot] = make_float4((float)(pa.x - g.r0), (float)(pa.y - g.z0),
                                                     (float)nq.x, (float)nq.y);
                         d.fastFL[slot] = (float)lq;
@@ -882,7 +897,7 @@ __global__ void __launch_bounds__(CB, 2) k_contact_pass(Dev d) {
                         s->fastOverflow = 1;
                     }
                 } else {
-                    atomicAdd(&d.bucketCount[bucket_of(d, g, cell)], 1);
+                    atomicAdd(&d.bucketCount[bucket], 1);
                 }
             }
         }
@@ -917,7 +932,8 @@ __global__ void __launch_bounds__(CB, 2) k_contact_pass(Dev d) {
     }
     BucketView view;
     if (direct) {
-        view = BucketView{nullptr, d.fastCount, nullptr, d.fastEntry, d.fastF, d.fastFL,
+        view = BucketView{nullptr, d.fastCount, folded ? d.fastCell : nullptr, d.fastEntry,
+                          d.fastF, d.fastFL,
                           d.fastAB, d.fastA, d.fastN, d.fastL, d.fastCap};
     } else {
         view = BucketView{d.bucketStart, nullptr, d.bucketCell, d.bucketEntry, d.bucketF,
@@ -925,34 +941,50 @@ __global__ void __launch_bounds__(CB, 2) k_contact_pass(Dev d) {
     }
 
     // the search and the pair forces: each warp searches 32 / SG slaves at a time, SG lanes
-    // each, and the groups' first lanes then compute the pairs' forces side by side (long
-    // dependent chains of divisions)
+    // each. Lane r of a group keeps what its round r found, and after SG rounds (or the last)
+    // every lane computes its pair's forces, side by side: they are long dependent chains of
+    // divisions, a dozen microseconds whether one lane or all have a pair. 15,300 surface nodes
+    // (two rounds): 44 us with the forces in every round, 33 us so.
     {
         const int warpsTotal = gridDim.x * CB_WARPS;
-        const int group = (threadIdx.x & 31) / SG;
-        for (int w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; w * (32 / SG) < nodeLen;
-             w += warpsTotal) {
-            const int idx = w * (32 / SG) + group;
-            double best;
-            int seg;
-            bool fell;
-            search_group(d, g, view, idx, nodeLen, best, seg, fell);
-            if ((threadIdx.x & (SG - 1)) == 0 && idx < nodeLen) {
-                const int n = d.nodeList[idx];
-                if (n >= 0) finish_slave(d, n, best, seg, fell);
+        const int lane = threadIdx.x & 31, group = lane / SG;
+        int w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+        while (w * (32 / SG) < nodeLen) {
+            const int first = w * (32 / SG) + group;
+            int found = NO_PAIR, r = 0;
+            for (; r < SG && w * (32 / SG) < nodeLen; r++, w += warpsTotal) {
+                const int f = search_group(d, g, view, w * (32 / SG) + group, nodeLen);
+                if ((lane & (SG - 1)) == r) found = f;
             }
+            const int mine = lane & (SG - 1);
+            const int idx = first + mine * warpsTotal * (32 / SG);
+            const int n = mine < r && idx < nodeLen ? d.nodeList[idx] : -1;
+            if (n >= 0) finish_slave(d, n, found);
+            __syncwarp();
         }
     }
     SYNC();
-    if (direct) FOR_GRID(c, (int)g.cells) d.fastCount[c] = 0;   // all zero again for the next step
+    if (direct) FOR_GRID(c, g.bucketN) d.fastCount[c] = 0;   // all zero again for the next step
     const bool friction = d.cFriction > 0.0;
-    // the pairs' spring energy and dissipation, summed over a fixed grid of node numbers
+    // the pairs' spring energy and dissipation, summed over a fixed grid of node numbers. The
+    // contact states (cleared by the step's gather) tell the pairs in a byte a node, read four
+    // rounds at a time: 1M nodes 9 us by pairNodes, 6 us so.
     {
         double energy = 0.0, diss = 0.0;
-        FOR_GRID(n, d.N) {
-            if (d.pairNodes[n].w) {
-                energy += d.pairEnergy[n];
-                diss += d.pairDiss[n];
+        const int stride = gridDim.x * CB;
+        for (int n0 = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+             n0 < d.N; n0 += 4 * stride) {
+            uint8_t pair[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                pair[k] = (long long)n0 + (long long)k * stride < d.N
+                              ? d.contactState[n0 + k * stride] : 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (pair[k]) {
+                    energy += d.pairEnergy[n0 + k * stride];
+                    diss += d.pairDiss[n0 + k * stride];
+                }
             }
         }
         const double e1 = block_sum_c(energy, shd);

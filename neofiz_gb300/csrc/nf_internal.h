@@ -170,16 +170,17 @@ struct Dev {
     double *bucketL;
     long long *bucketCell;                   // [8E] cell of each filed entry, by position
     long long *entryCell;                    // [8E] cell of each entry, by entry
-    // the direct-indexed grid: cell c's entries in slots [c fastCap, c fastCap + fastCount[c])
-    // when the grid has at most fastCells cells and none holds more than fastCap entries
-    int32_t *fastCount;                      // [fastCells]
+    // the direct-indexed grid: the entries of the cells whose low bits are b in slots
+    // [b fastCap, b fastCap + fastCount[b]) while none outgrows them
+    int32_t *fastCount;                      // [fastCells + 1]
+    long long *fastCell;                     // [fastCells x fastCap] the entry's cell
     int32_t *fastEntry;                      // [fastCells x fastCap]
     float4 *fastF;                           // [fastCells x fastCap] as bucketF
     float *fastFL;                           // [fastCells x fastCap] as bucketFL
     int2 *fastAB;                            // [fastCells x fastCap] as bucketAB
     double2 *fastA, *fastN;                  // [fastCells x fastCap] as bucketA, bucketN
     double *fastL;                           // [fastCells x fastCap] as bucketL
-    int fastCells, fastCap;                  // cells indexed directly, slots per cell
+    int fastCells, fastCap;                  // buckets (a power of two), slots per bucket
     int fastLimit;                           // slots a step may use, <= fastCap (nf_set_grid_slots)
     int bucketCap;
     // pair records, per node
