@@ -213,72 +213,6 @@ nf_status ensure_mixed_damage(Solver &S) {
     return NF_OK;
 }
 
-// lumpMass, ExplicitSolver.java:1559-1597: 2x2 Gauss lumping, in the reference's order.
-// emat may be NULL (every element material 0).
-void lumped_mass(const double *r, const double *z, const int32_t *conn, int E,
-                 const nf_material *materials, const int32_t *emat, bool axi, double thickness,
-                 double *mass) {
-    const double G = 0.5773502691896258;
-    const double gx[4] = {-G, G, G, -G}, ge[4] = {-G, -G, G, G};
-    for (int e = 0; e < E; e++) {
-        const double rho = materials[emat ? emat[e] : 0].density;
-        const int b = e * 4;
-        const int n0 = conn[b], n1 = conn[b + 1], n2 = conn[b + 2], n3 = conn[b + 3];
-        const double r0 = r[n0], r1 = r[n1], r2 = r[n2], r3 = r[n3];
-        const double z0 = z[n0], z1 = z[n1], z2 = z[n2], z3 = z[n3];
-        for (int g = 0; g < 4; g++) {
-            const double xi = gx[g], eta = ge[g];
-            const double xm = 1.0 - xi, xp = 1.0 + xi;
-            const double em = 1.0 - eta, ep = 1.0 + eta;
-            const double N0 = 0.25 * xm * em, N1 = 0.25 * xp * em;
-            const double N2 = 0.25 * xp * ep, N3 = 0.25 * xm * ep;
-            const double dN0x = -0.25 * em, dN1x = 0.25 * em, dN2x = 0.25 * ep, dN3x = -0.25 * ep;
-            const double dN0e = -0.25 * xm, dN1e = -0.25 * xp, dN2e = 0.25 * xp, dN3e = 0.25 * xm;
-            const double J00 = dN0x * r0 + dN1x * r1 + dN2x * r2 + dN3x * r3;
-            const double J01 = dN0x * z0 + dN1x * z1 + dN2x * z2 + dN3x * z3;
-            const double J10 = dN0e * r0 + dN1e * r1 + dN2e * r2 + dN3e * r3;
-            const double J11 = dN0e * z0 + dN1e * z1 + dN2e * z2 + dN3e * z3;
-            const double det = J00 * J11 - J01 * J10;
-            const double rg = N0 * r0 + N1 * r1 + N2 * r2 + N3 * r3;
-            const double dV = axi ? 2.0 * NF_PI * rg * det : thickness * det;
-            mass[n0] += rho * N0 * dV;
-            mass[n1] += rho * N1 * dV;
-            mass[n2] += rho * N2 * dV;
-            mass[n3] += rho * N3 * dV;
-        }
-    }
-}
-
-// buildNodeSlots, ExplicitSolver.java:347-366: per node its sources (element 8 e + corner,
-// then pressure-edge slots) in ascending order. slotStart has N + 1 entries, zeroed.
-void node_slots(const int32_t *conn, int N, int E, const int32_t *pedges, int K,
-                int32_t *slotStart, int32_t *slots) {
-    for (long long k = 0; k < 4LL * E; k++) slotStart[conn[k] + 1]++;
-    for (long long k = 0; k < 2LL * K; k++) slotStart[pedges[k] + 1]++;
-    for (int i = 0; i < N; i++) slotStart[i + 1] += slotStart[i];
-    std::vector<int32_t> cursor(slotStart, slotStart + N + 1);
-    for (int e = 0; e < E; e++)
-        for (int c = 0; c < 4; c++) slots[cursor[conn[e * 4 + c]]++] = e * 8 + c;
-    for (int k = 0; k < 2 * K; k += 2) {
-        const int slot = (E + k / 2) * 8;
-        slots[cursor[pedges[k]]++] = slot;
-        slots[cursor[pedges[k + 1]]++] = slot + 1;
-    }
-}
-
-// QuadMesh.minimumEdgeLength: the shortest element edge of the reference configuration.
-double min_edge_length(const double *r, const double *z, const int32_t *conn, int E) {
-    double edge = DBL_MAX;
-    for (int e = 0; e < E; e++)
-        for (int k = 0; k < 4; k++) {
-            const int i = conn[e * 4 + k], j = conn[e * 4 + (k + 1) % 4];
-            const double dr = r[j] - r[i], dz = z[j] - z[i];
-            const double len = sqrt(dr * dr + dz * dz);
-            if (len < edge) edge = len;
-        }
-    return edge;
-}
-
 // The FP32 copy of a material's constants (the mixed form).
 MatF mat_float(const MatDev &a) {
     MatF o{};
@@ -842,7 +776,7 @@ nf_status nf_set_damage(nf_solver *h, const double *gf, const double *eps) {
     }
     CK(&S, upload(S, d.dFail, eps, E));
     CK(&S, upload(S, d.dGf, gf, E));
-    launch_damage_geometry(S);
+    setup_damage_geometry(d, S.stream);
     d.hasDamage = 1;
     S.damageSet = true;
     if (d.mixed) {
@@ -1122,14 +1056,11 @@ nf_status nf_read_field(nf_solver *h, int32_t field, void *dst, size_t nbytes) {
     st = sync_check(S);
     if (st) return st;
     auto copy = [&](const void *src) -> nf_status {
-        // the destination's pages first: a copy of 32 MB into pages not mapped yet took 13.6 ms
-        // (the device faults them in one by one), with them touched it takes 1.3 ms
-        for (size_t i = 0; i < nbytes; i += 4096) ((volatile char *)dst)[i] = 0;
-        CK(&S, cudaMemcpyAsync(dst, src, nbytes, cudaMemcpyDeviceToHost, S.stream));
+        CK(&S, copy_to_host(dst, src, nbytes, S.stream));
         return sync_check(S);
     };
     auto pair = [&](const double2 *src, int comp) -> nf_status {
-        launch_component(S, src, S.stage, count, comp);
+        launch_component(src, S.stage, count, comp, S.stream);
         return copy(S.stage);
     };
     switch (field) {
@@ -1413,19 +1344,6 @@ MatF material_constants_f32(const MatDev &m) { return mat_float(m); }
 double element_signed_area(const double *r, const double *z, const int32_t *conn, int e) {
     return signed_area(r, z, conn, e);
 }
-void setup_lumped_mass(const double *r, const double *z, const int32_t *conn, int E,
-                       const nf_material *materials, const int32_t *emat, bool axi,
-                       double thickness, double *mass) {
-    lumped_mass(r, z, conn, E, materials, emat, axi, thickness, mass);
-}
-void setup_node_slots(const int32_t *conn, int N, int E, const int32_t *pedges, int K,
-                      int32_t *slotStart, int32_t *slots) {
-    node_slots(conn, N, E, pedges, K, slotStart, slots);
-}
-double setup_min_edge(const double *r, const double *z, const int32_t *conn, int E) {
-    return min_edge_length(r, z, conn, E);
-}
-// Helpers shared with the device film (k_film.cu).
 void solver_state_to_double(Solver &S) { mixed_to_double(S); }
 nf_status solver_fail(Solver &S, nf_status st, const char *message) {
     return fail(&S, st, "%s", message);

@@ -11,6 +11,7 @@
 #include <cfloat>
 #include <cstdarg>
 #include <cstdio>
+#include <cstring>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -41,6 +42,7 @@ struct Batch {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double lastMs = 0.0;
     long long launches = 0;
+    double *stage = nullptr;                 // a field on its way to the host
     std::vector<void *> allocs;
     // the adjoint's buffers (nf_batch_adjoint_*)
     AdjDev adj{};
@@ -341,19 +343,11 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
         return bfail(nullptr, NF_EDEVICE, "stream or event creation failed");
     }
 
-    // host set-up, instance by instance, as nf_create and the setters do it
+    // the instances' constants; the arrays over nodes and elements form on the device
     const bool axi = formulation == NF_AXISYMMETRIC;
-    std::vector<double2> X0(N), V(N);
-    std::vector<double> mass(N, 0.0), invMass(N);
-    std::vector<uint8_t> flags(N, 0);
-    std::vector<int4> conn(E);
-    std::vector<int32_t> emat(E), slotStart(N + 1, 0), slots(4LL * E + 2LL * K);
-    std::vector<int2> pedges(K);
-    std::vector<double> geom(damage ? 5LL * E : 0);
+    std::vector<double2> velocity(count);
     std::vector<MatDev> mats(count);
     std::vector<MatF> matsF(count);
-    std::vector<BatchScalars> sc(count);
-    std::vector<double> cost(count);
     B->inst.resize(count);
     int maxNodes = 1, maxElems = 1;
     for (int k = 0; k < count; k++) {
@@ -363,48 +357,12 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
         const int nn = n1 - n0, ne = e1 - e0;
         maxNodes = std::max(maxNodes, nn);
         maxElems = std::max(maxElems, ne);
-        const double *r = mesh->r + n0, *z = mesh->z + n0;
-        const int32_t *lc = mesh->conn + 4LL * e0;
         const int k0 = mesh->pressure_offset ? mesh->pressure_offset[k] : 0;
         const int nk = mesh->pressure_offset ? mesh->pressure_offset[k + 1] - k0 : 0;
-        const int32_t *lp = nk ? mesh->pressure_edges + 2LL * k0 : nullptr;
-        setup_lumped_mass(r, z, lc, ne, &p.material, nullptr, axi, thickness, mass.data() + n0);
-        std::vector<int32_t> ls(nn + 1, 0), lsl(4LL * ne + 2LL * nk);
-        setup_node_slots(lc, nn, ne, lp, nk, ls.data(), lsl.data());
-        const int slotBase = 4 * e0 + 2 * k0;
-        for (int i = 0; i < nn; i++) {
-            X0[n0 + i] = make_double2(r[i], z[i]);
-            V[n0 + i] = make_double2(p.velocity_r, p.velocity_z);
-            invMass[n0 + i] = 1.0 / mass[n0 + i];
-            flags[n0 + i] = mesh->fixed ? (uint8_t)(mesh->fixed[n0 + i] & 3) : 0;
-            slotStart[n0 + i + 1] = slotBase + ls[i + 1];
-        }
-        // local sources -> global: element slots shift by 8 e0, edge slots move past all elements
-        for (long long j = 0; j < 4LL * ne + 2LL * nk; j++) {
-            const int v = lsl[j];
-            slots[slotBase + j] = v < 8 * ne ? v + 8 * e0 : (E + k0 + (v >> 3) - ne) * 8 + (v & 7);
-        }
-        for (int j = 0; j < nk; j++) pedges[k0 + j] = make_int2(lp[2 * j] + n0, lp[2 * j + 1] + n0);
-        if (damage)
-            for (int e = 0; e < ne; e++) {                      // ExplicitSolver.java:767-789
-                const int b = 4 * e;
-                const int q0 = lc[b], q1 = lc[b + 1], q2 = lc[b + 2], q3 = lc[b + 3];
-                double *g = geom.data() + 5LL * (e0 + e);
-                g[1] = 0.5 * (r[q1] - r[q0] + r[q2] - r[q3]);
-                g[2] = 0.5 * (z[q1] - z[q0] + z[q2] - z[q3]);
-                g[3] = 0.5 * (r[q3] - r[q0] + r[q2] - r[q1]);
-                g[4] = 0.5 * (z[q3] - z[q0] + z[q2] - z[q1]);
-                g[0] = fabs(element_signed_area(r, z, lc, e));
-            }
-        for (int e = 0; e < ne; e++) {
-            conn[e0 + e] = make_int4(lc[4 * e] + n0, lc[4 * e + 1] + n0, lc[4 * e + 2] + n0,
-                                     lc[4 * e + 3] + n0);
-            emat[e0 + e] = k;
-        }
+        velocity[k] = make_double2(p.velocity_r, p.velocity_z);
         mats[k] = material_constants(p.material, formulation);
         matsF[k] = material_constants_f32(mats[k]);
         const double wave = material_wave(p.material);
-        const double edge = setup_min_edge(r, z, lc, ne);
         BatchInst &in = B->inst[k];
         in.n0 = n0; in.n1 = n1; in.e0 = e0; in.e1 = e1;
         in.k0 = k0; in.k1 = k0 + nk;
@@ -419,18 +377,7 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
         in.wallPlane = in.hasWall ? p.wall_plane : 0.0;
         in.wallFriction = in.hasWall ? p.wall_friction : 0.0;
         in.tEnd = p.t_end;
-        BatchScalars &s = sc[k];
-        s.minEdgeSquared = edge * edge;
-        s.dt = cfl_safety * edge / wave;                      // :333-338
-        s.dtPrevious = s.dt;
-        s.stepLimit = 0;
-        s.done = 1;
-        cost[k] = (double)ne * (p.t_end > 0.0 && s.dt > 0.0 ? p.t_end / s.dt : 1.0);
     }
-    std::vector<int32_t> order(count);
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return cost[a] > cost[c]; });
-    for (int k : order) B->elems.push_back(B->inst[k].e1 - B->inst[k].e0);
 
     d.N = N; d.E = E; d.K = K; d.ppe = 1;
     d.hasDamage = damage ? 1 : 0;
@@ -480,6 +427,13 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
     A(dOrder, count);
     A(b.queue, 1); A(b.remaining, 1);
     A(b.measure, 3LL * count);
+    int32_t *scratch = nullptr;
+    A(scratch, setup_scratch_ints(N, E));
+    A(B->stage, std::max<long long>(N, B->mixed ? 4LL * E : E));
+    unsigned long long *dEdges = nullptr;
+    A(dEdges, count);
+    double2 *dVelocity = nullptr;
+    A(dVelocity, count);
 #undef A
     if (e_ != cudaSuccess) {
         destroy(B);
@@ -492,27 +446,46 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
     b.maxElems = maxElems;
     e_ = cudaSuccess;
 #define U(dst, src, n) if (e_ == cudaSuccess) e_ = bupload(*B, dst, src, n)
-    U(d.X0, X0.data(), N); U(d.V, V.data(), N); U(d.mass, mass.data(), N);
-    U(d.invMass, invMass.data(), N); U(d.flags, flags.data(), N);
-    U(d.conn, conn.data(), E); U(d.emat, emat.data(), E); U(d.mats, mats.data(), count);
-    U(d.nodeSlotStart, slotStart.data(), N + 1); U(d.nodeSlot, slots.data(), 4LL * E + 2LL * K);
-    U(d.pedges, pedges.data(), K);
+    double *rz = reinterpret_cast<double *>(d.U);
+    std::vector<unsigned long long> edges(count, 0x7ff0000000000000ULL);
+    U(rz, mesh->r, N); U(rz + N, mesh->z, N);
+    if (mesh->fixed) U(d.flags, mesh->fixed, N);
+    U(reinterpret_cast<int32_t *>(d.conn), mesh->conn, 4LL * E); U(d.mats, mats.data(), count);
+    U(reinterpret_cast<int32_t *>(d.pedges), mesh->pressure_edges, 2LL * K);
+    U(dEdges, edges.data(), count); U(dVelocity, velocity.data(), count);
     if (damage) {
         U(d.dFail, mesh->failure_strain, E); U(d.dGf, mesh->fracture_energy, E);
-        U(d.dGeom, geom.data(), 5LL * E);
-        if (B->mixed) {
-            std::vector<float> f(E), gf(E), g5(5LL * E);
-            for (int e = 0; e < E; e++) {
-                f[e] = (float)mesh->failure_strain[e];
-                gf[e] = (float)mesh->fracture_energy[e];
-            }
-            for (size_t j = 0; j < g5.size(); j++) g5[j] = (float)geom[j];
-            U(d.dFailF, f.data(), E); U(d.dGfF, gf.data(), E); U(d.dGeomF, g5.data(), 5LL * E);
-            if (e_ == cudaSuccess) e_ = cudaStreamSynchronize(B->stream);   // f, gf, g5 die here
-        }
     }
     if (B->mixed) U(d.matsF, matsF.data(), count);
     U(dInst, B->inst.data(), count);
+    if (e_ == cudaSuccess) {
+        launch_batch_setup(d, dInst, count, dVelocity, dEdges, scratch, B->stream);
+        if (damage) setup_damage_geometry(d, B->stream);
+        e_ = cudaMemcpyAsync(edges.data(), dEdges, sizeof edges[0] * count, cudaMemcpyDeviceToHost,
+                             B->stream);
+    }
+    if (e_ == cudaSuccess) e_ = cudaStreamSynchronize(B->stream);
+    std::vector<BatchScalars> sc(count);
+    std::vector<double> cost(count);
+    std::vector<int32_t> order(count);
+    for (int k = 0; k < count; k++) {
+        const BatchInst &in = B->inst[k];
+        double edge = DBL_MAX;                                // the shortest one, as in nf_create
+        if (edges[k] < 0x7ff0000000000000ULL) {
+            memcpy(&edge, &edges[k], sizeof edge);
+            edge = sqrt(edge);
+        }
+        BatchScalars &s = sc[k];
+        s.minEdgeSquared = edge * edge;
+        s.dt = cfl_safety * edge / in.wave;                   // :333-338
+        s.dtPrevious = s.dt;
+        s.stepLimit = 0;
+        s.done = 1;
+        cost[k] = (double)(in.e1 - in.e0) * (in.tEnd > 0.0 && s.dt > 0.0 ? in.tEnd / s.dt : 1.0);
+    }
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return cost[a] > cost[c]; });
+    for (int k : order) B->elems.push_back(B->inst[k].e1 - B->inst[k].e0);
     U(b.sc, sc.data(), count);
     U(dOrder, order.data(), count);
 #undef U
@@ -714,24 +687,19 @@ nf_status nf_batch_read(nf_batch *h, int32_t field, void *dst, size_t nbytes) {
     if (nbytes < count * bytes)
         return bfail(&B, NF_EINVAL, "buffer of %zu bytes is smaller than the field (%zu)", nbytes,
                      count * bytes);
-    BCK(&B, cudaStreamSynchronize(B.stream));
+    if (count == 0) return NF_OK;
     const Dev &d = B.d;
-    double *o = (double *)dst;
-    auto pairs = [&](const double2 *src, int comp) -> nf_status {
-        std::vector<double2> t(count);
-        BCK(&B, cudaMemcpy(t.data(), src, 16 * count, cudaMemcpyDeviceToHost));
-        for (size_t i = 0; i < count; i++) o[i] = comp ? t[i].y : t[i].x;
-        return NF_OK;
-    };
     auto plain = [&](const void *src, size_t elem) -> nf_status {
-        BCK(&B, cudaMemcpy(dst, src, elem * count, cudaMemcpyDeviceToHost));
-        return NF_OK;
+        BCK(&B, copy_to_host(dst, src, elem * count, B.stream));
+        return bsync(B);
     };
-    auto widen = [&](const float *src) -> nf_status {
-        std::vector<float> t(count);
-        BCK(&B, cudaMemcpy(t.data(), src, 4 * count, cudaMemcpyDeviceToHost));
-        for (size_t i = 0; i < count; i++) o[i] = t[i];
-        return NF_OK;
+    auto pairs = [&](const double2 *src, int comp) -> nf_status {
+        launch_component(src, B.stage, count, comp, B.stream);
+        return plain(B.stage, 8);
+    };
+    auto widen = [&](const float *src, int stride = 1) -> nf_status {
+        launch_widen(src, B.stage, count, stride, B.stream);
+        return plain(B.stage, 8);
     };
     switch (field) {
         case NF_FIELD_UR: return pairs(d.U, 0);
@@ -743,11 +711,10 @@ nf_status nf_batch_read(nf_batch *h, int32_t field, void *dst, size_t nbytes) {
         case NF_FIELD_MASS: return plain(d.mass, 8);
         case NF_FIELD_WALL_STATE: return plain(d.wallState, 1);
         case NF_FIELD_FIXED: {
-            std::vector<uint8_t> f(count);
-            BCK(&B, cudaMemcpy(f.data(), d.flags, count, cudaMemcpyDeviceToHost));
+            st = plain(d.flags, 1);
             uint8_t *u = (uint8_t *)dst;
-            for (size_t i = 0; i < count; i++) u[i] = f[i] & 3;
-            return NF_OK;
+            for (size_t i = 0; i < count && !st; i++) u[i] &= 3;
+            return st;
         }
         case NF_FIELD_STRESS: return B.mixed ? widen(d.sigF) : plain(d.sig, 8);
         case NF_FIELD_BACK_STRESS: return B.mixed ? widen(d.backF) : plain(d.back, 8);
@@ -756,12 +723,7 @@ nf_status nf_batch_read(nf_batch *h, int32_t field, void *dst, size_t nbytes) {
         case NF_FIELD_HOURGLASS_STIFFNESS: return B.mixed ? widen(d.hgKF) : plain(d.hgK, 8);
         case NF_FIELD_HOURGLASS_R: case NF_FIELD_HOURGLASS_Z: {
             const int comp = field == NF_FIELD_HOURGLASS_Z;
-            if (B.mixed) {
-                std::vector<float2> t(count);
-                BCK(&B, cudaMemcpy(t.data(), d.hgF, 8 * count, cudaMemcpyDeviceToHost));
-                for (size_t i = 0; i < count; i++) o[i] = comp ? t[i].y : t[i].x;
-                return NF_OK;
-            }
+            if (B.mixed) return widen(reinterpret_cast<const float *>(d.hgF) + comp, 2);
             return pairs(d.hg, comp);
         }
         default: return bfail(&B, NF_EINVAL, "field %d is not readable from a batch", field);

@@ -1,11 +1,12 @@
-// k_setup.cu -- the arrays a scene derives from its mesh: node positions, shortest edge, the
-// sources of every node, the edge groups of the free surface, lumped masses, the damage model's
+// k_setup.cu -- the arrays a scene or a batch derives from its meshes: node positions, shortest
+// edge, the sources of every node, the edge groups of the free surface, lumped masses, the damage model's
 // element geometry and the surface's edge ends. Every value is the host expression's (no
 // contraction, sums in the same order), so the results are those of the serial loops.
 //
 // One core took 64 ms over these for 1M quads, half as long as the 400 steps that followed;
 // here they are 1 ms of kernels (each a pass or two over the mesh, bound by its gathers) behind
-// the upload of the mesh. Below about a thousand elements the launches cost what the host loops
+// the upload of the mesh (a batch of 512 rods, 580k quads:
+// 46 ms on one core and 15 so, which leaves the allocations, the checks and the upload). Below about a thousand elements the launches cost what the host loops
 // did (50 us). The orderings are counting sorts: an entry's place in its node's list is the
 // number of smaller entries there, which each entry counts for itself, so no list is walked by
 // one thread alone whatever the mesh's valences.
@@ -28,8 +29,9 @@ __global__ void __launch_bounds__(SB) k_positions(Dev d, const double *r, const 
     if (n < d.N) d.X0[n] = make_double2(r[n], z[n]);
 }
 
-// QuadMesh.minimumEdgeLength squared, as bits (a NaN is passed over).
-__global__ void __launch_bounds__(SB) k_shortest_edge(Dev d) {
+// QuadMesh.minimumEdgeLength squared, as bits (a NaN is passed over): of the scene, or of the
+// element's instance.
+__global__ void __launch_bounds__(SB) k_shortest_edge(Dev d, unsigned long long *instances) {
     const int e = blockIdx.x * SB + threadIdx.x;
     unsigned long long best = 0x7ff0000000000000ULL;
     if (e < d.E) {
@@ -43,7 +45,33 @@ __global__ void __launch_bounds__(SB) k_shortest_edge(Dev d) {
             best = q < best ? q : best;
         }
     }
-    commit_min_bits(best, &d.s->minEdgeBits);
+    if (!instances) {
+        commit_min_bits(best, &d.s->minEdgeBits);
+    } else if (e < d.E) {
+        unsigned long long *of = instances + d.emat[e];
+        if (best < __ldcg(of)) atomicMin(of, best);
+    }
+}
+
+// A block per instance: its elements' material, its nodes' velocity and fixed bits, and its
+// local node numbers moved to the batch's.
+__global__ void __launch_bounds__(SB) k_batch_fill(Dev d, const BatchInst *inst,
+                                                   const double2 *velocity) {
+    const BatchInst &in = inst[blockIdx.x];
+    const double2 v = velocity[blockIdx.x];
+    for (int n = in.n0 + threadIdx.x; n < in.n1; n += SB) {
+        d.V[n] = v;
+        d.flags[n] &= 3;
+    }
+    for (int e = in.e0 + threadIdx.x; e < in.e1; e += SB) {
+        const int4 c = d.conn[e];
+        d.conn[e] = make_int4(c.x + in.n0, c.y + in.n0, c.z + in.n0, c.w + in.n0);
+        d.emat[e] = blockIdx.x;
+    }
+    for (int k = in.k0 + threadIdx.x; k < in.k1; k += SB) {
+        const int2 p = d.pedges[k];
+        d.pedges[k] = make_int2(p.x + in.n0, p.y + in.n0);
+    }
 }
 
 // The sources of every node: element corner q (slot 8 e + corner), pressure-edge end k.
@@ -62,7 +90,7 @@ __global__ void __launch_bounds__(SB) k_count(Dev d, int *sources, int *edges) {
     const long long q = (long long)blockIdx.x * SB + threadIdx.x;
     if (q >= 4LL * d.E + 2LL * d.K) return;
     atomicAdd(&sources[source_node(d, q)], 1);
-    if (q < 4LL * d.E) atomicAdd(&edges[min(conn_at(d, q), edge_end(d, q))], 1);
+    if (edges && q < 4LL * d.E) atomicAdd(&edges[min(conn_at(d, q), edge_end(d, q))], 1);
 }
 // The most elements around a node (its corners, counted once each).
 __global__ void __launch_bounds__(SB) k_corners(Dev d, int *corners) {
@@ -81,7 +109,7 @@ __global__ void __launch_bounds__(SB) k_file(Dev d, int *sources, int *edges, co
     if (q >= 4LL * d.E + 2LL * d.K) return;
     const int n = source_node(d, q);
     sourceBin[d.nodeSlotStart[n] + atomicSub(&sources[n], 1) - 1] = source_slot(d, q);
-    if (q < 4LL * d.E) {
+    if (edges && q < 4LL * d.E) {
         const int lo = min(conn_at(d, q), edge_end(d, q));
         edgeBin[edgeStart[lo] + atomicSub(&edges[lo], 1) - 1] = (int)q;
     }
@@ -99,7 +127,7 @@ __global__ void __launch_bounds__(SB) k_rank(Dev d, const int *edgeStart, const 
         for (int j = begin; j < end; j++) rank += sourceBin[j] < slot;
         d.nodeSlot[begin + rank] = slot;
     }
-    if (q < 4LL * d.E) {
+    if (edgeStart && q < 4LL * d.E) {
         const int a = conn_at(d, q), b = edge_end(d, q);
         const int lo = min(a, b), hi = max(a, b);
         const int begin = edgeStart[lo], end = edgeStart[lo + 1];
@@ -204,12 +232,21 @@ __global__ void __launch_bounds__(SB) k_damage_geometry(Dev d) {
         const double2 i = p[k], j = p[(k + 1) & 3];
         a += i.x * j.y - j.x * i.y;
     }
-    double *o = d.dGeom + 5 * (size_t)e;
+    double o[5];
     o[0] = fabs(0.5 * a);
     o[1] = 0.5 * (p[1].x - p[0].x + p[2].x - p[3].x);
     o[2] = 0.5 * (p[1].y - p[0].y + p[2].y - p[3].y);
     o[3] = 0.5 * (p[3].x - p[0].x + p[2].x - p[1].x);
     o[4] = 0.5 * (p[3].y - p[0].y + p[2].y - p[1].y);
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        d.dGeom[5 * (size_t)e + k] = o[k];
+        if (d.dGeomF) d.dGeomF[5 * (size_t)e + k] = (float)o[k];
+    }
+    if (d.dGeomF) {
+        d.dFailF[e] = (float)d.dFail[e];
+        d.dGfF[e] = (float)d.dGf[e];
+    }
 }
 
 // The end nodes of every element edge (QuadMesh.surface's edge k of element e runs from corner
@@ -226,20 +263,24 @@ __global__ void __launch_bounds__(SB) k_component(const double2 *src, double *ds
     if (i < n) dst[i] = y ? src[i].y : src[i].x;
 }
 
+__global__ void __launch_bounds__(SB) k_widen(const float *src, double *dst, int n, int stride) {
+    const int i = blockIdx.x * SB + threadIdx.x;
+    if (i < n) dst[i] = src[(size_t)i * stride];
+}
+
 size_t setup_scratch_ints(int N, int E) {
     return scan_tmp_ints(std::max(4 * E, N + 1)) + 4 * ((size_t)N + 1) + 1;
 }
 
-// conn, emat, mats, pedges and s are uploaded, and r and z into U. The lists in between use
+// conn, emat, mats and pedges are in place, and r and z in U. The lists in between use
 // `contribution`, which like U is zeroed again, and `scratch` (setup_scratch_ints, zeroed).
-// Returns where the greatest number of elements around a node will be.
-int *launch_setup(Solver &S, int *scratch) {
-    Dev &d = S.d;
-    cudaStream_t st = S.stream;
+static void node_arrays(Dev &d, cudaStream_t st, int *scratch, bool surface,
+                        unsigned long long *instances) {
     const int N = d.N, E = d.E;
     const long long entries = 4LL * E + 2LL * d.K;
-    int *sources = scratch, *edges = sources + N + 1, *edgeStart = edges + N + 1;
-    int *corners = edgeStart + N + 1, *most = corners + N + 1, *tmp = most + 1;
+    int *sources = scratch, *edges = surface ? sources + N + 1 : nullptr;
+    int *edgeStart = surface ? edges + N + 1 : nullptr;
+    int *tmp = scratch + 4 * ((size_t)N + 1) + 1;
     int *sourceBin = reinterpret_cast<int *>(d.contribution), *edgeBin = sourceBin + entries;
     int *head = edgeBin + 4LL * E, *before = head + 4LL * E;   // 16 E + 2 K of 16 (E + K)
     const double *r = reinterpret_cast<const double *>(d.U);
@@ -247,35 +288,62 @@ int *launch_setup(Solver &S, int *scratch) {
     cudaMemsetAsync(d.U, 0, sizeof(double2) * (size_t)N, st);
     if (entries > 0) {
         const int grid = grid_for(entries, SB);
-        if (E > 0) k_shortest_edge<<<grid_for(E, SB), SB, 0, st>>>(d);
+        if (E > 0) k_shortest_edge<<<grid_for(E, SB), SB, 0, st>>>(d, instances);
         k_count<<<grid, SB, 0, st>>>(d, sources, edges);
-        if (E > 0) k_corners<<<grid_for(4LL * E, SB), SB, 0, st>>>(d, corners);
-        k_most<<<grid_for(N, SB), SB, 0, st>>>(N, corners, most);
         scan_exclusive(sources, d.nodeSlotStart, N + 1, nullptr, tmp, st, nullptr, nullptr);
-        scan_exclusive(edges, edgeStart, N + 1, nullptr, tmp, st, nullptr, nullptr);
+        if (surface) scan_exclusive(edges, edgeStart, N + 1, nullptr, tmp, st, nullptr, nullptr);
         k_file<<<grid, SB, 0, st>>>(d, sources, edges, edgeStart, sourceBin, edgeBin);
         k_rank<<<grid, SB, 0, st>>>(d, edgeStart, sourceBin, edgeBin);
     }
-    if (E > 0) {
+    if (E > 0 && surface) {
         const int grid = grid_for(4LL * E, SB);
         k_heads<<<grid, SB, 0, st>>>(d, head);
         scan_exclusive(head, before, 4 * E, nullptr, tmp, st, nullptr, nullptr);
         k_groups<<<grid, SB, 0, st>>>(d, head, before);
-        k_lump_volumes<<<grid_for(E, SB), SB, 0, st>>>(d, reinterpret_cast<double4 *>(d.contribution));
     }
-    if (N > 0)
-        k_lump<<<grid_for(N, SB), SB, 0, st>>>(d, reinterpret_cast<const double4 *>(d.contribution));
+    double4 *volumes = reinterpret_cast<double4 *>(d.contribution);
+    if (E > 0) k_lump_volumes<<<grid_for(E, SB), SB, 0, st>>>(d, volumes);
+    if (N > 0) k_lump<<<grid_for(N, SB), SB, 0, st>>>(d, volumes);
     cudaMemsetAsync(d.contribution, 0, sizeof(double) * 8 * ((size_t)E + d.K), st);
+}
+
+// A scene's arrays; its shortest edge goes to s. Returns where the greatest number of elements
+// around a node will be.
+int *launch_setup(Solver &S, int *scratch) {
+    Dev &d = S.d;
+    node_arrays(d, S.stream, scratch, true, nullptr);
+    int *corners = scratch + 3 * ((size_t)d.N + 1), *most = corners + d.N + 1;
+    if (d.E > 0) {
+        k_corners<<<grid_for(4LL * d.E, SB), SB, 0, S.stream>>>(d, corners);
+        k_most<<<grid_for(d.N, SB), SB, 0, S.stream>>>(d.N, corners, most);
+    }
     return most;
 }
-void launch_damage_geometry(Solver &S) {
-    if (S.d.E > 0) k_damage_geometry<<<grid_for(S.d.E, SB), SB, 0, S.stream>>>(S.d);
+// A batch's: conn and pedges arrive with the instances' local numbers, flags as the caller's
+// bytes, `edges` (per instance) at infinity.
+void launch_batch_setup(Dev &d, const BatchInst *inst, int count, const double2 *velocity,
+                        unsigned long long *edges, int *scratch, cudaStream_t st) {
+    k_batch_fill<<<count, SB, 0, st>>>(d, inst, velocity);
+    node_arrays(d, st, scratch, false, edges);
+}
+void setup_damage_geometry(Dev &d, cudaStream_t st) {
+    if (d.E > 0) k_damage_geometry<<<grid_for(d.E, SB), SB, 0, st>>>(d);
 }
 void launch_segments(Solver &S) {
     if (S.d.E > 0) k_segments<<<grid_for(4LL * S.d.E, SB), SB, 0, S.stream>>>(S.d);
 }
-void launch_component(Solver &S, const double2 *src, double *dst, size_t count, int y) {
-    k_component<<<grid_for((long long)count, SB), SB, 0, S.stream>>>(src, dst, (int)count, y);
+void launch_component(const double2 *src, double *dst, size_t count, int y, cudaStream_t st) {
+    k_component<<<grid_for((long long)count, SB), SB, 0, st>>>(src, dst, (int)count, y);
+}
+void launch_widen(const float *src, double *dst, size_t count, int stride, cudaStream_t st) {
+    k_widen<<<grid_for((long long)count, SB), SB, 0, st>>>(src, dst, (int)count, stride);
+}
+// The destination's pages first: a copy of 32 MB into pages not mapped yet took 13.6 ms (the
+// device faults them in one by one), with them touched it takes 1.3 ms.
+cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+    for (size_t i = 0; i < bytes; i += 4096) ((volatile char *)dst)[i] = 0;
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
 }
 
 }  // namespace nf

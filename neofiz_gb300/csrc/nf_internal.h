@@ -408,20 +408,18 @@ MatDev material_constants(const nf_material &m, int formulation);
 double material_wave(const nf_material &m);
 MatF material_constants_f32(const MatDev &m);
 double element_signed_area(const double *r, const double *z, const int32_t *conn, int e);
-void setup_lumped_mass(const double *r, const double *z, const int32_t *conn, int E,
-                       const nf_material *materials, const int32_t *emat, bool axi,
-                       double thickness, double *mass);
-void setup_node_slots(const int32_t *conn, int N, int E, const int32_t *pedges, int K,
-                      int32_t *slotStart, int32_t *slots);
-double setup_min_edge(const double *r, const double *z, const int32_t *conn, int E);
 void set_thread_error(const char *message);
 
 // Launchers (k_setup.cu)
 size_t setup_scratch_ints(int N, int E);
 int *launch_setup(Solver &S, int *scratch);
-void launch_damage_geometry(Solver &S);
+void launch_batch_setup(Dev &d, const BatchInst *inst, int count, const double2 *velocity,
+                        unsigned long long *edges, int *scratch, cudaStream_t st);
+void setup_damage_geometry(Dev &d, cudaStream_t st);
 void launch_segments(Solver &S);
-void launch_component(Solver &S, const double2 *src, double *dst, size_t count, int y);
+void launch_component(const double2 *src, double *dst, size_t count, int y, cudaStream_t st);
+void launch_widen(const float *src, double *dst, size_t count, int stride, cudaStream_t st);
+cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t st);
 
 // Launchers (k_step.cu). Each returns the number of kernels it enqueued.
 int launch_initial_assembly(Solver &S);
