@@ -2,9 +2,10 @@
 // thread through Sweep.over, src/main/java/org/neofiz/app/Sweep.java:82-105) stepped by one
 // persistent kernel.
 //
-// One block owns one instance at a time and runs its whole step with block barriers between
-// the phases: nodal update, element assembly with the block's exact minimum edge, the
-// per-node gather, the next CFL step. Blocks take instances from a queue (most expensive
+// One block, or for a batch with fewer instances than fill the device a cluster of up to eight
+// (choose_team), owns one instance at a time and runs its whole step with block or cluster
+// barriers between the phases: nodal update, element assembly with the block's exact minimum edge, the
+// per-node gather, the next CFL step. They take instances from a queue (most expensive
 // first), each for a chunk of steps, so uneven meshes and uneven step counts balance. Every
 // phase calls the same per-node and per-element bodies as the single-scene kernels
 // (nf_bodies.cuh), in the same order per node and per element, so an instance's trajectory is
@@ -12,7 +13,7 @@
 // impulse, energy loss, friction work) are summed per block in a fixed order: deterministic
 // for a given launch shape, but not in the single-scene kernels' association.
 //
-// Launch shape: block size (128, 256), whether the mixed form stages each instance's float
+// Launch shape: block size (32, 128, 256), whether the mixed form stages each instance's float
 // node geometry in shared memory, blocks per SM and the chunk length are chosen by the
 // autotuner (api_batch.cu); none of them changes the trajectory.
 #include "nf_batch_kernels.cuh"
@@ -228,17 +229,22 @@ void batch_teams(int mode, const BatchShape &s, int sms, int (&teams)[4]) {
     }
 }
 
-// Resident blocks per SM of a shape (0 when it cannot launch, e.g. too much shared memory).
+// Resident blocks per SM of a shape (0 when it cannot launch, e.g. too much shared memory). The
+// lone and the shared kernel are both made ready: which one a launch takes depends on the blocks
+// per SM that the answer bounds.
 int batch_max_blocks_per_sm(int mode, const BatchShape &s, int maxNodes, int maxElems) {
-    const void *k = select_kernel(mode, s, lone_warps(s, maxElems, 1), false);
     const size_t smem = batch_shared_bytes(mode, s, maxNodes);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return 0;
+    for (const bool lone : {false, true}) {
+        if (smem > 48 * 1024 &&
+            cudaFuncSetAttribute(select_kernel(mode, s, lone, false),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return 0;
+        }
     }
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, s.threads, smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &n, select_kernel(mode, s, lone_warps(s, maxElems, 1), false), s.threads, smem) != cudaSuccess) {
         (void)cudaGetLastError();
         return 0;
     }

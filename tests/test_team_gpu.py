@@ -55,3 +55,28 @@ def test_compensated_team_equals_one_block(gpu_lib):
             assert np.array_equal(few.readInstance(f, k), many.readInstance(f, k))
     few.close()
     many.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [_abi.PRECISION_FP64, _abi.PRECISION_MIXED,
+                                       _abi.PRECISION_COMPENSATED])
+def test_tuning_tries_staged_nodes_above_48_kb(gpu_lib, precision):
+    """2,525 nodes staged take 60 kB: every shape of the tuner launches, whichever of the lone
+    and the shared kernel its blocks per SM select, and the run goes on as if untuned."""
+    rods = scenes.taylor_sweep(3, seed=2, t_end=1.0)
+    for r in rods:
+        r.update(nr=24, nz=100)
+    batches = [BatchSolver(scenes.sweep_instances(rods), Formulation.AXISYMMETRIC, cfl=0.6,
+                           precision=precision) for _ in range(2)]
+    batches[0].tune(2)
+    if precision != _abi.PRECISION_COMPENSATED:           # its one-warp kernels round differently
+        for b in batches:
+            b.run(12)
+        for f in (_abi.FIELD_UR, _abi.FIELD_UZ, _abi.FIELD_STRESS):
+            assert np.array_equal(batches[0].read(f), batches[1].read(f)), f
+    if precision == _abi.PRECISION_MIXED:
+        for blocks in (1, 2):
+            batches[0].setConfig(128, 1, blocks, 8)
+            batches[0].run(8)
+    for b in batches:
+        b.close()
