@@ -41,8 +41,9 @@ L2_FLUSH_BYTES = 256 << 20
 # start + 6 and start + 7 (ncu cannot run inside the timed bench)
 ELEMENT_TRAFFIC_BYTES = {CELL: (43_483_904 + 173_568 + 43_474_176 + 36_864) // 2}
 # FP64-pipe warp instructions of one element-pass launch in the window: the mean of ncu's
-# smsp__inst_executed_pipe_fp64.sum over the same two launches
-ELEMENT_FP64_WARP_INST = {CELL: (3_078_533 + 3_061_133) // 2}
+# smsp__inst_executed_pipe_fp64.sum over ten launches (steps start + 6 to start + 15; 1.4216 to
+# 1.4281 M)
+ELEMENT_FP64_WARP_INST = {CELL: 1_424_664}
 
 
 def parse():
@@ -370,8 +371,8 @@ def fp64_roofline(elem_ms, cell):
         achieved = count / (elem_ms * 1e-3)
         out.update({"achieved": achieved, "frac": achieved / rate,
                     "fp64_warp_inst_per_launch": count,
-                    "count_source": "ncu smsp__inst_executed_pipe_fp64.sum, one launch of the "
-                                    "window"})
+                    "count_source": "ncu smsp__inst_executed_pipe_fp64.sum, the mean of ten "
+                                    "launches of the window"})
     return out
 
 
