@@ -32,13 +32,16 @@
 #define NF_LN2_128_1 0xefa39ef3u
 #define NF_LN2_128_2 0x0162e42fu
 
+/* A row of the logarithm's table; the device reads its first four words as one 16-byte load. */
+struct alignas(16) nf_log_row { uint32_t w[8]; };
+
 #if defined(__CUDACC__)
 #define NF_ILOG_SLOW static __host__ __device__ __noinline__
-static __device__ const uint32_t nf_log_words_d[8 * 128] = { NF_LOG_WORDS };
+static __device__ const nf_log_row nf_log_rows_d[128] = { NF_LOG_WORDS };
 #else
 #define NF_ILOG_SLOW static
 #endif
-static const uint32_t nf_log_words_h[8 * 128] = { NF_LOG_WORDS };
+static const nf_log_row nf_log_rows_h[128] = { NF_LOG_WORDS };
 
 /* Counts the slow paths in host tests. */
 #if !defined(__CUDA_ARCH__)
@@ -86,11 +89,11 @@ NF_IFP int nf_ilog_of(double x, nf_ilog *o) {
     const uint32_t j = (th >> 13) & 127u;
     const uint32_t hz = (uint32_t)(NF_LOG_OFF >> 32) + (th & 0xfffffu);
 #if defined(__CUDA_ARCH__)
-    const uint4 wa = __ldg(reinterpret_cast<const uint4 *>(nf_log_words_d) + 2 * j);
+    const uint4 wa = __ldg(reinterpret_cast<const uint4 *>(nf_log_rows_d[j].w));
     const uint32_t il = wa.x, ih = wa.y, c0 = wa.z, c1 = wa.w;
-    const uint32_t c2 = __ldg(nf_log_words_d + 8 * j + 4);
+    const uint32_t c2 = __ldg(nf_log_rows_d[j].w + 4);
 #else
-    const uint32_t *w = nf_log_words_h + 8 * j;
+    const uint32_t *w = nf_log_rows_h[j].w;
     const uint32_t il = w[0], ih = w[1], c0 = w[2], c1 = w[3], c2 = w[4];
 #endif
     /* P = (z 2^53) (invc 2^53), r = P 2^-106 - 1 in words p0, p1, t (signed) */
