@@ -400,7 +400,8 @@ typedef struct {
 typedef struct {
     int32_t threads;                 /* threads per block: 32, 128 or 256 */
     int32_t stage_nodes;             /* mixed form: node geometry staged in shared memory */
-    int32_t blocks_per_sm;           /* resident blocks per SM (1 .. occupancy limit) */
+    int32_t blocks_per_sm;           /* blocks per SM, 1 .. as many as are resident (FP64: up to
+                                        384 threads of them in any case) */
     int32_t chunk_steps;             /* steps an instance takes per launch */
 } nf_batch_config;
 

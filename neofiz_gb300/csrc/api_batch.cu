@@ -121,25 +121,34 @@ bool shape_valid(const Batch &B, const BatchShape &s) {
     if (s.threads != 32 && s.threads != 128 && s.threads != 256) return false;
     if (s.stage && !B.mixed) return false;
     if (s.chunk < 1 || s.blocksPerSm < 1) return false;
-    return batch_max_blocks_per_sm(B.mode, s, B.b.maxNodes, B.b.maxElems) >= s.blocksPerSm;
+    const int resident = batch_max_blocks_per_sm(B.mode, s, B.b.maxNodes, B.b.maxElems);
+    return resident > 0 && s.blocksPerSm <= std::max(resident, batch_blocks_promised(B.mode, s));
+}
+
+// The batch's shape as launched: no more blocks per SM than are resident.
+BatchShape launched_shape(const Batch &B) {
+    BatchShape s = B.shape;
+    const int resident = batch_max_blocks_per_sm(B.mode, s, B.b.maxNodes, B.b.maxElems);
+    if (resident > 0) s.blocksPerSm = std::min(s.blocksPerSm, resident);
+    return s;
 }
 
 // Blocks per instance while the `left` most expensive instances run (the cheap ones finish
 // first, and those left spread over more blocks), and the teams resident.
-int team_of(const Batch &B, int left, int *teams) {
+int team_of(const Batch &B, const BatchShape &shape, int left, int *teams) {
     int n[4];
-    batch_teams(B.mode, B.shape, B.sms, n);
+    batch_teams(B.mode, shape, B.sms, n);
     const int team = choose_team(B.elems.data(), std::max(1, std::min(left, B.count)), n);
     *teams = team == 1 ? n[0] : team == 2 ? n[1] : team == 4 ? n[2] : n[3];
     return team;
 }
 
 // The run's launches: reset the queue, launch one chunk; GRAPH_CHUNKS times.
-cudaError_t enqueue_chunks(Batch &B, int chunks, int team, int teams) {
+cudaError_t enqueue_chunks(Batch &B, const BatchShape &shape, int chunks, int team, int teams) {
     for (int c = 0; c < chunks; c++) {
         cudaError_t e = cudaMemsetAsync(B.b.queue, 0, sizeof(int32_t), B.stream);
         if (e != cudaSuccess) return e;
-        e = launch_batch_steps(B.d, B.b, B.mode, B.shape, team, teams, B.stream);
+        e = launch_batch_steps(B.d, B.b, B.mode, shape, team, teams, B.stream);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -149,14 +158,15 @@ nf_status ensure_graph(Batch &B, int left) {
     const bool sameShape = B.graph && memcmp(&B.graphShape, &B.shape, sizeof(BatchShape)) == 0;
     if (sameShape && B.graphLeft == left) return NF_OK;
     int teams = 1;
-    const int team = team_of(B, left, &teams);
+    const BatchShape shape = launched_shape(B);
+    const int team = team_of(B, shape, left, &teams);
     B.graphLeft = left;
     if (sameShape && B.graphTeam == team) return NF_OK;
     if (B.graph) cudaGraphExecDestroy(B.graph);
     B.graph = nullptr;
     cudaGraph_t g = nullptr;
     BCK(&B, cudaStreamBeginCapture(B.stream, cudaStreamCaptureModeThreadLocal));
-    const cudaError_t launched = enqueue_chunks(B, GRAPH_CHUNKS, team, teams);
+    const cudaError_t launched = enqueue_chunks(B, shape, GRAPH_CHUNKS, team, teams);
     const cudaError_t ended = cudaStreamEndCapture(B.stream, &g);
     if (launched != cudaSuccess || ended != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -627,8 +637,8 @@ nf_status nf_batch_tune(nf_batch *h, int32_t trial_steps, nf_batch_config *chose
             cudaEventRecord(B.ev0, B.stream);
             launch_batch_arm(B.b, trial_steps, B.stream);
             int teams = 1;
-            const int team = team_of(B, B.count, &teams);
-            cudaError_t e = enqueue_chunks(B, 1, team, teams);
+            const int team = team_of(B, B.shape, B.count, &teams);
+            cudaError_t e = enqueue_chunks(B, B.shape, 1, team, teams);
             cudaEventRecord(B.ev1, B.stream);
             B.launches += 2;
             if (e == cudaSuccess) e = cudaStreamSynchronize(B.stream);

@@ -251,6 +251,14 @@ int batch_max_blocks_per_sm(int mode, const BatchShape &s, int maxNodes, int max
     return n;
 }
 
+// Blocks per SM that a shape may ask for even where fewer are resident: the FP64 kernels once
+// took 168 registers a thread, 384 threads an SM (1, 3 and 12 blocks of 256, 128 and 32), and
+// shapes chosen then, by hand or by the tuner, stay valid. They launch what is resident: the
+// blocks share a queue, and further ones would find it empty.
+int batch_blocks_promised(int mode, const BatchShape &s) {
+    return mode == NF_PRECISION_FP64 ? 384 / s.threads : 0;
+}
+
 // team: blocks per instance (choose_team); teams: how many of them.
 cudaError_t launch_batch_steps(const Dev &d, const BatchDev &b, int mode, const BatchShape &s,
                                int team, int teams, cudaStream_t st) {

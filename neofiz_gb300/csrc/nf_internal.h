@@ -387,6 +387,7 @@ struct BatchShape {
 // Launchers (k_batch.cu).
 // mode: NF_PRECISION_FP64, NF_PRECISION_MIXED or NF_PRECISION_COMPENSATED
 int batch_max_blocks_per_sm(int mode, const BatchShape &shape, int maxNodes, int maxElems);
+int batch_blocks_promised(int mode, const BatchShape &shape);
 size_t batch_shared_bytes(int mode, const BatchShape &shape, int maxNodes);
 void launch_batch_initial(const Dev &d, const BatchDev &b, bool mixed, cudaStream_t st);
 void launch_batch_arm(const BatchDev &b, long long maxSteps, cudaStream_t st);

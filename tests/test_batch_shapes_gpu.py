@@ -1,0 +1,34 @@
+"""Launch shapes of the batch: which are accepted, and that they step the instances alike."""
+import numpy as np
+import pytest
+
+from neofiz_gb300 import _abi, scenes
+from neofiz_gb300.batch import BatchSolver
+from neofiz_gb300.materials import Formulation
+
+pytestmark = pytest.mark.gpu
+
+
+def batch(rods, precision=_abi.PRECISION_FP64):
+    return BatchSolver(scenes.sweep_instances(rods), Formulation.AXISYMMETRIC, cfl=0.6,
+                       precision=precision)
+
+
+@pytest.mark.parametrize("threads,blocks", [(256, 1), (128, 3), (32, 12)])
+def test_fp64_shapes_of_384_threads_per_sm_are_accepted(gpu_lib, threads, blocks):
+    """Shapes that FP64 batches took when their kernels held 168 registers a thread."""
+    rods = scenes.taylor_sweep(5, seed=4, t_end=1.0)
+    for r in rods:
+        r.update(nr=5, nz=23)
+    a, b = batch(rods), batch(rods)
+    a.setConfig(threads, 0, blocks, 16)
+    assert a.config() == {"threads": threads, "stage_nodes": 0, "blocks_per_sm": blocks,
+                          "chunk_steps": 16}
+    with pytest.raises(ValueError):
+        a.setConfig(threads, 0, blocks + 1, 16)
+    for s in (a, b):
+        s.run(30)
+    for f in (_abi.FIELD_UR, _abi.FIELD_UZ, _abi.FIELD_STRESS):
+        assert np.array_equal(a.read(f), b.read(f)), f
+    a.close()
+    b.close()
