@@ -2,7 +2,7 @@
 // measurement with respect to Johnson-Cook A, B, n, C, m, the kinematic hardening modulus and
 // the wall friction. There is no adjoint in the reference.
 //
-// One block owns one instance. The forward kernel runs the instance to its t_end with the
+// One block, or a cluster of them (choose_team), owns one instance. The forward kernel runs the instance to its t_end with the
 // batched step (nf_batch_step.cuh, bit-identical to the plain path) and saves the whole state
 // every `every` steps. The backward kernel walks the segments from the last: it restores the
 // segment's checkpoint, re-runs the segment saving the state before each step (the tape) and
@@ -10,7 +10,9 @@
 // update recomputed from the tape, the element reverse (its forward recomputed in the same
 // order, so every branch is the forward's), the per-node gather of the elements' adjoints in
 // the forward gather's order, the nodal reverse, and the CFL step's dependence on the
-// shortest edge. Per-thread parameter adjoints are summed by a fixed tree at the end.
+// shortest edge. Every sum over nodes or elements is team_sums', so an instance's gradients and
+// its sampled peak do not depend on its neighbours. The parameters' adjoints add up by lane in
+// global memory, in the thread that owns the element or node, over every step of the sweep.
 #include "nf_batch_step.cuh"
 #include "nf_adjoint.h"
 
@@ -28,13 +30,21 @@ struct StateBlock {
 
 __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~(size_t)15; }
 
+// The lanes that an instance's parameter adjoints are summed in (team_sums): whole warps.
+constexpr int PARAM_LANES = TEAM_MAX * ADJ_T;
+__host__ __device__ inline int param_lanes(int n, int e) {
+    const int items = ((n > e ? n : e) + 31) & ~31;
+    return items < PARAM_LANES ? items : PARAM_LANES;
+}
+
 size_t adj_state_bytes(int n, int e) {
     return 3 * al16(16 * (size_t)n) + 2 * al16(32 * (size_t)e) + al16(16 * (size_t)e)
            + 5 * al16(8 * (size_t)e) + 64 + al16((size_t)n);
 }
 size_t adj_bar_bytes(int n, int e, int k) {
     return 3 * al16(16 * (size_t)n) + 2 * al16(32 * (size_t)e) + al16(16 * (size_t)e)
-           + 4 * al16(8 * (size_t)e) + al16(128 * (size_t)e) + al16(32 * (size_t)k);
+           + 4 * al16(8 * (size_t)e) + al16(128 * (size_t)e) + al16(32 * (size_t)k)
+           + 8 * NF_ADJ_P_COUNT * (size_t)param_lanes(n, e);
 }
 size_t adj_seed_bytes(int n, int e) { return al16(16 * (size_t)n) + al16(32 * (size_t)e); }
 
@@ -62,6 +72,7 @@ struct BarBlock {
     double *sig, *back, *epsP, *wP, *corner;   // corner: 16 per element (4 corners x ur uz vr vz)
     double *dStr, *dSoft;                      // damage state
     double *edge;                              // 4 per pressure edge: a (r, z), b (r, z)
+    double *param;                             // the parameters' adjoints so far, by lane
 };
 
 __device__ BarBlock bar_at(char *p, int n, int e, int k) {
@@ -78,6 +89,7 @@ __device__ BarBlock bar_at(char *p, int n, int e, int k) {
     s.dSoft = (double *)p; p += al16(8 * (size_t)e);
     s.corner = (double *)p; p += al16(128 * (size_t)e);
     s.edge = (double *)p; p += al16(32 * (size_t)k);
+    s.param = (double *)p;
     return s;
 }
 
@@ -158,16 +170,17 @@ __device__ void elem_in(const Dev &d, const BatchInst &in, const StateBlock &pre
 }
 
 // BurstCase.loadCapacity (BurstCase.java:533-553) of the instance's current state: the hoop
-// stress times the current element area summed by a fixed tree, over the bore radius and the
-// height (exact extrema). Valid in every thread.
+// stress times the current element area (team_sums), over the bore radius and the height (exact
+// extrema). Valid in every thread.
 template <int T, bool TEAM>
 __device__ double capacity_of(const Team<TEAM> &team, const Dev &d, const BatchInst &in,
                               double *shRed) {
-    __shared__ double parts[TEAM ? TEAM_MAX : 1][4];     // hoop, bore, low, high of each block
+    __shared__ double parts[TEAM ? TEAM_MAX : 1][3];     // bore, low, high of each block
+    __shared__ double table[T * TEAM_MAX / 32][1];
     __shared__ double result;
     const int tid = team.tid(), stride = TEAM ? team.size * T : T;
-    double hoop = 0.0;
-    for (int e = in.e0 + tid; e < in.e1; e += stride) {
+    double hoop[SUM_SLOTS<TEAM>][1] = {};
+    for (int e = in.e0 + tid, slot = 0; e < in.e1; e += stride, slot = next_slot(team, slot)) {
         const int4 c = d.conn[e];
         const int nn[4] = {c.x, c.y, c.z, c.w};
         double sum = 0.0;
@@ -181,9 +194,8 @@ __device__ double capacity_of(const Team<TEAM> &team, const Dev &d, const BatchI
             }
             sum += ri * zj - rj * zi;
         }
-        hoop += d.sig[4 * (size_t)e + 2] * (0.5 * sum);
+        hoop[slot][0] += d.sig[4 * (size_t)e + 2] * (0.5 * sum);
     }
-    const double total = block_total<T>(hoop, shRed);
     double bore = DMAX, low = DMAX, high = -DMAX;
     for (int i = in.n0 + tid; i < in.n1; i += stride) {
         const double2 x = d.X0[i];
@@ -214,16 +226,14 @@ __device__ double capacity_of(const Team<TEAM> &team, const Dev &d, const BatchI
     if (threadIdx.x == 0)
         for (int r = 0; r < team.size; r++) {
             double *o = team.at(parts, r)[team.rank];
-            o[0] = total; o[1] = ext[0]; o[2] = ext[1]; o[3] = ext[2];
+            o[0] = ext[0]; o[1] = ext[1]; o[2] = ext[2];
         }
-    team.sync();
+    double total[1];
+    team_sums<TEAM, T, 1>(team, in.e1 - in.e0, hoop, table, total);
     if (threadIdx.x == 0) {
-        double sum = 0.0;
-        for (int r = 0; r < team.size; r++) {
-            sum += parts[r][0];
-            for (int q = 0; q < 3; q++) ext[q] = fmin(ext[q], parts[r][1 + q]);
-        }
-        result = sum / (ext[0] * (-ext[2] - ext[1]));
+        for (int r = 0; r < team.size; r++)
+            for (int q = 0; q < 3; q++) ext[q] = fmin(ext[q], parts[r][q]);
+        result = total[0] / (ext[0] * (-ext[2] - ext[1]));
     }
     team.sync();
     return result;
@@ -323,8 +333,8 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev
 // equal in all of them.
 template <bool INT, bool TEAM>
 __device__ void reverse_step(const Team<TEAM> &team, const Dev &d, const BatchInst &in,
-                             const MatDev &mat, StateBlock pre, BarBlock bar, double *pacc,
-                             double *shRed, double (*slots)[4], int *owner0, double *shDtb,
+                             const MatDev &mat, StateBlock pre, BarBlock bar,
+                             double (*table)[4], int *owner0, double *shDtb,
                              double *shDtPrevb, double *shTimeb, int *scratch) {
     const int n = in.n1 - in.n0, e = in.e1 - in.e0;
     const int tid = team.tid(), stride = TEAM ? team.size * ADJ_T : ADJ_T;
@@ -361,8 +371,9 @@ __device__ void reverse_step(const Team<TEAM> &team, const Dev &d, const BatchIn
     team.sync();
     const int owner = *owner0;
     const nf_adj_mat m = adj_mat_of(mat);
-    double dtb = 0.0;
-    for (int le = tid; le < e; le += stride) {
+    const int lanes = param_lanes(n, e);
+    double part[SUM_SLOTS<TEAM>][4] = {};    // the adjoints of decay, gain, dt and time
+    for (int le = tid, slot = 0; le < e; le += stride, slot = next_slot(team, slot)) {
         nf_adj_elem_in x;
         elem_in(d, in, pre, le, &x);
         nf_adj_elem_bar ab;
@@ -382,8 +393,14 @@ __device__ void reverse_step(const Team<TEAM> &team, const Dev &d, const BatchIn
         ab.softening = d.hasDamage ? bar.dSoft[le] : 0.0;
         ab.edgeOwner = le == owner ? nf_adj_edge_owner(&x, dt, finite, minEdge) : -1;
         ab.edgeb = edgeb;
+        double *const param = bar.param + (le & (PARAM_LANES - 1));
+        double pb[NF_ADJ_P_COUNT], dtb = part[slot][2];
+        for (int p = 0; p < NF_ADJ_P_COUNT; p++) pb[p] = param[p * lanes];
         nf_adj_element_reduced(&x, &m, dt, d.axi, finite, d.thickness, in.hourglass, &ab, &dtb,
-                               pacc);
+                               pb);
+        part[slot][2] = dtb;
+        for (int p = 0; p < NF_ADJ_P_COUNT; p++)
+            if (p != NF_ADJ_P_MU) param[p * lanes] = pb[p];
         for (int k = 0; k < 4; k++) {
             bar.sig[4 * le + k] = ab.sig[k];
             bar.back[4 * le + k] = ab.back[k];
@@ -399,21 +416,21 @@ __device__ void reverse_step(const Team<TEAM> &team, const Dev &d, const BatchIn
         }
     }
     // pressure edges, loaded at this step's end time (:1203-1207, :1511-1556)
-    double tpress = 0.0;
     const double tnow = pre.scal[2] + dt;
-    for (int j = tid; j < in.k1 - in.k0; j += stride) {
+    const int nk = in.k1 - in.k0;
+    for (int j = tid, slot = 0; j < nk; j += stride, slot = next_slot(team, slot)) {
         const int2 ed = d.pedges[in.k0 + j];
         const int la = ed.x - in.n0, lb = ed.y - in.n0;
         const double cb[4] = {bar.F[la].x, bar.F[lb].x, bar.F[la].y, bar.F[lb].y};
         const double2 xa = d.X0[ed.x], xb = d.X0[ed.y], ua = d.U[ed.x], ub = d.U[ed.y];
         nf_adj_pressure_edge(xa.x, xa.y, xb.x, xb.y, ua.x, ua.y, ub.x, ub.y, tnow, in.pressure,
                              in.ramp, d.axi, finite, d.thickness, cb, bar.edge + 4 * (size_t)j,
-                             bar.edge + 4 * (size_t)j + 2, &tpress);
+                             bar.edge + 4 * (size_t)j + 2, &part[slot][3]);
     }
     team.sync();
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int i = tid; i < n; i += stride) {
+    for (int i = tid, slot = 0; i < n; i += stride, slot = next_slot(team, slot)) {
         const int g = in.n0 + i;
+        double acc[4] = {part[slot][0], part[slot][1], part[slot][2], 0.0};
         double ub[2] = {bar.U[i].x, bar.U[i].y}, vb[2] = {bar.V[i].x, bar.V[i].y}, fb[2];
         for (int s = d.nodeSlotStart[g]; s < d.nodeSlotStart[g + 1]; s++) {
             const int slot = d.nodeSlot[s];
@@ -433,12 +450,14 @@ __device__ void reverse_step(const Team<TEAM> &team, const Dev &d, const BatchIn
         bar.U[i] = make_double2(ub[0], ub[1]);
         bar.V[i] = make_double2(vb[0], vb[1]);
         bar.F[i] = make_double2(fb[0], fb[1]);
+        for (int q = 0; q < 3; q++) part[slot][q] = acc[q];
+        if (acc[3] != 0.0) bar.param[NF_ADJ_P_MU * lanes + (i & (PARAM_LANES - 1))] += acc[3];
     }
-    pacc[NF_ADJ_P_MU] += acc[3];
-    double sums[4] = {dtb + acc[2], acc[0], acc[1], tpress};
-    team_totals<TEAM, ADJ_T, 4>(team, sums, shRed, slots);
+    double sums[4];
+    const int most = n > e ? n : e;
+    team_sums<TEAM, ADJ_T, 4>(team, most > nk ? most : nk, part, table, sums);
     if (threadIdx.x == 0) {
-        const double tDt = sums[0], tDecay = sums[1], tGain = sums[2], tTime = sums[3];
+        const double tDecay = sums[0], tGain = sums[1], tDt = sums[2], tTime = sums[3];
         const double dtAvgb = nf_adj_dtavg(tDecay, tGain, dtAvg, in.damping);
         *shTimeb += tTime;                      // time' = time + dt
         *shDtb = *shDtPrevb + tDt + 0.5 * dtAvgb + *shTimeb;
@@ -451,12 +470,11 @@ __device__ void reverse_step(const Team<TEAM> &team, const Dev &d, const BatchIn
 template <bool INT, bool TEAM>
 __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDev a) {
     __shared__ double shMin[ADJ_T / 32 + 1];
-    __shared__ double shRed[ADJ_T / 32 + 1];
     __shared__ int shOwner;
     __shared__ int scratch[3];                   // wall counts and status of recomputed steps
     __shared__ double shDtb[NF_ADJ_MAX_WIDTH], shDtPrevb[NF_ADJ_MAX_WIDTH];
     __shared__ double shTimeb[NF_ADJ_MAX_WIDTH];
-    __shared__ double slots[TEAM ? TEAM_MAX : 1][4], gradSlots[TEAM ? TEAM_MAX : 1][NF_ADJ_P_COUNT];
+    __shared__ double table[PARAM_LANES / 32][4], grads[PARAM_LANES / 32][NF_ADJ_P_COUNT];
     __shared__ BlockStep bs;
     const Team<TEAM> team;
     const int k = blockIdx.x / team.size;
@@ -470,10 +488,6 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDe
     char *ckpt = a.ckpt + a.ckptOff[k];
     char *tape = a.tape + a.tapeOff[k];
     const int nk = in.k1 - in.k0;
-    // per objective: its parameter adjoints, summed per thread over every step
-    double pacc[NF_ADJ_MAX_WIDTH][NF_ADJ_P_COUNT];
-    for (int w = 0; w < NF_ADJ_MAX_WIDTH; w++)
-        for (int p = 0; p < NF_ADJ_P_COUNT; p++) pacc[w][p] = 0.0;
     if (threadIdx.x == 0) {
         for (int w = 0; w < NF_ADJ_MAX_WIDTH; w++) shDtb[w] = shDtPrevb[w] = shTimeb[w] = 0.0;
         scratch[0] = scratch[1] = scratch[2] = 0;
@@ -524,17 +538,28 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDe
                 }
                 // the forward values each objective's reverse reads are recomputed from the
                 // same tape entry, so every objective sees the same bits
-                reverse_step<INT>(team, d, in, mat, pre, bar, pacc[w], shRed, slots, owner0, &shDtb[w],
-                             &shDtPrevb[w], &shTimeb[w], scratch);
+                reverse_step<INT>(team, d, in, mat, pre, bar, table, owner0, &shDtb[w], &shDtPrevb[w],
+                                  &shTimeb[w], scratch);
             }
         }
     }
-    for (int w = 0; w < W; w++) {
-        team_totals<TEAM, ADJ_T, NF_ADJ_P_COUNT>(team, pacc[w], shRed, gradSlots);
-        if (team.first())
-            for (int p = 0; p < NF_ADJ_P_COUNT; p++)
-                a.grad[((size_t)w * b.count + k) * NF_ADJ_P_COUNT + p] = pacc[w][p];
-        team.sync();
+    if (team.rank == 0) {                    // the gradients from the lanes, in the first block
+        const int lanes = param_lanes(n, e), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        for (int w = 0; w < W; w++) {
+            const BarBlock bar = bar_at(a.bar + w * a.barPlane + a.barOff[k], n, e, nk);
+            for (int v = warp; 32 * v < lanes; v += ADJ_T / 32)
+                for (int p = 0; p < NF_ADJ_P_COUNT; p++) {
+                    const double t = warp_sum(bar.param[p * lanes + 32 * v + lane]);
+                    if (lane == 0) grads[v][p] = t;
+                }
+            __syncthreads();
+            double g[NF_ADJ_P_COUNT];
+            if (warp == 0) table_sums<NF_ADJ_P_COUNT>(grads, lanes / 32, g);
+            if (threadIdx.x == 0)
+                for (int p = 0; p < NF_ADJ_P_COUNT; p++)
+                    a.grad[((size_t)w * b.count + k) * NF_ADJ_P_COUNT + p] = g[p];
+            __syncthreads();
+        }
     }
     // the solver arrays back to the forward's final state
     StateBlock fin = state_at(a.fin + a.finOff[k], n, e);

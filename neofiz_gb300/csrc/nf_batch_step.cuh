@@ -89,6 +89,55 @@ __device__ double block_total(double v, double *sh) {
     return t;
 }
 
+// Sums over an instance's items (nodes, elements, pressure edges) that do not depend on how many
+// blocks step it, and so not on its neighbours in the batch. The items are dealt to 8 T lanes,
+// T of them a block of the widest team: item j adds to lane j mod 8 T, item after item. A team
+// of fewer blocks gives each thread several lanes, one per slot: those of its first, second ...
+// item. Lanes add up by warps and the warps by one tree.
+template <bool TEAM>
+constexpr int SUM_SLOTS = TEAM ? TEAM_MAX / 2 : TEAM_MAX;
+template <bool TEAM>
+__device__ __forceinline__ int next_slot(const Team<TEAM> &team, int slot) {
+    return (slot + 1) & (TEAM_MAX / team.size - 1);
+}
+__device__ __forceinline__ double warp_sum(double v) {
+    // lanes of +0 alone add up to +0: the common case of sums that few items add to
+    if (!__any_sync(0xffffffffu, __double_as_longlong(v) != 0)) return v;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    return v;
+}
+// The tree over the warps' sums: `used` rows of the table, the others zero; valid in the calling
+// warp's first lane.
+template <int COUNT>
+__device__ __forceinline__ void table_sums(const double (*table)[COUNT], int used,
+                                           double (&out)[COUNT]) {
+    const int lane = threadIdx.x & 31;
+    for (int i = 0; i < COUNT; i++) {
+        const double low = lane < used ? table[lane][i] : 0.0;
+        const double high = lane + 32 < used ? table[lane + 32][i] : 0.0;
+        out[i] = warp_sum(low + high);
+    }
+}
+// COUNT sums of `items` items at most from the threads' slots, in out[] of every block's thread 0.
+// `table` has a row per warp of the widest team, block-shared; a team barrier separates one use
+// of it from the next.
+template <bool TEAM, int T, int COUNT>
+__device__ __forceinline__ void team_sums(const Team<TEAM> &team, int items,
+                                          const double (*part)[COUNT], double (*table)[COUNT],
+                                          double (&out)[COUNT]) {
+    const int warps = T / 32 * team.size, lane = threadIdx.x & 31, warp = team.tid() >> 5;
+    int slots = (items + 32 * warps - 1) / (32 * warps);
+    if (slots > TEAM_MAX / team.size) slots = TEAM_MAX / team.size;
+    for (int s = 0; s < slots; s++)
+        for (int i = 0; i < COUNT; i++) {
+            const double v = warp_sum(part[s][i]);
+            if (lane == 0)
+                for (int r = 0; r < team.size; r++) team.at(table, r)[s * warps + warp][i] = v;
+        }
+    team.sync();
+    if (threadIdx.x < 32) table_sums<COUNT>(table, slots * warps, out);
+}
+
 // COUNT block sums added over the team in rank order, in v[] of every block's thread 0.
 // `slots` is block-shared; a team barrier separates one use of it from the next.
 template <bool TEAM, int T, int COUNT>
