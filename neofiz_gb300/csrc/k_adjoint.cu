@@ -244,7 +244,7 @@ template <bool INT, bool TEAM>
 __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev a) {
     __shared__ double shMin[ADJ_T / 32 + 1];
     __shared__ int wallCount[2][2];
-    __shared__ double slots[TEAM ? TEAM_MAX : 1][3];
+    __shared__ double table[TEAM ? ADJ_T * TEAM_MAX / 32 : 1][3];
     __shared__ BlockStep bs;
     const Team<TEAM> team;
     const int k = blockIdx.x / team.size;
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev
     double dt = scp->dt, dtPrev = scp->dtPrevious, time = scp->time;
     double minEdge = scp->minEdgeSquared;
     long long steps = scp->steps;
-    double wall[3] = {0.0, 0.0, 0.0};        // impulse, energy loss, friction work
+    double wall[WALL_SLOTS<TEAM, ADJ_T>][3] = {};    // impulse, energy loss, friction work
     if (threadIdx.x == 0) {
         wallCount[0][0] = wallCount[0][1] = wallCount[1][0] = wallCount[1][1] = 0;
         block_step_init(bs, d, in, dt, dtPrev);
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev
         }
         minEdge = batch_step<false, ADJ_T, false, INT, TEAM>(
             team, d, in, dt, dtPrev, time, steps, none, nullptr, nullptr, 0, &scp->status,
-            &counts[par][0], &counts[par][1], wall[0], wall[1], wall[2], shMin, &bs);
+            &counts[par][0], &counts[par][1], wall, shMin, &bs);
         if (a.sampleEvery > 0 && steps % a.sampleEvery == 0) {
             team.sync();
             const double cap = capacity_of<ADJ_T>(team, d, in, shMin);
@@ -305,7 +305,8 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev
             }
         }
     }
-    team_totals<TEAM, ADJ_T, 3>(team, wall, shMin, slots);
+    double total[3];
+    wall_totals<TEAM, ADJ_T>(team, n, wall, shMin, table, total);
     StateBlock fin = state_at(a.fin + a.finOff[k], n, e);
     copy_state<ADJ_T>(team, d, in, fin, true);
     if (team.first()) {
@@ -315,7 +316,7 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev
             scp->wContact = wallCount[(taken - 1) & 1][0];
             scp->wStuck = wallCount[(taken - 1) & 1][1];
         }
-        scp->wImpulse += wall[0]; scp->wEnergyLoss += wall[1]; scp->wFriction += wall[2];
+        scp->wImpulse += total[0]; scp->wEnergyLoss += total[1]; scp->wFriction += total[2];
         scp->done = 1;
         a.steps[k] = steps;
         a.peakStep[k] = peakStep;
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDe
         team.sync();
         const long long start = sgi * a.every;
         const long long end = start + a.every < N ? start + a.every : N;
-        double i0 = 0.0, l0 = 0.0, f0 = 0.0;
+        double wall[WALL_SLOTS<TEAM, ADJ_T>][3] = {};   // not looked at
         for (long long j = start; j < end; j++) {
             StateBlock t = state_at(tape + (j - start) * bytes, n, e);
             copy_state<ADJ_T>(team, d, in, t, true);
@@ -515,7 +516,7 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDe
             }
             const double me = batch_step<false, ADJ_T, false, INT, TEAM>(
                 team, d, in, dt, dtPrev, time, steps, none, nullptr, nullptr, 0, scratchStatus,
-                &scratch[0], &scratch[1], i0, l0, f0, shMin, &bs);
+                &scratch[0], &scratch[1], wall, shMin, &bs);
             if (team.first()) t.scal[4] = me;
         }
         team.sync();

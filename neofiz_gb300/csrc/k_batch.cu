@@ -10,8 +10,11 @@
 // phase calls the same per-node and per-element bodies as the single-scene kernels
 // (nf_bodies.cuh), in the same order per node and per element, so an instance's trajectory is
 // bit-identical to the same scene run alone in the same precision. The audit totals (wall
-// impulse, energy loss, friction work) are summed per block in a fixed order: deterministic
-// for a given launch shape, but not in the single-scene kernels' association.
+// impulse, energy loss, friction work) are summed by lanes over the steps of a chunk and the lanes
+// in a fixed order (nf_batch_step.cuh): the same bits whatever the neighbours and so the blocks per
+// instance, and for every block width while an instance has no more nodes than eight blocks of it
+// have threads (one-warp blocks: while no two of its nodes at the wall are a multiple of 32
+// apart); but not in the single-scene kernels' association.
 //
 // Launch shape: block size (32, 128, 256), whether the mixed form stages each instance's float
 // node geometry in shared memory, blocks per SM and the chunk length are chosen by the

@@ -125,7 +125,7 @@ __device__ bool burst_sample(const Team<TEAM> &team, const Dev &d, const BatchDe
 template <bool MIXED, bool STAGE, int T, bool COMP, bool INT, bool TEAM>
 __device__ void run_instance(const Team<TEAM> &team, const Dev &d, const BatchDev &b, int k,
                              int chunk, float4 *sPMid, float2 *sVdt, double *shMin,
-                             int (*wallCount)[2], double (*slots)[3], BlockStep *bs) {
+                             int (*wallCount)[2], double (*table)[3], BlockStep *bs) {
     const BatchInst in = b.inst[k];
     BatchScalars *scp = b.sc + k;
     if (scp->done) return;
@@ -133,7 +133,7 @@ __device__ void run_instance(const Team<TEAM> &team, const Dev &d, const BatchDe
     double minEdge = scp->minEdgeSquared;
     long long steps = scp->steps;
     const long long limit = scp->stepLimit;
-    double wall[3] = {0.0, 0.0, 0.0};        // impulse, energy loss, friction work
+    double wall[WALL_SLOTS<TEAM, T>][3] = {};    // impulse, energy loss, friction work
     int(*counts)[2] = TEAM ? team.at(&wallCount[0], 0) : wallCount;   // the first block's
     if (threadIdx.x == 0) {
         wallCount[0][0] = wallCount[0][1] = 0;
@@ -163,11 +163,16 @@ __device__ void run_instance(const Team<TEAM> &team, const Dev &d, const BatchDe
         }
         minEdge = batch_step<MIXED, T, COMP, INT, TEAM>(
             team, d, in, dt, dtPrev, time, steps, geo, pMid, vdt, base, &scp->status,
-            &counts[par][0], &counts[par][1], wall[0], wall[1], wall[2], shMin, bs);
+            &counts[par][0], &counts[par][1], wall, shMin, bs);
         if (every > 0 && steps % every == 0)
             traversed = burst_sample<MIXED, COMP, T, TEAM>(team, d, b, in, k, time, shMin);
     }
-    team_totals<TEAM, T, 3>(team, wall, shMin, slots);
+    double total[3];
+    if constexpr (WALL_SLOTS<TEAM, T> == 1) {
+        for (int i = 0; i < 3; i++) total[i] = warp_sum(wall[0][i]);
+    } else {
+        wall_totals<TEAM, T>(team, in.n1 - in.n0, wall, shMin, table, total);
+    }
     if (team.first()) {
         scp->dt = dt;
         scp->dtPrevious = dtPrev;
@@ -178,9 +183,9 @@ __device__ void run_instance(const Team<TEAM> &team, const Dev &d, const BatchDe
             scp->wContact = wallCount[(taken - 1) & 1][0];
             scp->wStuck = wallCount[(taken - 1) & 1][1];
         }
-        scp->wImpulse += wall[0];
-        scp->wEnergyLoss += wall[1];
-        scp->wFriction += wall[2];
+        scp->wImpulse += total[0];
+        scp->wEnergyLoss += total[1];
+        scp->wFriction += total[2];
         const bool ended = every > 0 ? (steps % every == 0 && !(time < in.tEnd))
                                      : !(time < in.tEnd);
         if (ended || traversed || steps >= limit) {
@@ -198,7 +203,7 @@ __device__ __forceinline__ void batch_queue(const Dev &d, const BatchDev &b, int
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ double shMin[T / 32 + 1];
     __shared__ int wallCount[2][2];
-    __shared__ double slots[TEAM ? TEAM_MAX : 1][3];
+    __shared__ double table[TEAM ? T * TEAM_MAX / 32 : 1][3];
     __shared__ int next;
     __shared__ BlockStep bs;
     const Team<TEAM> team;
@@ -211,7 +216,7 @@ __device__ __forceinline__ void batch_queue(const Dev &d, const BatchDev &b, int
         team.sync();
         if (q >= b.count) return;
         run_instance<MIXED, STAGE, T, COMP, INT, TEAM>(team, d, b, b.order[q], chunk, sPMid, sVdt,
-                                                       shMin, wallCount, slots, &bs);
+                                                       shMin, wallCount, table, &bs);
     }
 }
 

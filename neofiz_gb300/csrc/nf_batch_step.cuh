@@ -74,26 +74,12 @@ __device__ double block_min_edge_f(float v, double *sh) {
     return block_min_edge<T>((double)v, sh);
 }
 
-// Fixed-tree block sum; valid in thread 0.
-template <int T>
-__device__ double block_total(double v, double *sh) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < T / 32; w++) t += sh[w];
-    __syncthreads();
-    return t;
-}
-
 // Sums over an instance's items (nodes, elements, pressure edges) that do not depend on how many
 // blocks step it, and so not on its neighbours in the batch. The items are dealt to 8 T lanes,
 // T of them a block of the widest team: item j adds to lane j mod 8 T, item after item. A team
 // of fewer blocks gives each thread several lanes, one per slot: those of its first, second ...
-// item. Lanes add up by warps and the warps by one tree.
+// item. Lanes add up by warps and the warps by one tree. Blocks of another width T deal the same
+// way while there are no more than 8 T items.
 template <bool TEAM>
 constexpr int SUM_SLOTS = TEAM ? TEAM_MAX / 2 : TEAM_MAX;
 template <bool TEAM>
@@ -138,25 +124,48 @@ __device__ __forceinline__ void team_sums(const Team<TEAM> &team, int items,
     if (threadIdx.x < 32) table_sums<COUNT>(table, slots * warps, out);
 }
 
-// COUNT block sums added over the team in rank order, in v[] of every block's thread 0.
-// `slots` is block-shared; a team barrier separates one use of it from the next.
-template <bool TEAM, int T, int COUNT>
-__device__ __forceinline__ void team_totals(const Team<TEAM> &team, double (&v)[COUNT], double *sh,
-                                            double (*slots)[COUNT]) {
-    double t[COUNT];
-    for (int i = 0; i < COUNT; i++) t[i] = block_total<T>(v[i], sh);
-    if (!TEAM) {
-        for (int i = 0; i < COUNT; i++) v[i] = t[i];
-        return;
-    }
-    if (threadIdx.x == 0)
-        for (int r = 0; r < team.size; r++)
-            for (int i = 0; i < COUNT; i++) team.at(slots, r)[team.rank][i] = t[i];
-    team.sync();
-    for (int i = 0; i < COUNT; i++) {
-        double sum = 0.0;
-        for (int r = 0; r < team.size; r++) sum += slots[r][i];
-        v[i] = sum;
+// The wall's impulse, energy loss and friction work go to the same lanes. One-warp blocks keep a
+// single sum a lane, in registers: they run instances of a few dozen nodes, none of whose lanes
+// have two at the wall, and they wait for instructions (2.8 of the 7 cycles between two), so that
+// eight slots cost them 3 % (512 burst slices: 87.3 ms, 89.9 with the slots).
+template <bool TEAM, int T>
+constexpr int WALL_SLOTS = T == 32 ? 1 : SUM_SLOTS<TEAM>;
+// Their totals over a chunk of steps, the warps added in turn, in out[] of the first block's first
+// thread. Out of line, once a chunk; the team by value, so that the caller's stays in registers.
+// sh: a row of T / 32; table: a row per warp of the widest team, used by teams alone, so that
+// the staged kernels' shared memory stays the nodes'.
+template <bool TEAM, int T>
+static __device__ __noinline__ void wall_totals(const Team<TEAM> team, int nodes,
+                                                const double (*part)[3], double *sh,
+                                                double (*table)[3], double (&out)[3]) {
+    const int warps = T / 32 * team.size, lane = threadIdx.x & 31, warp = team.tid() >> 5;
+    int slots = (nodes + 32 * warps - 1) / (32 * warps);
+    if (slots > TEAM_MAX / team.size) slots = TEAM_MAX / team.size;
+    out[0] = out[1] = out[2] = 0.0;
+#pragma unroll 1
+    for (int s = 0; s < slots; s++)
+#pragma unroll 1
+        for (int i = 0; i < 3; i++) {
+            const double v = warp_sum(part[s][i]);
+            if (TEAM) {
+                if (lane == 0) team.at(table, 0)[s * warps + warp][i] = v;
+            } else {
+                __syncthreads();
+                if (lane == 0) sh[warp] = v;
+                __syncthreads();
+                if (threadIdx.x == 0)
+                    for (int w = 0; w < warps; w++) out[i] += sh[w];
+            }
+        }
+    if (TEAM) {
+        team.sync();
+        if (team.rank == 0 && threadIdx.x < 32) {
+            double sum = 0.0;
+#pragma unroll 1
+            for (int row = 0; lane < 3 && row < slots * warps; row++) sum += table[row][lane];
+            __syncwarp();
+            for (int i = 0; i < 3; i++) out[i] = __shfl_sync(0xffffffffu, sum, i);
+        }
     }
 }
 
@@ -256,7 +265,8 @@ __device__ double team_min_edge_next_f(const Team<TEAM> &team, float v, double *
 // One step of instance `in` by its team of blocks, ExplicitSolver.step :940-991: the nodal update
 // (with the mixed form's float geometry when geo.pMid is set), the assembly with the exact
 // shortest squared edge, the per-node gather, the next CFL step. dt, dtPrev, time and steps
-// advance in place; returns the shortest squared edge. COMP (with MIXED): the compensated form's
+// advance in place; returns the shortest squared edge. wall: the threads' slots (team_sums) of the
+// wall's impulse, energy loss and friction work. COMP (with MIXED): the compensated form's
 // FP32 nodal update and gather (nf_bodies.cuh). INT: int_products. The step's coefficients and
 // the next step size come from bs, which each block's thread 0 keeps prepared.
 template <bool MIXED, int T, bool COMP, bool INT, bool TEAM>
@@ -265,19 +275,18 @@ __device__ __forceinline__ double batch_step(const Team<TEAM> &team, const Dev &
                                              double &time, long long &steps, const MixedGeo &geo,
                                              const float4 *pMid, const float2 *vdt, int base,
                                              uint32_t *status, int *wallContact, int *wallStuck,
-                                             double &impulse, double &loss, double &fric,
-                                             double *shMin, BlockStep *bs) {
+                                             double (*wall)[3], double *shMin, BlockStep *bs) {
     static_assert(!COMP || MIXED, "the compensated form assembles in FP32");
     const NodalCoef co{bs->decay, bs->gain, bs->dtAvg, dt};
     const WallRef w{in.hasWall, in.wallPlane, in.wallFriction, wallContact, wallStuck};
     const int tid = team.tid(), stride = TEAM ? team.size * T : T;
-    if (COMP) {
-        for (int i = in.n0 + tid; i < in.n1; i += stride)
+    for (int i = in.n0 + tid, slot = 0; i < in.n1; i += stride, slot = next_slot(team, slot)) {
+        double *const sum = wall[WALL_SLOTS<TEAM, T> == 1 ? 0 : slot];
+        if (COMP)
             nodal_node_comp(d, i, bs->fdecay, bs->fgain, bs->fdtAvg, bs->fdt, bs->plane,
-                            bs->friction, w, geo, status, impulse, loss, fric);
-    } else {
-        for (int i = in.n0 + tid; i < in.n1; i += stride)
-            nodal_node<INT>(d, i, co, w, geo, status, impulse, loss, fric);
+                            bs->friction, w, geo, status, sum[0], sum[1], sum[2]);
+        else
+            nodal_node<INT>(d, i, co, w, geo, status, sum[0], sum[1], sum[2]);
     }
     team.sync();
     time += dt;                                                       // :973-974

@@ -54,3 +54,36 @@ def test_sampled_peak_does_not_depend_on_the_neighbours(gpu_lib):
     for count in (40, 160):
         among = gradients([tube() for _ in range(count)], 0.5, objectives, sample=5)
         assert np.array_equal(alone[0], among[0]) and np.array_equal(alone[1], among[1]), count
+
+
+def wall_totals(instances, precision, config=None):
+    b = BatchSolver(instances, Formulation.AXISYMMETRIC, cfl=0.6, precision=precision)
+    if config:
+        b.setConfig(*config)
+    b.run(150)
+    b.run(75)
+    w = b.wallStats()[0]
+    b.close()
+    return w.impulse, w.energy_loss, w.friction_dissipation
+
+
+# every node of these rods' feet touches the wall: 161 and 25 of them, five warps and one. Blocks
+# of 32, 128 and 256 threads by turns, for the neighbours' size or because the shape asks for it
+@pytest.mark.parametrize("precision", [_abi.PRECISION_FP64, _abi.PRECISION_MIXED,
+                                       _abi.PRECISION_COMPENSATED])
+@pytest.mark.parametrize("nr,nz,config", [(160, 3, (128, 0, 1, 256)), (24, 1, (128, 0, 1, 256)),
+                                          (160, 14, (256, 0, 1, 256))])
+def test_wall_totals_do_not_depend_on_the_neighbours(gpu_lib, precision, nr, nz, config):
+    one = rod(nr, nz, 1.0)
+
+    def among(count, size):
+        rods = [one] + [one] * (count // 2) + others(count - count // 2, 1.0)
+        for r in rods[len(rods) - count // 3:]:
+            r.update(nr=size, nz=2 * size)
+        return scenes.sweep_instances(rods)
+
+    alone = wall_totals(scenes.sweep_instances([one]), precision)
+    assert all(t != 0.0 for t in alone)
+    assert alone == wall_totals(scenes.sweep_instances([one]), precision, config)
+    for count, size in ((3, 3), (40, 5), (40, 12), (160, 12), (700, 4)):
+        assert wall_totals(among(count, size), precision) == alone, (count, size)
