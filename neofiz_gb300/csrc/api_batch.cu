@@ -37,6 +37,8 @@ struct Batch {
     cudaGraphExec_t graph = nullptr;
     BatchShape graphShape{};
     int graphTeam = 0, graphLeft = -1;
+    BatchShape planned{}, launched{};        // the shape that launched and teams are of
+    int teams[4] = {0, 0, 0, 0};             // teams of 1, 2, 4 and 8 blocks resident
     std::vector<int> elems;                  // the instances' element counts, most expensive first
     int32_t *hostRemaining = nullptr;        // pinned
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -125,48 +127,52 @@ bool shape_valid(const Batch &B, const BatchShape &s) {
     return resident > 0 && s.blocksPerSm <= std::max(resident, batch_blocks_promised(B.mode, s));
 }
 
-// The batch's shape as launched: no more blocks per SM than are resident.
-BatchShape launched_shape(const Batch &B) {
-    BatchShape s = B.shape;
-    const int resident = batch_max_blocks_per_sm(B.mode, s, B.b.maxNodes, B.b.maxElems);
-    if (resident > 0) s.blocksPerSm = std::min(s.blocksPerSm, resident);
-    return s;
+bool same_shape(const BatchShape &a, const BatchShape &b) {
+    return memcmp(&a, &b, sizeof(BatchShape)) == 0;
+}
+
+// The batch's shape as launched, no more blocks per SM than are resident, and its teams.
+void plan_launch(Batch &B) {
+    if (same_shape(B.planned, B.shape)) return;
+    B.planned = B.launched = B.shape;
+    const int resident = batch_max_blocks_per_sm(B.mode, B.shape, B.b.maxNodes, B.b.maxElems);
+    if (resident > 0) B.launched.blocksPerSm = std::min(B.shape.blocksPerSm, resident);
+    batch_teams(B.mode, B.launched, B.sms, B.teams);
 }
 
 // Blocks per instance while the `left` most expensive instances run (the cheap ones finish
-// first, and those left spread over more blocks), and the teams resident.
-int team_of(const Batch &B, const BatchShape &shape, int left, int *teams) {
-    int n[4];
-    batch_teams(B.mode, shape, B.sms, n);
-    const int team = choose_team(B.elems.data(), std::max(1, std::min(left, B.count)), n);
-    *teams = team == 1 ? n[0] : team == 2 ? n[1] : team == 4 ? n[2] : n[3];
-    return team;
+// first, and those left spread over more blocks).
+int team_of(const Batch &B, int left) {
+    return choose_team(B.elems.data(), std::max(1, std::min(left, B.count)), B.teams);
 }
 
 // The run's launches: reset the queue, launch one chunk; GRAPH_CHUNKS times.
-cudaError_t enqueue_chunks(Batch &B, const BatchShape &shape, int chunks, int team, int teams) {
+cudaError_t enqueue_chunks(Batch &B, int chunks, int team) {
+    const int teams = B.teams[team == 1 ? 0 : team == 2 ? 1 : team == 4 ? 2 : 3];
     for (int c = 0; c < chunks; c++) {
         cudaError_t e = cudaMemsetAsync(B.b.queue, 0, sizeof(int32_t), B.stream);
         if (e != cudaSuccess) return e;
-        e = launch_batch_steps(B.d, B.b, B.mode, shape, team, teams, B.stream);
+        e = launch_batch_steps(B.d, B.b, B.mode, B.launched, team, teams, B.stream);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
+// Whether the captured launches are those of the batch's shape with `left` instances to go.
+bool graph_ready(const Batch &B, int left) {
+    return B.graph && same_shape(B.graphShape, B.shape) && B.graphLeft == left;
+}
+
 nf_status ensure_graph(Batch &B, int left) {
-    const bool sameShape = B.graph && memcmp(&B.graphShape, &B.shape, sizeof(BatchShape)) == 0;
-    if (sameShape && B.graphLeft == left) return NF_OK;
-    int teams = 1;
-    const BatchShape shape = launched_shape(B);
-    const int team = team_of(B, shape, left, &teams);
+    plan_launch(B);
+    const int team = team_of(B, left);
     B.graphLeft = left;
-    if (sameShape && B.graphTeam == team) return NF_OK;
+    if (B.graph && same_shape(B.graphShape, B.shape) && B.graphTeam == team) return NF_OK;
     if (B.graph) cudaGraphExecDestroy(B.graph);
     B.graph = nullptr;
     cudaGraph_t g = nullptr;
     BCK(&B, cudaStreamBeginCapture(B.stream, cudaStreamCaptureModeThreadLocal));
-    const cudaError_t launched = enqueue_chunks(B, shape, GRAPH_CHUNKS, team, teams);
+    const cudaError_t launched = enqueue_chunks(B, GRAPH_CHUNKS, team);
     const cudaError_t ended = cudaStreamEndCapture(B.stream, &g);
     if (launched != cudaSuccess || ended != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -179,7 +185,8 @@ nf_status ensure_graph(Batch &B, int left) {
     if (inst != cudaSuccess) return bfail(&B, NF_EDEVICE, "graph instantiate: %s", cudaGetErrorString(inst));
     B.graphShape = B.shape;
     B.graphTeam = team;
-    return NF_OK;
+    BCK(&B, cudaGraphUpload(B.graph, B.stream));
+    return bsync(B);
 }
 
 // The arrays a run changes, for the autotuner's save and restore.
@@ -558,33 +565,50 @@ nf_status nf_batch_run(nf_batch *h, int64_t max_steps) {
     Batch &B = *reinterpret_cast<Batch *>(h);
     B.lastMs = 0.0;
     if (max_steps <= 0) return NF_OK;
-    BCK(&B, cudaEventRecord(B.ev0, B.stream));
+    // the time counted is the device's: the host's building of a graph, before the first and
+    // whenever the instances left want another, stands between two spans
+    double total = 0.0;
+    auto begin = [&]() -> nf_status {
+        BCK(&B, cudaEventRecord(B.ev0, B.stream));
+        return NF_OK;
+    };
+    auto end = [&]() -> nf_status {
+        BCK(&B, cudaEventRecord(B.ev1, B.stream));
+        const nf_status synced = bsync(B);
+        if (synced) return synced;
+        float ms = 0.0f;
+        BCK(&B, cudaEventElapsedTime(&ms, B.ev0, B.ev1));
+        total += ms;
+        return NF_OK;
+    };
+    nf_status st = begin();
+    if (st) return st;
     launch_batch_arm(B.b, (long long)max_steps, B.stream);
     B.launches += 1;
     BCK(&B, cudaMemcpyAsync(B.hostRemaining, B.b.remaining, sizeof(int32_t),
                             cudaMemcpyDeviceToHost, B.stream));
-    nf_status st = bsync(B);
-    if (st) return st;
-    while (*B.hostRemaining > 0) {
-        st = ensure_graph(B, *B.hostRemaining);
-        if (st) return st;
+    st = bsync(B);
+    while (!st && *B.hostRemaining > 0) {
+        if (!graph_ready(B, *B.hostRemaining)) {
+            st = end();
+            if (!st) st = ensure_graph(B, *B.hostRemaining);
+            if (!st) st = begin();
+            if (st) break;
+        }
         BCK(&B, cudaGraphLaunch(B.graph, B.stream));
         B.launches += GRAPH_CHUNKS;
         BCK(&B, cudaMemcpyAsync(B.hostRemaining, B.b.remaining, sizeof(int32_t),
                                 cudaMemcpyDeviceToHost, B.stream));
         st = bsync(B);
-        if (st) return st;
     }
+    if (st) return st;
     if (B.comp) {                            // the FP64 arrays that reads see
         launch_batch_comp(B.d, false, B.stream);
         B.launches += 1;
     }
-    BCK(&B, cudaEventRecord(B.ev1, B.stream));
-    st = bsync(B);
+    st = end();
     if (st) return st;
-    float ms = 0.0f;
-    BCK(&B, cudaEventElapsedTime(&ms, B.ev0, B.ev1));
-    B.lastMs = ms;
+    B.lastMs = total;
     return NF_OK;
 }
 
@@ -634,11 +658,10 @@ nf_status nf_batch_tune(nf_batch *h, int32_t trial_steps, nf_batch_config *chose
     for (int round = 0; round < 2 && !st; round++)
         for (size_t i = 0; i < cands.size(); i++) {
             B.shape = cands[i];
+            plan_launch(B);
             cudaEventRecord(B.ev0, B.stream);
             launch_batch_arm(B.b, trial_steps, B.stream);
-            int teams = 1;
-            const int team = team_of(B, B.shape, B.count, &teams);
-            cudaError_t e = enqueue_chunks(B, B.shape, 1, team, teams);
+            cudaError_t e = enqueue_chunks(B, 1, team_of(B, B.count));
             cudaEventRecord(B.ev1, B.stream);
             B.launches += 2;
             if (e == cudaSuccess) e = cudaStreamSynchronize(B.stream);
