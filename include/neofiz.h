@@ -420,7 +420,8 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
 nf_status nf_batch_destroy(nf_batch *b);
 const char *nf_batch_last_error(const nf_batch *b);
 /* Autotuner: times every valid shape on trial_steps steps of the whole batch (state saved and
- * restored, so the trajectory is untouched), keeps the fastest and returns it. */
+ * restored, so the trajectory is untouched), keeps the fastest and returns it. For instances of
+ * uneven cost it times the shapes that can spread the last ones over several blocks. */
 nf_status nf_batch_tune(nf_batch *b, int32_t trial_steps, nf_batch_config *chosen);
 nf_status nf_batch_set_config(nf_batch *b, const nf_batch_config *config);
 nf_status nf_batch_get_config(nf_batch *b, nf_batch_config *config);

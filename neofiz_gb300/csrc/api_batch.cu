@@ -40,6 +40,7 @@ struct Batch {
     BatchShape planned{}, launched{};        // the shape that launched and teams are of
     int teams[4] = {0, 0, 0, 0};             // teams of 1, 2, 4 and 8 blocks resident
     std::vector<int> elems;                  // the instances' element counts, most expensive first
+    double spread = 1.0;                     // the most expensive instance's cost over the median one's
     int32_t *hostRemaining = nullptr;        // pinned
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double lastMs = 0.0;
@@ -503,6 +504,7 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return cost[a] > cost[c]; });
     for (int k : order) B->elems.push_back(B->inst[k].e1 - B->inst[k].e0);
+    B->spread = cost[order[0]] / cost[order[count / 2]];
     U(b.sc, sc.data(), count);
     U(dOrder, order.data(), count);
 #undef U
@@ -612,6 +614,21 @@ nf_status nf_batch_run(nf_batch *h, int64_t max_steps) {
     return NF_OK;
 }
 
+// Whether the batch's run ends with few of its instances over several blocks each: its costs are
+// ragged (twice the median one's and more) and an eighth of its instances would take teams. The
+// tuner's trial, of all instances, does not see that end, and only the 256-thread shapes without
+// staged nodes have it: 256 mixed rods of 180 to 2,880 elements took 350 ms with them and 804 with
+// the staged shape that the trial of all put 2 % ahead, 4,096 compensated ones 2.79 s and 4.03 with
+// blocks of 128, level in the trial.
+static bool ends_in_teams(Batch &B) {
+    if (!(B.spread >= 2.0)) return false;
+    BatchShape s{TEAM_THREADS, 0, 1, 1};
+    s.blocksPerSm = std::max(1, batch_max_blocks_per_sm(B.mode, s, B.b.maxNodes, B.b.maxElems));
+    int teams[4];
+    batch_teams(B.mode, s, B.sms, teams);
+    return choose_team(B.elems.data(), std::max(1, B.count / 8), teams) > 1;
+}
+
 nf_status nf_batch_tune(nf_batch *h, int32_t trial_steps, nf_batch_config *chosen) {
     Batch &B = *reinterpret_cast<Batch *>(h);
     if (trial_steps < 1) return bfail(&B, NF_EINVAL, "trial_steps must be positive");
@@ -630,11 +647,13 @@ nf_status nf_batch_tune(nf_batch *h, int32_t trial_steps, nf_batch_config *chose
         }
     };
     copy(true);
+    const bool teams = ends_in_teams(B);
     std::vector<BatchShape> cands;
     // one-warp blocks serve small instances (a burst slice has 16 elements): more of them
     // resident per SM instead of mostly idle 128-thread blocks
     for (int threads : {32, 128, 256})
         for (int stage = 0; stage <= (B.mixed ? 1 : 0); stage++) {
+            if (teams && (threads != TEAM_THREADS || stage)) continue;
             BatchShape s{threads, stage, 1, trial_steps};
             const int occ = batch_max_blocks_per_sm(B.mode, s, B.b.maxNodes, B.b.maxElems);
             bool atOcc = false;

@@ -47,3 +47,16 @@ def test_elapsed_leaves_out_the_building_of_graphs(gpu_lib):
         again.append(b.run(1))
     b.close()
     assert abs(np.median(anew) - np.median(again)) < 0.012, (np.median(anew), np.median(again))
+
+
+@pytest.mark.parametrize("precision,count", [(_abi.PRECISION_MIXED, 256),
+                                             (_abi.PRECISION_COMPENSATED, 512)])
+def test_tuning_a_ragged_batch_does_not_lose_to_the_default(gpu_lib, precision, count):
+    """Rods whose finest take four times the steps of the coarsest: the shape that tune keeps runs
+    them no slower than the untuned one, within a tenth."""
+    rods = scenes.taylor_sweep(count, seed=5, t_end=6.0e-6)
+    a, b = batch(rods, precision), batch(rods, precision)
+    b.tune()
+    assert b.run() < 1.1 * a.run()
+    a.close()
+    b.close()
