@@ -367,9 +367,7 @@ nf_status nf_create(const nf_mesh *mesh, const nf_material *materials, int32_t m
     A(d.pedges, K);
     A(d.partials, (size_t)PARTIAL_SLOTS * d.maxBlocks);
     A(d.edgeGroup, 4LL * E); A(d.groupStart, 4LL * E + 1); A(d.groupMember, 4LL * E);
-    A(S->stage, std::max(N, E));
-    int32_t *scratch = nullptr;
-    A(scratch, setup_scratch_ints(N, E));
+    A(S->stage, stage_doubles(std::max(N, E), N, E, true));
     A(d.s, 1);
     if (listed) {
         d.hotSmem = listed_pass_smem(S->device);
@@ -393,7 +391,7 @@ nf_status nf_create(const nf_mesh *mesh, const nf_material *materials, int32_t m
     DevScalars s0{};
     s0.minEdgeBits = 0x7ff0000000000000ULL;   // none yet
     upload(*S, d.s, &s0, 1);
-    const int *most = launch_setup(*S, scratch);
+    const int *most = launch_setup(*S);
     CK(nullptr, cudaMemcpyAsync(&S->maxCorners, most, sizeof(int), cudaMemcpyDeviceToHost, S->stream));
     nf_status st = read_scalars(*S, &s0);
     if (st) {

@@ -445,9 +445,7 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
     A(dOrder, count);
     A(b.queue, 1); A(b.remaining, 1);
     A(b.measure, 3LL * count);
-    int32_t *scratch = nullptr;
-    A(scratch, setup_scratch_ints(N, E));
-    A(B->stage, std::max<long long>(N, B->mixed ? 4LL * E : E));
+    A(B->stage, stage_doubles(std::max<long long>(N, B->mixed ? 4LL * E : E), N, E, false));
     unsigned long long *dEdges = nullptr;
     A(dEdges, count);
     double2 *dVelocity = nullptr;
@@ -477,7 +475,7 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
     if (B->mixed) U(d.matsF, matsF.data(), count);
     U(dInst, B->inst.data(), count);
     if (e_ == cudaSuccess) {
-        launch_batch_setup(d, dInst, count, dVelocity, dEdges, scratch, B->stream);
+        launch_batch_setup(d, dInst, count, dVelocity, dEdges, B->stage, B->stream);
         if (damage) setup_damage_geometry(d, B->stream);
         e_ = cudaMemcpyAsync(edges.data(), dEdges, sizeof edges[0] * count, cudaMemcpyDeviceToHost,
                              B->stream);

@@ -268,19 +268,23 @@ __global__ void __launch_bounds__(SB) k_widen(const float *src, double *dst, int
     if (i < n) dst[i] = src[(size_t)i * stride];
 }
 
-size_t setup_scratch_ints(int N, int E) {
-    return scan_tmp_ints(std::max(4 * E, N + 1)) + 4 * ((size_t)N + 1) + 1;
+// Doubles of a handle's staging buffer for fields on their way to the host, of `most` at a time:
+// the set-up works in it first (a count and, for a scene's surface, two ints more per node, and
+// the scan's space).
+size_t stage_doubles(size_t most, int N, int E, bool surface) {
+    const size_t ints = scan_tmp_ints(std::max(4 * E, N + 1)) + (surface ? 3 : 1) * ((size_t)N + 1) + 1;
+    return std::max(most, (ints + 1) / 2);
 }
 
 // conn, emat, mats and pedges are in place, and r and z in U. The lists in between use
-// `contribution`, which like U is zeroed again, and `scratch` (setup_scratch_ints, zeroed).
+// `contribution`, which like U is zeroed again, and the staging buffer, zeroed.
 static void node_arrays(Dev &d, cudaStream_t st, int *scratch, bool surface,
                         unsigned long long *instances) {
     const int N = d.N, E = d.E;
     const long long entries = 4LL * E + 2LL * d.K;
     int *sources = scratch, *edges = surface ? sources + N + 1 : nullptr;
     int *edgeStart = surface ? edges + N + 1 : nullptr;
-    int *tmp = scratch + 4 * ((size_t)N + 1) + 1;
+    int *tmp = scratch + (surface ? 3 : 1) * ((size_t)N + 1) + 1;
     int *sourceBin = reinterpret_cast<int *>(d.contribution), *edgeBin = sourceBin + entries;
     int *head = edgeBin + 4LL * E, *before = head + 4LL * E;   // 16 E + 2 K of 16 (E + K)
     const double *r = reinterpret_cast<const double *>(d.U);
@@ -308,11 +312,12 @@ static void node_arrays(Dev &d, cudaStream_t st, int *scratch, bool surface,
 }
 
 // A scene's arrays; its shortest edge goes to s. Returns where the greatest number of elements
-// around a node will be.
-int *launch_setup(Solver &S, int *scratch) {
+// around a node will be, in the staging buffer.
+int *launch_setup(Solver &S) {
     Dev &d = S.d;
+    int *scratch = reinterpret_cast<int *>(S.stage);
     node_arrays(d, S.stream, scratch, true, nullptr);
-    int *corners = scratch + 3 * ((size_t)d.N + 1), *most = corners + d.N + 1;
+    int *corners = scratch, *most = scratch + 3 * ((size_t)d.N + 1);   // the filing left zeros
     if (d.E > 0) {
         k_corners<<<grid_for(4LL * d.E, SB), SB, 0, S.stream>>>(d, corners);
         k_most<<<grid_for(d.N, SB), SB, 0, S.stream>>>(d.N, corners, most);
@@ -322,9 +327,9 @@ int *launch_setup(Solver &S, int *scratch) {
 // A batch's: conn and pedges arrive with the instances' local numbers, flags as the caller's
 // bytes, `edges` (per instance) at infinity.
 void launch_batch_setup(Dev &d, const BatchInst *inst, int count, const double2 *velocity,
-                        unsigned long long *edges, int *scratch, cudaStream_t st) {
+                        unsigned long long *edges, double *stage, cudaStream_t st) {
     k_batch_fill<<<count, SB, 0, st>>>(d, inst, velocity);
-    node_arrays(d, st, scratch, false, edges);
+    node_arrays(d, st, reinterpret_cast<int *>(stage), false, edges);
 }
 void setup_damage_geometry(Dev &d, cudaStream_t st) {
     if (d.E > 0) k_damage_geometry<<<grid_for(d.E, SB), SB, 0, st>>>(d);

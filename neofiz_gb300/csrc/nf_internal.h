@@ -412,10 +412,10 @@ double element_signed_area(const double *r, const double *z, const int32_t *conn
 void set_thread_error(const char *message);
 
 // Launchers (k_setup.cu)
-size_t setup_scratch_ints(int N, int E);
-int *launch_setup(Solver &S, int *scratch);
+size_t stage_doubles(size_t most, int N, int E, bool surface);
+int *launch_setup(Solver &S);
 void launch_batch_setup(Dev &d, const BatchInst *inst, int count, const double2 *velocity,
-                        unsigned long long *edges, int *scratch, cudaStream_t st);
+                        unsigned long long *edges, double *stage, cudaStream_t st);
 void setup_damage_geometry(Dev &d, cudaStream_t st);
 void launch_segments(Solver &S);
 void launch_component(const double2 *src, double *dst, size_t count, int y, cudaStream_t st);
