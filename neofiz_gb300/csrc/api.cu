@@ -456,7 +456,7 @@ nf_status nf_destroy(nf_solver *h) {
                     d.scanTmp, d.s, d.matsF, d.sigF, d.backF, d.epsPF, d.wPF, d.hgKF,
                     d.contribF, d.hgF, d.dStrF, d.dSoftF, d.dWidthF, d.dFailF, d.dGfF, d.dGeomF,
                     d.pMid, d.pCur, d.vdt, d.gaussVol, d.coopSums, d.incSlots, d.bucketF, d.bucketFL, d.bucketAB, d.bucketA, d.bucketN, d.bucketL,
-                    d.fastCount, d.fastCell, d.fastEntry, d.fastF, d.fastFL, d.fastAB, d.fastA, d.fastN,
+                    d.fastCount, d.fastEntry, d.fastF, d.fastFL, d.fastAB, d.fastA, d.fastN,
                     d.fastL, d.nodeCell,
                     d.hot, d.hotList, d.hotNext, d.hotStamp, d.jcYield};
     for (void *p : ptrs)                     // the arenas' arrays go with them
@@ -638,7 +638,6 @@ nf_status nf_set_contact(nf_solver *h, double friction, double damping, double s
         d.fastCap = NF_GRID_SLOTS;
         d.fastLimit = S.gridSlots;
         A(d.fastCount, d.fastCells + 1);
-        A(d.fastCell, (size_t)d.fastCells * d.fastCap);
         A(d.fastEntry, (size_t)d.fastCells * d.fastCap);
         A(d.fastF, (size_t)d.fastCells * d.fastCap); A(d.fastFL, (size_t)d.fastCells * d.fastCap);
         A(d.fastAB, (size_t)d.fastCells * d.fastCap);

@@ -418,10 +418,11 @@ __device__ void resolve_pair(const Dev &d, int n, int q) {
 // 2^-18 W (g.screen). The few that pass take the exact FP64 test, each lane its own. The
 // grid's buckets as the search reads them: the counting-sort layout (bucket b's entries at
 // [start[b], start[b + 1]), each with its cell) or the direct-indexed one (bucket b's entries at
-// [b cap, b cap + count[b]), with their cells where cells share buckets).
+// [b cap, b cap + count[b]); where cells share buckets the entry's node tells its cell).
 struct BucketView {
     const int32_t *start, *count;
-    const long long *cell;                     // null where a bucket holds one cell only
+    const long long *cell;                     // the counting-sort layout's
+    bool folded;                               // cells share the direct layout's buckets
     const int32_t *entry;
     const float4 *f;                           // first node - grid origin, normal (FP32)
     const float *fl;                           // length (FP32)
@@ -551,6 +552,10 @@ __device__ int search_group(const Dev &d, const Grid &g, const BucketView &v, in
         if (v.cell && v.cell[k] != cc) return;          // cells may share a bucket
         const int entry = v.entry[k];
         const int sg = entry >> 1;
+        if (v.folded) {
+            const int2 ends = v.ab[k], in = d.nodeCell[entry & 1 ? ends.y : ends.x];
+            if ((long long)in.y * g.cols + in.x != cc) return;
+        }
         const double2 pa = v.a[k], nq = v.n[k];
         const double dr = xn.x - pa.x, dz = xn.y - pa.y;
         const double gap = dr * nq.x + dz * nq.y;
@@ -835,8 +840,8 @@ __global__ void __launch_bounds__(CB, 2) k_contact_pass(Dev d) {
     // node under that cell. The cell's low bits index buckets of fixed size: each entry takes the
     // next of its bucket's slots (fastLimit of the fastCap reserved) and is filed there at once,
     // with the FP32 values the search's screen reads. In a grid of more than fastCells cells,
-    // bodies apart or a fine mesh, cells share buckets, and an entry keeps its cell for the
-    // search to tell them by: the surface is a line through the grid, so few do. 1M quads, 75k
+    // bodies apart or a fine mesh, cells share buckets, and the search tells them by the cell of
+    // the entry's node: the surface is a line through the grid, so few do. 1M quads, 75k
     // to 430k cells for 65,536 buckets: 58 us from the filing to the end of the search through
     // the counting sort, which such a grid took, and 44 us so. A hashed grid, or a bucket that
     // outgrows its slots, takes the counting sort: the counts, an exclusive scan, the filing.
@@ -885,7 +890,6 @@ __global__ void __launch_bounds__(CB, 2) k_contact_pass(Dev d) {
                         const double2 nq = make_double2(d.snr[q], d.snz[q]);
                         const double lq = d.slen[q];
                         d.fastEntry[slot] = entry;
-                        if (folded) d.fastCell[slot] = cell;
                         d.fastF[slot] = make_float4((float)(pa.x - g.r0), (float)(pa.y - g.z0),
                                                     (float)nq.x, (float)nq.y);
                         d.fastFL[slot] = (float)lq;
@@ -932,11 +936,10 @@ __global__ void __launch_bounds__(CB, 2) k_contact_pass(Dev d) {
     }
     BucketView view;
     if (direct) {
-        view = BucketView{nullptr, d.fastCount, folded ? d.fastCell : nullptr, d.fastEntry,
-                          d.fastF, d.fastFL,
+        view = BucketView{nullptr, d.fastCount, nullptr, folded, d.fastEntry, d.fastF, d.fastFL,
                           d.fastAB, d.fastA, d.fastN, d.fastL, d.fastCap};
     } else {
-        view = BucketView{d.bucketStart, nullptr, d.bucketCell, d.bucketEntry, d.bucketF,
+        view = BucketView{d.bucketStart, nullptr, d.bucketCell, false, d.bucketEntry, d.bucketF,
                           d.bucketFL, d.bucketAB, d.bucketA, d.bucketN, d.bucketL, 0};
     }
 

@@ -173,7 +173,6 @@ struct Dev {
     // the direct-indexed grid: the entries of the cells whose low bits are b in slots
     // [b fastCap, b fastCap + fastCount[b]) while none outgrows them
     int32_t *fastCount;                      // [fastCells + 1]
-    long long *fastCell;                     // [fastCells x fastCap] the entry's cell
     int32_t *fastEntry;                      // [fastCells x fastCap]
     float4 *fastF;                           // [fastCells x fastCap] as bucketF
     float *fastFL;                           // [fastCells x fastCap] as bucketFL

@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from neofiz_gb300 import ExplicitSolver, Formulation, Integration, Kinematics, QuadMesh
+from neofiz_gb300 import Contact, ExplicitSolver, Formulation, Integration, Kinematics, QuadMesh
 from neofiz_gb300 import _abi
 from neofiz_gb300.batch import BatchSolver, Instance
 from neofiz_gb300.materials import Material
@@ -54,3 +54,18 @@ def test_a_batch_holds_no_set_up_lists(gpu_lib):
     # some twenty allocations of their own, each rounded up to 2 MB at most
     assert held < 50 * (94 * m.nodeCount + 204 * m.elementCount) + 20 * 2 * MB // 2
 
+
+def test_contact_holds_no_cells_beside_its_slots(gpu_lib):
+    """65,536 buckets of 64 slots of 72 bytes; 901 bytes an element and 400 a node."""
+    def contact(nr, nz):
+        m = QuadMesh.solidCylinder(0.01, 0.1, nr, nz)
+        s = scene(m)
+        before = free()
+        s.setContact(Contact(m))
+        s.synchronize()
+        held = before - free()
+        s.close()
+        return held, m
+    contact(4, 8)
+    held, m = contact(100, 399)
+    assert held < 65536 * 64 * 72 + 901 * m.elementCount + 400 * m.nodeCount + 4 * MB
