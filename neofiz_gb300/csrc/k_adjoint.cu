@@ -240,7 +240,7 @@ __device__ double capacity_of(const Team<TEAM> &team, const Dev &d, const BatchI
 }
 
 // Forward: every instance to its t_end, a checkpoint every `every` steps, the final state.
-template <bool INT, bool TEAM>
+template <bool TEAM>
 __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev a) {
     __shared__ double shMin[ADJ_T / 32 + 1];
     __shared__ int wallCount[2][2];
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev
             wallCount[par ^ 1][0] = 0;
             wallCount[par ^ 1][1] = 0;
         }
-        minEdge = batch_step<false, ADJ_T, false, INT, TEAM>(
+        minEdge = batch_step<false, ADJ_T, false, false, TEAM>(
             team, d, in, dt, dtPrev, time, steps, none, nullptr, nullptr, 0, &scp->status,
             &counts[par][0], &counts[par][1], wall, shMin, &bs);
         if (a.sampleEvery > 0 && steps % a.sampleEvery == 0) {
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_forward(Dev d, BatchDev b, AdjDev
 // memory: atomics need a shared or global address).
 // owner0 is the first block's shared word; shDtb, shDtPrevb and shTimeb are each block's own and
 // equal in all of them.
-template <bool INT, bool TEAM>
+template <bool TEAM>
 __device__ void reverse_step(const Team<TEAM> &team, const Dev &d, const BatchInst &in,
                              const MatDev &mat, StateBlock pre, BarBlock bar,
                              double (*table)[4], int *owner0, double *shDtb,
@@ -354,7 +354,7 @@ __device__ void reverse_step(const Team<TEAM> &team, const Dev &d, const BatchIn
         for (int i = tid; i < n; i += stride) {
             const int g = in.n0 + i;
             d.U[g] = pre.U[i]; d.V[g] = pre.V[i]; d.F[g] = pre.F[i]; d.flags[g] = pre.flags[i];
-            nodal_node<INT>(d, g, co, w, none, reinterpret_cast<uint32_t *>(scratch + 2), i0, l0, f0);
+            nodal_node<false>(d, g, co, w, none, reinterpret_cast<uint32_t *>(scratch + 2), i0, l0, f0);
         }
     }
     if (team.first()) *owner0 = 0x7fffffff;
@@ -468,7 +468,7 @@ __device__ void reverse_step(const Team<TEAM> &team, const Dev &d, const BatchIn
 }
 
 // Backward: the reverse sweep over all steps of every instance, segment by segment.
-template <bool INT, bool TEAM>
+template <bool TEAM>
 __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDev a) {
     __shared__ double shMin[ADJ_T / 32 + 1];
     __shared__ int shOwner;
@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDe
             if (team.first()) {
                 t.scal[0] = dt; t.scal[1] = dtPrev; t.scal[2] = time; t.scal[3] = (double)steps;
             }
-            const double me = batch_step<false, ADJ_T, false, INT, TEAM>(
+            const double me = batch_step<false, ADJ_T, false, false, TEAM>(
                 team, d, in, dt, dtPrev, time, steps, none, nullptr, nullptr, 0, scratchStatus,
                 &scratch[0], &scratch[1], wall, shMin, &bs);
             if (team.first()) t.scal[4] = me;
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDe
                 }
                 // the forward values each objective's reverse reads are recomputed from the
                 // same tape entry, so every objective sees the same bits
-                reverse_step<INT>(team, d, in, mat, pre, bar, table, owner0, &shDtb[w], &shDtPrevb[w],
+                reverse_step(team, d, in, mat, pre, bar, table, owner0, &shDtb[w], &shDtPrevb[w],
                                   &shTimeb[w], scratch);
             }
         }
@@ -568,13 +568,11 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_backward(Dev d, BatchDev b, AdjDe
     team.sync();
 }
 
-static const void *forward_kernel(bool ints, bool team) {
-    if (team) return ints ? (const void *)k_adj_forward<true, true> : (const void *)k_adj_forward<false, true>;
-    return ints ? (const void *)k_adj_forward<true, false> : (const void *)k_adj_forward<false, false>;
+static const void *forward_kernel(bool team) {
+    return team ? (const void *)k_adj_forward<true> : (const void *)k_adj_forward<false>;
 }
-static const void *backward_kernel(bool ints, bool team) {
-    if (team) return ints ? (const void *)k_adj_backward<true, true> : (const void *)k_adj_backward<false, true>;
-    return ints ? (const void *)k_adj_backward<true, false> : (const void *)k_adj_backward<false, false>;
+static const void *backward_kernel(bool team) {
+    return team ? (const void *)k_adj_backward<true> : (const void *)k_adj_backward<false>;
 }
 
 // Raises the context's per-thread stack limit to what the adjoint kernels' frames need (the
@@ -582,10 +580,8 @@ static const void *backward_kernel(bool ints, bool team) {
 // lower. The device call graph has no cycles, so the frames are fixed at compile time.
 cudaError_t adjoint_reserve_stack() {
     size_t need = 0;
-    const void *kernels[] = {
-        forward_kernel(false, false), forward_kernel(true, false), forward_kernel(false, true),
-        forward_kernel(true, true), backward_kernel(false, false), backward_kernel(true, false),
-        backward_kernel(false, true), backward_kernel(true, true)};
+    const void *kernels[] = {forward_kernel(false), forward_kernel(true), backward_kernel(false),
+                             backward_kernel(true)};
     for (const void *f : kernels) {
         cudaFuncAttributes at;
         const cudaError_t e = cudaFuncGetAttributes(&at, f);
@@ -599,9 +595,8 @@ cudaError_t adjoint_reserve_stack() {
     return need > cur ? cudaDeviceSetLimit(cudaLimitStackSize, need) : cudaSuccess;
 }
 
-// One team of blocks per instance (choose_team), its products on the integer units where its
-// quarter SMs have more than one warp of elements (int_products). One block fits on an SM.
-static void launch_adjoint(const void *(*kernel)(bool, bool), const Dev &d, const BatchDev &b,
+// One team of blocks per instance (choose_team). One block fits on an SM.
+static void launch_adjoint(const void *(*kernel)(bool), const Dev &d, const BatchDev &b,
                            const AdjDev &a, const int *elems, int sms, cudaStream_t st) {
     if (b.count <= 0) return;
     Dev dd = d;
@@ -609,12 +604,10 @@ static void launch_adjoint(const void *(*kernel)(bool, bool), const Dev &d, cons
     AdjDev aa = a;
     void *args[] = {&dd, &bb, &aa};
     int teams[4] = {sms, 0, 0, 0};
-    for (int q = 1; q < 4; q++) teams[q] = max_teams(kernel(true, true), 1 << q, ADJ_T);
+    for (int q = 1; q < 4; q++) teams[q] = max_teams(kernel(true), 1 << q, ADJ_T);
     const int team = choose_team(elems, b.count, teams);
-    const int warps = (b.maxElems + 31) / 32 < ADJ_T / 32 * team ? (b.maxElems + 31) / 32 : ADJ_T / 32 * team;
-    const bool ints = int_products((warps + team - 1) / team, 1);
-    if (team > 1) launch_team(kernel(ints, true), b.count, team, ADJ_T, args, st);
-    else cudaLaunchKernel(kernel(ints, false), dim3(b.count), dim3(ADJ_T), args, 0, st);
+    if (team > 1) launch_team(kernel(true), b.count, team, ADJ_T, args, st);
+    else cudaLaunchKernel(kernel(false), dim3(b.count), dim3(ADJ_T), args, 0, st);
 }
 
 void launch_adjoint_forward(const Dev &d, const BatchDev &b, const AdjDev &a, const int *elems,

@@ -120,32 +120,38 @@ __global__ void __launch_bounds__(MEASURE_BLOCK) k_batch_measure(Dev d, BatchDev
 
 // ------------------------------------------------------------------------------------ launch
 
-template <bool MIXED, bool STAGE, bool INT>
-static const void *by_threads(int threads) {
-    if (threads == 32) return (const void *)k_batch_steps<MIXED, STAGE, 32, INT, false>;
-    return threads == 128 ? (const void *)k_batch_steps<MIXED, STAGE, 128, INT, false>
-                          : (const void *)k_batch_steps<MIXED, STAGE, TEAM_THREADS, INT, false>;
+template <bool MIXED, bool STAGE>
+static const void *by_threads(int threads, bool ints) {
+    if (threads == 32) return (const void *)k_batch_steps<MIXED, STAGE, 32, false, false>;
+    if (threads == 128) return (const void *)k_batch_steps<MIXED, STAGE, 128, false, false>;
+    if (MIXED && ints) return (const void *)k_batch_steps<MIXED, STAGE, TEAM_THREADS, MIXED, false>;
+    return (const void *)k_batch_steps<MIXED, STAGE, TEAM_THREADS, false, false>;
 }
 
-// The kernel of a shape; lone: its blocks give no quarter SM more than one warp of elements.
-static const void *select_kernel(int mode, const BatchShape &s, bool lone, bool team) {
+// The kernel of a shape. ints: the node products on the integer units (batch_int_products).
+static const void *select_kernel(int mode, const BatchShape &s, bool ints, bool team) {
     if (mode == NF_PRECISION_COMPENSATED) return comp_steps_kernel(s, team);
     if (mode == NF_PRECISION_MIXED) {
-        if (team) return lone ? (const void *)k_batch_steps<true, false, TEAM_THREADS, false, true>
-                              : (const void *)k_batch_steps<true, false, TEAM_THREADS, true, true>;
-        if (lone) return s.stage ? by_threads<true, true, false>(s.threads)
-                                 : by_threads<true, false, false>(s.threads);
-        return s.stage ? by_threads<true, true, true>(s.threads) : by_threads<true, false, true>(s.threads);
+        if (team) return ints ? (const void *)k_batch_steps<true, false, TEAM_THREADS, true, true>
+                              : (const void *)k_batch_steps<true, false, TEAM_THREADS, false, true>;
+        return s.stage ? by_threads<true, true>(s.threads, ints) : by_threads<true, false>(s.threads, ints);
     }
-    if (team) return lone ? (const void *)k_batch_steps<false, false, TEAM_THREADS, false, true>
-                          : (const void *)k_batch_steps<false, false, TEAM_THREADS, true, true>;
-    return lone ? by_threads<false, false, false>(s.threads) : by_threads<false, false, true>(s.threads);
+    return team ? (const void *)k_batch_steps<false, false, TEAM_THREADS, false, true>
+                : by_threads<false, false>(s.threads, false);
 }
-// Whether a shape keeps no more than one warp with elements on a quarter SM.
-static bool lone_warps(const BatchShape &s, int maxElems, int team) {
-    const int warps = (maxElems + 31) / 32 < s.threads / 32 * team ? (maxElems + 31) / 32
-                                                                   : s.threads / 32 * team;
-    return !int_products((long long)s.blocksPerSm * ((warps + team - 1) / team), 1);
+// Whether a shape's products go to the integer units: in the mixed form, whose products are the
+// nodes' alone, with blocks of 256 threads of which a quarter SM has more than one warp with
+// elements (150 rods of 24 x 120: 6.64 ms per 100 steps and 7.07 without, 256 ragged ones 26.9
+// and 27.4; narrower blocks lose, 1,200 rods of 10 x 30 in blocks of 128: 8.4 ms and 6.9). The
+// FP64 step has no room for it: its 255 registers leave a quarter SM two warps at most, and
+// with a whole element's products in integer code they wait for instructions: 1,200 rods of
+// 10 x 30: 99 ms and 55 without, 512 burst slices 6.7 and 4.8, 256 ragged rods 223 and 157, and no
+// size of 1 to 1,200 instances the other way round.
+static bool batch_int_products(int mode, const BatchShape &s, int maxElems, int team) {
+    if (mode != NF_PRECISION_MIXED || s.threads != TEAM_THREADS) return false;
+    const int most = s.threads / 32 * team, needed = (maxElems + 31) / 32;
+    const int warps = needed < most ? needed : most;
+    return int_products((long long)s.blocksPerSm * ((warps + team - 1) / team), 1);
 }
 
 size_t batch_shared_bytes(int mode, const BatchShape &s, int maxNodes) {
@@ -227,27 +233,27 @@ void batch_teams(int mode, const BatchShape &s, int sms, int (&teams)[4]) {
     for (int q = 1; q < 4; q++) {
         teams[q] = 0;
         if (s.threads != TEAM_THREADS || s.stage) continue;
-        const int n = max_teams(select_kernel(mode, s, false, true), 1 << q, TEAM_THREADS);
+        const int n = max_teams(select_kernel(mode, s, true, true), 1 << q, TEAM_THREADS);
         teams[q] = n < teams[0] >> q ? n : teams[0] >> q;
     }
 }
 
 // Resident blocks per SM of a shape (0 when it cannot launch, e.g. too much shared memory). The
-// lone and the shared kernel are both made ready: which one a launch takes depends on the blocks
-// per SM that the answer bounds.
+// kernels with and without integer products are both made ready: which one a launch takes depends
+// on the blocks per SM that the answer bounds.
 int batch_max_blocks_per_sm(int mode, const BatchShape &s, int maxNodes, int maxElems) {
     const size_t smem = batch_shared_bytes(mode, s, maxNodes);
-    for (const bool lone : {false, true}) {
+    for (const bool ints : {false, true}) {
         if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(select_kernel(mode, s, lone, false),
+            cudaFuncSetAttribute(select_kernel(mode, s, ints, false),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
             (void)cudaGetLastError();
             return 0;
         }
     }
+    const void *k = select_kernel(mode, s, batch_int_products(mode, s, maxElems, 1), false);
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &n, select_kernel(mode, s, lone_warps(s, maxElems, 1), false), s.threads, smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, s.threads, smem) != cudaSuccess) {
         (void)cudaGetLastError();
         return 0;
     }
@@ -269,13 +275,13 @@ cudaError_t launch_batch_steps(const Dev &d, const BatchDev &b, int mode, const 
     BatchDev bb = b;
     int chunk = s.chunk;
     void *args[] = {&dd, &bb, &chunk};
-    const bool lone = lone_warps(s, b.maxElems, team);
+    const bool ints = batch_int_products(mode, s, b.maxElems, team);
     if (teams > b.count) teams = b.count;
     if (teams < 1) teams = 1;
     if (team > 1)
-        return launch_team(select_kernel(mode, s, lone, true), teams, team, TEAM_THREADS, args, st);
+        return launch_team(select_kernel(mode, s, ints, true), teams, team, TEAM_THREADS, args, st);
     const size_t smem = batch_shared_bytes(mode, s, b.maxNodes);
-    return cudaLaunchKernel(select_kernel(mode, s, lone, false), dim3(teams), dim3(s.threads), args,
+    return cudaLaunchKernel(select_kernel(mode, s, ints, false), dim3(teams), dim3(s.threads), args,
                             smem, st);
 }
 

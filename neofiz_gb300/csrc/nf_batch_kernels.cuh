@@ -221,7 +221,7 @@ __device__ __forceinline__ void batch_queue(const Dev &d, const BatchDev &b, int
 }
 
 // The FP64 and mixed forms (the compiler's register choice).
-// INT: the FP64 products of elements and nodes on the integer units (int_products).
+// INT: the nodes' FP64 products on the integer units (batch_int_products; the mixed form alone).
 template <bool MIXED, bool STAGE, int T, bool INT, bool TEAM>
 __global__ void __launch_bounds__(T) k_batch_steps(Dev d, BatchDev b, int chunk) {
     batch_queue<MIXED, STAGE, T, false, INT, TEAM>(d, b, chunk);

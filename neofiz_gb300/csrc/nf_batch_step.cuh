@@ -267,7 +267,7 @@ __device__ double team_min_edge_next_f(const Team<TEAM> &team, float v, double *
 // shortest squared edge, the per-node gather, the next CFL step. dt, dtPrev, time and steps
 // advance in place; returns the shortest squared edge. wall: the threads' slots (team_sums) of the
 // wall's impulse, energy loss and friction work. COMP (with MIXED): the compensated form's
-// FP32 nodal update and gather (nf_bodies.cuh). INT: int_products. The step's coefficients and
+// FP32 nodal update and gather (nf_bodies.cuh). INT: batch_int_products. The step's coefficients and
 // the next step size come from bs, which each block's thread 0 keeps prepared.
 template <bool MIXED, int T, bool COMP, bool INT, bool TEAM>
 __device__ __forceinline__ double batch_step(const Team<TEAM> &team, const Dev &d,

@@ -306,9 +306,9 @@ static __device__ __forceinline__ double opposite_force(double t, double f, doub
 // The FP64 pipe issues one warp instruction per 64 to 76 cycles on a quarter SM, whatever the
 // operation, and bounds this code. So the quotients, the scalings by powers of two and, with INT,
 // the products run on the integer units (nf_ifp.h) beside the additions on the FP64 pipe, in
-// straight-line code. A product is 53 integer instructions: with two warps or more on a quarter
-// SM they fill the time between its FP64 instructions, but a lone warp issues them in between
-// and is faster without (int_products). An element with any operand outside their ranges (one
+// straight-line code. A product is 53 integer instructions: with several warps on a quarter SM they
+// fill the time between its FP64 instructions; a lone warp issues them in between and is faster
+// without (int_products), and so are the FP64 batches' kernels (batch_int_products). An element with any operand outside their ranges (one
 // test at the end of each half) is redone by strain_machine and forces_machine. Every value has
 // the bits of the reference's sequence:
 //  * -0.5 dt v is -(dt v) / 2 exactly, and 2 (0.5 spin) is spin;

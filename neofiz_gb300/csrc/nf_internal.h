@@ -462,9 +462,10 @@ size_t scan_tmp_ints(int n);
 
 int grid_for(long long n, int block);
 // Whether `warps` warps of elements or nodes give the quarter SMs more than one each at a time,
-// where their products go to the integer units (element_reduced, nodal_node): on a 200k-quad scene 143 us a
-// pass against 163 without, on 16-element batch instances alone on their quarter SM 99 us a step
-// against 74.
+// where a scene's products go to the integer units (element_reduced, nodal_node). FP64 rods of
+// linear hardening, us a step without and with them: 2,880 quads 30.8 and 33.2, 10,400 29.7 and
+// 32.3, 19,800 (the first above the line) 39.3 and 34.5, 260,000 176 and 150. Batches have a
+// rule of their own (batch_int_products).
 inline bool int_products(long long warps, int sms) { return warps > 4LL * sms; }
 // Fixed grids of the node and element kernels that reduce per block, striding over the items.
 // The nodal update takes one node per thread up to sixteen blocks per SM (two rounds of the
