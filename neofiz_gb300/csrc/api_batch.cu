@@ -516,13 +516,24 @@ nf_status nf_batch_create(const nf_batch_mesh *mesh, const nf_batch_instance *in
         launch_batch_comp(d, true, B->stream);
         B->launches += 1;
     }
-    // default shape: blocks of 256 threads, or no wider than the largest instance needs (a block's
-    // idle warps hold the registers of other instances' blocks: 512 wall slices of 16 elements
-    // take 220 ms in blocks of 256 and 87 in blocks of 32), and the most of them resident, up
-    // to 2048 threads per SM. The compensated one-warp kernels round differently from the wider
+    // default shape: blocks of 256 threads, or narrower ones for small instances, whose idle warps
+    // would hold the registers of other instances' blocks; and the most of them resident, up to
+    // 2048 threads per SM. A narrower block is no faster by itself, and a node loop of two rounds
+    // makes it slower, so it waits until the instances outnumber the wider blocks' places: mixed
+    // rods of 8 x 16 (153 nodes), 100 steps in blocks of 128 and 256: 150 of them 1.49 and 1.26 ms,
+    // 608 2.2 and 2.8; of 4 x 8 (45 nodes) in blocks of 32 and 128: 400 1.27 and 1.12, 1,200
+    // 1.65 and 2.38. Where all nodes fit in one round it costs nothing (7 x 12, 150 of them: 1.19
+    // and 1.20), nor do one-warp blocks in FP64, whose step is bound by the elements (4 x 8, 400 of
+    // them: 5.7 ms and 8.6). The compensated one-warp kernels round differently from the wider
     // ones, so that form stops at 128.
     BatchShape s{256, 0, 1, 256};
-    if (maxElems <= 128) s.threads = maxElems <= 32 && !B->comp ? 32 : 128;
+    auto outnumbered = [&] {
+        return count > (long long)B->sms * batch_max_blocks_per_sm(B->mode, s, maxNodes, maxElems);
+    };
+    if (maxElems <= 128 && (maxNodes <= 128 || outnumbered())) s.threads = 128;
+    if (s.threads == 128 && maxElems <= 32 && !B->comp &&
+        (!B->mixed || maxNodes <= 32 || outnumbered()))
+        s.threads = 32;
     const int occ = batch_max_blocks_per_sm(B->mode, s, maxNodes, maxElems);
     s.blocksPerSm = std::max(1, std::min(occ, 2048 / s.threads));
     B->shape = s;

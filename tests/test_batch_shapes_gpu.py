@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from neofiz_gb300 import _abi, scenes
+from neofiz_gb300 import ExplicitSolver, _abi, scenes
 from neofiz_gb300.batch import BatchSolver
 from neofiz_gb300.materials import Formulation
 
@@ -59,4 +59,29 @@ def test_tuning_a_ragged_batch_does_not_lose_to_the_default(gpu_lib, precision, 
     b.tune()
     assert b.run() < 1.1 * a.run()
     a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("precision,nr,nz,count,threads", [
+    (_abi.PRECISION_MIXED, 8, 16, 16, 256),       # 153 nodes: two rounds of 128 threads
+    (_abi.PRECISION_MIXED, 8, 16, 700, 128),      # more than the 256-thread blocks' 304 places
+    (_abi.PRECISION_MIXED, 7, 12, 16, 128),       # 104 nodes
+    (_abi.PRECISION_MIXED, 4, 8, 16, 128),        # 45 nodes: two rounds of 32 threads
+    (_abi.PRECISION_MIXED, 4, 8, 1200, 32),
+    (_abi.PRECISION_COMPENSATED, 8, 16, 16, 256),
+    (_abi.PRECISION_FP64, 4, 8, 16, 32),
+    (_abi.PRECISION_FP64, 10, 60, 700, 256)])
+def test_default_blocks_are_narrow_only_where_that_helps(gpu_lib, precision, nr, nz, count, threads):
+    rods = scenes.taylor_sweep(1, seed=4, t_end=1.0)
+    rods[0].update(nr=nr, nz=nz)
+    b = batch(rods * count, precision)
+    assert b.config()["threads"] == threads
+    b.run(9)
+    s, _, _ = scenes.sweep_rod(ExplicitSolver, rods[0])
+    if precision != _abi.PRECISION_COMPENSATED:           # which has no single scene
+        s.setPrecision(precision)
+        s.run(9)
+        for k in (0, count - 1):
+            assert np.array_equal(b.readInstance(_abi.FIELD_UZ, k), s.readField(_abi.FIELD_UZ))
+    s.close()
     b.close()
