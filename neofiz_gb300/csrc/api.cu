@@ -1054,11 +1054,11 @@ nf_status nf_read_field(nf_solver *h, int32_t field, void *dst, size_t nbytes) {
     if (st) return st;
     auto copy = [&](const void *src) -> nf_status {
         CK(&S, copy_to_host(dst, src, nbytes, S.stream));
-        return sync_check(S);
+        return NF_OK;
     };
     auto pair = [&](const double2 *src, int comp) -> nf_status {
-        launch_component(src, S.stage, count, comp, S.stream);
-        return copy(S.stage);
+        CK(&S, read_component(src, (double *)dst, count, comp, S.stage, S.stream));
+        return NF_OK;
     };
     switch (field) {
         case NF_FIELD_UR: return pair(d.U, 0);

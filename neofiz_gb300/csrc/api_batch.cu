@@ -752,15 +752,15 @@ nf_status nf_batch_read(nf_batch *h, int32_t field, void *dst, size_t nbytes) {
     const Dev &d = B.d;
     auto plain = [&](const void *src, size_t elem) -> nf_status {
         BCK(&B, copy_to_host(dst, src, elem * count, B.stream));
-        return bsync(B);
+        return NF_OK;
     };
     auto pairs = [&](const double2 *src, int comp) -> nf_status {
-        launch_component(src, B.stage, count, comp, B.stream);
-        return plain(B.stage, 8);
+        BCK(&B, read_component(src, (double *)dst, count, comp, B.stage, B.stream));
+        return NF_OK;
     };
     auto widen = [&](const float *src, int stride = 1) -> nf_status {
-        launch_widen(src, B.stage, count, stride, B.stream);
-        return plain(B.stage, 8);
+        BCK(&B, read_widened(src, (double *)dst, count, stride, B.stage, B.stream));
+        return NF_OK;
     };
     switch (field) {
         case NF_FIELD_UR: return pairs(d.U, 0);

@@ -337,18 +337,41 @@ void setup_damage_geometry(Dev &d, cudaStream_t st) {
 void launch_segments(Solver &S) {
     if (S.d.E > 0) k_segments<<<grid_for(4LL * S.d.E, SB), SB, 0, S.stream>>>(S.d);
 }
-void launch_component(const double2 *src, double *dst, size_t count, int y, cudaStream_t st) {
-    k_component<<<grid_for((long long)count, SB), SB, 0, st>>>(src, dst, (int)count, y);
-}
-void launch_widen(const float *src, double *dst, size_t count, int stride, cudaStream_t st) {
-    k_widen<<<grid_for((long long)count, SB), SB, 0, st>>>(src, dst, (int)count, stride);
-}
 // The destination's pages first: a copy of 32 MB into pages not mapped yet took 13.6 ms (the
 // device faults them in one by one), with them touched it takes 1.3 ms.
 cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t st) {
     for (size_t i = 0; i < bytes; i += 4096) ((volatile char *)dst)[i] = 0;
     const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
     return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
+// One component of a field of pairs, or a float field widened, in doubles: split on the device
+// through `stage`, or on the host where the field is small and a launch costs more than its copy
+// (45 nodes: 13 us a read by the copy, 20 by the kernel).
+constexpr size_t SMALL_READ = 4096;
+cudaError_t read_component(const double2 *src, double *dst, size_t count, int y, double *stage,
+                           cudaStream_t st) {
+    if (count <= SMALL_READ) {
+        std::vector<double2> pairs(count);
+        const cudaError_t e = copy_to_host(pairs.data(), src, sizeof(double2) * count, st);
+        for (size_t i = 0; i < count; i++) dst[i] = y ? pairs[i].y : pairs[i].x;
+        return e;
+    }
+    k_component<<<grid_for((long long)count, SB), SB, 0, st>>>(src, stage, (int)count, y);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? copy_to_host(dst, stage, sizeof(double) * count, st) : e;
+}
+cudaError_t read_widened(const float *src, double *dst, size_t count, int stride, double *stage,
+                         cudaStream_t st) {
+    if (count <= SMALL_READ) {
+        std::vector<float> values((count - 1) * stride + 1);
+        const cudaError_t e = copy_to_host(values.data(), src, sizeof(float) * values.size(), st);
+        for (size_t i = 0; i < count; i++) dst[i] = values[i * stride];
+        return e;
+    }
+    k_widen<<<grid_for((long long)count, SB), SB, 0, st>>>(src, stage, (int)count, stride);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? copy_to_host(dst, stage, sizeof(double) * count, st) : e;
 }
 
 }  // namespace nf

@@ -417,8 +417,10 @@ void launch_batch_setup(Dev &d, const BatchInst *inst, int count, const double2 
                         unsigned long long *edges, double *stage, cudaStream_t st);
 void setup_damage_geometry(Dev &d, cudaStream_t st);
 void launch_segments(Solver &S);
-void launch_component(const double2 *src, double *dst, size_t count, int y, cudaStream_t st);
-void launch_widen(const float *src, double *dst, size_t count, int stride, cudaStream_t st);
+cudaError_t read_component(const double2 *src, double *dst, size_t count, int y, double *stage,
+                           cudaStream_t st);
+cudaError_t read_widened(const float *src, double *dst, size_t count, int stride, double *stage,
+                         cudaStream_t st);
 cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t st);
 
 // Launchers (k_step.cu). Each returns the number of kernels it enqueued.
