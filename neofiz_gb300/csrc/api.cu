@@ -391,14 +391,15 @@ nf_status nf_create(const nf_mesh *mesh, const nf_material *materials, int32_t m
     DevScalars s0{};
     s0.minEdgeBits = 0x7ff0000000000000ULL;   // none yet
     upload(*S, d.s, &s0, 1);
-    const int *most = launch_setup(*S);
-    CK(nullptr, cudaMemcpyAsync(&S->maxCorners, most, sizeof(int), cudaMemcpyDeviceToHost, S->stream));
+    launch_setup(*S);
     nf_status st = read_scalars(*S, &s0);
     if (st) {
         g_err = S->err;
         nf_destroy(reinterpret_cast<nf_solver *>(S));
         return st;
     }
+    S->maxCorners = s0.surfNodes;
+    s0.surfNodes = 0;
 
     // initial step, QuadMesh.minimumEdgeLength + ExplicitSolver.java:333-338: the root of the
     // least square is the least root

@@ -6,8 +6,8 @@
 // One core took 64 ms over these for 1M quads, half as long as the 400 steps that followed;
 // here they are 1 ms of kernels (each a pass or two over the mesh, bound by its gathers) behind
 // the upload of the mesh (a batch of 512 rods, 580k quads:
-// 46 ms on one core and 15 so, which leaves the allocations, the checks and the upload). Below about a thousand elements the launches cost what the host loops
-// did (50 us). The orderings are counting sorts: an entry's place in its node's list is the
+// 46 ms on one core and 15 so, which leaves the allocations, the checks and the upload). A scene of
+// up to a thousand nodes takes one block and one launch (k_set_up_small). The orderings are counting sorts: an entry's place in its node's list is the
 // number of smaller entries there, which each entry counts for itself, so no list is walked by
 // one thread alone whatever the mesh's valences.
 #include "nf_bodies.cuh"
@@ -24,27 +24,35 @@ __device__ __forceinline__ int edge_end(const Dev &d, long long q) {
     return conn_at(d, (q & ~3LL) + ((q + 1) & 3));
 }
 
-__global__ void __launch_bounds__(SB) k_positions(Dev d, const double *r, const double *z) {
-    const int n = blockIdx.x * SB + threadIdx.x;
-    if (n < d.N) d.X0[n] = make_double2(r[n], z[n]);
+// The passes, each for one item; the kernels below run them over a grid, or (set_up_small) all of
+// them in one block.
+__device__ __forceinline__ void position(const Dev &d, int n) {
+    const double *r = reinterpret_cast<const double *>(d.U);
+    d.X0[n] = make_double2(r[n], r[d.N + n]);
 }
 
-// QuadMesh.minimumEdgeLength squared, as bits (a NaN is passed over): of the scene, or of the
-// element's instance.
+// QuadMesh.minimumEdgeLength squared, as bits (a NaN is passed over).
+__device__ __forceinline__ unsigned long long shortest_edge(const Dev &d, int e) {
+    unsigned long long best = 0x7ff0000000000000ULL;
+    const int4 c = d.conn[e];
+    const int nn[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const double2 a = d.X0[nn[k]], b = d.X0[nn[(k + 1) & 3]];
+        const double dr = b.x - a.x, dz = b.y - a.y;
+        const unsigned long long q = __double_as_longlong(dr * dr + dz * dz);
+        best = q < best ? q : best;
+    }
+    return best;
+}
+__global__ void __launch_bounds__(SB) k_positions(Dev d) {
+    const int n = blockIdx.x * SB + threadIdx.x;
+    if (n < d.N) position(d, n);
+}
+// The scene's shortest edge, or the element's instance's.
 __global__ void __launch_bounds__(SB) k_shortest_edge(Dev d, unsigned long long *instances) {
     const int e = blockIdx.x * SB + threadIdx.x;
-    unsigned long long best = 0x7ff0000000000000ULL;
-    if (e < d.E) {
-        const int4 c = d.conn[e];
-        const int nn[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const double2 a = d.X0[nn[k]], b = d.X0[nn[(k + 1) & 3]];
-            const double dr = b.x - a.x, dz = b.y - a.y;
-            const unsigned long long q = __double_as_longlong(dr * dr + dz * dz);
-            best = q < best ? q : best;
-        }
-    }
+    const unsigned long long best = e < d.E ? shortest_edge(d, e) : 0x7ff0000000000000ULL;
     if (!instances) {
         commit_min_bits(best, &d.s->minEdgeBits);
     } else if (e < d.E) {
@@ -86,27 +94,13 @@ __device__ __forceinline__ int source_slot(const Dev &d, long long q) {
     return (int)((d.E + (k >> 1)) * 8 + (k & 1));
 }
 
-__global__ void __launch_bounds__(SB) k_count(Dev d, int *sources, int *edges) {
-    const long long q = (long long)blockIdx.x * SB + threadIdx.x;
-    if (q >= 4LL * d.E + 2LL * d.K) return;
+__device__ __forceinline__ void count_source(const Dev &d, long long q, int *sources, int *edges) {
     atomicAdd(&sources[source_node(d, q)], 1);
     if (edges && q < 4LL * d.E) atomicAdd(&edges[min(conn_at(d, q), edge_end(d, q))], 1);
 }
-// The most elements around a node (its corners, counted once each).
-__global__ void __launch_bounds__(SB) k_corners(Dev d, int *corners) {
-    const long long q = (long long)blockIdx.x * SB + threadIdx.x;
-    if (q < 4LL * d.E) atomicAdd(&corners[conn_at(d, q)], 1);
-}
-__global__ void __launch_bounds__(SB) k_most(int n, const int *corners, int *most) {
-    const int i = blockIdx.x * SB + threadIdx.x;
-    const int m = __reduce_max_sync(0xffffffffu, i < n ? corners[i] : 0);
-    if ((threadIdx.x & 31) == 0 && m > __ldcg(most)) atomicMax(most, m);
-}
 // Into the nodes' ranges in any order; the counts run down to zero.
-__global__ void __launch_bounds__(SB) k_file(Dev d, int *sources, int *edges, const int *edgeStart,
-                                             int *sourceBin, int *edgeBin) {
-    const long long q = (long long)blockIdx.x * SB + threadIdx.x;
-    if (q >= 4LL * d.E + 2LL * d.K) return;
+__device__ __forceinline__ void file_source(const Dev &d, long long q, int *sources, int *edges,
+                                            const int *edgeStart, int *sourceBin, int *edgeBin) {
     const int n = source_node(d, q);
     sourceBin[d.nodeSlotStart[n] + atomicSub(&sources[n], 1) - 1] = source_slot(d, q);
     if (edges && q < 4LL * d.E) {
@@ -116,10 +110,8 @@ __global__ void __launch_bounds__(SB) k_file(Dev d, int *sources, int *edges, co
 }
 // buildNodeSlots (ExplicitSolver.java:347-366): a node's sources ascending; and the edges of one
 // lower node by higher node, then by element edge.
-__global__ void __launch_bounds__(SB) k_rank(Dev d, const int *edgeStart, const int *sourceBin,
-                                             const int *edgeBin) {
-    const long long q = (long long)blockIdx.x * SB + threadIdx.x;
-    if (q >= 4LL * d.E + 2LL * d.K) return;
+__device__ __forceinline__ void rank_source(const Dev &d, long long q, const int *edgeStart,
+                                            const int *sourceBin, const int *edgeBin) {
     {
         const int n = source_node(d, q), slot = source_slot(d, q);
         const int begin = d.nodeSlotStart[n], end = d.nodeSlotStart[n + 1];
@@ -140,20 +132,17 @@ __global__ void __launch_bounds__(SB) k_rank(Dev d, const int *edgeStart, const 
     }
 }
 // Equal undirected node pairs are neighbours now: a group starts where the pair changes.
-__global__ void __launch_bounds__(SB) k_heads(Dev d, int *head) {
-    const long long i = (long long)blockIdx.x * SB + threadIdx.x;
-    if (i >= 4LL * d.E) return;
+__device__ __forceinline__ int group_head(const Dev &d, long long i) {
     int first = 1;
     if (i > 0) {
         const int q = d.groupMember[i], p = d.groupMember[i - 1];
         const int a = conn_at(d, q), b = edge_end(d, q), f = conn_at(d, p), g = edge_end(d, p);
         first = min(a, b) != min(f, g) || max(a, b) != max(f, g);
     }
-    head[i] = first;
+    return first;
 }
-__global__ void __launch_bounds__(SB) k_groups(Dev d, const int *head, const int *before) {
-    const long long i = (long long)blockIdx.x * SB + threadIdx.x;
-    if (i >= 4LL * d.E) return;
+__device__ __forceinline__ void file_group(const Dev &d, long long i, const int *head,
+                                           const int *before) {
     const int g = before[i] + head[i] - 1;
     d.edgeGroup[d.groupMember[i]] = g;
     if (head[i]) d.groupStart[g] = (int)i;
@@ -163,9 +152,7 @@ __global__ void __launch_bounds__(SB) k_groups(Dev d, const int *head, const int
 // lumpMass, ExplicitSolver.java:1559-1597: 2x2 Gauss lumping. The four points' volumes by
 // element, then each node adds its corners' shares: in element order, for each element point by
 // point, and where an element has the node at several corners, those in turn within the point.
-__global__ void __launch_bounds__(SB) k_lump_volumes(Dev d, double4 *volumes) {
-    const int e = blockIdx.x * SB + threadIdx.x;
-    if (e >= d.E) return;
+__device__ __forceinline__ double4 lump_volumes(const Dev &d, int e) {
     const double G = 0.5773502691896258;
     const double gx[4] = {-G, G, G, -G}, ge[4] = {-G, -G, G, G};
     const int4 c = d.conn[e];
@@ -188,16 +175,16 @@ __global__ void __launch_bounds__(SB) k_lump_volumes(Dev d, double4 *volumes) {
         const double rg = N0 * p0.x + N1 * p1.x + N2 * p2.x + N3 * p3.x;
         v[g] = d.axi ? 2.0 * NF_PI * rg * det : d.thickness * det;
     }
-    volumes[e] = make_double4(v[0], v[1], v[2], v[3]);
+    return make_double4(v[0], v[1], v[2], v[3]);
 }
-__global__ void __launch_bounds__(SB) k_lump(Dev d, const double4 *volumes) {
-    const int n = blockIdx.x * SB + threadIdx.x;
-    if (n >= d.N) return;
+// Returns how many elements are around the node (its corners, counted once each).
+__device__ __forceinline__ int lump_node(const Dev &d, int n, const double4 *volumes) {
     const double G = 0.5773502691896258;
     const double gx[4] = {-G, G, G, -G}, ge[4] = {-G, -G, G, G};
     double m = 0.0;
-    const int end = d.nodeSlotStart[n + 1];
-    for (int k = d.nodeSlotStart[n]; k < end;) {
+    const int begin = d.nodeSlotStart[n], end = d.nodeSlotStart[n + 1];
+    int k = begin;
+    while (k < end) {
         const int e = d.nodeSlot[k] >> 3;
         if (e >= d.E) break;                              // pressure edges come last
         int corners = 0;
@@ -218,6 +205,106 @@ __global__ void __launch_bounds__(SB) k_lump(Dev d, const double4 *volumes) {
     }
     d.mass[n] = m;
     d.invMass[n] = 1.0 / m;                               // nodalUpdate's 1/m, once
+    return k - begin;
+}
+
+__global__ void __launch_bounds__(SB) k_count(Dev d, int *sources, int *edges) {
+    const long long q = (long long)blockIdx.x * SB + threadIdx.x;
+    if (q < 4LL * d.E + 2LL * d.K) count_source(d, q, sources, edges);
+}
+__global__ void __launch_bounds__(SB) k_file(Dev d, int *sources, int *edges, const int *edgeStart,
+                                             int *sourceBin, int *edgeBin) {
+    const long long q = (long long)blockIdx.x * SB + threadIdx.x;
+    if (q < 4LL * d.E + 2LL * d.K) file_source(d, q, sources, edges, edgeStart, sourceBin, edgeBin);
+}
+__global__ void __launch_bounds__(SB) k_rank(Dev d, const int *edgeStart, const int *sourceBin,
+                                             const int *edgeBin) {
+    const long long q = (long long)blockIdx.x * SB + threadIdx.x;
+    if (q < 4LL * d.E + 2LL * d.K) rank_source(d, q, edgeStart, sourceBin, edgeBin);
+}
+__global__ void __launch_bounds__(SB) k_heads(Dev d, int *head) {
+    const long long i = (long long)blockIdx.x * SB + threadIdx.x;
+    if (i < 4LL * d.E) head[i] = group_head(d, i);
+}
+__global__ void __launch_bounds__(SB) k_groups(Dev d, const int *head, const int *before) {
+    const long long i = (long long)blockIdx.x * SB + threadIdx.x;
+    if (i < 4LL * d.E) file_group(d, i, head, before);
+}
+__global__ void __launch_bounds__(SB) k_lump_volumes(Dev d, double4 *volumes) {
+    const int e = blockIdx.x * SB + threadIdx.x;
+    if (e < d.E) volumes[e] = lump_volumes(d, e);
+}
+__global__ void __launch_bounds__(SB) k_lump(Dev d, const double4 *volumes, int *most) {
+    const int n = blockIdx.x * SB + threadIdx.x;
+    const int corners = n < d.N ? lump_node(d, n, volumes) : 0;
+    if (!most) return;
+    const int m = __reduce_max_sync(0xffffffffu, corners);
+    if ((threadIdx.x & 31) == 0 && m > __ldcg(most)) atomicMax(most, m);
+}
+
+// All of a small scene's passes in one block, a barrier between two of them: their dozen and a
+// half launches took 75 us, a third of creating a scene of 32 quads.
+constexpr int SMALL_BLOCK = 1024;
+constexpr int SMALL_NODES = 1024;                          // and as many elements and pressure edges
+__device__ void small_scan(const int *in, int *out, int n) {     // exclusive
+    __shared__ int warps[SMALL_BLOCK / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int per = (n + SMALL_BLOCK - 1) / SMALL_BLOCK;
+    const int begin = min((int)threadIdx.x * per, n), end = min(begin + per, n);
+    int own = 0;
+    for (int i = begin; i < end; i++) own += in[i];
+    int sum = own;                                         // inclusive in the warp
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += t;
+    }
+    if (lane == 31) warps[warp] = sum;
+    __syncthreads();
+    if (warp == 0) {
+        int w = warps[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += t;
+        }
+        warps[lane] = w;
+    }
+    __syncthreads();
+    int at = sum - own + (warp ? warps[warp - 1] : 0);
+    for (int i = begin; i < end; i++) {
+        const int v = in[i];
+        out[i] = at;
+        at += v;
+    }
+    __syncthreads();
+}
+__global__ void __launch_bounds__(SMALL_BLOCK) k_set_up_small(Dev d, int *sources, int *edges,
+                                                              int *edgeStart, int *most,
+                                                              int *sourceBin, int *edgeBin,
+                                                              int *head, int *before) {
+    const int N = d.N, E = d.E, entries = 4 * E + 2 * d.K, t = threadIdx.x;
+    double4 *volumes = reinterpret_cast<double4 *>(d.contribution);
+    for (int n = t; n < N; n += SMALL_BLOCK) position(d, n);
+    for (int q = t; q < entries; q += SMALL_BLOCK) count_source(d, q, sources, edges);
+    __syncthreads();
+    for (int n = t; n < N; n += SMALL_BLOCK) d.U[n] = make_double2(0.0, 0.0);
+    for (int e = t; e < E; e += SMALL_BLOCK) atomicMin(&d.s->minEdgeBits, shortest_edge(d, e));
+    small_scan(sources, d.nodeSlotStart, N + 1);
+    small_scan(edges, edgeStart, N + 1);
+    for (int q = t; q < entries; q += SMALL_BLOCK)
+        file_source(d, q, sources, edges, edgeStart, sourceBin, edgeBin);
+    __syncthreads();
+    for (int q = t; q < entries; q += SMALL_BLOCK) rank_source(d, q, edgeStart, sourceBin, edgeBin);
+    __syncthreads();
+    for (int i = t; i < 4 * E; i += SMALL_BLOCK) head[i] = group_head(d, i);
+    __syncthreads();
+    small_scan(head, before, 4 * E);
+    for (int i = t; i < 4 * E; i += SMALL_BLOCK) file_group(d, i, head, before);
+    __syncthreads();                                       // the lists in `contribution` are done
+    for (int e = t; e < E; e += SMALL_BLOCK) volumes[e] = lump_volumes(d, e);
+    __syncthreads();
+    for (int n = t; n < N; n += SMALL_BLOCK) atomicMax(most, lump_node(d, n, volumes));
+    __syncthreads();
+    for (int i = t; i < 8 * (E + d.K); i += SMALL_BLOCK) d.contribution[i] = 0.0;
 }
 
 // The damage model's element geometry, ExplicitSolver.java:767-789.
@@ -272,23 +359,27 @@ __global__ void __launch_bounds__(SB) k_widen(const float *src, double *dst, int
 // the set-up works in it first (a count and, for a scene's surface, two ints more per node, and
 // the scan's space).
 size_t stage_doubles(size_t most, int N, int E, bool surface) {
-    const size_t ints = scan_tmp_ints(std::max(4 * E, N + 1)) + (surface ? 3 : 1) * ((size_t)N + 1) + 1;
+    const size_t ints = scan_tmp_ints(std::max(4 * E, N + 1)) + (surface ? 3 : 1) * ((size_t)N + 1);
     return std::max(most, (ints + 1) / 2);
 }
 
 // conn, emat, mats and pedges are in place, and r and z in U. The lists in between use
 // `contribution`, which like U is zeroed again, and the staging buffer, zeroed.
-static void node_arrays(Dev &d, cudaStream_t st, int *scratch, bool surface,
+static void node_arrays(Dev &d, cudaStream_t st, int *scratch, bool surface, int *most,
                         unsigned long long *instances) {
     const int N = d.N, E = d.E;
     const long long entries = 4LL * E + 2LL * d.K;
     int *sources = scratch, *edges = surface ? sources + N + 1 : nullptr;
     int *edgeStart = surface ? edges + N + 1 : nullptr;
-    int *tmp = scratch + (surface ? 3 : 1) * ((size_t)N + 1) + 1;
+    int *tmp = scratch + (surface ? 3 : 1) * ((size_t)N + 1);
     int *sourceBin = reinterpret_cast<int *>(d.contribution), *edgeBin = sourceBin + entries;
     int *head = edgeBin + 4LL * E, *before = head + 4LL * E;   // 16 E + 2 K of 16 (E + K)
-    const double *r = reinterpret_cast<const double *>(d.U);
-    if (N > 0) k_positions<<<grid_for(N, SB), SB, 0, st>>>(d, r, r + N);
+    if (surface && E > 0 && N <= SMALL_NODES && E <= SMALL_NODES && d.K <= SMALL_NODES) {
+        k_set_up_small<<<1, SMALL_BLOCK, 0, st>>>(d, sources, edges, edgeStart, most, sourceBin,
+                                                  edgeBin, head, before);
+        return;
+    }
+    if (N > 0) k_positions<<<grid_for(N, SB), SB, 0, st>>>(d);
     cudaMemsetAsync(d.U, 0, sizeof(double2) * (size_t)N, st);
     if (entries > 0) {
         const int grid = grid_for(entries, SB);
@@ -307,29 +398,21 @@ static void node_arrays(Dev &d, cudaStream_t st, int *scratch, bool surface,
     }
     double4 *volumes = reinterpret_cast<double4 *>(d.contribution);
     if (E > 0) k_lump_volumes<<<grid_for(E, SB), SB, 0, st>>>(d, volumes);
-    if (N > 0) k_lump<<<grid_for(N, SB), SB, 0, st>>>(d, volumes);
+    if (N > 0) k_lump<<<grid_for(N, SB), SB, 0, st>>>(d, volumes, most);
     cudaMemsetAsync(d.contribution, 0, sizeof(double) * 8 * ((size_t)E + d.K), st);
 }
 
-// A scene's arrays; its shortest edge goes to s. Returns where the greatest number of elements
-// around a node will be, in the staging buffer.
-int *launch_setup(Solver &S) {
-    Dev &d = S.d;
-    int *scratch = reinterpret_cast<int *>(S.stage);
-    node_arrays(d, S.stream, scratch, true, nullptr);
-    int *corners = scratch, *most = scratch + 3 * ((size_t)d.N + 1);   // the filing left zeros
-    if (d.E > 0) {
-        k_corners<<<grid_for(4LL * d.E, SB), SB, 0, S.stream>>>(d, corners);
-        k_most<<<grid_for(d.N, SB), SB, 0, S.stream>>>(d.N, corners, most);
-    }
-    return most;
+// A scene's arrays; its shortest edge goes to s, and the most elements around a node to surfNodes
+// there, one read of both.
+void launch_setup(Solver &S) {
+    node_arrays(S.d, S.stream, reinterpret_cast<int *>(S.stage), true, &S.d.s->surfNodes, nullptr);
 }
 // A batch's: conn and pedges arrive with the instances' local numbers, flags as the caller's
 // bytes, `edges` (per instance) at infinity.
 void launch_batch_setup(Dev &d, const BatchInst *inst, int count, const double2 *velocity,
                         unsigned long long *edges, double *stage, cudaStream_t st) {
     k_batch_fill<<<count, SB, 0, st>>>(d, inst, velocity);
-    node_arrays(d, st, reinterpret_cast<int *>(stage), false, edges);
+    node_arrays(d, st, reinterpret_cast<int *>(stage), false, nullptr, edges);
 }
 void setup_damage_geometry(Dev &d, cudaStream_t st) {
     if (d.E > 0) k_damage_geometry<<<grid_for(d.E, SB), SB, 0, st>>>(d);

@@ -412,7 +412,7 @@ void set_thread_error(const char *message);
 
 // Launchers (k_setup.cu)
 size_t stage_doubles(size_t most, int N, int E, bool surface);
-int *launch_setup(Solver &S);
+void launch_setup(Solver &S);
 void launch_batch_setup(Dev &d, const BatchInst *inst, int count, const double2 *velocity,
                         unsigned long long *edges, double *stage, cudaStream_t st);
 void setup_damage_geometry(Dev &d, cudaStream_t st);
