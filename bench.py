@@ -39,7 +39,7 @@ L2_FLUSH_BYTES = 256 << 20
 # DRAM bytes (read + write) of one element-pass launch of this workload in the window, from
 # ncu's dram__bytes_read.sum + dram__bytes_write.sum, the mean over the launches of steps
 # start + 6 and start + 7 (ncu cannot run inside the timed bench)
-ELEMENT_TRAFFIC_BYTES = {CELL: (43_483_904 + 173_568 + 43_474_176 + 36_864) // 2}
+ELEMENT_TRAFFIC_BYTES = {CELL: (43_563_008 + 143_616 + 43_574_272 + 160_000) // 2}
 # FP64-pipe warp instructions of one element-pass launch in the window: the mean of ncu's
 # smsp__inst_executed_pipe_fp64.sum over ten launches (steps start + 6 to start + 15; 1.4216 to
 # 1.4281 M)

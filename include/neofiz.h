@@ -396,7 +396,9 @@ typedef struct {
     double damping_omega;
 } nf_batch_instance;
 
-/* A launch shape of the batched step; any valid shape gives the same trajectories. */
+/* A launch shape of the batched step. Any valid shape gives the same trajectories in FP64 and in
+ * the mixed form; in the compensated form those of 32 threads round differently from the others
+ * (within that form's error). */
 typedef struct {
     int32_t threads;                 /* threads per block: 32, 128 or 256 */
     int32_t stage_nodes;             /* mixed form: node geometry staged in shared memory */

@@ -18,7 +18,8 @@
 //
 // Launch shape: block size (32, 128, 256), whether the mixed form stages each instance's float
 // node geometry in shared memory, blocks per SM and the chunk length are chosen by the
-// autotuner (api_batch.cu); none of them changes the trajectory.
+// autotuner (api_batch.cu). None of them changes an FP64 or mixed trajectory; the compensated
+// one-warp kernels, which the tuner may choose, round differently from that form's wider ones.
 #include "nf_batch_kernels.cuh"
 
 #include <algorithm>
@@ -188,10 +189,11 @@ int max_teams(const void *k, int team, int threads) {
 // part and its elements' rounds over the team's threads, half a round at least (below four warps
 // a block its quarter SMs have one warp each already): 0.6 + elements / (256 team). Teams take
 // the instances in this order, each the next when it is free; the time until the last is done,
-// plus half the longest instance's (which goes on when most have ended), is compared. On 60
-// timings (10 to 600 ragged rods in three forms and 16 equal ones, 1 to 8 blocks each; e.g. 64
-// FP64 rods 65, 44 and 59 ms with 2, 4 and 8 blocks, 256 mixed rods 328, 197 and 173 with 1, 2
-// and 4) this picks the fastest, or one within 2 % of it, of every group.
+// plus half the longest instance's (which goes on when most have ended), is compared. The constants
+// are fitted, to runs of 10 to 1,500 ragged rods in three forms and of 16 equal ones, with 1 to
+// 8 blocks each (profiles/batch_teams.md): this picks the fastest, or one within 2 % of it, of 21
+// groups of 22 (64 FP64 rods 196, 106, 62 and 85 ms with 1, 2, 4 and 8 blocks, 256 mixed ones 44.6,
+// 27.2, 26.9 and 37.9), and in the other, 1,500 compensated rods, 52.5 ms where one block takes 49.8.
 int choose_team(const int *elems, int count, const int (&teams)[4]) {
     if (count >= 8 * teams[0]) return 1;     // long queues: nothing to share out
     int best = 1;

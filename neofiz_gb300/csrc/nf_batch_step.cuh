@@ -1,4 +1,4 @@
-// nf_batch_step.cuh -- one step of one batched instance by a whole block, shared by the
+// nf_batch_step.cuh -- one step of one batched instance by a block or a cluster of them, shared by the
 // batched kernel (k_batch.cu) and the adjoint kernels (k_adjoint.cu).
 #pragma once
 
