@@ -163,8 +163,9 @@ public final class GpuBatch implements AutoCloseable {
         return count;
     }
 
-    /** The autotuner: times every valid launch shape on trialSteps steps (the trajectory is
-     * untouched) and keeps the fastest. */
+    /** The autotuner: times the valid launch shapes on trialSteps steps (the trajectory is
+     * untouched) and keeps the fastest; for instances of uneven cost those shapes that can spread
+     * the last ones over several blocks. */
     public void tune(int trialSteps) {
         try (Arena a = Arena.ofConfined()) {
             MemorySegment cfg = a.allocate(BATCH_CONFIG);

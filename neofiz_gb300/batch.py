@@ -152,7 +152,8 @@ class BatchSolver:
     # ------------------------------------------------------------------ shapes
 
     def tune(self, trial_steps: int = 32) -> dict:
-        """The autotuner: times every valid launch shape, keeps the fastest."""
+        """The autotuner: times the launch shapes (for instances of uneven cost those that can
+        spread the last ones over several blocks), keeps the fastest."""
         c = _abi.BatchConfig()
         self._check(self._api.batch_tune(self._handle, int(trial_steps), C.byref(c)))
         return self.config()

@@ -377,7 +377,7 @@ void launch_adjoint_backward(const Dev &d, const BatchDev &b, const AdjDev &a, c
 
 // A launch configuration of the batched step (chosen by the autotuner).
 struct BatchShape {
-    int threads;                             // 128 or 256
+    int threads;                             // 32, 128 or 256
     int stage;                               // mixed: node geometry in shared memory
     int blocksPerSm;
     int chunk;                               // steps per instance per launch
